@@ -2,6 +2,7 @@
 // on one tile, FP32 and FP64) and the whole-matrix tiled factorisation and
 // triangular solves composed from them.  Every entry point only enqueues work
 // on the caller's stream and returns; nothing here synchronises or allocates.
+#include "kernels/chol_panel.cuh"
 #include "kernels/simt_blas.cuh"
 #include "kernels/trsv_sweep.cuh"
 #include "gb300_internal.h"
@@ -35,7 +36,17 @@ static void gemm_launch(cudaStream_t s, bool lower, int m, int n, int k, T alpha
 }
 
 template <typename T> struct simt_cfg;
-// FP32: 128x128 block tiles, 8x8 per thread; narrow variant for few columns (RHS blocks).
+// CTAs of a product in bm x bm block tiles
+static long gemm_ctas(bool lower, int m, int n, int bm)
+{
+    const long tm = cdiv(m, bm), tn = cdiv(n, bm);
+    return lower ? tm * (tm + 1) / 2 : tm * tn;
+}
+
+// FP32: 128x128 block tiles, 8x8 per thread, when they make at least half a
+// wave; smaller ones otherwise (the 64 and 32 tiles take a third and an eighth
+// of the 128 tile's time each, so up to two waves of them are faster).
+// Narrow variant for few columns.
 template <> struct simt_cfg<float> {
     template <bool TA, bool TB>
     static void run(cudaStream_t s, bool lower, int m, int n, int k, float al, const float *A, long lda,
@@ -43,11 +54,16 @@ template <> struct simt_cfg<float> {
     {
         if (!lower && n <= 32)
             gemm_launch<float, TA, TB, 128, 32, 8, 8, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else
+        else if (gemm_ctas(lower, m, n, 128) > 76)
             gemm_launch<float, TA, TB, 128, 128, 8, 8, 8>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
+        else if (gemm_ctas(lower, m, n, 64) > 76)
+            gemm_launch<float, TA, TB, 64, 64, 16, 4, 4>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
+        else
+            gemm_launch<float, TA, TB, 32, 32, 32, 2, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
     }
 };
-// FP64: 64x64 block tiles, 4x4 per thread.
+// FP64: 64x64 block tiles, 4x4 per thread, for several waves of them; 32x32
+// tiles below that, so that every SM's FP64 units (2 FMA per clock) have work.
 template <> struct simt_cfg<double> {
     template <bool TA, bool TB>
     static void run(cudaStream_t s, bool lower, int m, int n, int k, double al, const double *A, long lda,
@@ -55,8 +71,10 @@ template <> struct simt_cfg<double> {
     {
         if (!lower && n <= 16)
             gemm_launch<double, TA, TB, 64, 16, 8, 4, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else
+        else if (gemm_ctas(lower, m, n, 64) >= 4 * 152)
             gemm_launch<double, TA, TB, 64, 64, 8, 4, 4>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
+        else
+            gemm_launch<double, TA, TB, 32, 32, 16, 2, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
     }
 };
 
@@ -119,21 +137,27 @@ void trtri_lower(cudaStream_t s, int n, const T *L, long ldl, T *Linv, long ldi,
     }
 }
 
-// B[m x nc] <- B * L^{-T}, blocked by SMALL_W columns: small triangular solve
-// of one column block, then a GEMM update of the remaining columns.
+// B[m x nc] <- B * L^{-T}: one launch per CP_TRSM_MAXN columns (rows are
+// independent), then a GEMM update of the remaining columns.
+template <typename T, int SR>
+static void trsm_slab(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb)
+{
+    const size_t smem = cp_trsm_smem<T, SR>(n);
+    if (gb300_func_dyn_smem((const void *)trsm_slab_kernel<T, SR>, (int)cp_trsm_smem<T, SR>(CP_TRSM_MAXN))) return;
+    gb300_count_launch(), trsm_slab_kernel<T, SR><<<cdiv(m, SR), 256, smem, s>>>(m, n, L, ldl, B, ldb);
+}
+
 template <typename T>
 void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long ldb)
 {
     if (m <= 0 || nc <= 0) return;
-    constexpr int SMALL_W = small_w<T>::value;
-    for (int j0 = 0; j0 < nc; j0 += SMALL_W) {
-        const int w = std::min(SMALL_W, nc - j0);
+    for (int j0 = 0; j0 < nc; j0 += CP_TRSM_MAXN) {
+        const int w = std::min(CP_TRSM_MAXN, nc - j0);
         const T *Ljj = L + j0 + (long)j0 * ldl;
         T *Bj = B + (long)j0 * ldb;
-        if (w == SMALL_W)
-            gb300_count_launch(), trsm_rltn_small_kernel<T, SMALL_W, true><<<cdiv(m, 128), 128, 0, s>>>(m, w, Ljj, ldl, Bj, ldb);
-        else
-            gb300_count_launch(), trsm_rltn_small_kernel<T, SMALL_W, false><<<cdiv(m, 128), 128, 0, s>>>(m, w, Ljj, ldl, Bj, ldb);
+        // 16 rows per CTA once that fills the GPU, else 4
+        if (m >= 16 * 128) trsm_slab<T, 16>(s, m, w, Ljj, ldl, Bj, ldb);
+        else trsm_slab<T, 4>(s, m, w, Ljj, ldl, Bj, ldb);
         const int rest = nc - j0 - w;
         if (rest > 0)
             gemm<T>(s, false, true, false, m, rest, w, T(-1), Bj, ldb, L + (j0 + w) + (long)j0 * ldl, ldl, T(1),
@@ -145,19 +169,18 @@ void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long l
 // column panel below it, then the lower-triangular trailing update.  This is
 // the loop of examples/cholesky/cholesky_implicit.c:244-318 with the tasks of
 // one step k fused into whole-panel launches.  Diagonal blocks larger than
-// SMALL_W are themselves factored by the same algorithm with tile SMALL_W.
+// the leaf (CP_W) are themselves factored by the same algorithm with tile CP_W.
 template <typename T>
 void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
 {
-    constexpr int SMALL_W = small_w<T>::value;
     if (nb <= 0) nb = n;
     for (int k0 = 0; k0 < n; k0 += nb) {
         const int kb = std::min(nb, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
-        if (kb <= SMALL_W)
-            gb300_count_launch(), potf2_small_kernel<T, SMALL_W><<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
+        if (kb <= CP_W)
+            gb300_count_launch(), potf2_leaf_kernel<T><<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
         else
-            potrf_tiled<T>(s, kb, Akk, lda, SMALL_W, info, info_base + k0);
+            potrf_tiled<T>(s, kb, Akk, lda, CP_W, info, info_base + k0);
         const int m = n - k0 - kb;
         if (m > 0) {
             T *P = A + (k0 + kb) + (long)k0 * lda;
@@ -169,42 +192,37 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
 }
 
 // POTRS with a lower factor: L y = b (forward), then L^T x = y (backward),
-// blocked by SMALL_W rows; min-dgels/base/SRC/dpotrs.c does the same two
-// sweeps through dtrsm.
-// Block width of the POTRS sweeps: 128 rows (FP32) / 64 rows (FP64) per
-// diagonal solve, so a sweep over n rows costs n / W diagonal solves and
-// n / W GEMM updates.
-template <typename T> struct potrs_w { static constexpr int value = 128; };
-template <> struct potrs_w<double> { static constexpr int value = 64; };
-
-template <typename T, bool TRANS>
-static void trsv_block(cudaStream_t s, int w, int nrhs, const T *L, long ldl, T *B, long ldb)
+// in blocks of CP_SB rows: solve the block, update the rows to come.
+// min-dgels/base/SRC/dpotrs.c does the same two sweeps through dtrsm.
+template <typename T, int C, bool TRANS>
+static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
-    constexpr int W = potrs_w<T>::value;
-    constexpr size_t smem = (size_t)(W * (W + 1) + W * 16) * sizeof(T);
-    if (gb300_func_dyn_smem((const void *)trsv_block_kernel<T, W, TRANS>, (int)smem)) return;
-    gb300_count_launch(), trsv_block_kernel<T, W, TRANS><<<cdiv(nrhs, 16), 128, smem, s>>>(w, nrhs, L, ldl, B, ldb);
+    constexpr size_t sm_blk = cp_trsv_smem<T, C>(TRANS), sm_upd = cp_upd_smem<T, C>(TRANS);
+    if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, C, TRANS>, (int)sm_blk) ||
+        gb300_func_dyn_smem((const void *)trsv_upd_kernel<T, C, TRANS>, (int)sm_upd))
+        return;
+    const int nblk = (n + CP_SB - 1) / CP_SB;
+    for (int b = 0; b < nblk; ++b) {
+        const int j0 = (TRANS ? nblk - 1 - b : b) * CP_SB, w = std::min(CP_SB, n - j0);
+        gb300_count_launch(), trsv_blk_kernel<T, C, TRANS>
+            <<<cdiv(nrhs, C), 256, sm_blk, s>>>(w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
+        const int rest = TRANS ? j0 : n - j0 - w;
+        if (rest <= 0) continue;
+        gb300_count_launch(), trsv_upd_kernel<T, C, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, C)), 256, sm_upd, s>>>(
+            rest, w, nrhs, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl, ldl, B + j0, TRANS ? B : B + j0 + w, ldb);
+    }
 }
 
 template <typename T>
 void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
     if (n <= 0 || nrhs <= 0) return;
-    constexpr int W = potrs_w<T>::value;
-    for (int j0 = 0; j0 < n; j0 += W) {
-        const int w = std::min(W, n - j0);
-        trsv_block<T, false>(s, w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
-        const int rest = n - j0 - w;
-        if (rest > 0)
-            gemm<T>(s, false, false, false, rest, nrhs, w, T(-1), L + (j0 + w) + (long)j0 * ldl, ldl, B + j0, ldb,
-                    T(1), B + j0 + w, ldb);
-    }
-    const int last = ((n - 1) / W) * W;
-    for (int j0 = last; j0 >= 0; j0 -= W) {
-        const int w = std::min(W, n - j0);
-        trsv_block<T, true>(s, w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
-        if (j0 > 0)
-            gemm<T>(s, true, false, false, j0, nrhs, w, T(-1), L + j0, ldl, B + j0, ldb, T(1), B, ldb);
+    if (nrhs == 1) {
+        potrs_sweep_blocks<T, 1, false>(s, n, nrhs, L, ldl, B, ldb);
+        potrs_sweep_blocks<T, 1, true>(s, n, nrhs, L, ldl, B, ldb);
+    } else {
+        potrs_sweep_blocks<T, 4, false>(s, n, nrhs, L, ldl, B, ldb);
+        potrs_sweep_blocks<T, 4, true>(s, n, nrhs, L, ldl, B, ldb);
     }
 }
 
@@ -283,7 +301,7 @@ int starpu_gb300_spotrf_tile(void *stream, int n, float *A, int lda, int *d_info
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, small_w<float>::value, d_info, 0);
+    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0);
     return gb300_last_launch_status();
 }
 
@@ -291,21 +309,21 @@ int starpu_gb300_dpotrf_tile(void *stream, int n, double *A, int lda, int *d_inf
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, small_w<double>::value, d_info, 0);
+    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0);
     return gb300_last_launch_status();
 }
 
 int starpu_gb300_spotrf_tile_status(void *stream, int n, float *A, int lda, int *d_status)
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
-    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, small_w<float>::value, d_status, 0);
+    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0);
     return gb300_last_launch_status();
 }
 
 int starpu_gb300_dpotrf_tile_status(void *stream, int n, double *A, int lda, int *d_status)
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
-    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, small_w<double>::value, d_status, 0);
+    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0);
     return gb300_last_launch_status();
 }
 

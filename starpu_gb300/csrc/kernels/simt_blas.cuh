@@ -182,101 +182,6 @@ gemm_simt_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long lda
 }
 
 // ---------------------------------------------------------------------------
-// Unblocked Cholesky of one n x n (n <= NMAX) diagonal block, lower, held in
-// registers.  Same arithmetic as the reference CPU codelet loop
-// (examples/cholesky/cholesky_kernels.c:329-342): lambda = sqrt(a_zz),
-// scale the column by 1/lambda, rank-1 update of the trailing lower part.
-// A non-positive (or NaN) pivot records info = info_base + z + 1 (LAPACK
-// convention, first failure wins) in *info; the kernel never traps.
-// ---------------------------------------------------------------------------
-template <typename T, int NMAX>
-__global__ void __launch_bounds__(256) potf2_small_kernel(int n, T *__restrict__ A, long lda, int *info, int info_base)
-{
-    // 256 threads as NMAX rows x CL column lanes; thread (ti, tc) keeps row ti,
-    // columns tc, tc + CL, ... in registers.  The step loop is unrolled so
-    // that column z lives in a fixed register of its owners; the owners
-    // publish column z through a double-buffered shared vector (one barrier
-    // per step), every thread scales its two factors by 1/sqrt(a_zz) itself.
-    constexpr int CL = 256 / NMAX, NC = NMAX / CL;
-    __shared__ T col[2][NMAX];
-    const int tid = threadIdx.x;
-    const int ti = tid % NMAX, tc = tid / NMAX;
-    T a[NC];
-#pragma unroll
-    for (int q = 0; q < NC; ++q) {
-        const int c = tc + q * CL;
-        a[q] = (ti < n && c <= ti) ? A[(long)ti + (long)c * lda] : T(0);
-    }
-    bool bad = false;
-#pragma unroll
-    for (int z = 0; z < NMAX; ++z) {
-        if (z >= n) break;
-        T *cz = col[z & 1];
-        if (tc == z % CL) cz[ti] = a[z / CL];  // owners of column z publish it (rows < z hold 0)
-        __syncthreads();
-        const T d = cz[z];
-        if (!(d > T(0)) && !bad) {
-            bad = true;
-            if (tid == 0 && info) atomicCAS(info, 0, info_base + z + 1);
-        }
-        const T lzz = sqrt(d);
-        const T inv = T(1) / lzz;
-        const T li = cz[ti] * inv;
-        if (tc == z % CL) a[z / CL] = (ti == z) ? lzz : (ti > z ? li : a[z / CL]);
-        if (ti > z) {
-#pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                const int c = tc + q * CL;
-                if (c > z && c <= ti) a[q] = fma(-li, cz[c] * inv, a[q]);
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < NC; ++q) {
-        const int c = tc + q * CL;
-        if (ti < n && c <= ti) A[(long)ti + (long)c * lda] = a[q];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// B[m x w] <- B * L^{-T}, L w x w lower non-unit (w <= W): the right-side
-// TRSM of the panel (cublasStrsm(R,L,T,N), cholesky_kernels.c:258) for one
-// column block.  Every row of B is an independent forward substitution; one
-// thread owns one row in registers.  Column-oriented order like reference
-// BLAS strsm: x_j *= 1/L_jj, then x_c -= L_cj * x_j for c > j.
-// ---------------------------------------------------------------------------
-template <typename T, int W, bool FULL>
-__global__ void __launch_bounds__(128) trsm_rltn_small_kernel(int m, int w, const T *__restrict__ L, long ldl,
-                                                              T *__restrict__ B, long ldb)
-{
-    __shared__ T Ls[W][W + 1];
-    __shared__ T invd[W];
-    const int tid = threadIdx.x;
-    const int ww = FULL ? W : w;
-    for (int idx = tid; idx < W * W; idx += blockDim.x) {
-        int i = idx % W, j = idx / W;
-        Ls[i][j] = (i < ww && j < ww && i >= j) ? L[(long)i + (long)j * ldl] : T(0);
-    }
-    __syncthreads();
-    for (int j = tid; j < W; j += blockDim.x) invd[j] = (j < ww) ? T(1) / Ls[j][j] : T(0);
-    __syncthreads();
-    const long r = (long)blockIdx.x * blockDim.x + tid;
-    if (r >= m) return;
-    T x[W];
-#pragma unroll
-    for (int c = 0; c < W; ++c) x[c] = (FULL || c < ww) ? B[r + (long)c * ldb] : T(0);
-#pragma unroll
-    for (int j = 0; j < W; ++j) {
-        x[j] *= invd[j];
-#pragma unroll
-        for (int c = j + 1; c < W; ++c) x[c] = fma(-Ls[c][j], x[j], x[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < W; ++c)
-        if (FULL || c < ww) B[r + (long)c * ldb] = x[c];
-}
-
-// ---------------------------------------------------------------------------
 // Left-side small triangular solves on a w x nrhs block (w <= W), one thread
 // per right-hand side.  Used by the blocked POTRS (forward L y = b, backward
 // L^T x = y), mirroring LAPACK dpotrs (min-dgels/base/SRC/dpotrs.c): two
@@ -316,60 +221,6 @@ __global__ void __launch_bounds__(64) trsm_left_small_kernel(int w, int nrhs, co
 #pragma unroll
     for (int i = 0; i < W; ++i)
         if (i < w) B[(long)i + (long)c * ldb] = x[i];
-}
-
-// ---------------------------------------------------------------------------
-// Diagonal-block solve of the blocked POTRS with wide blocks (w <= W, W up
-// to 128): L_ii (w x w) and 16 right-hand-side columns of the block are
-// staged in shared memory; each column is owned by 8 consecutive lanes that
-// compute one row at a time as a dot product split 8 ways and reduced with
-// shuffles, so rows advance with warp-level synchronisation only.
-//   TRANS = false: y_r = (b_r - sum_{c<r} L_rc y_c) / L_rr,  r = 0..w-1
-//   TRANS = true : x_r = (y_r - sum_{c>r} L_cr x_c) / L_rr,  r = w-1..0
-// Launch: ceil(nrhs / 16) CTAs of 128 threads, dynamic shared memory
-// (W * (W + 1) + W * 16) * sizeof(T).
-// ---------------------------------------------------------------------------
-template <typename T, int W, bool TRANS>
-__global__ void __launch_bounds__(128) trsv_block_kernel(int w, int nrhs, const T *__restrict__ L, long ldl,
-                                                         T *__restrict__ B, long ldb)
-{
-    extern __shared__ __align__(16) unsigned char trsv_smem[];
-    T *Ls = (T *)trsv_smem;            // [W][W+1], Ls[r * (W+1) + c] = L(r, c)
-    T *Ys = Ls + W * (W + 1);          // [16][W]
-    const int tid = threadIdx.x;
-    const int col0 = blockIdx.x * 16;
-    for (int idx = tid; idx < w * w; idx += blockDim.x) {
-        const int r = idx % w, c = idx / w;
-        Ls[r * (W + 1) + c] = (r >= c) ? L[(long)r + (long)c * ldl] : T(0);
-    }
-    for (int idx = tid; idx < 16 * w; idx += blockDim.x) {
-        const int r = idx % w, j = idx / w;
-        Ys[j * W + r] = (col0 + j < nrhs) ? B[(long)r + (long)(col0 + j) * ldb] : T(0);
-    }
-    __syncthreads();
-    const int j = tid >> 3;      // right-hand side owned by this group of 8 lanes
-    const int l8 = tid & 7;
-    T *y = Ys + j * W;
-    const unsigned gmask = 0xFFu << ((tid & 31) & ~7);
-    for (int s = 0; s < w; ++s) {
-        const int r = TRANS ? (w - 1 - s) : s;
-        T acc = T(0);
-        if (!TRANS) {
-            for (int c = l8; c < r; c += 8) acc = fma(Ls[r * (W + 1) + c], y[c], acc);
-        } else {
-            for (int c = r + 1 + l8; c < w; c += 8) acc = fma(Ls[c * (W + 1) + r], y[c], acc);
-        }
-        acc += __shfl_xor_sync(gmask, acc, 1);
-        acc += __shfl_xor_sync(gmask, acc, 2);
-        acc += __shfl_xor_sync(gmask, acc, 4);
-        if (l8 == 0) y[r] = (y[r] - acc) / Ls[r * (W + 1) + r];
-        __syncwarp(gmask);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < 16 * w; idx += blockDim.x) {
-        const int r = idx % w, jj = idx / w;
-        if (col0 + jj < nrhs) B[(long)r + (long)(col0 + jj) * ldb] = Ys[jj * W + r];
-    }
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,113 @@
+"""Plain FP32 / FP64 factorisation and solve kernels at the sizes where their
+blocking changes: leaf and panel remainders, the row counts that pick the
+panel solve's slab, the product tiles, and the solve's block and column groups.
+Reference: numpy in FP64."""
+import numpy as np
+import pytest
+
+from starpu_gb300 import DeviceBuffer
+from starpu_gb300.native import check
+
+pytestmark = pytest.mark.gpu
+
+EPS = {np.float32: 2.0**-24, np.float64: 2.0**-53}
+P = {np.float32: "s", np.float64: "d"}
+BOTH = pytest.mark.parametrize("dtype", [np.float32, np.float64])
+
+
+def up(a):
+    return DeviceBuffer.from_array(np.asfortranarray(a))
+
+
+def spd(n, seed, scale=None):
+    rng = np.random.default_rng(seed)
+    b = rng.standard_normal((n, n))
+    a = b @ b.T / n + np.eye(n)
+    return a if scale is None else a * scale[:, None] * scale[None, :]
+
+
+def fn(gpu, dtype, name):
+    return getattr(gpu, "starpu_gb300_" + P[dtype] + name)
+
+
+@BOTH
+@pytest.mark.parametrize("m,n", [(1, 1), (3, 64), (17, 127), (2047, 70), (2048, 64), (2049, 130), (5, 1025), (2100, 1100)])
+def test_trsm_slabs(gpu, dtype, m, n):
+    l = np.linalg.cholesky(spd(n, n)).astype(dtype)
+    b = np.random.default_rng(m).uniform(-1, 1, (m, n)).astype(dtype)
+    dl, db = up(l), up(np.vstack([b, np.full((2, n), 7, dtype)]))  # two rows of padding below
+    check(fn(gpu, dtype, "trsm_rltn_tile")(None, m, n, 1.0, dl.ptr, n, db.ptr, m + 2))
+    out = db.download((m + 2, n), dtype)
+    assert np.all(out[m:] == 7)
+    x = out[:m].astype(np.float64)
+    # each row solves L x = b with backward error <= c n eps |L| |x|
+    bound = 4 * n * EPS[dtype] * (np.abs(x) @ np.abs(l.astype(np.float64)).T + np.abs(b))
+    assert np.all(np.abs(x @ l.astype(np.float64).T - b) <= bound)
+
+
+@BOTH
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (31, 3), (33, 4), (256, 1), (257, 5), (511, 17), (700, 64), (1030, 2)])
+def test_potrs_blocks(gpu, dtype, n, nrhs):
+    l = np.linalg.cholesky(spd(n, n)).astype(dtype)
+    l[np.triu_indices(n, 1)] = np.nan  # never read
+    b = np.random.default_rng(n + nrhs).uniform(-1, 1, (n, nrhs)).astype(dtype)
+    dl, db = up(l), up(b)
+    check(fn(gpu, dtype, "potrs")(None, n, nrhs, dl.ptr, n, db.ptr, n))
+    x = db.download((n, nrhs), dtype).astype(np.float64)
+    l = np.tril(np.nan_to_num(l)).astype(np.float64)
+    y = np.abs(l.T) @ np.abs(x)
+    bound = 8 * n * EPS[dtype] * (np.abs(l) @ y + np.abs(b))
+    assert np.all(np.abs(l @ (l.T @ x) - b) <= bound)
+
+
+@BOTH
+@pytest.mark.parametrize("m,n,k", [(33, 31, 64), (300, 290, 65), (640, 700, 33), (1200, 1100, 64), (1700, 1650, 17)])
+@pytest.mark.parametrize("lower", [False, True])
+def test_product_tiles(gpu, dtype, m, n, k, lower):
+    n = m if lower else n
+    rng = np.random.default_rng(m + k)
+    a, b, c = (rng.standard_normal(s).astype(dtype) for s in ((m, k), (n, k), (m, n)))
+    b = a if lower else b
+    da, db, dc = up(a), up(b), up(c)
+    if lower:
+        check(fn(gpu, dtype, "syrk_ln_tile")(None, n, k, -1.0, da.ptr, n, 1.0, dc.ptr, n))
+    else:
+        check(fn(gpu, dtype, "gemm_nt_tile")(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    out = dc.download((m, n), dtype).astype(np.float64)
+    a, b, c = (v.astype(np.float64) for v in (a, b, c))
+    ref, bound = c - a @ b.T, (k + 2) * EPS[dtype] * (np.abs(c) + np.abs(a) @ np.abs(b).T)
+    keep = np.tril(np.ones((m, n), bool)) if lower else np.ones((m, n), bool)
+    assert np.all(np.abs(out - ref)[keep] <= bound[keep])
+    assert np.array_equal(out[~keep], c[~keep])
+
+
+@BOTH
+@pytest.mark.parametrize("n,nb", [(63, 64), (65, 16), (127, 64), (191, 64), (192, 512), (193, 512), (321, 100), (700, 512), (1281, 256), (3001, 512)])
+def test_potrf_blocks(gpu, dtype, n, nb):
+    # rows and columns scaled over 12 orders of magnitude (FP32: 6)
+    d = np.power(10.0, np.random.default_rng(n).uniform(-6, 6, n) * (1.0 if dtype == np.float64 else 0.5))
+    a = spd(n, n, d).astype(dtype)
+    lda = n + 1
+    pad = np.full((lda, n), 3, dtype, order="F")
+    pad[:n] = a
+    da, info = up(pad), up(np.full(1, 9, np.int32))
+    check(fn(gpu, dtype, "potrf")(None, n, da.ptr, lda, nb, info.ptr))
+    out = da.download((lda, n), dtype)
+    assert info.download((1,), np.int32)[0] == 0
+    iu = np.triu_indices(n, 1)
+    assert np.array_equal(out[:n][iu], a[iu]) and np.all(out[n] == 3)
+    l = np.tril(out[:n]).astype(np.float64)
+    a = a.astype(np.float64)
+    # |A - L L^T| <= c (n + 1) eps |L| |L|^T, and |L| |L|^T <= sqrt(a_ii a_jj)
+    s = np.sqrt(np.diag(a))
+    assert np.all(np.abs(np.tril(a - l @ l.T)) <= 2 * (n + 1) * EPS[dtype] * s[:, None] * s[None, :])
+
+
+@BOTH
+@pytest.mark.parametrize("n,k", [(1, 1), (40, 3), (64, 64), (100, 65), (500, 130), (500, 331), (1000, 1000)])
+def test_first_bad_pivot_is_reported(gpu, dtype, n, k):
+    a = spd(n, n).astype(dtype)
+    a[k - 1, k - 1] = -1.0
+    da, info = up(a), up(np.zeros(1, np.int32))
+    check(fn(gpu, dtype, "potrf")(None, n, da.ptr, n, 256, info.ptr))
+    assert info.download((1,), np.int32)[0] == k
