@@ -4,6 +4,7 @@
 // on the caller's stream and returns; nothing here synchronises or allocates.
 #include "kernels/chol_panel.cuh"
 #include "kernels/simt_blas.cuh"
+#include "kernels/slice_update.cuh"
 #include "kernels/trsv_sweep.cuh"
 #include "gb300_internal.h"
 #include "starpu_gb300_kernels.h"
@@ -12,6 +13,9 @@
 #include <type_traits>
 
 namespace gb300 {
+
+// smallest trailing matrix whose FP64 update runs on the tensor cores
+constexpr int SLICE_MIN_M = 128;
 
 static inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 
@@ -165,6 +169,48 @@ void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long l
     }
 }
 
+// C[m x n] -= A B^T in FP64 on the tensor cores (kernels/slice_update.cuh), A
+// m x k and B n x k with the given element strides, k cut into launches of 64.
+static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const double *A, long a_rs, long a_ks,
+                         const double *B, long b_rs, long b_ks, double *C, long ldc, int *err)
+{
+    if (m <= 0 || n <= 0 || k <= 0) return;
+    if (gb300_func_dyn_smem((const void *)slice_update_kernel, SU_SMEM)) return;
+    SliceUpdateArgs a;
+    a.a_rs = a_rs, a.a_ks = a_ks, a.b_rs = b_rs, a.b_ks = b_ks;
+    a.C = C, a.ldc = ldc, a.m = m, a.n = n, a.lower = lower ? 1 : 0;
+    a.row_blocks = (m + SU_BM - 1) / SU_BM;
+    a.col_tiles = (n + SU_BN - 1) / SU_BN;
+    a.err = err;
+    a.wait_budget_ns = 2000000000ull;  // 2 s per wait: far above any legitimate stall
+    const int sms = gb300_device_sms();
+    auto tiles = [&](int rb) { return lower ? std::min(a.col_tiles, (SU_BM / SU_BN) * (rb + 1)) : a.col_tiles; };
+    long total = 0;
+    for (int rb = 0; rb < a.row_blocks; ++rb) total += tiles(rb);
+    // a work item cuts its 128 rows of A once (about the time of a tile):
+    // long items, but four or more per SM to balance them
+    a.seg = (int)std::max(1L, std::min(16L, total / (4L * sms)));
+    a.items = 0;
+    for (int rb = 0; rb < a.row_blocks; ++rb) a.items += (tiles(rb) + a.seg - 1) / a.seg;
+    for (int k0 = 0; k0 < k; k0 += SU_K) {
+        a.A = A + k0 * a_ks;
+        a.B = B + k0 * b_ks;
+        a.k = std::min(SU_K, k - k0);
+        gb300_count_launch(), slice_update_kernel<<<std::min(a.items, sms), SU_THREADS, SU_SMEM, s>>>(a);
+    }
+}
+
+// Trailing update of one step: C (m x m, lower) -= P P^T, P m x k.
+static void trailing_update(cudaStream_t s, int m, int k, const float *P, long ldp, float *C, long ldc, int *)
+{
+    gemm<float>(s, false, true, true, m, m, k, -1.0f, P, ldp, P, ldp, 1.0f, C, ldc);
+}
+static void trailing_update(cudaStream_t s, int m, int k, const double *P, long ldp, double *C, long ldc, int *err)
+{
+    if (m < SLICE_MIN_M) gemm<double>(s, false, true, true, m, m, k, -1.0, P, ldp, P, ldp, 1.0, C, ldc);
+    else slice_update(s, true, m, m, k, P, 1, ldp, P, 1, ldp, C, ldc, err);
+}
+
 // Right-looking tiled Cholesky with tile nb: POTRF(k), TRSM of the whole
 // column panel below it, then the lower-triangular trailing update.  This is
 // the loop of examples/cholesky/cholesky_implicit.c:244-318 with the tasks of
@@ -174,6 +220,8 @@ template <typename T>
 void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
 {
     if (nb <= 0) nb = n;
+    // FP64: the FP64 units would bound wider panels, the tensor-core update takes 64 columns
+    if (std::is_same<T, double>::value) nb = std::min(nb, CP_W);
     for (int k0 = 0; k0 < n; k0 += nb) {
         const int kb = std::min(nb, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
@@ -185,8 +233,7 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
         if (m > 0) {
             T *P = A + (k0 + kb) + (long)k0 * lda;
             trsm_rltn<T>(s, m, kb, Akk, lda, P, lda);
-            gemm<T>(s, false, true, true, m, m, kb, T(-1), P, lda, P, lda, T(1), A + (k0 + kb) + (long)(k0 + kb) * lda,
-                    lda);
+            trailing_update(s, m, kb, P, lda, A + (k0 + kb) + (long)(k0 + kb) * lda, lda, info);
         }
     }
 }

@@ -1,6 +1,7 @@
 """Plain FP32 / FP64 factorisation and solve kernels at the sizes where their
 blocking changes: leaf and panel remainders, the row counts that pick the
-panel solve's slab, the product tiles, and the solve's block and column groups.
+panel solve's slab, the product tiles, the solve's block and column groups,
+and the FP64 update on the tensor cores (tile, segment and row-block edges).
 Reference: numpy in FP64."""
 import numpy as np
 import pytest
@@ -111,3 +112,15 @@ def test_first_bad_pivot_is_reported(gpu, dtype, n, k):
     da, info = up(a), up(np.zeros(1, np.int32))
     check(fn(gpu, dtype, "potrf")(None, n, da.ptr, n, 256, info.ptr))
     assert info.download((1,), np.int32)[0] == k
+
+
+def test_fp64_update_keeps_nan_in_its_row(gpu):
+    n, i = 400, 250
+    a = spd(n, n)
+    a[i, 10] = a[10, i] = np.nan
+    da, info = up(a), up(np.zeros(1, np.int32))
+    check(gpu.starpu_gb300_dpotrf(None, n, da.ptr, n, 64, info.ptr))
+    out = da.download((n, n), np.float64)
+    assert info.download((1,), np.int32)[0] == i + 1
+    ref = np.linalg.cholesky(spd(n, n)[:i, :i])
+    assert np.allclose(np.tril(out[:i, :i]), ref, rtol=0, atol=1e-13)
