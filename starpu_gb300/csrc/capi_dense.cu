@@ -16,6 +16,11 @@ namespace gb300 {
 
 // smallest trailing matrix whose FP64 update runs on the tensor cores
 constexpr int SLICE_MIN_M = 128;
+// largest FP32 matrix (or diagonal tile) that one cooperative launch factors:
+// 1522 us at n = 4096 against 2417 us in tiles of 256 with a launch per tile,
+// panel and update; beyond, its 64-wide updates would read and write the
+// trailing matrix too often
+constexpr int COOP_MAX_N = 4096;
 
 static inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 
@@ -214,12 +219,14 @@ static void trailing_update(cudaStream_t s, int m, int k, const double *P, long 
 // Right-looking tiled Cholesky with tile nb: POTRF(k), TRSM of the whole
 // column panel below it, then the lower-triangular trailing update.  This is
 // the loop of examples/cholesky/cholesky_implicit.c:244-318 with the tasks of
-// one step k fused into whole-panel launches.  Diagonal blocks larger than
-// the leaf (CP_W) are themselves factored by the same algorithm with tile CP_W.
+// one step k fused into whole-panel launches.  FP32 diagonal blocks, and whole
+// matrices up to COOP_MAX_N, are factored by one cooperative launch
+// (kernels/diag_coop.cuh); FP64 goes in panels of CP_W columns.
 template <typename T>
 void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
 {
     if (nb <= 0) nb = n;
+    if (std::is_same<T, float>::value && n <= COOP_MAX_N) nb = n;
     // FP64: the FP64 units would bound wider panels, the tensor-core update takes 64 columns
     if (std::is_same<T, double>::value) nb = std::min(nb, CP_W);
     for (int k0 = 0; k0 < n; k0 += nb) {
@@ -227,6 +234,8 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
         T *Akk = A + k0 + (long)k0 * lda;
         if (kb <= CP_W)
             gb300_count_launch(), potf2_leaf_kernel<T><<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
+        else if (std::is_same<T, float>::value && kb <= COOP_MAX_N)
+            potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0);
         else
             potrf_tiled<T>(s, kb, Akk, lda, CP_W, info, info_base + k0);
         const int m = n - k0 - kb;

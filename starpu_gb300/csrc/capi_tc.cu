@@ -388,7 +388,7 @@ static int diag_factor_inverse(cudaStream_t s, int n, float *A, long lda, float 
     const int sms = max_sms > 0 ? std::min(max_sms, num_sms()) : num_sms();
     const int grid = std::max(1, std::min(work, sms * std::max(occ, 1)));
     if (invert) cudaMemset2DAsync(Linv, ldi * sizeof(float), 0, n * sizeof(float), n, s);
-    cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
+    if (bar) cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
     DiagCoopArgs a;
     a.n = n;
     a.A = A;
@@ -405,6 +405,11 @@ static int diag_factor_inverse(cudaStream_t s, int n, float *A, long lda, float 
     gb300_count_launch();
     return gb300_record_cuda_error(
         cudaLaunchCooperativeKernel((const void *)diag_coop_kernel, dim3(grid), dim3(DC_T), args, 0, s));
+}
+
+int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base)
+{
+    return diag_factor_inverse(s, n, A, lda, nullptr, 0, nullptr, nullptr, info, info_base, nullptr, false);
 }
 
 // A high-priority stream and a fork / join event pair per host thread and

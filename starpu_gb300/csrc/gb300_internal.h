@@ -11,6 +11,10 @@ namespace gb300 {
 // largest diagonal tile the cooperative factor-and-invert kernel handles
 constexpr int GB300_DIAG_TILE_MAX = 1024;
 
+// FP32 lower Cholesky of the whole n x n matrix in one cooperative launch,
+// no workspace (capi_tc.cu)
+int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base);
+
 // residual partials P_z = -(A X) on the tensor cores (capi_tc.cu)
 size_t residual_tc_a_bytes(int n);
 int residual_tc_slice_a(cudaStream_t s, int n, const double *A, long lda, const unsigned long long *amax_bits,

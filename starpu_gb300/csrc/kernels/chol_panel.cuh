@@ -9,6 +9,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
+
 namespace gb300 {
 
 constexpr int CP_W = 64;  // order of a leaf and width of a panel step
@@ -18,26 +20,28 @@ template <typename T> struct alignas(16) Quad {
     T v[4];
 };
 
-// 1 / sqrt(d) to about one ulp: the hardware approximation and one correction
-// step, which keeps the pivot chain of the leaf short (a square root and a
-// division cost several times as much).  Outside the normal range, and for
-// d <= 0 or NaN, the plain functions give what the unblocked loop gives.
+// 1 / sqrt(d) to about one ulp for d in the normal range (cp_normal): the
+// hardware approximation and one correction step, which keeps the pivot chain
+// of the leaf short (a square root and a division cost several times as much).
+__device__ __forceinline__ bool cp_normal(float d) { return d >= 1.17549435e-38f && d <= 1.7014118e38f; }
+__device__ __forceinline__ bool cp_normal(double d) { return d >= 2.3e-308 && d <= 1.7e308; }
 __device__ __forceinline__ float cp_rsqrt(float d)
 {
-    if (!(d >= 1.17549435e-38f && d <= 3.0e38f)) return 1.0f / sqrtf(d);
-    const float r = rsqrtf(d);
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(0.5f * r, fmaf(-d * r, r, 1.0f), r);
 }
 // r from the approximation with relative error below 2^-19, then
 // r (1 + e/2 + 3 e^2/8) with e = 1 - d r^2: the next term is (5/16) e^3 < 2^-55
 __device__ __forceinline__ double cp_rsqrt(double d)
 {
-    if (!(d >= 2.3e-308 && d <= 1.7e308)) return 1.0 / sqrt(d);
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
     const double e = fma(-d * r, r, 1.0);
     return fma(r * e, fma(0.375, e, 0.5), r);
 }
+// outside it, and for d <= 0 or NaN: what the unblocked loop gives
+template <typename T> __device__ __noinline__ T cp_rsqrt_any(T d) { return T(1) / sqrt(d); }
 
 template <typename T> __device__ __forceinline__ T cp_dot_sub(T c, const Quad<T> &a, const Quad<T> &b)
 {
@@ -47,107 +51,231 @@ template <typename T> __device__ __forceinline__ T cp_dot_sub(T c, const Quad<T>
 }
 
 // ---------------------------------------------------------------------------
-// Cholesky of the n x n (n <= 64) lower block A, in place, by one CTA of 8
-// warps.  Lane = row (two rows per lane), warp w owns columns 4w .. 4w+3 and
-// 32 + 4w .. 32 + 4w + 3, in registers.  The 64 columns go four at a time
-// (16 steps, one barrier each): the warp that owns the step's columns fetches
-// their 4 x 4 diagonal block with ten shuffles, every lane factors it for
-// itself (no shuffle or barrier inside the pivot chain), solves its own two
-// rows and publishes them; then every warp applies the rank-4 update to the
-// columns it still has to the right.  Bound by the chain of 64 dependent
-// pivots.  Same operations as the reference codelet loop
+// The panel of one 64-column step, by one CTA of 8 warps: Cholesky of the n x
+// n (n <= 64) block d and, when NX = 2, the solve x <- x L^-T of 64 rows x
+// along with it.  Blocks are held in registers: lane = row (two per lane),
+// warp w owns columns 4w .. 4w + 3 and 32 + 4w .. 32 + 4w + 3.
+//
+// The columns go four at a time (16 steps).  The warp that owns a step's
+// columns factors their 4 x 4 diagonal block, solves its rows and publishes
+// the four columns in shared memory (a buffer and an mbarrier per step, so no
+// CTA barrier); the other warps apply the rank-4 update to the columns they
+// still have to the right.  The owner of the next step updates those columns
+// first, publishes, and catches up on its others afterwards: the chain of one
+// step is wait, update of 4 columns, factor, solve, publish.  Bound by that
+// chain of 16 steps.  Same operations as the reference codelet loop
 // (cholesky_kernels.c:329-342), four columns at a time; a non-positive (or
 // NaN) pivot records info_base + its 1-based column in *info, first one wins.
 // ---------------------------------------------------------------------------
-// steps 8 G0 .. 8 G0 + 7 of the leaf (columns 32 G0 .. 32 G0 + 31)
-template <typename T, int G0>
-__device__ __forceinline__ void cp_leaf_steps(T (&a)[2][4][2], Quad<T> (*pan)[CP_W], int n, int *info, int info_base)
+template <typename T> using CpBlock = T[2][4][2];  // [column group][column][row half]
+
+// the published columns of every step: rows 0 .. 63 of d, then those of x
+template <typename T, int NX> using CpPanel = Quad<T>[16][CP_W + 32 * NX];
+
+constexpr int CP_ERR_TIMEOUT = -1000;
+
+// Once per kernel, before a CTA barrier.
+__device__ __forceinline__ void cp_panel_init(uint64_t (&bar)[16])
+{
+    if (threadIdx.x < 16) ptx::mbar_init(&bar[threadIdx.x], 32);
+    ptx::fence_mbarrier_init();
+}
+
+// One thread's elements of a block: f(value, row, column)
+template <typename T, typename F> __device__ __forceinline__ void cp_each(CpBlock<T> &v, F f)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int steps = min(8, (n - 32 * G0 + 3) / 4);
-#pragma unroll 1
-    for (int ow = 0; ow < steps; ++ow) {
-        Quad<T> *p = pan[ow & 1];
-        if (warp == ow) {
-            T d[4][4], r[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+    for (int g = 0; g < 2; ++g)
 #pragma unroll
-                for (int j = 0; j <= i; ++j) d[i][j] = __shfl_sync(0xffffffffu, a[G0][j][G0], 4 * ow + i);
-            int bad = -1;
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (!(d[j][j] > T(0)) && bad < 0) bad = j;
-                r[j] = cp_rsqrt(d[j][j]);
+            for (int h = 0; h < 2; ++h) f(v[g][c][h], 32 * h + lane, 32 * g + 4 * warp + c);
+}
+
+// the published columns of step s (bounded: the publisher never waits for this warp)
+__device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity)
+{
+    for (int i = 0; i < (1 << 22); ++i)
+        if (ptx::mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+
+// rank-4 update of the column groups G .. LAST by a published step
+template <typename T, int NX, int G, int LAST>
+__device__ __forceinline__ void cp_update(CpBlock<T> &d, CpBlock<T> &x, const Quad<T> *p)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Quad<T> ld[2], lx[2];
 #pragma unroll
-                for (int i = j + 1; i < 4; ++i) d[i][j] *= r[j];
+    for (int h = G; h < 2; ++h) ld[h] = p[32 * h + lane];
 #pragma unroll
-                for (int k = j + 1; k < 4; ++k)
+    for (int h = 0; h < NX; ++h) lx[h] = p[CP_W + 32 * h + lane];
 #pragma unroll
-                    for (int i = k; i < 4; ++i) d[i][k] = fma(-d[i][j], d[k][j], d[i][k]);
-            }
-            if (bad >= 0 && lane == 0 && info) {
-                const int col = 32 * G0 + 4 * ow + bad;
-                if (col < n) atomicCAS(info, 0, info_base + col + 1);
-            }
+    for (int g = G; g <= LAST; ++g)
 #pragma unroll
-            for (int h = G0; h < 2; ++h) {
-                Quad<T> x;
+        for (int c = 0; c < 4; ++c) {
+            const Quad<T> lc = p[32 * g + 4 * warp + c];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    T v = a[G0][j][h];
+            for (int h = g; h < 2; ++h) d[g][c][h] = cp_dot_sub(d[g][c][h], ld[h], lc);
 #pragma unroll
-                    for (int q = 0; q < j; ++q) v = fma(-x.v[q], d[j][q], v);
-                    x.v[j] = v * r[j];
-                    a[G0][j][h] = x.v[j];
-                }
-                p[32 * h + lane] = x;
-            }
+            for (int h = 0; h < NX; ++h) x[g][c][h] = cp_dot_sub(x[g][c][h], lx[h], lc);
         }
-        __syncthreads();
-        Quad<T> li[2];
+}
+
+// FP32: the four lanes that hold the rows of the 4 x 4 diagonal block pass it
+// through shared memory; every lane factors it for itself and solves its
+// rows, so nothing is exchanged inside the pivot chain.
+template <bool ANY> __device__ __forceinline__ void cp_factor4(float (&l)[4][4], float (&r)[4])
+{
 #pragma unroll
-        for (int h = G0; h < 2; ++h) li[h] = p[32 * h + lane];
+    for (int j = 0; j < 4; ++j) {
+        r[j] = ANY && !cp_normal(l[j][j]) ? cp_rsqrt_any(l[j][j]) : cp_rsqrt(l[j][j]);
 #pragma unroll
-        for (int g = G0; g < 2; ++g) {
-            if (g == G0 && warp <= ow) continue;
+        for (int i = j + 1; i < 4; ++i) l[i][j] *= r[j];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const Quad<T> lc = p[32 * g + 4 * warp + c];
+        for (int k = j + 1; k < 4; ++k)
 #pragma unroll
-                for (int h = g; h < 2; ++h) a[g][c][h] = cp_dot_sub(a[g][c][h], li[h], lc);
-            }
-        }
+            for (int i = k; i < 4; ++i) l[i][k] = fmaf(-l[i][j], l[k][j], l[i][k]);
     }
 }
 
+template <int NX, int G>
+__device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Quad<float> *p)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float l[4][4], r[4];
+    auto fetch = [&] {
+        const int row = 32 * G + 4 * warp;
+        if ((lane >> 2) == warp) p[32 * G + lane] = {d[G][0][G], d[G][1][G], d[G][2][G], d[G][3][G]};
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const Quad<float> v = p[row + i];
+#pragma unroll
+            for (int j = 0; j <= i; ++j) l[i][j] = v.v[j];
+        }
+        __syncwarp();
+    };
+    fetch();
+    cp_factor4<false>(l, r);
+    // pivots outside the normal range (their bits, less those of the smallest
+    // normal number, exceed the range's): again, with the plain functions
+    int bad = -1;
+    unsigned off = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) off = max(off, __float_as_uint(l[j][j]) - 0x00800000u);
+    if (off > 0x7E000000u) {
+        fetch();
+        cp_factor4<true>(l, r);
+#pragma unroll
+        for (int j = 3; j >= 0; --j)
+            if (!(l[j][j] > 0.0f)) bad = j;
+    }
+    auto solve = [&](float(&c)[4][2], int h, int row) {
+        Quad<float> y;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float v = c[j][h];
+#pragma unroll
+            for (int q = 0; q < j; ++q) v = fmaf(-y.v[q], l[j][q], v);
+            y.v[j] = v * r[j];
+            c[j][h] = y.v[j];
+        }
+        p[row] = y;
+    };
+#pragma unroll
+    for (int h = G; h < 2; ++h) solve(d[G], h, 32 * h + lane);
+#pragma unroll
+    for (int h = 0; h < NX; ++h) solve(x[G], h, CP_W + 32 * h + lane);
+    return bad;
+}
+
+// FP64: an instruction takes a sub-partition's FP64 unit for 64 clocks
+// whatever the number of lanes, so the four columns go one by one, each lane
+// on its own rows: 20 + 5 operations per row half instead of 36 + 10.
+template <int NX, int G>
+__device__ __forceinline__ int cp_solve4(CpBlock<double> &d, CpBlock<double> &x, Quad<double> *p)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int bad = -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const double piv = __shfl_sync(0xffffffffu, d[G][j][G], 4 * warp + j);
+        if (!(piv > 0.0) && bad < 0) bad = j;
+        const double r = cp_normal(piv) ? cp_rsqrt(piv) : cp_rsqrt_any(piv);
+#pragma unroll
+        for (int h = G; h < 2; ++h) d[G][j][h] *= r;
+#pragma unroll
+        for (int h = 0; h < NX; ++h) x[G][j][h] *= r;
+#pragma unroll
+        for (int q = j + 1; q < 4; ++q) {
+            const double l = __shfl_sync(0xffffffffu, d[G][j][G], 4 * warp + q);
+#pragma unroll
+            for (int h = G; h < 2; ++h) d[G][q][h] = fma(-d[G][j][h], l, d[G][q][h]);
+#pragma unroll
+            for (int h = 0; h < NX; ++h) x[G][q][h] = fma(-x[G][j][h], l, x[G][q][h]);
+        }
+    }
+#pragma unroll
+    for (int h = G; h < 2; ++h) p[32 * h + lane] = {d[G][0][h], d[G][1][h], d[G][2][h], d[G][3][h]};
+#pragma unroll
+    for (int h = 0; h < NX; ++h) p[CP_W + 32 * h + lane] = {x[G][0][h], x[G][1][h], x[G][2][h], x[G][3][h]};
+    return bad;
+}
+
+// The whole panel; `phase` is the parity of the mbarriers (0 for the first
+// panel of a kernel, then in turn), with a CTA barrier between two panels.
+// False: a wait ran out.
+template <typename T, int NX>
+__device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T, NX> &pan, uint64_t (&bar)[16], uint32_t phase,
+                                         int n, int *info, int info_base, bool report)
+{
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int steps = (n + 3) / 4;
+    bool ok = true;
+    auto own = [&](int step, int bad) {
+        ptx::mbar_arrive(&bar[step]);
+        if (bad >= 0 && report && lane == 0 && info && 4 * step + bad < n) atomicCAS(info, 0, info_base + 4 * step + bad + 1);
+    };
+#pragma unroll 1
+    for (int i = 0; i < min(w, steps) - 1; ++i) {
+        ok = cp_wait(&bar[i], phase) && ok;
+        cp_update<T, NX, 0, 1>(d, x, pan[i]);
+    }
+    if (w > 0 && w <= steps) {
+        ok = cp_wait(&bar[w - 1], phase) && ok;
+        cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
+    }
+    if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w]));
+    __syncwarp();
+    if (steps <= 8) return ok;
+    if (w > 0) cp_update<T, NX, 1, 1>(d, x, pan[w - 1]);
+    cp_update<T, NX, 1, 1>(d, x, pan[w]);
+#pragma unroll 1
+    for (int i = w + 1; i < min(8 + w, steps); ++i) {
+        ok = cp_wait(&bar[i], phase) && ok;
+        cp_update<T, NX, 1, 1>(d, x, pan[i]);
+    }
+    if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w]));
+    return ok;
+}
+
+// Cholesky of the n x n (n <= 64) lower block A, in place, by one CTA.
 template <typename T>
 __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, T *__restrict__ A, long lda, int *info, int info_base)
 {
-    __shared__ Quad<T> pan[2][CP_W];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T a[2][4][2];  // [column group][column][row half]
-#pragma unroll
-    for (int g = 0; g < 2; ++g)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = 32 * h + lane, col = 32 * g + 4 * warp + c;
-                // rows and columns past n continue the block as the identity
-                a[g][c][h] = (h >= g && r < n && col <= r) ? A[r + (long)col * lda] : T(r == col ? 1 : 0);
-            }
-    cp_leaf_steps<T, 0>(a, pan, n, info, info_base);
-    cp_leaf_steps<T, 1>(a, pan, n, info, info_base);
-#pragma unroll
-    for (int g = 0; g < 2; ++g)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int h = g; h < 2; ++h) {
-                const int r = 32 * h + lane, col = 32 * g + 4 * warp + c;
-                if (r < n && col <= r) A[r + (long)col * lda] = a[g][c][h];
-            }
+    __shared__ CpPanel<T, 0> pan;
+    __shared__ uint64_t bar[16];
+    CpBlock<T> a;
+    cp_panel_init(bar);
+    // rows and columns past n continue the block as the identity
+    cp_each<T>(a, [&](T &v, int r, int c) { v = (r < n && c <= r) ? A[r + (long)c * lda] : T(r == c ? 1 : 0); });
+    __syncthreads();
+    if (!cp_panel<T, 0>(a, a, pan, bar, 0, n, info, info_base, true) && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
+    cp_each<T>(a, [&](T &v, int r, int c) {
+        if (r < n && c <= r) A[r + (long)c * lda] = v;
+    });
 }
 
 // ---------------------------------------------------------------------------

@@ -1,16 +1,19 @@
-// One cooperative launch that factors an FP32 diagonal tile of order
-// n <= 1024 (lower Cholesky, in place) and writes its lower-triangular
-// inverse: the POTRF of the mixed solve's diagonal tile and the operand of
-// its tensor-core panel TRSM (P <- P L_kk^-T as P * Linv^T).
+// One cooperative launch that factors an FP32 matrix (lower Cholesky, in
+// place) and, on request, builds its lower-triangular inverse (order <= 1024):
+// the POTRF of the mixed solve's diagonal tile with the operand of its
+// tensor-core panel TRSM (P <- P L_kk^-T as P * Linv^T), and the plain FP32
+// factorisation of tiles and small matrices.
 //
-// The tile is handled in 64 x 64 blocks, right-looking, as the tile loop of
+// The matrix is handled in 64 x 64 blocks, right-looking, as the tile loop of
 // examples/cholesky/cholesky_implicit.c:244-318 with the POTRF/TRSM/SYRK/GEMM
-// codelet arithmetic of cholesky_kernels.c (unblocked POTRF leaf: scale by
-// 1/l_zz, rank-1 update; column-oriented TRSM; GEMM updates).  Step k:
-//   A  every CTA with a block row i >= k loads the diagonal block and factors
-//      it in shared memory (the same instructions in every CTA, so every copy
-//      is bit-identical); the CTA of row k stores it and inverts it, the
-//      others solve their block L_ik = A_ik L_kk^-T;
+// codelet arithmetic of cholesky_kernels.c.  Step k:
+//   A  every CTA with a block row i >= k loads the diagonal block and its own
+//      64 rows into registers and takes both through the leaf's 16 steps of
+//      four columns together (chol_panel.cuh): the diagonal block is factored
+//      by the same instructions in every CTA (bit-identical copies), the own
+//      rows become L_ik = A_ik L_kk^-T on the way.  The CTA of row k solves
+//      the identity instead, which gives the block's inverse, and stores the
+//      factored block after the phase's barrier, when every CTA has read it;
 //   B  the trailing blocks A_ij -= L_ik L_jk^T (k < j <= i) are spread over
 //      the grid.
 // The inverse X = L^-1 is built on the way, block row by block row from
@@ -19,14 +22,21 @@
 // step k+1, both in CTAs the factorisation leaves idle; only the last block
 // row follows the factorisation.
 //
-// Phases are separated by grid barriers: a launch counter that each CTA
-// bumps, waited on with acquire loads.  The launch is cooperative (every CTA
-// resident), each wait is bounded by %globaltimer; on a timeout the CTA sets
-// *err and returns, and the CTAs still waiting time out in turn.  Data other
+// Bound by the chain of n / 64 steps: 16 dependent four-column steps, two
+// grid barriers and two rounds of loads each.
+//
+// Phases are separated by grid barriers.  With a.bar: a launch counter that
+// each CTA bumps, waited on with acquire loads, each wait bounded by
+// %globaltimer; on a timeout the CTA sets *err and returns, and the CTAs
+// still waiting time out in turn.  Without (callers that have no workspace):
+// the cooperative launch's own barrier, which every CTA reaches.  Data other
 // CTAs wrote is read through L2 (ld.global.cg), never from a stale L1 line.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "chol_panel.cuh"
 
 namespace gb300 {
 
@@ -53,8 +63,8 @@ struct DiagCoopArgs {
     float *T;  // scratch of the inverse's block products: n * n floats
     int *info;
     int info_base;
-    unsigned *bar;  // barrier counter, zero at launch
-    int *err;
+    unsigned *bar;  // barrier counter, zero at launch; null: the launch's own grid barrier
+    int *err;       // (with bar)
     int invert;  // 0: factor only (no inverse is written)
 };
 
@@ -69,11 +79,14 @@ __device__ __forceinline__ unsigned dc_ld_acquire(const unsigned *p)
 // another CTA has flagged an error -- the caller returns.
 __device__ __forceinline__ bool dc_sync(const DiagCoopArgs &a, unsigned phase, int *s_ok)
 {
+    if (!a.bar) {
+        cooperative_groups::this_grid().sync();
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();
-        atomicAdd(a.bar, 1u);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
         const unsigned target = phase * gridDim.x;
         if (dc_ld_acquire(a.bar) < target) {
             const uint64_t t0 = dc_timer();
@@ -83,168 +96,61 @@ __device__ __forceinline__ bool dc_sync(const DiagCoopArgs &a, unsigned phase, i
                     ok = 0;
                     break;
                 }
-                __nanosleep(32);
             }
         }
-        __threadfence();
         *s_ok = ok;
     }
     __syncthreads();
     return *s_ok != 0;
 }
 
-// rows x cols block of a column-major global matrix into a 64 x 64 shared
-// tile, zero outside.
-__device__ __forceinline__ void dc_load(float *s, const float *g, long ld, int rows, int cols)
-{
-    for (int e = threadIdx.x; e < DC_B * DC_B; e += DC_T) {
-        const int r = e & (DC_B - 1), c = e >> 6;
-        s[c * DC_LD + r] = (r < rows && c < cols) ? __ldcg(g + r + (long)c * ld) : 0.0f;
-    }
-}
-
-// Cholesky of the nb x nb (nb <= 32) lower block of D at offset `off`, in
-// place, by one warp: lane i holds row i in registers, the step loop is
-// unrolled (static register indices) and column values travel by shuffles,
-// so no CTA barrier sits on the chain.  Lanes i >= nb hold identity rows.
-// 1/l_zz comes from rsqrtf: this factor is the mixed solve's FP32 working
-// factor, refined afterwards, so the last ulp of the pivots does not matter.
-// invd[i] = 1 / l_ii.  The first non-positive pivot sets *info (first wins).
-__device__ __noinline__ void dc_potf2_32(float *D, int off, int nb, float *invd, int *info, int info_base,
-                                            bool report)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int i = threadIdx.x & 31;
-    float a[32];
+// One thread's 16 elements of a 64 x 64 tile (rows x cols of a column-major
+// global matrix, zero outside): all loads in flight together, 16 bytes each
+// where the tile is whole and aligned (vec).
+struct DcTile {
+    float4 v[4];
+    __device__ __forceinline__ void load(const float *g, long ld, int rows, int cols, bool vec)
+    {
+        if (vec && rows == DC_B && cols == DC_B) {
 #pragma unroll
-    for (int c = 0; c < 32; ++c) a[c] = (i < nb) ? ((c <= i) ? D[off + c * DC_LD + i] : 0.0f) : (c == i ? 1.0f : 0.0f);
-    int badz = -1;
-    float myinv = 1.0f;
-#pragma unroll
-    for (int z = 0; z < 32; ++z) {
-        const float d = __shfl_sync(FULL, a[z], z);
-        if (!(d > 0.0f) && badz < 0) badz = z;
-        const float inv = rsqrtf(d);
-        const float li = a[z] * inv;
-        if (i == z) {
-            a[z] = d * inv;
-            myinv = inv;
-        } else if (i > z) {
-            a[z] = li;
-        }
-#pragma unroll
-        for (int c = z + 1; c < 32; ++c) {
-            const float lc = __shfl_sync(FULL, li, c);
-            if (i >= c) a[c] = fmaf(-li, lc, a[c]);
-        }
-    }
-    if (i < nb) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (c <= i) D[off + c * DC_LD + i] = a[c];
-    }
-    invd[i] = myinv;
-    if (report && i == 0 && badz >= 0 && badz < nb && info) atomicCAS(info, 0, info_base + badz + 1);
-}
-
-// Cholesky of the bk x bk (bk <= 64) lower block in D (shared), in place:
-// 32 x 32 blocks -- warp 0 factors L11, warp 1 solves L21 = A21 L11^-T (lane
-// = row, unrolled column-oriented substitution), the CTA updates
-// A22 -= L21 L21^T, warp 0 factors L22.  invd[j] = 1 / l_jj (1 for j >= bk).
-__device__ __forceinline__ void dc_potf2(float *D, int bk, float *invd, int *info, int info_base, bool report)
-{
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 0) dc_potf2_32(D, 0, min(bk, 32), invd, info, info_base, report);
-    __syncthreads();
-    if (bk > 32) {
-        if (warp == 1) {
-            const int r = 32 + lane;
-            float x[32];
-#pragma unroll
-            for (int c = 0; c < 32; ++c) x[c] = D[c * DC_LD + r];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                x[j] *= invd[j];
-#pragma unroll
-                for (int c = j + 1; c < 32; ++c) x[c] = fmaf(-D[j * DC_LD + c], x[j], x[c]);
+            for (int q = 0; q < 4; ++q) {
+                const int e = threadIdx.x + q * DC_T, r4 = e & 15, c = e >> 4;
+                v[q] = __ldcg(reinterpret_cast<const float4 *>(g + 4 * r4 + (long)c * ld));
             }
-            if (r < bk) {
+        } else {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) D[c * DC_LD + r] = x[c];
+            for (int q = 0; q < 4; ++q) {
+                const int e = threadIdx.x + q * DC_T, r = 4 * (e & 15), c = e >> 4;
+                const float *p = g + r + (long)c * ld;
+                const bool in = c < cols;
+                v[q].x = in && r < rows ? __ldcg(p) : 0.0f;
+                v[q].y = in && r + 1 < rows ? __ldcg(p + 1) : 0.0f;
+                v[q].z = in && r + 2 < rows ? __ldcg(p + 2) : 0.0f;
+                v[q].w = in && r + 3 < rows ? __ldcg(p + 3) : 0.0f;
             }
         }
-        __syncthreads();
-        for (int e = tid; e < 32 * 32; e += DC_T) {
-            const int r = 32 + (e & 31), c = 32 + (e >> 5);
-            if (c <= r && r < bk) {
-                float acc = D[c * DC_LD + r];
-#pragma unroll 8
-                for (int p = 0; p < 32; ++p) acc = fmaf(-D[p * DC_LD + r], D[p * DC_LD + c], acc);
-                D[c * DC_LD + r] = acc;
-            }
-        }
-        __syncthreads();
-        if (warp == 0) dc_potf2_32(D, 32 * DC_LD + 32, bk - 32, invd + 32, info, info_base + 32, report);
-    } else if (tid >= 32 && tid < 64) {
-        invd[tid] = 1.0f;
     }
-    __syncthreads();
-}
-
-// Forward substitution with the factored 64 x 64 block L in D, one system
-// per group of four lanes: lane l of the group holds entries 16 l .. 16 l + 15
-// of the group's vector x, which on return is L^-1 x (column-oriented:
-// x_j *= 1/l_jj, then x_c -= l_cj x_j for c > j).  The owner of x_j is lane
-// j / 16, its register j % 16 (a static index: j runs as 4 rolled groups of
-// 16 unrolled steps); x_j reaches the other lanes by a shuffle.
-__device__ __forceinline__ void dc_fwd_subst(const float *D, const float *invd, float x[16])
-{
-    const int l = threadIdx.x & 3, src0 = threadIdx.x & 28;
-#pragma unroll 1
-    for (int G = 0; G < 4; ++G) {
+    // to a shared tile: column-major (s[c * DC_LD + r]), or p-major (s[r * DC_LD + c])
+    __device__ __forceinline__ void store(float *s) const
+    {
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-            const int j = 16 * G + jj;
-            const float xo = x[jj] * invd[j];
-            if (l == G) x[jj] = xo;
-            const float xj = __shfl_sync(0xffffffffu, xo, src0 | G);
-            const float *Dj = D + j * DC_LD + 16 * l;
-#pragma unroll
-            for (int q = 0; q < 16; ++q)
-                if (l > G || (l == G && q > jj)) x[q] = fmaf(-Dj[q], xj, x[q]);
+        for (int q = 0; q < 4; ++q) {
+            const int e = threadIdx.x + q * DC_T;
+            *reinterpret_cast<float4 *>(s + (e >> 4) * DC_LD + 4 * (e & 15)) = v[q];
         }
     }
-}
-
-// Bs (64 rows, bk columns, shared) <- Bs L^-T with L the factored block in D:
-// row r of Bs is the system of lane group r (threads 4r .. 4r + 3).
-__device__ __forceinline__ void dc_trsm(const float *D, float *Bs, const float *invd)
-{
-    const int r = threadIdx.x >> 2, l = threadIdx.x & 3;
-    float x[16];
+    __device__ __forceinline__ void store_t(float *s) const
+    {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) x[q] = Bs[(16 * l + q) * DC_LD + r];
-    dc_fwd_subst(D, invd, x);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) Bs[(16 * l + q) * DC_LD + r] = x[q];
-    __syncthreads();
-}
-
-// X = L^-1 of the factored bk x bk block in D, written to the global block g
-// (ld ldg, lower part only): column c of X solves L x = e_c in lane group c.
-__device__ __forceinline__ void dc_trtri(const float *D, int bk, const float *invd, float *g, long ldg)
-{
-    const int c = threadIdx.x >> 2, l = threadIdx.x & 3;
-    float x[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) x[q] = (16 * l + q == c) ? 1.0f : 0.0f;
-    dc_fwd_subst(D, invd, x);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int r = 16 * l + q;
-        if (r < bk && c < bk && r >= c) g[r + (long)c * ldg] = x[q];
+        for (int q = 0; q < 4; ++q) {
+            const int e = threadIdx.x + q * DC_T, c = e >> 4, r = 4 * (e & 15);
+            s[r * DC_LD + c] = v[q].x;
+            s[(r + 1) * DC_LD + c] = v[q].y;
+            s[(r + 2) * DC_LD + c] = v[q].z;
+            s[(r + 3) * DC_LD + c] = v[q].w;
+        }
     }
-}
+};
 
 // acc += As * Bs for 64 x 64 shared tiles: As column-major (As[p * DC_LD + r]
 // = A(r, p)), Bs stored p-major (Bs[p * DC_LD + c] = B(p, c)) -- which is how
@@ -266,17 +172,6 @@ __device__ __forceinline__ void dc_mma(const float *As, const float *Bs, float a
     }
 }
 
-// rows x cols block of a column-major global matrix into a shared tile
-// stored p-major (s[r * DC_LD + c] = g(r, c)), zero outside: the B operand
-// of an NN product.
-__device__ __forceinline__ void dc_load_t(float *s, const float *g, long ld, int rows, int cols)
-{
-    for (int e = threadIdx.x; e < DC_B * DC_B; e += DC_T) {
-        const int r = e & (DC_B - 1), c = e >> 6;
-        s[r * DC_LD + c] = (r < rows && c < cols) ? __ldcg(g + r + (long)c * ld) : 0.0f;
-    }
-}
-
 // row index ii, column index jj <= ii of the t-th block of a lower triangle
 // (row by row: (0,0), (1,0), (1,1), (2,0), ...)
 __device__ __forceinline__ void dc_tri_index(int t, int &ii, int &jj)
@@ -288,29 +183,44 @@ __device__ __forceinline__ void dc_tri_index(int t, int &ii, int &jj)
     jj = t - i * (i + 1) / 2;
 }
 
-// C (rows x cols of a column-major global matrix) -= acc, where the mask
-// `lower` keeps only elements on or below the diagonal.  vec: C and ld allow
-// float4 accesses along the thread's four rows.
-__device__ __forceinline__ void dc_sub_store(float *C, long ld, int rows, int cols, bool lower, bool vec,
-                                             const float acc[4][4])
+// The thread's 4 x 4 elements of C (rows x cols of a column-major global
+// matrix; `lower` keeps only those on or below the diagonal), read before the
+// product and written after it.  whole: every element, 16 bytes at a time.
+__device__ __forceinline__ bool dc_whole(int rows, int cols, bool lower, bool vec)
 {
-    const int tr = threadIdx.x & 15, tn = threadIdx.x >> 4, r0 = 4 * tr;
+    return vec && rows == DC_B && cols == DC_B && !lower;
+}
+__device__ __forceinline__ void dc_sub_load(const float *C, long ld, int rows, int cols, bool lower, bool whole,
+                                            float (&c)[4][4])
+{
+    const int r0 = 4 * (threadIdx.x & 15), c0 = 4 * (threadIdx.x >> 4);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const int c = 4 * tn + j;
-        if (c >= cols) continue;
-        float *p = C + r0 + (long)c * ld;
-        if (vec && r0 + 3 < rows && (!lower || c <= r0)) {
-            float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
-            v.x -= acc[0][j];
-            v.y -= acc[1][j];
-            v.z -= acc[2][j];
-            v.w -= acc[3][j];
-            *reinterpret_cast<float4 *>(p) = v;
+        const float *p = C + r0 + (long)(c0 + j) * ld;
+        if (whole) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
+            c[0][j] = v.x, c[1][j] = v.y, c[2][j] = v.z, c[3][j] = v.w;
         } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (r0 + i < rows && (!lower || c <= r0 + i)) p[i] = __ldcg(p + i) - acc[i][j];
+                c[i][j] = c0 + j < cols && r0 + i < rows && (!lower || c0 + j <= r0 + i) ? __ldcg(p + i) : 0.0f;
+        }
+    }
+}
+__device__ __forceinline__ void dc_sub_store(float *C, long ld, int rows, int cols, bool lower, bool whole,
+                                             const float (&c)[4][4], const float (&acc)[4][4])
+{
+    const int r0 = 4 * (threadIdx.x & 15), c0 = 4 * (threadIdx.x >> 4);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float *p = C + r0 + (long)(c0 + j) * ld;
+        if (whole) {
+            *reinterpret_cast<float4 *>(p) = make_float4(c[0][j] - acc[0][j], c[1][j] - acc[1][j], c[2][j] - acc[2][j],
+                                                         c[3][j] - acc[3][j]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c0 + j < cols && r0 + i < rows && (!lower || c0 + j <= r0 + i)) p[i] = c[i][j] - acc[i][j];
         }
     }
 }
@@ -322,12 +232,16 @@ __device__ __forceinline__ float *dc_slot(const DiagCoopArgs &a, int j, int p)
 }
 
 // slot(j, p) = L_kp X_pj (rows of block row k: rk), X_pj the inverse block
-__device__ __forceinline__ void dc_inv_product(const DiagCoopArgs &a, int k, int j, int p, float *s0, float *s1)
+__device__ __forceinline__ void dc_inv_product(const DiagCoopArgs &a, int k, int j, int p, float *s0, float *s1, bool vec,
+                                               bool vec_inv)
 {
     const int rk = min(DC_B, a.n - k * DC_B);
+    DcTile l, x;
+    l.load(a.A + k * DC_B + (long)(p * DC_B) * a.lda, a.lda, rk, DC_B, vec);
+    x.load(a.Linv + p * DC_B + (long)(j * DC_B) * a.ldi, a.ldi, DC_B, DC_B, vec_inv);
     __syncthreads();  // shared tiles free
-    dc_load(s0, a.A + k * DC_B + (long)(p * DC_B) * a.lda, a.lda, rk, DC_B);
-    dc_load_t(s1, a.Linv + p * DC_B + (long)(j * DC_B) * a.ldi, a.ldi, DC_B, DC_B);
+    l.store(s0);
+    x.store_t(s1);
     __syncthreads();
     float acc[4][4] = {};
     dc_mma(s0, s1, acc);
@@ -340,16 +254,24 @@ __device__ __forceinline__ void dc_inv_product(const DiagCoopArgs &a, int k, int
 }
 
 // X_kj = -X_kk (sum_{p = j}^{k-1} slot(j, p)), summed in p order
-__device__ __forceinline__ void dc_inv_combine(const DiagCoopArgs &a, int k, int j, float *s0, float *s1)
+__device__ __forceinline__ void dc_inv_combine(const DiagCoopArgs &a, int k, int j, float *s0, float *s1, bool vec_inv)
 {
     const int rk = min(DC_B, a.n - k * DC_B);
-    __syncthreads();  // shared tiles free
-    for (int e = threadIdx.x; e < DC_B * DC_B; e += DC_T) {
-        float v = 0.0f;
-        for (int p = j; p < k; ++p) v += __ldcg(dc_slot(a, j, p) + e);
-        s1[(e & (DC_B - 1)) * DC_LD + (e >> 6)] = v;
+    DcTile x;
+    x.load(a.Linv + k * DC_B + (long)(k * DC_B) * a.ldi, a.ldi, rk, rk, vec_inv);
+    float v[DC_B * DC_B / DC_T] = {};
+    for (int p = j; p < k; ++p) {
+        const float *S = dc_slot(a, j, p) + threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < DC_B * DC_B / DC_T; ++q) v[q] += __ldcg(S + q * DC_T);
     }
-    dc_load(s0, a.Linv + k * DC_B + (long)(k * DC_B) * a.ldi, a.ldi, rk, rk);
+    __syncthreads();  // shared tiles free
+#pragma unroll
+    for (int q = 0; q < DC_B * DC_B / DC_T; ++q) {
+        const int e = threadIdx.x + q * DC_T;
+        s1[(e & (DC_B - 1)) * DC_LD + (e >> 6)] = v[q];
+    }
+    x.store(s0);
     __syncthreads();
     float acc[4][4] = {};
     dc_mma(s0, s1, acc);
@@ -370,76 +292,90 @@ __device__ __forceinline__ void dc_inv_combine(const DiagCoopArgs &a, int k, int
 // (L X = I, block row k), in CTAs the factorisation leaves idle; only the
 // last row runs after the factorisation.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(DC_T) diag_coop_kernel(DiagCoopArgs a)
+__global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
 {
-    __shared__ __align__(16) float s0[DC_B * DC_LD];
-    __shared__ __align__(16) float s1[DC_B * DC_LD];
-    __shared__ float invd[DC_B];
+    // two operand tiles, or the panel's published columns (never both at a time)
+    constexpr int TILE = DC_B * DC_LD * sizeof(float);
+    __shared__ __align__(16) unsigned char shared[2 * TILE > sizeof(CpPanel<float, 2>) ? 2 * TILE : sizeof(CpPanel<float, 2>)];
+    float *s0 = (float *)shared, *s1 = (float *)(shared + TILE);
+    CpPanel<float, 2> &pan = *(CpPanel<float, 2> *)shared;
+    __shared__ uint64_t bar[16];
     __shared__ int s_ok;
     const int n = a.n, nblk = (n + DC_B - 1) / DC_B, G = gridDim.x, b = blockIdx.x;
-    const int tid = threadIdx.x;
     const bool vec = ((reinterpret_cast<uintptr_t>(a.A) & 15) == 0) && ((a.lda & 3) == 0);
-    unsigned phase = 0;
+    const bool vec_inv = ((reinterpret_cast<uintptr_t>(a.Linv) & 15) == 0) && ((a.ldi & 3) == 0);
+    unsigned phase = 0, panels = 0;
+    cp_panel_init(bar);
+    __syncthreads();
 
     for (int k = 0; k < nblk; ++k) {
         const int k0 = k * DC_B, bk = min(DC_B, n - k0);
         float *Akk = a.A + k0 + (long)k0 * a.lda;
         // ---- phase A
         const int nf = nblk - k, nc = (a.invert && k >= 2) ? k - 1 : 0;
-        bool factored = false;
+        CpBlock<float> d, x;
         for (int t = b; t < nf + nc; t += G) {
             if (t < nf) {
-                if (!factored) {
-                    dc_load(s0, Akk, a.lda, bk, bk);
-                    __syncthreads();
-                    dc_potf2(s0, bk, invd, a.info, a.info_base + k0, b == 0);
-                    factored = true;
-                }
-                const int i = k + t;
-                if (i == k) {
-                    for (int e = tid; e < DC_B * DC_B; e += DC_T) {
-                        const int r = e & 63, c = e >> 6;
-                        if (r < bk && c <= r) Akk[r + (long)c * a.lda] = s0[c * DC_LD + r];
-                    }
-                    if (a.invert) dc_trtri(s0, bk, invd, a.Linv + k0 + (long)k0 * a.ldi, a.ldi);
-                } else {
-                    const int i0 = i * DC_B, ri = min(DC_B, n - i0);
-                    float *Aik = a.A + i0 + (long)k0 * a.lda;
-                    __syncthreads();  // s1 of the previous block row has been stored
-                    dc_load(s1, Aik, a.lda, ri, bk);
-                    __syncthreads();
-                    dc_trsm(s0, s1, invd);
-                    for (int e = tid; e < DC_B * DC_B; e += DC_T) {
-                        const int r = e & 63, c = e >> 6;
-                        if (r < ri && c < bk) Aik[r + (long)c * a.lda] = s1[c * DC_LD + r];
-                    }
-                }
+                const int i0 = (k + t) * DC_B, ri = min(DC_B, n - i0);
+                float *Aik = a.A + i0 + (long)k0 * a.lda;
+                // the block (identity past bk, zeros above) and this CTA's rows
+                cp_each<float>(d, [&](float &v, int r, int c) {
+                    v = (r < bk && c <= r) ? __ldcg(Akk + r + (long)c * a.lda) : (r == c ? 1.0f : 0.0f);
+                });
+                cp_each<float>(x, [&](float &v, int r, int c) {
+                    if (t == 0) v = r == c ? 1.0f : 0.0f;
+                    else v = (r < ri && c < bk) ? __ldcg(Aik + r + (long)c * a.lda) : 0.0f;
+                });
+                __syncthreads();  // pan of the previous task is free
+                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, bk, a.info, a.info_base + k0, t == 0) && a.err)
+                    atomicCAS(a.err, 0, DC_ERR_TIMEOUT);
+                ++panels;
+                if (t > 0)
+                    cp_each<float>(x, [&](float &v, int r, int c) {
+                        if (r < ri && c < bk) Aik[r + (long)c * a.lda] = v;
+                    });
+                else if (a.invert)  // I L^-T = X_kk^T
+                    cp_each<float>(x, [&](float &v, int r, int c) {
+                        if (c >= r && c < bk) a.Linv[(k0 + c) + (long)(k0 + r) * a.ldi] = v;
+                    });
             } else {
-                dc_inv_combine(a, k - 1, t - nf, s0, s1);  // factor tasks come first: s0 is free
+                dc_inv_combine(a, k - 1, t - nf, s0, s1, vec_inv);
             }
         }
         if (!dc_sync(a, ++phase, &s_ok)) return;
+        if (b == 0)  // the factored block: every CTA has read the unfactored one
+            cp_each<float>(d, [&](float &v, int r, int c) {
+                if (r < bk && c <= r) Akk[r + (long)c * a.lda] = v;
+            });
         if (k == nblk - 1) break;
         // ---- phase B
+        // (CTA 0, which stores the factored block, takes its tile last)
         const int m = nblk - k - 1, nu = m * (m + 1) / 2;
         const int np = (a.invert && k >= 1) ? k * (k + 1) / 2 : 0;
-        for (int t = b; t < nu + np; t += G) {
+        for (int t = (b + G - 1) % G; t < nu + np; t += G) {
             if (t < nu) {
                 int ii, jj;
                 dc_tri_index(t, ii, jj);
                 const int bi = k + 1 + ii, bj = k + 1 + jj;
                 const int i0 = bi * DC_B, j0 = bj * DC_B, ri = min(DC_B, n - i0), rj = min(DC_B, n - j0);
+                float *C = a.A + i0 + (long)j0 * a.lda;
+                const bool whole = dc_whole(ri, rj, bi == bj, vec);
+                DcTile li, lj;
+                float c[4][4];
+                li.load(a.A + i0 + (long)k0 * a.lda, a.lda, ri, bk, vec);
+                lj.load(a.A + j0 + (long)k0 * a.lda, a.lda, rj, bk, vec);
+                dc_sub_load(C, a.lda, ri, rj, bi == bj, whole, c);
                 __syncthreads();  // the previous task's shared operands are free
-                dc_load(s0, a.A + i0 + (long)k0 * a.lda, a.lda, ri, bk);
-                dc_load(s1, a.A + j0 + (long)k0 * a.lda, a.lda, rj, bk);
+                li.store(s0);
+                lj.store(s1);
                 __syncthreads();
                 float acc[4][4] = {};
                 dc_mma(s0, s1, acc);
-                dc_sub_store(a.A + i0 + (long)j0 * a.lda, a.lda, ri, rj, bi == bj, vec, acc);
+                dc_sub_store(C, a.lda, ri, rj, bi == bj, whole, c, acc);
             } else {
                 int p, j;
                 dc_tri_index(t - nu, p, j);
-                dc_inv_product(a, k, j, p, s0, s1);
+                dc_inv_product(a, k, j, p, s0, s1, vec, vec_inv);
             }
         }
         if (!dc_sync(a, ++phase, &s_ok)) return;
@@ -451,10 +387,10 @@ __global__ void __launch_bounds__(DC_T) diag_coop_kernel(DiagCoopArgs a)
         for (int t = b; t < k * (k + 1) / 2; t += G) {
             int p, j;
             dc_tri_index(t, p, j);
-            dc_inv_product(a, k, j, p, s0, s1);
+            dc_inv_product(a, k, j, p, s0, s1, vec, vec_inv);
         }
         if (!dc_sync(a, ++phase, &s_ok)) return;
-        for (int t = b; t < k; t += G) dc_inv_combine(a, k, t, s0, s1);
+        for (int t = b; t < k; t += G) dc_inv_combine(a, k, t, s0, s1, vec_inv);
     }
 }
 

@@ -83,7 +83,7 @@ def test_product_tiles(gpu, dtype, m, n, k, lower):
 
 
 @BOTH
-@pytest.mark.parametrize("n,nb", [(63, 64), (65, 16), (127, 64), (191, 64), (192, 512), (193, 512), (321, 100), (700, 512), (1281, 256), (3001, 512)])
+@pytest.mark.parametrize("n,nb", [(63, 64), (65, 16), (127, 64), (191, 64), (192, 512), (193, 512), (321, 100), (700, 512), (1281, 256), (3001, 512), (4097, 1024)])
 def test_potrf_blocks(gpu, dtype, n, nb):
     # rows and columns scaled over 12 orders of magnitude (FP32: 6)
     d = np.power(10.0, np.random.default_rng(n).uniform(-6, 6, n) * (1.0 if dtype == np.float64 else 0.5))
