@@ -146,32 +146,58 @@ void trtri_lower(cudaStream_t s, int n, const T *L, long ldl, T *Linv, long ldi,
     }
 }
 
-// B[m x nc] <- B * L^{-T}: one launch per CP_TRSM_MAXN columns (rows are
-// independent), then a GEMM update of the remaining columns.
-template <typename T, int SR>
-static void trsm_slab(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb)
+// One launch of the slab solve X M^T = B (SlabArgs), n <= CP_TRSM_MAXN.
+template <typename T, int SR> static void slab_launch(cudaStream_t s, const SlabArgs<T> &a)
 {
-    const size_t smem = cp_trsm_smem<T, SR>(n);
     if (gb300_func_dyn_smem((const void *)trsm_slab_kernel<T, SR>, (int)cp_trsm_smem<T, SR>(CP_TRSM_MAXN))) return;
-    gb300_count_launch(), trsm_slab_kernel<T, SR><<<cdiv(m, SR), 256, smem, s>>>(m, n, L, ldl, B, ldb);
+    gb300_count_launch(), trsm_slab_kernel<T, SR><<<cdiv(a.m, SR), 256, cp_trsm_smem<T, SR>(a.n), s>>>(a);
 }
 
+// X M^T = B in place: one launch per CP_TRSM_MAXN columns (rows are
+// independent), then a GEMM update of the remaining columns.
+template <typename T> void trsm_slab(cudaStream_t s, const SlabArgs<T> &a)
+{
+    if (a.m <= 0 || a.n <= 0) return;
+    SlabArgs<T> c = a;
+    for (int j0 = 0; j0 < a.n; j0 += CP_TRSM_MAXN) {
+        c.n = std::min(CP_TRSM_MAXN, a.n - j0);
+        c.M = a.M + j0 * (a.m_js + a.m_ps);
+        c.B = a.B + j0 * a.b_js;
+        // 16 rows per CTA once that fills the GPU; below, 4 spread the products
+        // over more SMs (8 when one 64-column block has none)
+        if (a.m >= 16 * 128) slab_launch<T, 16>(s, c);
+        else if (a.n <= CP_W && a.m > 4 * 152) slab_launch<T, 8>(s, c);
+        else slab_launch<T, 4>(s, c);
+        const int rest = a.n - j0 - c.n;
+        if (rest <= 0) break;
+        // B_rest -= X M_rest^T
+        const T *M2 = c.M + c.n * a.m_js;
+        T *B2 = c.B + c.n * a.b_js;
+        if (a.b_js == 1 && a.m_js == 1)  // transposed: B2^T (rest x m) -= M_rest X^T
+            gemm<T>(s, false, false, false, rest, a.m, c.n, T(-1), M2, a.m_ps, c.B, a.b_rs, T(1), B2, a.b_rs);
+        else
+            gemm<T>(s, false, a.m_js == 1, false, a.m, rest, c.n, T(-1), c.B, a.b_js, M2, a.m_js == 1 ? a.m_ps : a.m_js,
+                    T(1), B2, a.b_js);
+    }
+}
+
+// B[m x nc] <- B * L^{-T}
 template <typename T>
 void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long ldb)
 {
-    if (m <= 0 || nc <= 0) return;
-    for (int j0 = 0; j0 < nc; j0 += CP_TRSM_MAXN) {
-        const int w = std::min(CP_TRSM_MAXN, nc - j0);
-        const T *Ljj = L + j0 + (long)j0 * ldl;
-        T *Bj = B + (long)j0 * ldb;
-        // 16 rows per CTA once that fills the GPU, else 4
-        if (m >= 16 * 128) trsm_slab<T, 16>(s, m, w, Ljj, ldl, Bj, ldb);
-        else trsm_slab<T, 4>(s, m, w, Ljj, ldl, Bj, ldb);
-        const int rest = nc - j0 - w;
-        if (rest > 0)
-            gemm<T>(s, false, true, false, m, rest, w, T(-1), Bj, ldb, L + (j0 + w) + (long)j0 * ldl, ldl, T(1),
-                    B + (long)(j0 + w) * ldb, ldb);
-    }
+    trsm_slab<T>(s, {m, nc, L, 1, ldl, B, 1, ldb, false});
+}
+
+// B[m x n] <- L^{-1} B (LU block row)
+template <typename T> void trsm_llnn(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb)
+{
+    trsm_slab<T>(s, {n, m, L, 1, ldl, B, ldb, 1, false});
+}
+
+// B[m x n] <- B U^{-1}, U unit upper (LU block column)
+template <typename T> void trsm_runu(cudaStream_t s, int m, int n, const T *U, long ldu, T *B, long ldb)
+{
+    trsm_slab<T>(s, {m, n, U, ldu, 1, B, 1, ldb, true});
 }
 
 // C[m x n] -= A B^T in FP64 on the tensor cores (kernels/slice_update.cuh), A
@@ -250,36 +276,43 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
 // POTRS with a lower factor: L y = b (forward), then L^T x = y (backward),
 // in blocks of CP_SB rows: solve the block, update the rows to come.
 // min-dgels/base/SRC/dpotrs.c does the same two sweeps through dtrsm.
-template <typename T, int C, bool TRANS>
+// CB right-hand sides per CTA in the block solve, CU in the update.
+template <typename T, int CB, int CU, bool TRANS>
 static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
-    constexpr size_t sm_blk = cp_trsv_smem<T, C>(TRANS), sm_upd = cp_upd_smem<T, C>(TRANS);
-    if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, C, TRANS>, (int)sm_blk) ||
-        gb300_func_dyn_smem((const void *)trsv_upd_kernel<T, C, TRANS>, (int)sm_upd))
+    constexpr size_t sm_blk = cp_trsv_smem<T, CB>(TRANS), sm_upd = cp_upd_smem<T, CU>(TRANS);
+    if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, CB, TRANS>, (int)sm_blk) ||
+        gb300_func_dyn_smem((const void *)trsv_upd_kernel<T, CU, TRANS>, (int)sm_upd))
         return;
     const int nblk = (n + CP_SB - 1) / CP_SB;
     for (int b = 0; b < nblk; ++b) {
         const int j0 = (TRANS ? nblk - 1 - b : b) * CP_SB, w = std::min(CP_SB, n - j0);
-        gb300_count_launch(), trsv_blk_kernel<T, C, TRANS>
-            <<<cdiv(nrhs, C), 256, sm_blk, s>>>(w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
+        gb300_count_launch(), trsv_blk_kernel<T, CB, TRANS>
+            <<<cdiv(nrhs, CB), 256, sm_blk, s>>>(w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
         const int rest = TRANS ? j0 : n - j0 - w;
         if (rest <= 0) continue;
-        gb300_count_launch(), trsv_upd_kernel<T, C, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, C)), 256, sm_upd, s>>>(
+        gb300_count_launch(), trsv_upd_kernel<T, CU, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, CU)), 256, sm_upd, s>>>(
             rest, w, nrhs, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl, ldl, B + j0, TRANS ? B : B + j0 + w, ldb);
     }
+}
+
+template <typename T, int CB, int CU>
+static void potrs_sweeps(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
+{
+    potrs_sweep_blocks<T, CB, CU, false>(s, n, nrhs, L, ldl, B, ldb);
+    potrs_sweep_blocks<T, CB, CU, true>(s, n, nrhs, L, ldl, B, ldb);
 }
 
 template <typename T>
 void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
     if (n <= 0 || nrhs <= 0) return;
-    if (nrhs == 1) {
-        potrs_sweep_blocks<T, 1, false>(s, n, nrhs, L, ldl, B, ldb);
-        potrs_sweep_blocks<T, 1, true>(s, n, nrhs, L, ldl, B, ldb);
-    } else {
-        potrs_sweep_blocks<T, 4, false>(s, n, nrhs, L, ldl, B, ldb);
-        potrs_sweep_blocks<T, 4, true>(s, n, nrhs, L, ldl, B, ldb);
-    }
+    // The block solve takes one right-hand side per CTA while there are SMs for
+    // them: its rows' products share one SM's FMA units.
+    if (nrhs == 1) potrs_sweeps<T, 1, 1>(s, n, nrhs, L, ldl, B, ldb);
+    else if (nrhs <= 4) potrs_sweeps<T, 1, 4>(s, n, nrhs, L, ldl, B, ldb);
+    else if (nrhs <= 152) potrs_sweeps<T, 1, 8>(s, n, nrhs, L, ldl, B, ldb);
+    else potrs_sweeps<T, 4, 8>(s, n, nrhs, L, ldl, B, ldb);
 }
 
 // ---- single-launch POTRS sweeps with inverted 64 x 64 diagonal blocks ------
@@ -337,6 +370,10 @@ template void gemm<double>(cudaStream_t, bool, bool, bool, int, int, int, double
                            const double *, long, double, double *, long);
 template void trsm_rltn<float>(cudaStream_t, int, int, const float *, long, float *, long);
 template void trsm_rltn<double>(cudaStream_t, int, int, const double *, long, double *, long);
+template void trsm_llnn<float>(cudaStream_t, int, int, const float *, long, float *, long);
+template void trsm_llnn<double>(cudaStream_t, int, int, const double *, long, double *, long);
+template void trsm_runu<float>(cudaStream_t, int, int, const float *, long, float *, long);
+template void trsm_runu<double>(cudaStream_t, int, int, const double *, long, double *, long);
 template void potrf_tiled<float>(cudaStream_t, int, float *, long, int, int *, int);
 template void trtri_lower<float>(cudaStream_t, int, const float *, long, float *, long, float *);
 template void potrf_tiled<double>(cudaStream_t, int, double *, long, int, int *, int);

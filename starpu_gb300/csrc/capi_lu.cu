@@ -14,46 +14,8 @@ namespace gb300 {
 
 static inline unsigned lu_cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 
-// B[m x n] <- L^{-1} B, L m x m lower non-unit, blocked by SMALL_W rows:
-// diagonal-block solve (one thread per column of B), then the GEMM update of
-// the rows below.
-template <typename T>
-static void trsm_llnn(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb)
-{
-    constexpr int W = small_w<T>::value;
-    for (int r0 = 0; r0 < m; r0 += W) {
-        const int w = std::min(W, m - r0);
-        gb300_count_launch(), trsm_left_small_kernel<T, W, false>
-            <<<lu_cdiv(n, 64), 64, 0, s>>>(w, n, L + r0 + (long)r0 * ldl, ldl, B + r0, ldb);
-        const int rest = m - r0 - w;
-        if (rest > 0)
-            gemm<T>(s, false, false, false, rest, n, w, T(-1), L + (r0 + w) + (long)r0 * ldl, ldl, B + r0, ldb, T(1),
-                    B + r0 + w, ldb);
-    }
-}
-
-// B[m x n] <- B U^{-1}, U n x n unit upper, blocked by SMALL_W columns.
-template <typename T>
-static void trsm_runu(cudaStream_t s, int m, int n, const T *U, long ldu, T *B, long ldb)
-{
-    constexpr int W = small_w<T>::value;
-    for (int c0 = 0; c0 < n; c0 += W) {
-        const int w = std::min(W, n - c0);
-        if (w == W)
-            gb300_count_launch(), trsm_runu_small_kernel<T, W, true>
-                <<<lu_cdiv(m, 128), 128, 0, s>>>(m, w, U + c0 + (long)c0 * ldu, ldu, B + (long)c0 * ldb, ldb);
-        else
-            gb300_count_launch(), trsm_runu_small_kernel<T, W, false>
-                <<<lu_cdiv(m, 128), 128, 0, s>>>(m, w, U + c0 + (long)c0 * ldu, ldu, B + (long)c0 * ldb, ldb);
-        const int rest = n - c0 - w;
-        if (rest > 0)
-            gemm<T>(s, false, false, false, m, rest, w, T(-1), B + (long)c0 * ldb, ldb, U + c0 + (long)(c0 + w) * ldu,
-                    ldu, T(1), B + (long)(c0 + w) * ldb, ldb);
-    }
-}
-
 // Blocked right-looking LU of one n x n tile (A = L U, L non-unit, U unit):
-// per SMALL_W block, the register-resident leaf, U12 = L11^-1 A12,
+// per block (64 in FP32, 32 in FP64, whose leaf would spill), the register-resident leaf, U12 = L11^-1 A12,
 // L21 = A21 U11^-1, A22 -= L21 U12.  thr > 0 records the first step whose
 // pivot falls below thr into *d_first (the diagonal block of a step is fully
 // updated when its leaf runs, so the test sees the same values as the
@@ -61,11 +23,14 @@ static void trsm_runu(cudaStream_t s, int m, int n, const T *U, long ldu, T *B, 
 template <typename T>
 static void getrf_blocked(cudaStream_t s, int n, T *A, long lda, T thr, int *d_first, int *info)
 {
-    constexpr int W = small_w<T>::value;
+    constexpr int W = sizeof(T) == 4 ? 64 : 32;
     for (int k0 = 0; k0 < n; k0 += W) {
         const int kb = std::min(W, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
-        gb300_count_launch(), getf2_small_kernel<T, W><<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0);
+        if constexpr (sizeof(T) == 4)
+            gb300_count_launch(), getf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0);
+        else
+            gb300_count_launch(), getf2_small_kernel<T, W><<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0);
         const int rest = n - k0 - kb;
         if (rest <= 0) break;
         T *A12 = A + k0 + (long)(k0 + kb) * lda, *A21 = A + (k0 + kb) + (long)k0 * lda;

@@ -454,7 +454,7 @@ static LookaheadStream *lookahead_stream()
 // runs on the defaults below.  The model balances the update's 3 m2^2 kb
 // flops on the remaining SMs, at the split-precision tensor rate of this
 // kernel (default 1.45 PFLOP/s on the whole GPU), against the panel's
-// latency-bound diagonal tile (default about 0.75 ms) plus its 6 m2 kb^2
+// latency-bound diagonal tile (default 0.3 ms) plus its 6 m2 kb^2
 // TRSM flops and the panel splits, which together run at a fraction of that
 // rate per SM (default GB300_PANEL_RATE or 0.4: the per-step timeline of the
 // n = 32768 solve gave 2.02 ms for a 27648-row panel on 38 SMs).
@@ -480,7 +480,7 @@ static int lookahead_sms(int m2, int kb)
     }();
     const int S = num_sms();
     if (fixed >= 0) return fixed >= S ? 0 : fixed;
-    double rate = 1.45e15, t_diag = 0.75e-3, panel_rate = panel_rate_env;
+    double rate = 1.45e15, t_diag = 0.3e-3, panel_rate = panel_rate_env;
     const int trial = g_la_trial;
     if (trial >= 0) return trial >= S ? 0 : trial;
     if (trial == -1) {
@@ -495,10 +495,11 @@ static int lookahead_sms(int m2, int kb)
     if (S < 32 || m2 <= 0) return 0;
     const double R = rate / S;
     const double f_upd = 3.0 * m2 * (double)m2 * kb, f_trsm = 6.0 * m2 * (double)kb * kb / panel_rate;
-    // below about a quarter of the GPU the diagonal-tile kernel itself slows down
-    int best = S / 4;
+    // at least a sixth of the GPU: n = 32768 took 61.8 ms from 24 SMs up, 62.2
+    // from 16 and 62.6 from 38 (a quarter)
+    int best = S / 6;
     double best_t = 1e30;
-    for (int L = S / 4; L <= S - 16; L += 8) {
+    for (int L = S / 6; L <= S - 16; L += 8) {
         const double t = std::max(f_upd / (R * (S - L)), t_diag + f_trsm / (R * L));
         if (t < best_t) {
             best_t = t;

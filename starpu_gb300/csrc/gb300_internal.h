@@ -80,16 +80,12 @@ struct DenseTuning {
 bool dense_tuning(int nb, DenseTuning *out);
 int dense_tuning_store(const DenseTuning &d);
 
-// Width of the register-blocked small triangular kernels and of the
-// unblocked diagonal POTRF leaf: 64 columns in FP32, 32 in FP64 (a 64-wide
-// FP64 row does not fit the register file without spilling).
-template <typename T> struct small_w { static constexpr int value = 64; };
-template <> struct small_w<double> { static constexpr int value = 32; };
-
 template <typename T>
 void gemm(cudaStream_t s, bool ta, bool tb, bool lower, int m, int n, int k, T alpha, const T *A, long lda,
           const T *B, long ldb, T beta, T *C, long ldc);
 template <typename T> void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long ldb);
+template <typename T> void trsm_llnn(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb);
+template <typename T> void trsm_runu(cudaStream_t s, int m, int n, const T *U, long ldu, T *B, long ldb);
 template <typename T> void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base);
 // Linv = inverse of the lower triangle of L (n x n, ld ldi, upper part zeroed); scratch >= n*n/4 elements
 template <typename T> void trtri_lower(cudaStream_t s, int n, const T *L, long ldl, T *Linv, long ldi, T *scratch);

@@ -279,58 +279,149 @@ __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, T *__restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// B[m x n] <- B L^{-T}, L n x n lower non-unit: rows of B are independent, so
-// a CTA takes SR rows through all n columns in one launch (left-looking over
-// 64-column blocks, the solved part of its rows in shared memory).
-//   update  block columns j: B_j -= X_{<j} L_{j,<j}^T, thread = one column
-//           and every fourth k, SR accumulators, L read along its columns
-//           (coalesced, from L2: every CTA reads all of L);
-//   solve   16 lanes per row, 4 columns each: the owner of the next four
-//           columns finishes them, shuffles pass them on (no barrier).
-// SR: 16 rows, or 4 where 16 would leave most SMs without a CTA.
+// X M^T = B for a lower triangular M (n x n), B m x n overwritten by X, with
+// M(j, p) at M[j m_js + p m_ps] and B(r, j) at B[r b_rs + j b_js]:
+//   B <- B L^{-T}   M = L                    (the Cholesky panel, STRSM R, L, T, N)
+//   B <- L^{-1} B   M = L, B transposed      (LU block row, STRSM L, L, N, N)
+//   B <- B U^{-1}   M = U^T, unit diagonal   (LU block column, STRSM R, U, N, U)
+// Rows are independent, so a CTA takes SR of them through all n columns in one
+// launch (left-looking over 64-column blocks, its solved part in shared memory):
+//   update  block columns j: B_j -= X_{<j} M_{j,<j}^T, thread = one column
+//           and every fourth p, SR accumulators, M from L2 (every CTA reads all
+//           of it); the next block's diagonal tile and right-hand sides are
+//           already on their way;
+//   solve   16 lanes per row, 4 columns each, passed on by shuffles (no
+//           barrier).  FP32: 4 neighbouring columns per lane, 4 at a time.
+//           FP64: every 16th column, one at a time, on M scaled to a unit
+//           diagonal: 164 FP64 operations per row pair instead of 416.
+// SR is 16 where that fills the GPU, else 8 or 4.
 // ---------------------------------------------------------------------------
 constexpr int CP_TRSM_MAXN = 1024;  // columns of one launch (shared memory: SR n elements)
-constexpr int CP_LP = CP_W + 4;     // pitch of the staged diagonal block
+constexpr int CP_LP = CP_W + 4;     // pitch of the staged diagonal block and rows
+
+template <typename T> struct SlabArgs {
+    int m, n;
+    const T *M;
+    long m_js, m_ps;
+    T *B;
+    long b_rs, b_js;
+    bool unit;
+};
 
 template <typename T, int SR> constexpr size_t cp_trsm_smem(int n)
 {
-    return ((size_t)((n + CP_W - 1) / CP_W * CP_W) * SR + (size_t)CP_W * CP_LP + CP_W + 4 * CP_W * (SR + 1)) * sizeof(T);
+    return ((size_t)((n + CP_W - 1) / CP_W * CP_W) * SR + (size_t)CP_W * CP_LP + CP_W + (size_t)SR * CP_LP +
+            4 * CP_W * (SR + 1)) * sizeof(T);
 }
 
-template <typename T, int SR>
-__global__ void __launch_bounds__(256) trsm_slab_kernel(int m, int n, const T *__restrict__ L, long ldl,
-                                                        T *__restrict__ B, long ldb)
+// 16 lanes per row: the solve of one 64-column block (rows S, block Ls, inverse diagonal inv)
+template <int SR> __device__ __forceinline__ void cp_slab_solve(float *S, const float *Ls, const float *inv)
+{
+    const int r = threadIdx.x >> 4, l = threadIdx.x & 15, src = threadIdx.x & 16;
+    Quad<float> x = *reinterpret_cast<const Quad<float> *>(S + r * CP_LP + 4 * l);
+#pragma unroll 2
+    for (int s = 0; s < 16; ++s) {
+        const float *D = Ls + (4 * s) * CP_LP + 4 * s;
+        float y[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float v = x.v[c];
+#pragma unroll
+            for (int q = 0; q < c; ++q) v = fmaf(-y[q], D[q * CP_LP + c], v);
+            y[c] = v * inv[4 * s + c];
+        }
+        if (l == s)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x.v[c] = y[c];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) y[c] = __shfl_sync(0xffffffffu, y[c], src | s);
+        if (l > s)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const Quad<float> lv = *reinterpret_cast<const Quad<float> *>(Ls + (4 * s + q) * CP_LP + 4 * l);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) x.v[c] = fmaf(-y[q], lv.v[c], x.v[c]);
+            }
+    }
+    *reinterpret_cast<Quad<float> *>(S + r * CP_LP + 4 * l) = x;
+}
+template <int SR> __device__ __forceinline__ void cp_slab_solve(double *S, const double *Ls, const double *inv)
+{
+    const int r = threadIdx.x >> 4, l = threadIdx.x & 15, src = threadIdx.x & 16;
+    double x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = S[r * CP_LP + 16 * q + l] * inv[16 * q + l];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+#pragma unroll 4
+        for (int s = 0; s < 16; ++s) {
+            const double y = __shfl_sync(0xffffffffu, x[g], src | s);
+            const double *D = Ls + (16 * g + s) * CP_LP + l;
+#pragma unroll
+            for (int q = g; q < 4; ++q)
+                if (q > g || l > s) x[q] = fma(-y, D[16 * q], x[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) S[r * CP_LP + 16 * q + l] = x[q];
+}
+
+template <typename T, int SR> __global__ void __launch_bounds__(256) trsm_slab_kernel(const SlabArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char cp_smem[];
-    const int npad = (n + CP_W - 1) / CP_W * CP_W;
-    T *Xs = (T *)cp_smem;                // [npad][SR]: solved rows, column by column
-    T *Ls = Xs + (size_t)npad * SR;      // [64][CP_LP]: diagonal block, Ls[c * CP_LP + r] = L(r, c)
-    T *inv = Ls + CP_W * CP_LP;          // [64]
-    T *red = inv + CP_W;                 // [4][64][SR + 1]
+    constexpr bool SCALED = sizeof(T) == 8;
+    const int npad = (a.n + CP_W - 1) / CP_W * CP_W;
+    T *Xs = (T *)cp_smem;             // [npad][SR]: solved rows, column by column
+    T *Ls = Xs + (size_t)npad * SR;   // [64][CP_LP]: diagonal block, Ls[c * CP_LP + r] = M(r, c), r > c
+    T *inv = Ls + CP_W * CP_LP;       // [64]
+    T *S = inv + CP_W;                // [SR][CP_LP]: the block's rows
+    T *red = S + SR * CP_LP;          // [4][64][SR + 1]
     const int tid = threadIdx.x, col = tid & 63, kg = tid >> 6;
     const int r0 = blockIdx.x * SR;
-    for (int j0 = 0; j0 < n; j0 += CP_W) {
-        const int w = min(CP_W, n - j0);
-        // the diagonal block (identity past w) and the block's right-hand sides
-        for (int e = tid; e < CP_W * CP_W; e += 256) {
-            const int r = e & 63, c = e >> 6;
-            Ls[c * CP_LP + r] = (r < w && c < r) ? L[(j0 + r) + (long)(j0 + c) * ldl] : T(0);
+    const bool b_along = a.b_js == 1;  // neighbouring threads on neighbouring elements of B
+    T lreg[16], b[SR / 4], dg = T(1);
+    auto bidx = [&](int i, int &r, int &c) {
+        const int e = tid + 256 * i;
+        r = b_along ? e / CP_W : e % SR;
+        c = b_along ? e % CP_W : e / SR;
+    };
+    auto fetch = [&](int j0) {
+        const int w = min(CP_W, a.n - j0);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int r = a.m_js == 1 ? col : 4 * i + kg, c = a.m_js == 1 ? 4 * i + kg : col;
+            lreg[i] = (r < w && c < r) ? a.M[(j0 + r) * a.m_js + (j0 + c) * a.m_ps] : T(0);
         }
-        if (tid < CP_W) inv[tid] = tid < w ? T(1) / L[(j0 + tid) + (long)(j0 + tid) * ldl] : T(1);
-        T b[SR / 4];
+        if (tid < CP_W) dg = (tid < w && !a.unit) ? a.M[(j0 + tid) * (a.m_js + a.m_ps)] : T(1);
 #pragma unroll
         for (int i = 0; i < SR / 4; ++i) {
-            const int e = tid + 256 * i, r = e % SR, c = e / SR;
-            b[i] = (c < w && r0 + r < m) ? B[(r0 + r) + (long)(j0 + c) * ldb] : T(0);
+            int r, c;
+            bidx(i, r, c);
+            b[i] = (c < w && r0 + r < a.m) ? a.B[(r0 + r) * a.b_rs + (j0 + c) * a.b_js] : T(0);
         }
+    };
+    fetch(0);
+    for (int j0 = 0; j0 < a.n; j0 += CP_W) {
+        const int w = min(CP_W, a.n - j0);
+        if (tid < CP_W) inv[tid] = T(1) / dg;
+        if (SCALED) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int r = a.m_js == 1 ? col : 4 * i + kg, c = a.m_js == 1 ? 4 * i + kg : col;
+            Ls[c * CP_LP + r] = SCALED ? lreg[i] * inv[r] : lreg[i];
+        }
+        T cur[SR / 4];
+#pragma unroll
+        for (int i = 0; i < SR / 4; ++i) cur[i] = b[i];
+        if (j0 + CP_W < a.n) fetch(j0 + CP_W);
         if (j0 > 0) {
             T acc[SR];
 #pragma unroll
             for (int r = 0; r < SR; ++r) acc[r] = T(0);
-            const T *Lc = L + j0 + min(col, w - 1);
+            const T *Mc = a.M + (j0 + min(col, w - 1)) * a.m_js;
 #pragma unroll 8
             for (int p = kg; p < j0; p += 4) {
-                const T l = Lc[(long)p * ldl];
+                const T l = Mc[p * a.m_ps];
                 const Quad<T> *x = reinterpret_cast<const Quad<T> *>(Xs + (size_t)p * SR);
 #pragma unroll
                 for (int q = 0; q < SR / 4; ++q) {
@@ -341,57 +432,30 @@ __global__ void __launch_bounds__(256) trsm_slab_kernel(int m, int n, const T *_
             }
 #pragma unroll
             for (int r = 0; r < SR; ++r) red[(kg * CP_W + col) * (SR + 1) + r] = acc[r];
+            __syncthreads();
         }
-        __syncthreads();
 #pragma unroll
         for (int i = 0; i < SR / 4; ++i) {
-            const int e = tid + 256 * i, r = e % SR, c = e / SR;
-            T v = b[i];
+            int r, c;
+            bidx(i, r, c);
+            T v = cur[i];
             if (j0 > 0)
                 v -= (red[(0 * CP_W + c) * (SR + 1) + r] + red[(1 * CP_W + c) * (SR + 1) + r]) +
                      (red[(2 * CP_W + c) * (SR + 1) + r] + red[(3 * CP_W + c) * (SR + 1) + r]);
-            Xs[(size_t)(j0 + c) * SR + r] = v;
+            S[r * CP_LP + c] = v;
         }
         __syncthreads();
-        if (tid < 16 * SR) {
-            const int r = tid >> 4, l = tid & 15, src = tid & 16;
-            // a warp is two rows of 16 lanes; SR >= 4 keeps whole warps here
-            T x[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) x[c] = Xs[(size_t)(j0 + 4 * l + c) * SR + r];
-#pragma unroll 2
-            for (int s = 0; s < 16; ++s) {
-                const T *D = Ls + (4 * s) * CP_LP + 4 * s;
-                T y[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    T v = x[c];
-#pragma unroll
-                    for (int q = 0; q < c; ++q) v = fma(-y[q], D[q * CP_LP + c], v);
-                    y[c] = v * inv[4 * s + c];
-                }
-                if (l == s)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) x[c] = y[c];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) y[c] = __shfl_sync(0xffffffffu, y[c], src | s);
-                if (l > s)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const Quad<T> lv = *reinterpret_cast<const Quad<T> *>(Ls + (4 * s + q) * CP_LP + 4 * l);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) x[c] = fma(-y[q], lv.v[c], x[c]);
-                    }
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) Xs[(size_t)(j0 + 4 * l + c) * SR + r] = x[c];
-        }
+        if (tid < 16 * SR) cp_slab_solve<SR>(S, Ls, inv);  // whole warps: two rows each
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < SR / 4; ++i) {
-            const int e = tid + 256 * i, r = e % SR, c = e / SR;
-            if (c < w && r0 + r < m) B[(r0 + r) + (long)(j0 + c) * ldb] = Xs[(size_t)(j0 + c) * SR + r];
+            int r, c;
+            bidx(i, r, c);
+            const T v = S[r * CP_LP + c];
+            Xs[(size_t)(j0 + c) * SR + r] = v;
+            if (c < w && r0 + r < a.m) a.B[(r0 + r) * a.b_rs + (j0 + c) * a.b_js] = v;
         }
+        __syncthreads();
     }
 }
 
@@ -404,13 +468,14 @@ __global__ void __launch_bounds__(256) trsm_slab_kernel(int m, int n, const T *_
 // 32-row pieces: warp c solves column c's piece by shuffles (lane = row)
 // while the CTA's loads of the piece's off-diagonal part are in flight, then
 // thread = row (forward) or column (backward) applies them.  Bound by the
-// chain of dependent rows.
+// chain of dependent rows.  FP64 solves a piece scaled to a unit diagonal, one
+// operation (64 clocks) per row in the chain instead of three.
 // ---------------------------------------------------------------------------
 constexpr int CP_SB = 256;
 
 template <typename T, int C> constexpr size_t cp_trsv_smem(bool trans)
 {
-    return ((size_t)C * CP_SB + 32 * 33 + (trans ? (size_t)CP_SB * 33 : 0)) * sizeof(T);
+    return ((size_t)(C + 1) * CP_SB + 32 * 33 + (trans ? (size_t)CP_SB * 33 : 0)) * sizeof(T);
 }
 
 template <typename T, int C, bool TRANS>
@@ -419,7 +484,8 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, int nrhs, const T 
 {
     extern __shared__ __align__(16) unsigned char cp_smem[];
     T *xs = (T *)cp_smem;         // [C][CP_SB]
-    T *Ld = xs + C * CP_SB;       // [32][33]: forward Ld[j][i] = L(i, j), backward Ld[j][i] = L(j, i)
+    T *dinv = xs + C * CP_SB;     // [CP_SB]: 1 / L(r, r)
+    T *Ld = dinv + CP_SB;         // [32][33]: forward Ld[j][i] = L(i, j), backward Ld[j][i] = L(j, i)
     T *Lt = Ld + 32 * 33;         // backward: [CP_SB][33], Lt[c][i] = L(piece row i, c)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c0 = blockIdx.x * C, nc = min(C, nrhs - c0);
@@ -427,6 +493,9 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, int nrhs, const T 
         const int r = e % CP_SB, c = e / CP_SB;
         xs[e] = (r < w && c < nc) ? B[r + (long)(c0 + c) * ldb] : T(0);
     }
+    dinv[tid] = tid < w ? T(1) / L[tid + (long)tid * ldl] : T(1);
+    __syncthreads();
+    constexpr bool SCALED = sizeof(T) == 8;
     const int np = (w + 31) / 32;
     for (int s = 0; s < np; ++s) {
         const int p0 = 32 * (TRANS ? np - 1 - s : s), pw = min(32, w - p0);
@@ -445,14 +514,27 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, int nrhs, const T 
         }
         for (int e = tid; e < 32 * 32; e += 256) {
             const int i = e & 31, j = e >> 5;  // L(i, j) of the piece's diagonal block
-            const T v = (i < pw && j <= i) ? L[(p0 + i) + (long)(p0 + j) * ldl] : T(i == j ? 1 : 0);
+            T v = (i < pw && j <= i) ? L[(p0 + i) + (long)(p0 + j) * ldl] : T(i == j ? 1 : 0);
+            if (SCALED) v *= dinv[p0 + (TRANS ? j : i)];
             Ld[TRANS ? i * 33 + j : j * 33 + i] = v;
         }
         __syncthreads();
         for (int c = warp; c < C; c += 8) {
             // the products are summed apart from the right-hand side, so that
             // each rounding is relative to their (smaller) sum
-            const T v = xs[c * CP_SB + p0 + lane], d = T(1) / Ld[lane * 33 + lane];
+            const T d = dinv[p0 + lane];
+            if (SCALED) {
+                T v = xs[c * CP_SB + p0 + lane] * d;
+#pragma unroll 8
+                for (int i = 0; i < 32; ++i) {
+                    const int j = TRANS ? 31 - i : i;
+                    const T xj = __shfl_sync(0xffffffffu, v, j);
+                    if (TRANS ? lane < j : lane > j) v = fma(-Ld[j * 33 + lane], xj, v);
+                }
+                xs[c * CP_SB + p0 + lane] = v;
+                continue;
+            }
+            const T v = xs[c * CP_SB + p0 + lane];
             T acc = T(0);
             if (!TRANS) {
 #pragma unroll 8

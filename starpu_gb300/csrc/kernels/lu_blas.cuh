@@ -9,6 +9,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chol_panel.cuh"
+
 namespace gb300 {
 
 // 1 / d rounded to T the way the reference forms its scale factor: in double,
@@ -81,36 +83,154 @@ __global__ void __launch_bounds__(256) getf2_small_kernel(int n, T *__restrict__
 }
 
 // ---------------------------------------------------------------------------
-// B[m x w] <- B * U^{-1}, U w x w unit upper (w <= W): the right-side TRSM of
-// the LU's block column (cublasStrsm(R, U, N, U), xlu_kernels.c:281-289).
-// One thread per row of B, column-oriented like reference BLAS strsm.
-// FULL (w == W) keeps every index static, which keeps x[] in registers.
+// The FP32 leaf: unblocked LU of one n x n (n <= 64) block by one CTA of 8
+// warps, the columns four at a time as the Cholesky panel takes them
+// (chol_panel.cuh: lane = row, warp w owns columns 4w .. and 32 + 4w .., a
+// buffer and an mbarrier per step instead of CTA barriers).  The owner of a
+// step factors its 4 x 4 block in every lane, forms its columns of L and
+// publishes them with the reciprocal pivots; the others form their elements
+// of the four rows of U from the 4 x 4 block (four shuffles per column) and
+// apply the rank-4 update.  Bound by the chain of 16 steps: 10 us against 36
+// for a barrier and a double-precision reciprocal per column.  Same status words
+// and threshold as getf2_small_kernel.
 // ---------------------------------------------------------------------------
-template <typename T, int W, bool FULL>
-__global__ void __launch_bounds__(128) trsm_runu_small_kernel(int m, int w, const T *__restrict__ U, long ldu,
-                                                              T *__restrict__ B, long ldb)
+struct GetfPanel {
+    Quad<float> pan[16][CP_W];  // L of the step's columns, 0 above its rows
+    Quad<float> inv[16];        // 1 / pivots
+    uint64_t bar[16];
+};
+
+template <int G> __device__ __forceinline__ void getf_update(CpBlock<float> &a, const GetfPanel &s, int step)
 {
-    __shared__ T Us[W][W + 1];
-    const int tid = threadIdx.x;
-    const int ww = FULL ? W : w;
-    for (int idx = tid; idx < W * W; idx += blockDim.x) {
-        const int i = idx % W, j = idx / W;
-        Us[i][j] = (i < ww && j < ww && i < j) ? U[(long)i + (long)j * ldu] : T(0);
+    const int lane = threadIdx.x & 31, hs = step >> 3, blk = step & 7;
+    const Quad<float> *p = s.pan[step];
+    Quad<float> li[2], l[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) li[h] = p[32 * h + lane];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) l[i] = p[4 * step + i];
+    const Quad<float> inv = s.inv[step];
+    const bool in = (lane >> 2) == blk;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float v = hs ? a[G][c][1] : a[G][c][0];
+        Quad<float> u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float t = __shfl_sync(0xffffffffu, v, 4 * blk + i);
+#pragma unroll
+            for (int q = 0; q < i; ++q) t = fmaf(-l[i].v[q], u.v[q], t);
+            u.v[i] = t * inv.v[i];
+        }
+        const float mine = (lane & 2) ? ((lane & 1) ? u.v[3] : u.v[2]) : ((lane & 1) ? u.v[1] : u.v[0]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (in && h == hs) a[G][c][h] = mine;
+            else if (h >= hs) a[G][c][h] = cp_dot_sub(a[G][c][h], li[h], u);
     }
+}
+
+// the owner's part of step 8 G + warp
+template <int G>
+__device__ __forceinline__ void getf_own(CpBlock<float> &a, GetfPanel &s, int n, float thr, int *d_first, int *info,
+                                         int info_base)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, step = 8 * G + warp;
+    Quad<float> *p = s.pan[step];
+    const bool in = (lane >> 2) == warp;
+    if (in) p[32 * G + lane] = {a[G][0][G], a[G][1][G], a[G][2][G], a[G][3][G]};
+    __syncwarp();
+    float l[4][4], inv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const Quad<float> v = p[4 * step + i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) l[i][j] = v.v[j];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        inv[j] = __frcp_rn(l[j][j]);
+#pragma unroll
+        for (int k = j + 1; k < 4; ++k) l[j][k] *= inv[j];
+#pragma unroll
+        for (int i = j + 1; i < 4; ++i)
+#pragma unroll
+            for (int k = j + 1; k < 4; ++k) l[i][k] = fmaf(-l[i][j], l[j][k], l[i][k]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        Quad<float> y;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float v = a[G][j][h];
+#pragma unroll
+            for (int q = 0; q < j; ++q) v = fmaf(-y.v[q], l[q][j], v);
+            y.v[j] = v;
+        }
+        if (h < G || (h == G && lane < 4 * warp)) {  // rows above: U already, no part in this step
+            y = {0.0f, 0.0f, 0.0f, 0.0f};
+        } else if (h == G && in) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if ((lane & 3) == i) {
+                        a[G][j][h] = l[i][j];
+                        y.v[j] = j <= i ? l[i][j] : 0.0f;
+                    }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) a[G][j][h] = y.v[j];
+        }
+        p[32 * h + lane] = y;
+    }
+    if (lane == 0) s.inv[step] = {inv[0], inv[1], inv[2], inv[3]};
+    ptx::mbar_arrive(&s.bar[step]);
+    if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int z = 4 * step + j;
+            if (z >= n) break;
+            if (l[j][j] == 0.0f && info) atomicCAS(info, 0, info_base + z + 1);
+            if (thr > 0.0f && !(fabsf(l[j][j]) >= thr) && d_first) atomicMin(d_first, info_base + z);
+        }
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restrict__ A, long lda, float thr, int *d_first,
+                                                         int *info, int info_base)
+{
+    __shared__ GetfPanel s;
+    const int w = threadIdx.x >> 5, steps = (n + 3) / 4;
+    CpBlock<float> a;
+    cp_panel_init(s.bar);
+    cp_each<float>(a, [&](float &v, int r, int c) { v = (r < n && c < n) ? A[r + (long)c * lda] : (r == c ? 1.0f : 0.0f); });
     __syncthreads();
-    const long r = (long)blockIdx.x * blockDim.x + tid;
-    if (r >= m) return;
-    T x[W];
-#pragma unroll
-    for (int c = 0; c < W; ++c) x[c] = (FULL || c < ww) ? B[r + (long)c * ldb] : T(0);
-#pragma unroll
-    for (int j = 0; j < W; ++j) {
-#pragma unroll
-        for (int c = j + 1; c < W; ++c) x[c] = fma(-Us[j][c], x[j], x[c]);
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < min(w, steps); ++i) {
+        ok = cp_wait(&s.bar[i], 0) && ok;
+        getf_update<0>(a, s, i);
+        if (i < w - 1) getf_update<1>(a, s, i);  // the next owner publishes first
     }
-#pragma unroll
-    for (int c = 0; c < W; ++c)
-        if (FULL || c < ww) B[r + (long)c * ldb] = x[c];
+    if (w < steps) getf_own<0>(a, s, n, thr, d_first, info, info_base);
+    if (steps > 8) {
+        if (w > 0) getf_update<1>(a, s, w - 1);
+        getf_update<1>(a, s, w);
+#pragma unroll 1
+        for (int i = w + 1; i < min(8 + w, steps); ++i) {
+            ok = cp_wait(&s.bar[i], 0) && ok;
+            getf_update<1>(a, s, i);
+        }
+        if (8 + w < steps) getf_own<1>(a, s, n, thr, d_first, info, info_base);
+    }
+    if (!ok && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
+    cp_each<float>(a, [&](float &v, int r, int c) {
+        if (r < n && c < n) A[r + (long)c * lda] = v;
+    });
 }
 
 // ---------------------------------------------------------------------------

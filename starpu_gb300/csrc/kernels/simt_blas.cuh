@@ -182,48 +182,6 @@ gemm_simt_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long lda
 }
 
 // ---------------------------------------------------------------------------
-// Left-side small triangular solves on a w x nrhs block (w <= W), one thread
-// per right-hand side.  Used by the blocked POTRS (forward L y = b, backward
-// L^T x = y), mirroring LAPACK dpotrs (min-dgels/base/SRC/dpotrs.c): two
-// triangular sweeps with the Cholesky factor.
-// ---------------------------------------------------------------------------
-template <typename T, int W, bool TRANS>
-__global__ void __launch_bounds__(64) trsm_left_small_kernel(int w, int nrhs, const T *__restrict__ L, long ldl,
-                                                             T *__restrict__ B, long ldb)
-{
-    __shared__ T Ls[W][W + 1];
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < W * W; idx += blockDim.x) {
-        int i = idx % W, j = idx / W;
-        Ls[i][j] = (i < w && j < w && i >= j) ? L[(long)i + (long)j * ldl] : T(i == j ? 1 : 0);
-    }
-    __syncthreads();
-    const int c = blockIdx.x * blockDim.x + tid;
-    if (c >= nrhs) return;
-    T x[W];
-#pragma unroll
-    for (int i = 0; i < W; ++i) x[i] = (i < w) ? B[(long)i + (long)c * ldb] : T(0);
-    if (!TRANS) {
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            x[j] = x[j] / Ls[j][j];
-#pragma unroll
-            for (int i = j + 1; i < W; ++i) x[i] = fma(-Ls[i][j], x[j], x[i]);
-        }
-    } else {
-#pragma unroll
-        for (int j = W - 1; j >= 0; --j) {
-            x[j] = x[j] / Ls[j][j];
-#pragma unroll
-            for (int i = 0; i < j; ++i) x[i] = fma(-Ls[j][i], x[j], x[i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < W; ++i)
-        if (i < w) B[(long)i + (long)c * ldb] = x[i];
-}
-
-// ---------------------------------------------------------------------------
 // Elementwise helpers.
 // ---------------------------------------------------------------------------
 template <typename TO, typename TI>

@@ -124,3 +124,36 @@ def test_fp64_update_keeps_nan_in_its_row(gpu):
     assert info.download((1,), np.int32)[0] == i + 1
     ref = np.linalg.cholesky(spd(n, n)[:i, :i])
     assert np.allclose(np.tril(out[:i, :i]), ref, rtol=0, atol=1e-13)
+
+
+@BOTH
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 33, 36, 63, 64, 65, 130])
+def test_getrf_blocks(gpu, dtype, n):
+    a = (np.random.default_rng(n).uniform(-1, 1, (n, n)) + n * np.eye(n)).astype(dtype)
+    da, info = up(a), up(np.full(1, 5, np.int32))
+    check(fn(gpu, dtype, "getrf_tile")(None, n, da.ptr, n, info.ptr))
+    out = da.download((n, n), dtype).astype(np.float64)
+    assert info.download((1,), np.int32)[0] == 0
+    l, u = np.tril(out), np.triu(out, 1) + np.eye(n)
+    bound = 2 * (n + 1) * EPS[dtype] * (np.abs(l) @ np.abs(u))
+    assert np.all(np.abs(l @ u - a) <= bound)
+
+
+@BOTH
+@pytest.mark.parametrize("m,n", [(1, 1100), (64, 65), (70, 700), (700, 70), (1030, 33)])
+def test_lu_panel_solves(gpu, dtype, m, n):
+    rng = np.random.default_rng(m + n)
+    for name, k in (("trsm_llnn_tile", m), ("trsm_runu_tile", n)):
+        t = rng.uniform(-1, 1, (k, k)) / k
+        t = np.tril(t) + np.eye(k) if k == m and name == "trsm_llnn_tile" else np.triu(t, 1)
+        b = rng.uniform(-1, 1, (m, n))
+        t, b = t.astype(dtype), b.astype(dtype)
+        dt, db = up(t), up(b)
+        check(fn(gpu, dtype, name)(None, m, n, dt.ptr, k, db.ptr, m))
+        x, t64 = db.download((m, n), dtype).astype(np.float64), t.astype(np.float64)
+        if name == "trsm_llnn_tile":
+            got, mag = t64 @ x, np.abs(t64) @ np.abs(x)
+        else:
+            u = t64 + np.eye(k)
+            got, mag = x @ u, np.abs(x) @ np.abs(u)
+        assert np.all(np.abs(got - b) <= 4 * k * EPS[dtype] * (mag + np.abs(b)))
