@@ -125,23 +125,51 @@ __device__ __forceinline__ int f16_row_exp(float bound)
     return e - 15;
 }
 
-// rk[i] from the actual row maxima (the inverse of a diagonal tile, whose
-// elements have no bound from the matrix): 32 rows per CTA, the k loop split
-// over 8 thread rows.
-__global__ void panel_row_scale_kernel(int m, int k, const float *__restrict__ P, long ldp, int *__restrict__ rk,
-                                       float *__restrict__ rs)
+// The split with rk from the actual row maxima (the inverse of a diagonal
+// tile, whose elements have no bound from the matrix; codelet tiles): 32 rows
+// per CTA of 32 x 32 threads, the row maxima in a first pass over the k columns
+// (a thread every 32nd column, eight loads in flight), the split in a second
+// pass that finds them in L2.  One launch instead of a row-maximum launch
+// (12 us for a 1024 x 1024 tile, one load in flight) and a split (6 us).
+__global__ void __launch_bounds__(1024) split_f16s_rowmax_kernel(int m, int k, const float *__restrict__ P, long ldp,
+                                                                 int *__restrict__ rk, float *__restrict__ rs,
+                                                                 __half *__restrict__ h, __half *__restrict__ l, long ldk)
 {
-    __shared__ float red[8][33];
-    const int r = blockIdx.x * 32 + threadIdx.x;
+    __shared__ float t[32][33];
+    __shared__ int sh[32];
+    const int r0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y, r = r0 + tx;
     float mx = 0.0f;
-    if (r < m)
-        for (int c = threadIdx.y; c < k; c += 8) mx = fmaxf(mx, fabsf(P[r + (long)c * ldp]));
-    red[threadIdx.y][threadIdx.x] = mx;
+    if (r < m) {
+#pragma unroll 8
+        for (int c = ty; c < k; c += 32) mx = fmaxf(mx, fabsf(P[r + (long)c * ldp]));
+    }
+    t[ty][tx] = mx;
     __syncthreads();
-    if (threadIdx.y == 0 && r < m) {
-        for (int y = 1; y < 8; ++y) mx = fmaxf(mx, red[y][threadIdx.x]);
-        rk[r] = f16_row_exp(mx);
-        rs[r] = pow2f(rk[r]);
+    if (ty == 0) {
+        for (int y = 1; y < 32; ++y) mx = fmaxf(mx, t[y][tx]);
+        const int e = f16_row_exp(mx);
+        sh[tx] = -e;
+        if (r < m && blockIdx.y == 0) {
+            rk[r] = e;
+            rs[r] = pow2f(e);
+        }
+    }
+    __syncthreads();
+    const int rr = r0 + ty;
+    const int sx = sh[ty];
+    const float sc = (sx >= -126 && sx <= 127) ? __int_as_float((sx + 127) << 23) : 0.0f;
+    for (int c0 = 32 * blockIdx.y; c0 < ldk; c0 += 32 * gridDim.y) {
+        __syncthreads();
+        t[ty][tx] = (r < m && c0 + ty < k) ? P[r + (long)(c0 + ty) * ldp] : 0.0f;
+        __syncthreads();
+        if (rr < m && c0 + tx < ldk) {
+            const float v = t[tx][ty];
+            const float x = sc != 0.0f ? v * sc : ldexpf(v, sx);
+            const __half hh = __float2half_rn(x);
+            const long o = (long)rr * ldk + c0 + tx;
+            h[o] = hh;
+            l[o] = __float2half_rn(x - __half2float(hh));
+        }
     }
 }
 
@@ -167,11 +195,10 @@ __global__ void diag_bounds_kernel(int n, const float *__restrict__ A, long lda,
     if (threadIdx.x == 0) dtile[t] = red[0];
 }
 
-// the split; rk given (from_bounds = 0) or computed from d / f (from_bounds = 1:
-// rows r0.. of the matrix, d indexed by matrix row, *f or 1 when f is NULL)
+// the split with rk from the bounds d / f (rows r0.. of the matrix, d indexed
+// by matrix row, *f or 1 when f is NULL)
 __global__ void split_f16s_kmajor_kernel(int m, int k, const float *__restrict__ P, long ldp, int *__restrict__ rk,
-                                         float *__restrict__ rs,
-                                         int from_bounds, const float *__restrict__ d, int r0,
+                                         float *__restrict__ rs, const float *__restrict__ d, int r0,
                                          const float *__restrict__ f, __half *__restrict__ h, __half *__restrict__ l,
                                          long ldk)
 {
@@ -180,17 +207,12 @@ __global__ void split_f16s_kmajor_kernel(int m, int k, const float *__restrict__
     const int rb = blockIdx.x * 32, c0 = blockIdx.y * 32;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     if (tid < 32 && rb + tid < m) {
-        int e;
-        if (from_bounds) {
-            // sqrt(d_r) sqrt(f): no underflow or overflow of the product for
-            // matrices scaled far from 1
-            e = f16_row_exp(sqrtf(fmaxf(d[r0 + rb + tid], 0.0f)) * (f ? sqrtf(*f) : 1.0f));
-            if (blockIdx.y == 0) {
-                rk[rb + tid] = e;
-                rs[rb + tid] = pow2f(e);
-            }
-        } else {
-            e = rk[rb + tid];
+        // sqrt(d_r) sqrt(f): no underflow or overflow of the product for
+        // matrices scaled far from 1
+        const int e = f16_row_exp(sqrtf(fmaxf(d[r0 + rb + tid], 0.0f)) * (f ? sqrtf(*f) : 1.0f));
+        if (blockIdx.y == 0) {
+            rk[rb + tid] = e;
+            rs[rb + tid] = pow2f(e);
         }
         sh[tid] = -e;
     }
@@ -218,11 +240,16 @@ static int split_f16s(cudaStream_t s, int m, int k, const float *P, long ldp, co
                       const float *d = nullptr, int r0 = 0, const float *f = nullptr)
 {
     if (m <= 0 || k <= 0) return GB300_OK;
-    if (!d)
-        gb300_count_launch(), panel_row_scale_kernel<<<(m + 31) / 32, dim3(32, 8), 0, s>>>(m, k, P, ldp, o.rk, o.rs);
+    if (!d) {
+        // few row blocks: several CTAs share one (each finds the maxima for itself)
+        const int gx = (m + 31) / 32, gy = std::max(1, std::min((int)((ldk + 31) / 32), 2 * num_sms() / gx));
+        gb300_count_launch(), split_f16s_rowmax_kernel<<<dim3(gx, gy), dim3(32, 32), 0, s>>>(m, k, P, ldp, o.rk, o.rs, o.h,
+                                                                                          o.l, ldk);
+        return gb300_last_launch_status();
+    }
     dim3 g((m + 31) / 32, (unsigned)((ldk + 31) / 32));
-    gb300_count_launch(), split_f16s_kmajor_kernel<<<g, dim3(32, 8), 0, s>>>(m, k, P, ldp, o.rk, o.rs, d ? 1 : 0, d, r0, f,
-                                                                           o.h, o.l, ldk);
+    gb300_count_launch(), split_f16s_kmajor_kernel<<<g, dim3(32, 8), 0, s>>>(m, k, P, ldp, o.rk, o.rs, d, r0, f, o.h, o.l,
+                                                                           ldk);
     return gb300_last_launch_status();
 }
 
@@ -239,6 +266,35 @@ struct TcOperand {
     const float *rs;
 };
 
+// The kernels' shared-memory limits on the current device.
+static int tcu_prepare()
+{
+    if (int rc = gb300_func_dyn_smem((const void *)tc_update_kernel<TCU_BN>, TcuCfg<TCU_BN>::SMEM)) return rc;
+    return gb300_func_dyn_smem((const void *)tc_update_kernel<TCU_BN_NARROW>, TcuCfg<TCU_BN_NARROW>::SMEM);
+}
+
+// tiles of 128 x bn an update covers
+static long tcu_tiles(int m, int n, int lower, int bn)
+{
+    const long tm = (m + TCU_BM - 1) / TCU_BM, tn = (n + bn - 1) / bn;
+    if (!lower) return tm * tn;
+    long cnt = 0;
+    for (long c = 0; c < tn; ++c) cnt += std::max(0L, tm - c * bn / TCU_BM);
+    return cnt;
+}
+
+// The tile width of an update on `ctas` SMs: a wide tile takes about 2.6 times
+// as long as a narrow one (both measured on a 1024 x 1024 x 1024 update, where
+// the narrow ones are faster by the number of waves), so the fewer waves by
+// that weight win.  A range of tiles [t0, t1) counts in wide ones.
+static int tcu_bn(int m, int n, int lower, int ctas, int t0, int t1)
+{
+    if (t0 > 0 || t1 >= 0) return TCU_BN;
+    const long w = (tcu_tiles(m, n, lower, TCU_BN) + ctas - 1) / ctas;
+    const long v = (tcu_tiles(m, n, lower, TCU_BN_NARROW) + ctas - 1) / ctas;
+    return 10 * v < 26 * w ? TCU_BN_NARROW : TCU_BN;
+}
+
 // max_grid > 0 caps the persistent grid (CTAs, one per SM): the trailing
 // update that runs beside the next panel leaves that panel's SMs free.
 // f16s: both operands are scaled FP16 panels.  [t0, t1) (t1 < 0: to the end)
@@ -252,13 +308,15 @@ static int tc_update_op(cudaStream_t s, int m, int n, int K, const TcOperand &A,
     if ((nterms != 1 && nterms != 3) || (nterms == 3 && (!A.lo || !B.lo)) || (lower && m != n) || !d_err ||
         (f16s && (!A.rs || !B.rs)))
         return GB300_EINVAL;
+    const int sms = num_sms(), max_ctas = max_grid > 0 ? std::min(max_grid, sms) : sms;
+    const int bn = tcu_bn(m, n, lower, max_ctas, t0, t1);
     CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
     int rc;
     if ((rc = make_kmajor_map(&ta_hi, A.hi, m, K, lda, TCU_BM))) return rc;
-    if ((rc = make_kmajor_map(&tb_hi, B.hi, n, K, ldb, TCU_BN))) return rc;
+    if ((rc = make_kmajor_map(&tb_hi, B.hi, n, K, ldb, bn))) return rc;
     if (nterms == 3) {
         if ((rc = make_kmajor_map(&ta_lo, A.lo, m, K, lda, TCU_BM))) return rc;
-        if ((rc = make_kmajor_map(&tb_lo, B.lo, n, K, ldb, TCU_BN))) return rc;
+        if ((rc = make_kmajor_map(&tb_lo, B.lo, n, K, ldb, bn))) return rc;
     } else {
         ta_lo = ta_hi;
         tb_lo = tb_hi;
@@ -278,23 +336,21 @@ static int tc_update_op(cudaStream_t s, int m, int n, int K, const TcOperand &A,
     a.store = store;
     a.b_lower = b_lower ? 1 : 0;
     a.tiles_m = (m + TCU_BM - 1) / TCU_BM;
-    a.tiles_n = (n + TCU_BN - 1) / TCU_BN;
-    if (lower) {
-        long cnt = 0;
-        for (int tn = 0; 2 * tn < a.tiles_m; ++tn) cnt += a.tiles_m - 2 * tn;
-        a.num_tiles = (int)cnt;
-    } else {
-        a.num_tiles = a.tiles_m * a.tiles_n;
-    }
+    a.tiles_n = (n + bn - 1) / bn;
+    a.num_tiles = (int)tcu_tiles(m, n, lower, bn);
     a.tile_begin = std::max(0, std::min(t0, a.num_tiles));
     a.tile_end = t1 < 0 ? a.num_tiles : std::max(a.tile_begin, std::min(t1, a.num_tiles));
     if (a.tile_end <= a.tile_begin) return GB300_OK;
     a.err = d_err;
     a.wait_budget_ns = 2000000000ull;  // 2 s per wait: far above any legitimate stall
-    if (int rc = gb300_func_dyn_smem((const void *)tc_update_kernel, TCU_SMEM)) return rc;
-    const int ntl = a.tile_end - a.tile_begin;
-    const int grid = std::min(ntl, max_grid > 0 ? std::min(max_grid, num_sms()) : num_sms());
-    gb300_count_launch(), tc_update_kernel<<<grid, TCU_THREADS, TCU_SMEM, s>>>(ta_hi, ta_lo, tb_hi, tb_lo, a);
+    if ((rc = tcu_prepare())) return rc;
+    const int grid = std::min(a.tile_end - a.tile_begin, max_ctas);
+    if (bn == TCU_BN)
+        gb300_count_launch(), tc_update_kernel<TCU_BN>
+            <<<grid, TCU_THREADS, TcuCfg<TCU_BN>::SMEM, s>>>(ta_hi, ta_lo, tb_hi, tb_lo, a);
+    else
+        gb300_count_launch(), tc_update_kernel<TCU_BN_NARROW>
+            <<<grid, TCU_THREADS, TcuCfg<TCU_BN_NARROW>::SMEM, s>>>(ta_hi, ta_lo, tb_hi, tb_lo, a);
     return gb300_last_launch_status();
 }
 
@@ -877,7 +933,7 @@ size_t starpu_gb300_tile_tc_workspace(int nmax)
 
 int starpu_gb300_tile_tc_prepare(void)
 {
-    return gb300_func_dyn_smem((const void *)tc_update_kernel, TCU_SMEM);
+    return gb300::tcu_prepare();
 }
 
 int starpu_gb300_sgemm_nt_tile_tc(void *stream, int m, int n, int k, const float *A, int lda, const float *B,

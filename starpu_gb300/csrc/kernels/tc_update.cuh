@@ -28,11 +28,14 @@
 //
 // CTA = 6 warps, one CTA per SM (persistent, static round-robin over tiles):
 //   warp 0  TMA producer     (one elected lane)
-//   warp 1  MMA issuer       (one elected lane) + TMEM owner (512 columns)
+//   warp 1  MMA issuer       (one elected lane) + TMEM owner
 //   warps 2-5 epilogue       (tcgen05.ld: warp w reads TMEM lanes 32*(w%4)..+31)
-// Shared memory: STAGES x (A 128x64 + B 256x64 BF16) = STAGES x 48 KB.
-// TMEM: two 128x256 FP32 accumulators so the epilogue of tile i overlaps the
-// main loop of tile i+1.
+// Tiles of 128 x BN, BN = 256 (4 stages of 48 KB) or 64 (8 of 24 KB); TMEM holds
+// two 128 x BN FP32 accumulators so the epilogue of tile i overlaps the main loop
+// of tile i+1.  A 64-column tile reads its A operand four times as often (its
+// MMAs are bound by shared memory at two thirds of the tensor rate) but makes
+// four times as many tiles: tcu_narrow() takes it where the wide tiles leave SMs
+// idle.  Every element's products are added in the same order either way.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -43,14 +46,17 @@
 namespace gb300 {
 
 constexpr int TCU_BM = 128;
-constexpr int TCU_BN = 256;
+constexpr int TCU_BN = 256;       // the wide tile
+constexpr int TCU_BN_NARROW = 64;
 constexpr int TCU_BK = 64;        // 64 BF16 = one 128-byte swizzle row
-constexpr int TCU_STAGES = 4;
 constexpr int TCU_THREADS = 192;
 constexpr int TCU_A_BYTES = TCU_BM * TCU_BK * 2;   // 16 KB
-constexpr int TCU_B_BYTES = TCU_BN * TCU_BK * 2;   // 32 KB
-constexpr int TCU_SMEM = TCU_STAGES * (TCU_A_BYTES + TCU_B_BYTES) + 1024 /*align*/ + 256 /*barriers*/;
-constexpr uint32_t TCU_TMEM_COLS = 512;
+template <int BN> struct TcuCfg {
+    static constexpr int STAGES = BN == TCU_BN ? 4 : 8;
+    static constexpr int B_BYTES = BN * TCU_BK * 2;
+    static constexpr int SMEM = STAGES * (TCU_A_BYTES + B_BYTES) + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr uint32_t TMEM_COLS = 2 * BN;
+};
 
 // error codes written to *err
 constexpr int TCU_ERR_TIMEOUT_PRODUCER = 1;
@@ -71,22 +77,21 @@ struct TcUpdateArgs {
     int tiles_m, tiles_n, num_tiles;
     int tile_begin, tile_end;  // the launch covers tiles [tile_begin, tile_end) of the num_tiles
     // 1: B is lower triangular in (row, k) (B(c, k) = 0 for k > c, the panel TRSM's
-    // inverse), so a tile of columns n0 .. n0 + 255 stops at k = n0 + 255
+    // inverse), so a tile of columns n0 .. n0 + BN - 1 stops at k = n0 + BN - 1
     int b_lower;
     int *err;
     unsigned long long wait_budget_ns;
 };
 
 // K blocks a tile of columns n0 .. needs (all of them unless B is lower triangular)
-__device__ __forceinline__ int tcu_tile_kblocks(const TcUpdateArgs &a, int kblocks, int n0)
+template <int BN> __device__ __forceinline__ int tcu_tile_kblocks(const TcUpdateArgs &a, int kblocks, int n0)
 {
-    return a.b_lower ? min(kblocks, (n0 + TCU_BN + TCU_BK - 1) / TCU_BK) : kblocks;
+    return a.b_lower ? min(kblocks, (n0 + BN + TCU_BK - 1) / TCU_BK) : kblocks;
 }
 
-// Map a linear tile index to (tm, tn).  Lower: column tn holds tiles
-// tm = 2*tn .. tiles_m-1 (a 128-row tile crosses the diagonal of a 256-column
-// tile only from tm = 2*tn on).
-__device__ __forceinline__ void tcu_tile_coords(const TcUpdateArgs &a, int t, int &tm, int &tn)
+// Map a linear tile index to (tm, tn).  Lower: column tn holds the row tiles
+// from the one that holds its first diagonal element on.
+template <int BN> __device__ __forceinline__ void tcu_tile_coords(const TcUpdateArgs &a, int t, int &tm, int &tn)
 {
     if (!a.lower) {
         tm = t % a.tiles_m;
@@ -95,9 +100,9 @@ __device__ __forceinline__ void tcu_tile_coords(const TcUpdateArgs &a, int t, in
     }
     int col = 0, acc = 0;
     for (;;) {
-        int cnt = a.tiles_m - 2 * col;
+        const int first = col * BN / TCU_BM, cnt = a.tiles_m - first;
         if (t < acc + cnt) {
-            tm = 2 * col + (t - acc);
+            tm = first + (t - acc);
             tn = col;
             return;
         }
@@ -106,11 +111,13 @@ __device__ __forceinline__ void tcu_tile_coords(const TcUpdateArgs &a, int t, in
     }
 }
 
+template <int BN>
 __global__ void __launch_bounds__(TCU_THREADS, 1)
 tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
                  const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
                  const TcUpdateArgs args)
 {
+    constexpr int TCU_STAGES = TcuCfg<BN>::STAGES, TCU_B_BYTES = TcuCfg<BN>::B_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-byte aligned tile area (required by the 128B swizzle atoms)
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -150,7 +157,7 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
         }
     }
     if (warp == 1) {
-        ptx::tmem_alloc(tmem_slot, TCU_TMEM_COLS);
+        ptx::tmem_alloc(tmem_slot, TcuCfg<BN>::TMEM_COLS);
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
@@ -169,9 +176,9 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
             bool ok = true;
             for (int t = args.tile_begin + blockIdx.x; t < args.tile_end && ok; t += gridDim.x) {
                 int tm, tn;
-                tcu_tile_coords(args, t, tm, tn);
-                const int m0 = tm * TCU_BM, n0 = tn * TCU_BN;
-                const int kbt = tcu_tile_kblocks(args, kblocks, n0), total_kb = kbt * args.nterms;
+                tcu_tile_coords<BN>(args, t, tm, tn);
+                const int m0 = tm * TCU_BM, n0 = tn * BN;
+                const int kbt = tcu_tile_kblocks<BN>(args, kblocks, n0), total_kb = kbt * args.nterms;
                 for (int kb = 0; kb < total_kb; ++kb) {
                     if (!ptx::wait_parity(&empty[stage], phase ^ 1, abort_flag, args.wait_budget_ns)) {
                         ok = false;
@@ -217,8 +224,8 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
     } else if (warp == 1) {
         // ------------------------------------------------------- MMA issuer
         if (ptx::elect_one()) {
-            const uint32_t idesc = args.f16s ? ptx::make_idesc(TCU_BM, TCU_BN, ptx::FMT_F16)
-                                             : ptx::make_idesc(TCU_BM, TCU_BN, ptx::FMT_BF16);
+            const uint32_t idesc = args.f16s ? ptx::make_idesc(TCU_BM, BN, ptx::FMT_F16)
+                                             : ptx::make_idesc(TCU_BM, BN, ptx::FMT_BF16);
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -230,10 +237,10 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                     break;
                 }
                 ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * TCU_BN);
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
                 int tm, tn;
-                tcu_tile_coords(args, t, tm, tn);
-                const int total_kb = tcu_tile_kblocks(args, kblocks, tn * TCU_BN) * args.nterms;
+                tcu_tile_coords<BN>(args, t, tm, tn);
+                const int total_kb = tcu_tile_kblocks<BN>(args, kblocks, tn * BN) * args.nterms;
                 for (int kb = 0; kb < total_kb; ++kb) {
                     if (!ptx::wait_parity(&full[stage], phase, abort_flag, args.wait_budget_ns)) {
                         ok = false;
@@ -280,30 +287,30 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
         bool ok = true;
         for (int t = args.tile_begin + blockIdx.x; t < args.tile_end; t += gridDim.x) {
             int tm, tn;
-            tcu_tile_coords(args, t, tm, tn);
+            tcu_tile_coords<BN>(args, t, tm, tn);
             const int row = tm * TCU_BM + row_in_tile;
-            const int n0 = tn * TCU_BN;
+            const int n0 = tn * BN;
             if (!ptx::wait_parity(&acc_full[acc], acc_phase, abort_flag, args.wait_budget_ns)) {
                 ok = false;
                 break;
             }
             ptx::tc_fence_after();
-            const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TCU_BN);
+            const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
             float *crow = args.C + row;
             const bool row_ok = row < args.m;
             // scaled FP16: the row's scale (the columns' below)
             const float rsc = (args.f16s && row_ok) ? args.rs_a[row] : 1.0f;
 #pragma unroll 1
-            for (int ch = 0; ch < TCU_BN / 32; ++ch) {
+            for (int ch = 0; ch < BN / 32; ++ch) {
                 uint32_t r[32];
                 ptx::tmem_ld_32x32b_x32(tbase + ch * 32, r);
                 ptx::tmem_ld_wait();
-                if (ch == TCU_BN / 32 - 1) {
+                if (ch == BN / 32 - 1) {
                     ptx::tc_fence_before();
                     ptx::mbar_arrive(&acc_empty[acc]);
                 }
                 const int c0 = n0 + ch * 32;
-                if (row_ok) {
+                if (row_ok && c0 < args.n) {
                     float cv[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
@@ -360,7 +367,7 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    if (warp == 1) ptx::tmem_dealloc(tmem_base, TCU_TMEM_COLS);
+    if (warp == 1) ptx::tmem_dealloc(tmem_base, TcuCfg<BN>::TMEM_COLS);
 }
 
 } // namespace gb300
