@@ -26,7 +26,8 @@
 
 namespace gb300 {
 
-static const int kBuckets = 6;                      // n <= 32, 64, 128, 256, 512, 1024
+static const int kBuckets = BAT_BUCKETS;            // n <= 32, 64, 128, 256, 512, 1024
+static const int kBucketMax[kBuckets] = {32, 64, 128, 256, 512, 1024};
 static signed char g_nb_table[kBuckets] = {16, 32, 32, 64, 64, 64};
 static double g_nb_us[kBuckets] = {0, 0, 0, 0, 0, 0};
 static bool g_nb_tuned = false;
@@ -35,8 +36,6 @@ static DenseTuning g_dense[kDense];
 static int g_ndense = 0;
 static bool g_table_loaded = false;
 static std::mutex g_table_mu;
-
-static size_t smem_bytes() { return (size_t)(64 * 65 + 2 * 64 * BAT_TP) * sizeof(float); }
 
 // the existing table file, else where a new one is written
 static void tuning_path(char *path, size_t len)
@@ -91,11 +90,10 @@ static int write_table_locked()
     snprintf(tmp, sizeof tmp, "%s.tmp", path);
     FILE *f = fopen(tmp, "w");
     if (!f) return GB300_EINVAL;
-    static const int maxn_of[kBuckets] = {32, 64, 128, 256, 512, 1024};
     if (g_nb_tuned) {
         fprintf(f, "# GB300 batched Cholesky tuning: diagonal/panel block size per size bucket\n");
         fprintf(f, "# bucket max_n nb time_us\n");
-        for (int b = 0; b < kBuckets; ++b) fprintf(f, "%d %d %d %.3f\n", b, maxn_of[b], (int)g_nb_table[b], g_nb_us[b]);
+        for (int b = 0; b < kBuckets; ++b) fprintf(f, "%d %d %d %.3f\n", b, kBucketMax[b], (int)g_nb_table[b], g_nb_us[b]);
     }
     if (g_ndense) {
         fprintf(f, "# GB300 mixed-solve schedule per tile size (lookahead_sms -1: chosen per step by the model)\n");
@@ -136,30 +134,35 @@ int dense_tuning_store(const DenseTuning &d)
     return write_table_locked();
 }
 
-// Persistent grid of the batched kernel on the current device: the SMs times
-// the CTAs resident per SM (the shared memory limit is set per device first).
-static int batched_grid()
+// Resident CTAs of the batched kernel on the current device (the shared
+// memory limit is set per device first): the most a cooperative launch takes.
+template <int NR> static int batched_resident()
 {
-    if (gb300_func_dyn_smem((const void *)batched_dposv_kernel, (int)smem_bytes())) return 0;
+    constexpr int smem = (int)BatSmem<NR>::BYTES;
+    if (gb300_func_dyn_smem((const void *)batched_dposv_kernel<NR>, smem)) return 0;
     int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batched_dposv_kernel, BAT_THREADS, smem_bytes()) !=
-        cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batched_dposv_kernel<NR>, BAT_THREADS, smem) != cudaSuccess) {
         cudaGetLastError();
         per = 1;
     }
     return gb300_device_sms() * std::max(1, per);
 }
 
+static int batched_grid() { return batched_resident<4>(); }
+
 struct BatWs {
-    int *n, *order, *status;
-    long long *a_off, *b_off;
+    BatchedSystem *sys;
+    int *cnt, *status;
+    BatchedState *state;  // followed by `active`: zeroed together
+    unsigned *active;
     double *berr, *R;
-    float *W, *Y;
-    unsigned *ticket;
-    signed char *nb;
+    float *W, *D;
 };
 
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// floats of a system's W
+static long long w_size(int n) { return (long long)bat_ldw(n) * n; }
 
 static size_t bat_layout(int nsys, long long wtotal, long long btotal, void *base, BatWs *ws)
 {
@@ -169,24 +172,22 @@ static size_t bat_layout(int nsys, long long wtotal, long long btotal, void *bas
         off = al(off + b);
         return o;
     };
-    size_t on = take(sizeof(int) * nsys), oo = take(sizeof(int) * nsys), os = take(sizeof(int) * nsys);
-    size_t oa = take(sizeof(long long) * nsys), ob = take(sizeof(long long) * nsys);
-    size_t oe = take(sizeof(double) * nsys), oR = take(sizeof(double) * btotal);
-    size_t oW = take(sizeof(float) * wtotal), oY = take(sizeof(float) * btotal);
-    size_t ot = take(sizeof(unsigned)), onb = take(kBuckets);
+    size_t oy = take(sizeof(BatchedSystem) * nsys), oc = take(sizeof(int) * kBuckets * BAT_CNT);
+    size_t os = take(sizeof(int) * nsys), oe = take(sizeof(double) * nsys);
+    size_t ot = take(sizeof(BatchedState) * nsys), oa = take(3 * sizeof(unsigned));
+    size_t oR = take(sizeof(double) * btotal), oW = take(sizeof(float) * wtotal);
+    size_t oD = take(sizeof(float) * DC_B * DC_B * nsys);
     if (base && ws) {
         char *b = (char *)base;
-        ws->n = (int *)(b + on);
-        ws->order = (int *)(b + oo);
+        ws->sys = (BatchedSystem *)(b + oy);
+        ws->cnt = (int *)(b + oc);
         ws->status = (int *)(b + os);
-        ws->a_off = (long long *)(b + oa);
-        ws->b_off = (long long *)(b + ob);
         ws->berr = (double *)(b + oe);
+        ws->state = (BatchedState *)(b + ot);
+        ws->active = (unsigned *)(b + oa);
         ws->R = (double *)(b + oR);
         ws->W = (float *)(b + oW);
-        ws->Y = (float *)(b + oY);
-        ws->ticket = (unsigned *)(b + ot);
-        ws->nb = (signed char *)(b + onb);
+        ws->D = (float *)(b + oD);
     }
     return off;
 }
@@ -195,11 +196,42 @@ static void totals(int nsys, const int *n, int nrhs, long long *wt, long long *b
 {
     long long w = 0, b = 0;
     for (int i = 0; i < nsys; ++i) {
-        w += (long long)n[i] * n[i];
+        w += w_size(n[i]);
         b += (long long)n[i] * nrhs;
     }
     *wt = w;
     *bt = b;
+}
+
+// The most tasks a phase has (it bounds the grid: a small batch is not made
+// to wait at barriers of the whole GPU).
+static long long widest_phase(const BatchedArgs &a, const std::vector<int> &cnt)
+{
+    auto count = [&](int b, int v) { return v >= BAT_MAXN ? 0 : cnt[b * BAT_CNT + v / BAT_GRAIN]; };
+    long long rows = 0, most = a.nsys;
+    for (int b = 0; b < kBuckets; ++b)
+        for (int v = 0; v < BAT_MAXN; v += 64) rows += count(b, v);
+    most = std::max(most, rows);
+    for (int k = 0; k < a.steps; ++k) {
+        long long upd = 0;
+        for (int b = 0; b < kBuckets; ++b) {
+            upd += count(b, k * a.nb[b]);
+            for (int i = 0; i < BAT_MAXN / 64; ++i) upd += (i + 1LL) * count(b, (k + 1) * a.nb[b] + 64 * i);
+        }
+        most = std::max(most, upd);
+    }
+    return most;
+}
+
+template <int NR> static int launch_batched(cudaStream_t s, BatchedArgs &a, long long tasks)
+{
+    const int resident = batched_resident<NR>();
+    if (resident <= 0) return GB300_ECUDA;  // the attribute set-up failed; its message is recorded
+    void *args[] = {&a};
+    gb300_count_launch();
+    return gb300_record_cuda_error(cudaLaunchCooperativeKernel((const void *)batched_dposv_kernel<NR>,
+                                                               dim3((unsigned)std::min<long long>(tasks, resident)),
+                                                               dim3(BAT_THREADS), args, BatSmem<NR>::BYTES, s));
 }
 
 // Launch over systems whose metadata is in host arrays; synchronous.
@@ -213,41 +245,50 @@ static int run_batched(cudaStream_t s, int nsys, const int *n, const double *A, 
     if (lwork < bat_layout(nsys, wt, bt, nullptr, nullptr)) return GB300_EINVAL;
     BatWs ws;
     bat_layout(nsys, wt, bt, work, &ws);
-    // W / Y / R reuse the caller's offsets, which index A / B (elements)
     std::vector<int> order(nsys);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return n[x] > n[y]; });
-    std::vector<long long> aoff(a_off, a_off + nsys), boff(b_off, b_off + nsys);
-    int rc;
-    if ((rc = gb300_record_cuda_error(cudaMemcpyAsync(ws.n, n, sizeof(int) * nsys, cudaMemcpyHostToDevice, s)))) return rc;
-    cudaMemcpyAsync(ws.order, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(ws.a_off, aoff.data(), sizeof(long long) * nsys, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(ws.b_off, boff.data(), sizeof(long long) * nsys, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(ws.nb, nb_table, kBuckets, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(ws.ticket, 0, sizeof(unsigned), s);
+    std::vector<BatchedSystem> sys(nsys);
+    std::vector<int> cnt(kBuckets * BAT_CNT, 0);
     BatchedArgs a;
+    a.steps = 0;
+    for (int b = 0; b < kBuckets; ++b) a.first[b] = nsys, a.nb[b] = nb_table[b];
+    long long wo = 0, ro = 0;
+    for (int p = 0; p < nsys; ++p) {
+        const int i = order[p];
+        int b = 0;
+        while (n[i] > kBucketMax[b]) ++b;
+        sys[p] = {n[i], i, a_off[i], b_off[i], wo, ro};
+        wo += w_size(n[i]);
+        ro += (long long)n[i] * nrhs;
+        a.first[b] = std::min(a.first[b], p);
+        a.steps = std::max(a.steps, (n[i] + a.nb[b] - 1) / a.nb[b]);
+        ++cnt[b * BAT_CNT + (n[i] - 1) / BAT_GRAIN];  // counts n > 16 v for every v up to here
+    }
+    for (int b = 0; b < kBuckets; ++b)
+        for (int v = BAT_CNT - 2; v >= 0; --v) cnt[b * BAT_CNT + v] += cnt[b * BAT_CNT + v + 1];
+    int rc;
+    if ((rc = gb300_record_cuda_error(
+             cudaMemcpyAsync(ws.sys, sys.data(), sizeof(BatchedSystem) * nsys, cudaMemcpyHostToDevice, s))))
+        return rc;
+    cudaMemcpyAsync(ws.cnt, cnt.data(), sizeof(int) * cnt.size(), cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(ws.state, 0, (char *)(ws.active + 3) - (char *)ws.state, s);
     a.nsys = nsys;
-    a.n = ws.n;
-    a.a_off = ws.a_off;
-    a.b_off = ws.b_off;
-    a.order = ws.order;
-    a.smem_bytes = smem_bytes();
+    a.nrhs = nrhs;
+    a.max_iter = max_iter;
+    a.tol = tol;
+    a.sys = ws.sys;
+    a.state = ws.state;
+    a.cnt = ws.cnt;
     a.A = A;
     a.B = B;
     a.X = X;
     a.W = ws.W;
-    a.Y = ws.Y;
+    a.D = ws.D;
     a.R = ws.R;
-    a.nrhs = nrhs;
-    a.tol = tol;
-    a.max_iter = max_iter;
     a.status = ws.status;
     a.berr = ws.berr;
-    a.ticket = ws.ticket;
-    a.nb_of_bucket = ws.nb;
-    const int bgrid = batched_grid();
-    if (bgrid <= 0) return GB300_ECUDA;  // the attribute set-up failed; its message is recorded
-    const int grid = std::min(nsys, bgrid);
+    a.active = ws.active;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (kernel_ms) {
         cudaEventCreate(&e0);
@@ -255,15 +296,18 @@ static int run_batched(cudaStream_t s, int nsys, const int *n, const double *A, 
         cudaEventRecord(e0, s);
     }
     int slot = gb300_prof_begin(s, GB300_PROF_BATCHED);
-    gb300_count_launch(), batched_dposv_kernel<<<grid, BAT_THREADS, smem_bytes(), s>>>(a);
+    const long long tasks = widest_phase(a, cnt);
+    rc = nrhs <= 4 ? launch_batched<4>(s, a, tasks) : launch_batched<8>(s, a, tasks);
     double fl = 0;
     for (int i = 0; i < nsys; ++i) fl += (double)n[i] * n[i] * n[i] / 3.0 + 2.0 * (double)n[i] * n[i] * nrhs;
     gb300_prof_end(s, slot, fl, 8.0 * (double)wt);
     if (kernel_ms) cudaEventRecord(e1, s);
-    if ((rc = gb300_last_launch_status())) return rc;
-    if (status) cudaMemcpyAsync(status, ws.status, sizeof(int) * nsys, cudaMemcpyDeviceToHost, s);
-    if (berr) cudaMemcpyAsync(berr, ws.berr, sizeof(double) * nsys, cudaMemcpyDeviceToHost, s);
-    rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
+    if (!rc) rc = gb300_last_launch_status();
+    if (!rc) {
+        if (status) cudaMemcpyAsync(status, ws.status, sizeof(int) * nsys, cudaMemcpyDeviceToHost, s);
+        if (berr) cudaMemcpyAsync(berr, ws.berr, sizeof(double) * nsys, cudaMemcpyDeviceToHost, s);
+        rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
+    }
     if (kernel_ms) {
         cudaEventElapsedTime(kernel_ms, e0, e1);
         cudaEventDestroy(e0);
@@ -334,12 +378,11 @@ int starpu_gb300_batched_autotune(int systems_per_bucket, int reps)
     if (reps <= 0) reps = 2;
     cudaStream_t s = nullptr;
     const int nrhs = 4;
-    const int maxn_of[kBuckets] = {32, 64, 128, 256, 512, 1024};
     const int cands[3] = {16, 32, 64};
     signed char best_nb[kBuckets];
     double best_us[kBuckets];
     for (int b = 0; b < kBuckets; ++b) {
-        const int n = maxn_of[b] * 3 / 4;  // a size inside the bucket
+        const int n = kBucketMax[b] * 3 / 4;  // a size inside the bucket
         const int nsys = b >= 4 ? std::max(1, systems_per_bucket / (b == 5 ? 4 : 2)) : systems_per_bucket;
         std::vector<int> ns(nsys, n);
         std::vector<long long> ao(nsys), bo(nsys);
@@ -362,7 +405,7 @@ int starpu_gb300_batched_autotune(int systems_per_bucket, int reps)
         best_us[b] = INFINITY;
         best_nb[b] = g_nb_table[b];
         for (int c = 0; c < 3; ++c) {
-            if (cands[c] > 2 * maxn_of[b]) continue;
+            if (cands[c] > 2 * kBucketMax[b]) continue;
             signed char table[kBuckets];
             memcpy(table, g_nb_table, kBuckets);
             table[b] = (signed char)cands[c];

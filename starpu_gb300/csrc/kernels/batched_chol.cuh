@@ -1,544 +1,549 @@
-// Persistent batched SPD solve: one launch factors and solves many
-// independent systems of different sizes (n <= 1024), FP32 blocked Cholesky
-// + FP64 iterative refinement, one CTA per system at a time.
+// Persistent batched SPD solve: one cooperative launch factors and solves
+// many independent systems of different sizes (n <= 1024), FP32 blocked
+// Cholesky + FP64 iterative refinement.
 //
-// Work distribution: systems are visited in the order given by `order`
-// (largest first); each CTA takes the next system with an atomic ticket, so
-// big systems start early and the small ones fill the tail.  A CTA runs the
-// whole pipeline for its system with a fixed sequence of operations, so a
-// system's result does not depend on which other systems share the launch.
+// All systems go through the same phases together, a grid barrier between
+// two phases, so that a large system's work is spread over the GPU instead of
+// being one CTA's latency (a system of order 1024 took 17 ms alone in its CTA,
+// the time of a whole batch of 1024 systems):
+//   convert   W = fp32(lower A), row sums of |A|; task = 64 rows of a system
+//   step k    panel: the NB columns from k NB on; task = 64 rows below the
+//             diagonal block, which every task factors for itself together
+//             with its rows (chol_panel.cuh); the factored block goes to a
+//             scratch tile, since others still read the unfactored one
+//             update: W_ij -= L_i L_j^T; task = 64 x 64 tile of the trailing
+//             triangle (or the scratch tile's copy to W)
+//   round r   solve: task = one system in one CTA: backward error of the last
+//             solution, x += L^-T L^-1 r in shared memory
+//             residual: r = b - A x; task = 64 rows of a system
+// Systems are sorted by order, largest first, in size buckets with a block
+// width NB each (16, 32 or 64, the tuned parameter); a phase's tasks are found
+// from the number of systems of a bucket larger than a given order.  Every
+// task is a fixed sequence of operations on its system's data, so a system's
+// result does not depend on which other systems share the launch.
 //
-// Per system (256 threads, FP32 work copy W of the lower triangle):
-//   W = fp32(A), ||A||_inf                        (A FP64, column-major, ld = n)
-//   right-looking blocked Cholesky with block NB (the tuned parameter):
-//     POTRF of the NB x NB diagonal block in shared memory
-//     TRSM of the panel rows, one row per thread, registers
-//     lower-triangular trailing update in 64 x 64 tiles staged in shared memory,
-//       on the tensor cores (warp-level TF32 MMAs on split operands)
-//   x = fp64(L^-T L^-1 fp32(b)); repeat r = b - A x, berr, x += corr.
-//   The residual runs in double-float arithmetic on the FP32 pipe (A split
-//   per element, X split once per residual into shared memory, FP64 flush
-//   every 128 terms; ~2^-47 relative per block), GB300 issuing FP64 FMAs at
-//   ~1/60 of its FP32 rate; with more right-hand sides than the shared
-//   memory holds it runs in FP64.
+// The residual runs in double-float arithmetic on the FP32 pipe (A split per
+// element, X split once per task into shared memory, FP64 flush every 128
+// terms; ~2^-47 relative per block): the FP64 pipe is 64 times slower.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chol_panel.cuh"
 #include "df_arith.cuh"
+#include "tile64.cuh"
 
 namespace gb300 {
 
 constexpr int BAT_THREADS = 256;
 constexpr int BAT_MAXN = 1024;
 constexpr int BAT_MAXRHS = 8;
-constexpr int BAT_TILE = 64;
-constexpr int BAT_TP = 72;  // pitch of a staged panel slice row (64 + 8): conflict-free MMA fragment loads
+constexpr int BAT_BUCKETS = 6;            // n <= 32, 64, 128, 256, 512, 1024
+constexpr int BAT_GRAIN = 16;             // cnt is kept for every multiple of this order
+constexpr int BAT_CNT = BAT_MAXN / BAT_GRAIN + 1;
 
-struct BatchedArgs {
-    int nsys;
-    const int *n;                 // [nsys]
-    const long long *a_off;       // offset (doubles) of system i in A / (floats) in W
-    const long long *b_off;       // offset (doubles) of system i in B and X
-    const int *order;             // visiting order (largest first)
-    const double *A;
-    const double *B;
-    double *X;
-    float *W;                     // FP32 work copies (same offsets as A)
-    float *Y;                     // FP32 rhs/corrections (same offsets as B)
-    double *R;                    // FP64 residuals (same offsets as B)
-    int nrhs;
-    double tol;
-    int max_iter;
-    int *status;                  // [nsys] iterations (>= 0) or -(info) / -1000 not converged
-    double *berr;                 // [nsys] final max backward error
-    unsigned *ticket;
-    const signed char *nb_of_bucket;  // block size per size bucket (log2 of ceil(n/32))
-    size_t smem_bytes;                // dynamic shared memory of the launch
+// W's leading dimension: columns start 16-byte aligned
+__host__ __device__ __forceinline__ int bat_ldw(int n) { return (n + 3) & ~3; }
+
+struct BatchedSystem {
+    int n, index;              // order, position in the caller's arrays
+    long long a_off, b_off;    // the caller's offsets (elements of A; of B and X)
+    long long w_off, r_off;    // W (floats, n columns of bat_ldw(n)) and R (doubles)
 };
 
-__device__ __forceinline__ int bucket_of(int n)
+// Per-system state, by sorted position.
+struct BatchedState {
+    unsigned long long anorm;               // ||A||_inf as FP64 bits
+    unsigned long long rmax[BAT_MAXRHS];    // max |r| of the last residual, FP64 bits
+    double xmax[BAT_MAXRHS], bmax[BAT_MAXRHS];
+    int info, done;
+};
+
+struct BatchedArgs {
+    int nsys, nrhs, max_iter, steps;
+    double tol;
+    const BatchedSystem *sys;   // [nsys] largest first
+    BatchedState *state;        // [nsys], zeroed
+    const int *cnt;             // [BAT_BUCKETS][BAT_CNT]: systems of the bucket with n > 16 v
+    int first[BAT_BUCKETS];     // sorted position of the bucket's first system
+    int nb[BAT_BUCKETS];        // block width
+    const double *A, *B;
+    double *X;
+    float *W;
+    float *D;                   // [nsys] 64 x 64 scratch tiles
+    double *R;
+    int *status;                // [nsys] by caller's index: corrections (>= 0), -(info), -1000 not converged
+    double *berr;               // [nsys] final max backward error
+    unsigned *active;           // [3] systems still iterating, in turn; zeroed
+};
+
+// Task t of a phase as (system, i, j); t is reduced by the tasks passed over.
+struct BatTask {
+    int pos, i, j, k0, nb;
+};
+
+__device__ __forceinline__ int bat_count(const int *cnt, int b, int v)
 {
-    int b = 0;
-    int t = (n + 31) / 32;
-    while ((1 << b) < t) ++b;
-    return b > 5 ? 5 : b;  // 32, 64, 128, 256, 512, 1024
+    return v >= BAT_MAXN ? 0 : cnt[b * BAT_CNT + v / BAT_GRAIN];
 }
 
-// TF32 split of x: hi = tf32(x) (round to nearest), lo = tf32(x - hi)
-__device__ __forceinline__ void bat_split_tf32(float x, uint32_t &hi, uint32_t &lo)
+// 64-row blocks of every system: i-th block of the systems with n > 64 i
+__device__ __forceinline__ bool bat_find_rows(const BatchedArgs &a, const int *cnt, int t, BatTask &o)
 {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    const float r = x - __uint_as_float(hi);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+    for (int b = BAT_BUCKETS - 1; b >= 0; --b)
+        for (int i = 0;; ++i) {
+            const int c = bat_count(cnt, b, 64 * i);
+            if (c == 0) break;
+            if (t < c) {
+                o.pos = a.first[b] + t;
+                o.i = i;
+                return true;
+            }
+            t -= c;
+        }
+    return false;
 }
 
-// d += a b for one 16 x 8 x 8 TF32 tile (warp-wide, FP32 accumulation)
-__device__ __forceinline__ void bat_mma_tf32(float d[4], const uint32_t a[4], const uint32_t b[2])
+// panel of step k: i = 0 the diagonal block alone, i > 0 with the i-th 64 rows below it
+__device__ __forceinline__ bool bat_find_panel(const BatchedArgs &a, const int *cnt, int k, int t, BatTask &o)
 {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-                 "{%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// ----------------------------------------------------------------- factor
-template <int NB>
-__device__ int bat_factor(float *W, int n, float *smem)
-{
-    float(*D)[NB + 1] = reinterpret_cast<float(*)[NB + 1]>(smem);   // diagonal block
-    float *As = smem + NB * (NB + 1);                                  // [NB][BAT_TP] panel slice (k-major)
-    float *Bs = As + NB * BAT_TP;                                      // [NB][BAT_TP]
-    __shared__ int s_info;
-    const int tid = threadIdx.x;
-    if (tid == 0) s_info = 0;
-    __syncthreads();
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        const int kb = min(NB, n - k0);
-        // ---- POTRF of the diagonal block
-        for (int idx = tid; idx < NB * NB; idx += BAT_THREADS) {
-            const int i = idx % NB, j = idx / NB;
-            D[i][j] = (i < kb && j < kb && i >= j) ? W[(k0 + i) + (long)(k0 + j) * n] : 0.0f;
-        }
-        __syncthreads();
-        constexpr int CL = BAT_THREADS / NB;  // column lanes for the rank-1 update
-        const int ti = tid % NB, tc = tid / NB;
-        for (int z = 0; z < kb; ++z) {
-            if (tid == 0) {
-                const float d = D[z][z];
-                if (!(d > 0.0f) && s_info == 0) s_info = k0 + z + 1;
-                D[z][z] = sqrtf(d);
+    for (int b = BAT_BUCKETS - 1; b >= 0; --b) {
+        const int nb = a.nb[b], k0 = k * nb;
+        for (int i = 0;; ++i) {
+            const int c = bat_count(cnt, b, i == 0 ? k0 : k0 + nb + 64 * (i - 1));
+            if (c == 0) break;
+            if (t < c) {
+                o.pos = a.first[b] + t;
+                o.i = i;
+                o.k0 = k0;
+                o.nb = nb;
+                return true;
             }
-            __syncthreads();
-            const float inv = 1.0f / D[z][z];
-            if (tc == 0 && ti > z && ti < kb) D[ti][z] *= inv;
-            __syncthreads();
-            if (ti > z && ti < kb) {
-                const float liz = D[ti][z];
-                for (int c = z + 1 + tc; c <= ti; c += CL) D[ti][c] = fmaf(-liz, D[c][z], D[ti][c]);
-            }
-            __syncthreads();
-        }
-        for (int idx = tid; idx < kb * kb; idx += BAT_THREADS) {
-            const int i = idx % kb, j = idx / kb;
-            if (i >= j) W[(k0 + i) + (long)(k0 + j) * n] = D[i][j];
-        }
-        if (s_info) break;
-        const int r0 = k0 + kb, m = n - r0;
-        if (m <= 0) break;
-        // ---- TRSM: W[i, k0:k0+kb] <- W[i, k0:k0+kb] L_kk^-T, one row per thread
-        for (int i = r0 + tid; i < n; i += BAT_THREADS) {
-            float x[NB];
-#pragma unroll
-            for (int c = 0; c < NB; ++c) x[c] = (c < kb) ? W[i + (long)(k0 + c) * n] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (j < kb) {
-                    x[j] = x[j] / D[j][j];
-#pragma unroll
-                    for (int c = j + 1; c < NB; ++c) x[c] = fmaf(-D[c][j], x[j], x[c]);
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < NB; ++c)
-                if (c < kb) W[i + (long)(k0 + c) * n] = x[c];
-        }
-        __syncthreads();
-        // ---- trailing update of the lower triangle, 64 x 64 tiles, on the
-        // tensor cores: warp-level m16n8k8 TF32 MMAs, three per tile on the
-        // split x = hi + lo of both operands (about 21 significant bits, the
-        // FP32 factor's working accuracy; the refinement recovers FP64).
-        // Warp w owns rows 16 (w % 4) .. + 15 and columns 32 (w / 4) .. + 31
-        // of the tile (four n8 fragments); K = the block width, padded to 8
-        // with zeros.
-        const int nt = (m + BAT_TILE - 1) / BAT_TILE;
-        const int kp = (kb + 7) & ~7;
-        const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-        const int wr = 16 * (warp & 3), wc = 32 * (warp >> 2);
-        for (int tj = 0; tj < nt; ++tj) {
-            // stage the panel rows of tile column tj once per column
-#pragma unroll 4
-            for (int idx = tid; idx < kp * BAT_TILE; idx += BAT_THREADS) {
-                const int rr = idx % BAT_TILE, p = idx / BAT_TILE;
-                const int row = r0 + tj * BAT_TILE + rr;
-                Bs[p * BAT_TP + rr] = (p < kb && row < n) ? W[row + (long)(k0 + p) * n] : 0.0f;
-            }
-            for (int ti2 = tj; ti2 < nt; ++ti2) {
-#pragma unroll 4
-                for (int idx = tid; idx < kp * BAT_TILE; idx += BAT_THREADS) {
-                    const int rr = idx % BAT_TILE, p = idx / BAT_TILE;
-                    const int row = r0 + ti2 * BAT_TILE + rr;
-                    As[p * BAT_TP + rr] = (p < kb && row < n) ? W[row + (long)(k0 + p) * n] : 0.0f;
-                }
-                __syncthreads();
-                // this thread's 16 elements of the tile, loaded before the products
-                float cv[4][4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int col = r0 + tj * BAT_TILE + wc + 8 * j + 2 * t4 + (q & 1);
-                        const int row = r0 + ti2 * BAT_TILE + wr + g + 8 * (q >> 1);
-                        cv[j][q] = (col < n && row < n && row >= col) ? W[row + (long)col * n] : 0.0f;
-                    }
-                float acc[4][4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[j][q] = 0.0f;
-                for (int p = 0; p < kp; p += 8) {
-                    uint32_t ah[4], al[4];
-                    bat_split_tf32(As[(p + t4) * BAT_TP + wr + g], ah[0], al[0]);
-                    bat_split_tf32(As[(p + t4) * BAT_TP + wr + g + 8], ah[1], al[1]);
-                    bat_split_tf32(As[(p + t4 + 4) * BAT_TP + wr + g], ah[2], al[2]);
-                    bat_split_tf32(As[(p + t4 + 4) * BAT_TP + wr + g + 8], ah[3], al[3]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint32_t bh[2], bl[2];
-                        bat_split_tf32(Bs[(p + t4) * BAT_TP + wc + 8 * j + g], bh[0], bl[0]);
-                        bat_split_tf32(Bs[(p + t4 + 4) * BAT_TP + wc + 8 * j + g], bh[1], bl[1]);
-                        bat_mma_tf32(acc[j], al, bh);  // the small terms first
-                        bat_mma_tf32(acc[j], ah, bl);
-                        bat_mma_tf32(acc[j], ah, bh);
-                    }
-                }
-                // fragment element q of n-tile j: row wr + g + 8 (q / 2), column wc + 8 j + 2 t4 + q % 2
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int col = r0 + tj * BAT_TILE + wc + 8 * j + 2 * t4 + (q & 1);
-                        const int row = r0 + ti2 * BAT_TILE + wr + g + 8 * (q >> 1);
-                        if (col < n && row < n && row >= col) W[row + (long)col * n] = cv[j][q] - acc[j][q];
-                    }
-                __syncthreads();
-            }
+            t -= c;
         }
     }
-    __syncthreads();
-    return s_info;
+    return false;
 }
 
-// --------------------------------------------------------------- solves
-// Mirror the factor into the upper triangle of W (W[j, i] = L[i, j]) so that
-// both sweeps below read contiguous columns.
-__device__ void bat_mirror_upper(float *W, int n, float *smem)
+// update of step k: i = -1 the diagonal block's copy, else tile (i, j) of the trailing triangle
+__device__ __forceinline__ bool bat_find_update(const BatchedArgs &a, const int *cnt, int k, int t, BatTask &o)
 {
-    // 32 x 32 tiles below the diagonal, transposed through shared memory so
-    // that both the reads (down the columns of L) and the writes (down the
-    // columns of the upper part) are coalesced; 8 warps, one tile row each
-    float(*T)[33] = reinterpret_cast<float(*)[33]>(smem) + (threadIdx.x >> 5) * 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = (n + 31) / 32;
-    for (int t = warp; t < nt * (nt + 1) / 2; t += BAT_THREADS / 32) {
-        int ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-        while (ti * (ti + 1) / 2 > t) --ti;
-        while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-        const int tj = t - ti * (ti + 1) / 2;  // tile (ti, tj), tj <= ti
-        const int r0 = 32 * ti, c0 = 32 * tj;
-        for (int c = 0; c < 32; ++c)
-            T[c][lane] = (r0 + lane < n && c0 + c < n) ? W[r0 + lane + (long)(c0 + c) * n] : 0.0f;
-        __syncwarp();
-        // W(c0 + lane, r0 + r) = L(r0 + r, c0 + lane) for c0 + lane < r0 + r
-        for (int r = 0; r < 32; ++r)
-            if (r0 + r < n && c0 + lane < n && c0 + lane < r0 + r) W[c0 + lane + (long)(r0 + r) * n] = T[lane][r];
-        __syncwarp();
+    for (int b = BAT_BUCKETS - 1; b >= 0; --b) {
+        const int nb = a.nb[b], k0 = k * nb;
+        for (int i = -1;; ++i) {
+            const int c = bat_count(cnt, b, i < 0 ? k0 : k0 + nb + 64 * i), tiles = i < 0 ? 1 : i + 1;
+            if (c == 0) break;
+            if (t < c * tiles) {
+                o.pos = a.first[b] + t % c;
+                o.i = i;
+                o.j = t / c;
+                o.k0 = k0;
+                o.nb = nb;
+                return true;
+            }
+            t -= c * tiles;
+        }
     }
-    __syncthreads();
+    return false;
 }
 
-// Y (n x nrhs, ld n) <- L^-T L^-1 Y, in blocks of 32 columns.  Per block,
-// the 32 x 32 diagonal block is staged in shared memory (coalesced) and warp
-// 0 solves it (lane = row, the solved entry broadcast by shuffles) into
-// shared memory; then every thread updates its rows outside the block with
-// the block's 32 columns of L (forward) or of L^T (backward, read from the
-// mirrored upper triangle), all 32 loads of a row in flight at once.  Each
-// row sees its updates in the same column order as a column-by-column
-// substitution.
-__device__ void bat_potrs(const float *W, int n, float *Y, int nrhs, float *smem)
+__device__ __forceinline__ double bat_warp_max(double m)
 {
-    const int tid = threadIdx.x, lane = tid & 31;
-    float(*D)[33] = reinterpret_cast<float(*)[33]>(smem);  // D[c][r] = block (r, c)
-    float *ys = smem + 32 * 33;                             // ys[j * BAT_MAXRHS + c]: the solved block
-    for (int pass = 0; pass < 2; ++pass) {
-        const bool fwd = pass == 0;
-        const int nblk = (n + 31) / 32;
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
+
+// shared memory of a CTA: the widest phase's
+template <int NR> struct BatSmem {
+    static constexpr size_t TILES = 2 * DC_B * DC_LD * sizeof(float);
+    static constexpr size_t PAN = sizeof(CpPanel<float, 2>);
+    // solve: right-hand sides, diagonal block, its inverse pivots, the block's rows
+    static constexpr size_t SOLVE = ((size_t)NR * BAT_MAXN + CP_W * CP_LP + CP_W + 8 * CP_LP) * sizeof(float);
+    // residual: X split, partial sums
+    static constexpr size_t RES = (size_t)NR * BAT_MAXN * sizeof(float2) + 4 * 64 * NR * sizeof(double);
+    static constexpr size_t M1 = TILES > PAN ? TILES : PAN, M2 = SOLVE > RES ? SOLVE : RES;
+    static constexpr size_t BYTES = M1 > M2 ? M1 : M2;
+};
+
+// df_split_scaled for the usual exponents without branches
+__device__ __forceinline__ float2 bat_split(double a, int ea)
+{
+    const uint32_t whi = (uint32_t)__double2hiint(a), wlo = (uint32_t)__double2loint(a);
+    const int fe = (int)((whi >> 20) & 0x7FF) - (896 + ea);  // biased FP32 exponent of a 2^-ea
+    if ((unsigned)(fe - 53) >= 202u) return df_split_scaled(a, ea);
+    const uint32_t sign = whi & 0x80000000u;
+    const float r = __uint2float_rn(wlo & 0x1FFFFFFFu);  // the 29 bits below the high part's 24
+    return make_float2(__uint_as_float(sign | ((uint32_t)fe << 23) | (__funnelshift_l(wlo, whi, 3) & 0x7FFFFFu)),
+                       __uint_as_float(sign | __float_as_uint(__fmul_rn(r, __uint_as_float((uint32_t)(fe - 52) << 23)))));
+}
+
+// ---- convert: 64 rows of one system.  The row sums run in double-float
+// relative to the largest diagonal element (FP64 additions and conversions,
+// one each per element, took 530 us for 1024 systems: the FP64 pipe's time).
+__device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
+{
+    const BatchedSystem s = a.sys[t.pos];
+    const int n = s.n, ldw = bat_ldw(n), row = 64 * t.i + (threadIdx.x & 63), cg = threadIdx.x >> 6;
+    const double *A0 = a.A + s.a_off, *A = A0 + row;
+    float *W = a.W + s.w_off + row;
+    unsigned dm = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) dm = max(dm, (unsigned)__double2hiint(A0[(long)i * (n + 1)]) & 0x7FFFFFFFu);
+    dm = __reduce_max_sync(0xffffffffu, dm);
+    const int ex = (int)(dm >> 20), ea = ex == 0 || ex == 0x7FF ? 0 : ex - 1023;
+    const bool plain = ea < -100 || ea > 100;  // 2^ea leaves FP32's range: convert element by element
+    const float back = plain ? 0.0f : __int_as_float((ea + 127) << 23);
+    float sh = 0.0f, sl = 0.0f;
+    if (row < n)
+        for (int c0 = cg; c0 < n; c0 += 64) {
+            double v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) v[u] = c0 + 4 * u < n ? A[(long)(c0 + 4 * u) * n] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                const float2 p = bat_split(v[u], ea);
+                const float h = fabsf(p.x), l = fabsf(p.y), q = __fadd_rn(sh, h), z = __fsub_rn(q, sh);
+                sl = __fadd_rn(sl, __fadd_rn(l, __fadd_rn(__fsub_rn(sh, __fsub_rn(q, z)), __fsub_rn(h, z))));
+                sh = q;
+                if (c0 + 4 * u <= row) W[(long)(c0 + 4 * u) * ldw] = plain ? (float)v[u] : __fmul_rn(__fadd_rn(p.x, p.y), back);
+            }
+        }
+    __syncthreads();
+    red[threadIdx.x] = ldexp((double)sh + (double)sl, ea);
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        double m = (red[threadIdx.x] + red[64 + threadIdx.x]) + (red[128 + threadIdx.x] + red[192 + threadIdx.x]);
+        m = bat_warp_max(m);
+        if ((threadIdx.x & 31) == 0) atomicMax(&a.state[t.pos].anorm, (unsigned long long)__double_as_longlong(m));
+    }
+}
+
+// ---- panel: diagonal block and (i > 0) 64 rows below it
+__device__ void bat_panel(const BatchedArgs &a, const BatTask &t, CpPanel<float, 2> &pan, uint64_t (&bar)[16], uint32_t phase)
+{
+    const BatchedSystem s = a.sys[t.pos];
+    const int n = s.n, ld = bat_ldw(n), bk = min(t.nb, n - t.k0), r0 = t.k0 + t.nb + 64 * (t.i - 1), rows = t.i > 0 ? min(64, n - r0) : 0;
+    float *W = a.W + s.w_off;
+    const float *Dg = W + t.k0 + (long)t.k0 * ld;
+    float *P = W + r0 + (long)t.k0 * ld;
+    CpBlock<float> d, x;
+    cp_each<float>(d, [&](float &v, int r, int c) {
+        v = (r < bk && c <= r) ? __ldcg(Dg + r + (long)c * ld) : (r == c ? 1.0f : 0.0f);
+    });
+    cp_each<float>(x, [&](float &v, int r, int c) { v = (r < rows && c < bk) ? __ldcg(P + r + (long)c * ld) : 0.0f; });
+    __syncthreads();  // pan of the previous task is free
+    if (!cp_panel<float, 2>(d, x, pan, bar, phase, bk, &a.state[t.pos].info, t.k0, t.i == 0))
+        atomicCAS(&a.state[t.pos].info, 0, BAT_MAXN + 1);  // a wait ran out: the system is reported as failed
+    if (t.i > 0) {
+        cp_each<float>(x, [&](float &v, int r, int c) {
+            if (r < rows && c < bk) P[r + (long)c * ld] = v;
+        });
+    } else {
+        float *D = a.D + (long)t.pos * (DC_B * DC_B);
+        cp_each<float>(d, [&](float &v, int r, int c) { D[r + DC_B * c] = v; });
+    }
+}
+
+// ---- update: one 64 x 64 tile of the trailing triangle, or the diagonal block's copy
+__device__ void bat_update(const BatchedArgs &a, const BatTask &t, float *s0, float *s1)
+{
+    const BatchedSystem s = a.sys[t.pos];
+    const int n = s.n, ld = bat_ldw(n), bk = min(t.nb, n - t.k0);
+    float *W = a.W + s.w_off;
+    if (t.i < 0) {
+        const float *D = a.D + (long)t.pos * (DC_B * DC_B);
+        for (int e = threadIdx.x; e < DC_B * DC_B; e += BAT_THREADS) {
+            const int r = e & 63, c = e >> 6;
+            if (r < bk && c <= r) W[(t.k0 + r) + (long)(t.k0 + c) * ld] = __ldcg(D + e);
+        }
+        return;
+    }
+    const int r0 = t.k0 + t.nb, i0 = r0 + 64 * t.i, j0 = r0 + 64 * t.j, ri = min(64, n - i0), rj = min(64, n - j0);
+    const bool lower = t.i == t.j, whole = dc_whole(ri, rj, lower, true);
+    float *C = W + i0 + (long)j0 * ld;
+    const float *P = W + (long)t.k0 * ld;
+    DcTile li, lj;
+    float c[4][4];
+    li.load(P + i0, ld, ri, bk, true);
+    lj.load(P + j0, ld, rj, bk, true);
+    dc_sub_load(C, ld, ri, rj, lower, whole, c);
+    __syncthreads();  // the previous task's operands are free
+    li.store(s0);
+    lj.store(s1);
+    __syncthreads();
+    float acc[4][4] = {};
+    dc_mma(s0, s1, acc, (bk + 7) & ~7);
+    dc_sub_store(C, ld, ri, rj, lower, whole, c, acc);
+}
+
+// ---- solve: Y <- L^-T L^-1 Y in shared memory (ys[c * n + i]), 64 rows at a time
+template <int NR> __device__ void bat_potrs(const float *W, int n, int ld, float *ys, float *Ls, float *inv, float *S)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nblk = (n + CP_W - 1) / CP_W;
+    for (int e = tid; e < 8 * CP_LP; e += BAT_THREADS) S[e] = 0.0f;
+    for (int pass = 0; pass < 2; ++pass)
         for (int bb = 0; bb < nblk; ++bb) {
-            const int j0 = fwd ? 32 * bb : 32 * (nblk - 1 - bb), jb = min(32, n - j0);
-            // stage the diagonal block (forward: L, backward: the mirrored U = L^T)
-            for (int e = tid; e < 32 * 32; e += BAT_THREADS) {
-                const int r = e & 31, c = e >> 5;
-                D[c][r] = (r < jb && c < jb) ? W[j0 + r + (long)(j0 + c) * n] : 0.0f;
+            const bool fwd = pass == 0;
+            const int j0 = CP_W * (fwd ? bb : nblk - 1 - bb), w = min(CP_W, n - j0);
+            // the diagonal block (backward: reversed, so that the same forward
+            // substitution solves with its transpose)
+            float l[16], d = 1.0f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int r = tid & 63, c = 4 * i + (tid >> 6);
+                l[i] = (r < w && c < r) ? W[(j0 + r) + (long)(j0 + c) * ld] : 0.0f;
             }
-            __syncthreads();
-            if (tid < 32) {
-                float y[BAT_MAXRHS];
+            if (tid < w) d = W[(j0 + tid) * (long)(ld + 1)];
+            float dot[8][NR];
+            if (!fwd) {
+                // sums of the rows below over the block's columns, 8 columns per warp
 #pragma unroll
-                for (int c = 0; c < BAT_MAXRHS; ++c)
-                    y[c] = (c < nrhs && lane < jb) ? Y[j0 + lane + (long)c * n] : 0.0f;
-                for (int q = 0; q < jb; ++q) {
-                    const int j = fwd ? q : jb - 1 - q;
-                    const float l = D[j][lane];  // (lane, j) of the block
-                    if (lane == j) {
+                for (int u = 0; u < 8; ++u)
 #pragma unroll
-                        for (int c = 0; c < BAT_MAXRHS; ++c) y[c] /= l;
-                    }
+                    for (int c = 0; c < NR; ++c) dot[u][c] = 0.0f;
+                const float *Wc = W + (long)(j0 + 8 * warp) * ld;
+                for (int r = j0 + CP_W + lane; r < n; r += 128) {
+                    float v[4][8];  // 32 loads in flight
 #pragma unroll
-                    for (int c = 0; c < BAT_MAXRHS; ++c) {
-                        const float yj = __shfl_sync(0xffffffffu, y[c], j);
-                        if (fwd ? lane > j : lane < j) y[c] = fmaf(-l, yj, y[c]);
-                    }
-                }
-                if (lane < jb) {
+                    for (int k = 0; k < 4; ++k)
 #pragma unroll
-                    for (int c = 0; c < BAT_MAXRHS; ++c) {
-                        ys[lane * BAT_MAXRHS + c] = y[c];
-                        if (c < nrhs) Y[j0 + lane + (long)c * n] = y[c];
-                    }
-                }
-            }
-            __syncthreads();
-            // rows outside the block: below it (forward) or above it (backward)
-            const int i_lo = fwd ? j0 + jb : 0, i_hi = fwd ? n : j0;
-            for (int i = i_lo + tid; i < i_hi; i += BAT_THREADS) {
-                float l[32];
+                        for (int u = 0; u < 8; ++u) v[k][u] = r + 32 * k < n ? Wc[r + 32 * k + (long)u * ld] : 0.0f;
 #pragma unroll
-                for (int q = 0; q < 32; ++q) l[q] = q < jb ? W[i + (long)(j0 + q) * n] : 0.0f;
-                float y[BAT_MAXRHS];
+                    for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int c = 0; c < BAT_MAXRHS; ++c) y[c] = c < nrhs ? Y[i + (long)c * n] : 0.0f;
+                        for (int c = 0; c < NR; ++c) {
+                            const float y = r + 32 * k < n ? ys[c * n + r + 32 * k] : 0.0f;
 #pragma unroll
-                for (int q = 0; q < 32; ++q) {
-                    const int j = fwd ? q : 31 - q;
-                    if (j < jb) {
-#pragma unroll
-                        for (int c = 0; c < BAT_MAXRHS; ++c) y[c] = fmaf(-l[j], ys[j * BAT_MAXRHS + c], y[c]);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < BAT_MAXRHS; ++c)
-                    if (c < nrhs) Y[i + (long)c * n] = y[c];
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// R = B - A X (n x nrhs) in double-float arithmetic on the FP32 pipe: A
-// scaled by 2^-ea (ea = exponent of ||A||_inf, an upper bound of |a_ij|) and
-// split per element by bit operations, each column of X scaled by 2^-ex_c
-// and split once into shared memory (Xs[k nrhs + c]); per row (one thread)
-// and right-hand side an error-free running sum, flushed to FP64 every 128
-// terms, in a fixed order (deterministic).
-__device__ void bat_residual_df(const double *A, int n, const double *X, const double *B, double *R, int nrhs,
-                                double anorm, float *smem)
-{
-    __shared__ int s_ex[BAT_MAXRHS];
-    __shared__ double s_xm[BAT_THREADS / 32];
-    const int tid = threadIdx.x;
-    float2 *Xs = reinterpret_cast<float2 *>(smem);
-    for (int c = 0; c < nrhs; ++c) {
-        double m = 0.0;
-        for (int k = tid; k < n; k += BAT_THREADS) m = fmax(m, fabs(X[k + (long)c * n]));
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((tid & 31) == 0) s_xm[tid >> 5] = m;
-        __syncthreads();
-        if (tid == 0) {
-            for (int w = 1; w < BAT_THREADS / 32; ++w) m = fmax(m, s_xm[w]);
-            s_ex[c] = df_scale_exp(m);
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < n * nrhs; e += BAT_THREADS) {
-        const int k = e / nrhs, c = e - k * nrhs;
-        Xs[e] = df_split_scaled(X[k + (long)c * n], s_ex[c]);
-    }
-    __syncthreads();
-    const int ea = df_scale_exp(anorm);
-    for (int i = tid; i < n; i += BAT_THREADS) {
-        double acc[BAT_MAXRHS];
-        float sh[BAT_MAXRHS], sl[BAT_MAXRHS];
-#pragma unroll
-        for (int c = 0; c < BAT_MAXRHS; ++c) {
-            acc[c] = c < nrhs ? B[i + (long)c * n] : 0.0;
-            sh[c] = 0.0f;
-            sl[c] = 0.0f;
-        }
-        for (int j0 = 0; j0 < n; j0 += 128) {
-            const int j1 = min(n, j0 + 128);
-            for (int j = j0; j < j1; j += 8) {
-                // eight loads of the row in flight before their products
-                double av8[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) av8[u] = j + u < j1 ? A[i + (long)(j + u) * n] : 0.0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (j + u >= j1) break;
-                    const float2 av = df_split_scaled(av8[u], ea);
-#pragma unroll
-                    for (int c = 0; c < BAT_MAXRHS; ++c)
-                        if (c < nrhs) {
-                            const float2 xv = Xs[(j + u) * nrhs + c];
-                            df_mac(sh[c], sl[c], av.x, av.y, xv.x, xv.y);
+                            for (int u = 0; u < 8; ++u) dot[u][c] = fmaf(v[k][u], y, dot[u][c]);
                         }
                 }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+#pragma unroll
+                    for (int c = 0; c < NR; ++c)
+                        for (int o = 16; o > 0; o >>= 1) dot[u][c] += __shfl_xor_sync(0xffffffffu, dot[u][c], o);
             }
+            __syncthreads();  // the first block: ys and S are filled
 #pragma unroll
-            for (int c = 0; c < BAT_MAXRHS; ++c)
-                if (c < nrhs) {
-                    acc[c] -= ldexp((double)sh[c] + (double)sl[c], ea + s_ex[c]);
-                    sh[c] = 0.0f;
-                    sl[c] = 0.0f;
+            for (int i = 0; i < 16; ++i) {
+                const int r = tid & 63, c = 4 * i + (tid >> 6);
+                if (fwd) Ls[c * CP_LP + r] = l[i];
+                else if (r < w && c < w) Ls[(w - 1 - r) * CP_LP + (w - 1 - c)] = l[i];
+            }
+            if (tid < CP_W) inv[fwd || tid >= w ? tid : w - 1 - tid] = 1.0f / d;
+            if (fwd) {
+                for (int e = tid; e < NR * CP_W; e += BAT_THREADS) {
+                    const int c = e / CP_W, i = e % CP_W;
+                    S[c * CP_LP + i] = i < w ? ys[c * n + j0 + i] : 0.0f;
                 }
-        }
+            } else {
 #pragma unroll
-        for (int c = 0; c < BAT_MAXRHS; ++c)
-            if (c < nrhs) R[i + (long)c * n] = acc[c];
-    }
-    __syncthreads();
+                for (int u = 0; u < 8; ++u)
+#pragma unroll
+                    for (int c = 0; c < NR; ++c)
+                        if (lane == (u * NR + c) % 32) {
+                            const int i = 8 * warp + u;
+                            if (i < w) S[c * CP_LP + w - 1 - i] = ys[c * n + j0 + i] - dot[u][c];
+                            else S[c * CP_LP + i] = 0.0f;
+                        }
+                // past w the reversed block continues as the identity
+                if (w < CP_W)
+                    for (int e = tid; e < CP_W * CP_W; e += BAT_THREADS) {
+                        const int r = e & 63, c = e >> 6;
+                        if (r >= w || c >= w) Ls[c * CP_LP + r] = 0.0f;
+                    }
+            }
+            __syncthreads();
+            if (tid < 16 * 8) cp_slab_solve<8>(S, Ls, inv);
+            __syncthreads();
+            for (int e = tid; e < NR * CP_W; e += BAT_THREADS) {
+                const int c = e / CP_W, i = e % CP_W;
+                if (i < w) ys[c * n + j0 + i] = S[c * CP_LP + (fwd ? i : w - 1 - i)];
+            }
+            if (fwd)
+                for (int i = j0 + CP_W + tid; i < n; i += BAT_THREADS) {
+                    float acc[NR], v[CP_W];  // a row's 64 loads in flight
+                    const float *Wi = W + i + (long)j0 * ld;
+#pragma unroll
+                    for (int q = 0; q < CP_W; ++q) v[q] = Wi[(long)q * ld];
+#pragma unroll
+                    for (int c = 0; c < NR; ++c) acc[c] = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < CP_W; q += 4)
+#pragma unroll
+                        for (int c = 0; c < NR; ++c) {
+                            const Quad<float> y = *reinterpret_cast<const Quad<float> *>(S + c * CP_LP + q);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) acc[c] = fmaf(v[q + u], y.v[u], acc[c]);
+                        }
+#pragma unroll
+                    for (int c = 0; c < NR; ++c) ys[c * n + i] -= acc[c];
+                }
+            __syncthreads();
+        }
 }
 
-// -------------------------------------------------------------- kernel
-__global__ void __launch_bounds__(BAT_THREADS, 2) batched_dposv_kernel(BatchedArgs a)
+// One round of one system: the backward error of its solution (after the
+// first round), then the next correction.
+template <int NR> __device__ void bat_round(const BatchedArgs &a, int pos, int round, float *smem, double *red)
 {
-    extern __shared__ __align__(16) float bat_smem[];
-    __shared__ unsigned s_sys;
-    __shared__ double s_red[4][BAT_THREADS / 32];
-    __shared__ double s_anorm;
-    __shared__ int s_done;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_sys = atomicAdd(a.ticket, 1u);
-        __syncthreads();
-        const unsigned t = s_sys;
-        __syncthreads();
-        if (t >= (unsigned)a.nsys) return;
-        const int sys = a.order[t];
-        const int n = a.n[sys];
-        const double *A = a.A + a.a_off[sys];
-        float *W = a.W + a.a_off[sys];
-        const double *B = a.B + a.b_off[sys];
-        double *X = a.X + a.b_off[sys];
-        float *Y = a.Y + a.b_off[sys];
-        double *R = a.R + a.b_off[sys];
-        const int nrhs = a.nrhs;
-        // W = fp32(lower A); row sums of |A| -> ||A||_inf
-        double rowmax = 0.0;
-        for (int i = tid; i < n; i += BAT_THREADS) {
-            double s = 0.0;
-            for (int j = 0; j < n; j += 8) {
-                double v8[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v8[u] = j + u < n ? A[i + (long)(j + u) * n] : 0.0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    s += fabs(v8[u]);
-                    if (j + u < n && i >= j + u) W[i + (long)(j + u) * n] = (float)v8[u];
-                }
-            }
-            rowmax = fmax(rowmax, s);
-        }
-        for (int o = 16; o > 0; o >>= 1) rowmax = fmax(rowmax, __shfl_xor_sync(0xffffffffu, rowmax, o));
-        if ((tid & 31) == 0) s_red[0][tid >> 5] = rowmax;
-        __syncthreads();
+    const BatchedSystem s = a.sys[pos];
+    BatchedState &st = a.state[pos];
+    const int n = s.n, nrhs = a.nrhs, tid = threadIdx.x;
+    if (__ldcg(&st.done)) return;
+    const int info = round == 0 ? __ldcg(&st.info) : 0;
+    if (info) {
         if (tid == 0) {
-            double m = 0;
-            for (int w = 0; w < BAT_THREADS / 32; ++w) m = fmax(m, s_red[0][w]);
-            s_anorm = m;
+            a.status[s.index] = info > BAT_MAXN ? -1000 : -info;
+            a.berr[s.index] = INFINITY;
+            st.done = 1;
         }
-        __syncthreads();
-        const int nb = a.nb_of_bucket[bucket_of(n)];
-        int info;
-        if (nb == 16) info = bat_factor<16>(W, n, bat_smem);
-        else if (nb == 32) info = bat_factor<32>(W, n, bat_smem);
-        else info = bat_factor<64>(W, n, bat_smem);
-        if (info) {
+        return;
+    }
+    if (round > 0) {
+        const double anorm = __longlong_as_double((long long)__ldcg(&st.anorm));
+        double worst = 0.0;
+        for (int c = 0; c < nrhs; ++c) {
+            const double rm = __longlong_as_double((long long)__ldcg(&st.rmax[c])), den = anorm * __ldcg(&st.xmax[c]) + __ldcg(&st.bmax[c]);
+            worst = fmax(worst, den > 0 ? rm / den : (rm > 0 ? INFINITY : 0.0));
+        }
+        if (worst <= a.tol || round > a.max_iter) {
+            __syncthreads();  // every thread has read done
             if (tid == 0) {
-                a.status[sys] = -info;
-                a.berr[sys] = INFINITY;
+                a.status[s.index] = worst <= a.tol ? round - 1 : -1000;
+                a.berr[s.index] = worst;
+                st.done = 1;
             }
-            __syncthreads();
-            continue;
+            return;
         }
-        bat_mirror_upper(W, n, bat_smem);
-        // initial solve
-        for (int idx = tid; idx < n * nrhs; idx += BAT_THREADS) Y[idx] = (float)B[idx];
-        __syncthreads();
-        bat_potrs(W, n, Y, nrhs, bat_smem);
-        for (int idx = tid; idx < n * nrhs; idx += BAT_THREADS) X[idx] = (double)Y[idx];
-        __syncthreads();
-        int it = 0;
-        double worst = INFINITY;
-        // the double-float residual's X split fits the shared memory
-        const bool df = (size_t)n * nrhs * sizeof(float2) <= a.smem_bytes;
-        for (;; ++it) {
-            if (df) {
-                bat_residual_df(A, n, X, B, R, nrhs, s_anorm, bat_smem);
-            } else
-            // R = B - A X, columns of A streamed, one row per thread (coalesced)
-            for (int i = tid; i < n; i += BAT_THREADS) {
-                double acc[BAT_MAXRHS];
-#pragma unroll
-                for (int c = 0; c < BAT_MAXRHS; ++c) acc[c] = (c < nrhs) ? B[i + (long)c * n] : 0.0;
-                for (int j = 0; j < n; ++j) {
-                    const double av = A[i + (long)j * n];
-#pragma unroll
-                    for (int c = 0; c < BAT_MAXRHS; ++c)
-                        if (c < nrhs) acc[c] = fma(-av, X[j + (long)c * n], acc[c]);
-                }
-#pragma unroll
-                for (int c = 0; c < BAT_MAXRHS; ++c)
-                    if (c < nrhs) R[i + (long)c * n] = acc[c];
-            }
-            __syncthreads();
-            // backward error per right-hand side, max over them
-            double w = 0.0;
-            for (int c = 0; c < nrhs; ++c) {
-                double rm = 0, xm = 0, bm = 0;
-                for (int i = tid; i < n; i += BAT_THREADS) {
-                    rm = fmax(rm, fabs(R[i + (long)c * n]));
-                    xm = fmax(xm, fabs(X[i + (long)c * n]));
-                    bm = fmax(bm, fabs(B[i + (long)c * n]));
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    rm = fmax(rm, __shfl_xor_sync(0xffffffffu, rm, o));
-                    xm = fmax(xm, __shfl_xor_sync(0xffffffffu, xm, o));
-                    bm = fmax(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-                }
-                if ((tid & 31) == 0) {
-                    s_red[0][tid >> 5] = rm;
-                    s_red[1][tid >> 5] = xm;
-                    s_red[2][tid >> 5] = bm;
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    for (int q = 1; q < BAT_THREADS / 32; ++q) {
-                        rm = fmax(rm, s_red[0][q]);
-                        xm = fmax(xm, s_red[1][q]);
-                        bm = fmax(bm, s_red[2][q]);
-                    }
-                    const double den = s_anorm * xm + bm;
-                    const double e = den > 0 ? rm / den : (rm > 0 ? INFINITY : 0.0);
-                    s_red[3][0] = fmax(c == 0 ? 0.0 : s_red[3][0], e);
-                }
-                __syncthreads();
-            }
-            w = s_red[3][0];
-            worst = w;
-            if (tid == 0) s_done = (w <= a.tol) || it >= a.max_iter;
-            __syncthreads();
-            if (s_done) break;
-            __syncthreads();
-            for (int idx = tid; idx < n * nrhs; idx += BAT_THREADS) Y[idx] = (float)R[idx];
-            __syncthreads();
-            bat_potrs(W, n, Y, nrhs, bat_smem);
-            for (int idx = tid; idx < n * nrhs; idx += BAT_THREADS) X[idx] += (double)Y[idx];
-            __syncthreads();
+    }
+    float *ys = smem, *Ls = ys + NR * BAT_MAXN, *inv = Ls + CP_W * CP_LP, *S = inv + CP_W;
+    const double *B = a.B + s.b_off, *R = a.R + s.r_off;
+    double *X = a.X + s.b_off;
+    __syncthreads();  // shared memory of the previous task is free
+    for (int e = tid; e < NR * n; e += BAT_THREADS)
+        ys[e] = e < nrhs * n ? (float)(round == 0 ? B[e] : __ldcg(R + e)) : 0.0f;
+    bat_potrs<NR>(a.W + s.w_off, n, bat_ldw(n), ys, Ls, inv, S);
+    for (int c = 0; c < nrhs; ++c) {
+        double xm = 0.0, bm = 0.0;
+        for (int i = tid; i < n; i += BAT_THREADS) {
+            const int e = c * n + i;
+            const double x = (round == 0 ? 0.0 : X[e]) + (double)ys[e];
+            X[e] = x;
+            xm = fmax(xm, fabs(x));
+            if (round == 0) bm = fmax(bm, fabs(B[e]));
         }
+        xm = bat_warp_max(xm);
+        bm = bat_warp_max(bm);
+        __syncthreads();
+        if ((tid & 31) == 0) red[tid >> 5] = xm, red[8 + (tid >> 5)] = bm;
+        __syncthreads();
         if (tid == 0) {
-            a.status[sys] = (worst <= a.tol) ? it : -1000;
-            a.berr[sys] = worst;
+            for (int w = 1; w < BAT_THREADS / 32; ++w) xm = fmax(xm, red[w]), bm = fmax(bm, red[8 + w]);
+            st.xmax[c] = xm;
+            if (round == 0) st.bmax[c] = bm;
+            st.rmax[c] = 0;
         }
-        __syncthreads();
+    }
+    if (tid == 0) atomicAdd(&a.active[round % 3], 1u);
+}
+
+// ---- residual: 64 rows of R = B - A X in double-float arithmetic on the
+// FP32 pipe (A scaled by the exponent of ||A||_inf and split per element by bit
+// operations, each column of X scaled by its own exponent), thread = row and
+// every fourth column, the four sums added in a fixed order.
+template <int NR> __device__ void bat_residual(const BatchedArgs &a, const BatTask &t, float *smem)
+{
+    const BatchedSystem s = a.sys[t.pos];
+    BatchedState &st = a.state[t.pos];
+    if (__ldcg(&st.done)) return;
+    const int n = s.n, nrhs = a.nrhs, tid = threadIdx.x;
+    float2 *Xs = reinterpret_cast<float2 *>(smem);                       // [n][NR]
+    double *part = reinterpret_cast<double *>(Xs + (size_t)NR * BAT_MAXN);  // [4][NR][64]
+    const double *X = a.X + s.b_off, *B = a.B + s.b_off;
+    int ex[NR];
+#pragma unroll
+    for (int c = 0; c < NR; ++c) ex[c] = c < nrhs ? df_scale_exp(__ldcg(&st.xmax[c])) : 0;
+    const int ea = df_scale_exp(__longlong_as_double((long long)__ldcg(&st.anorm)));
+    __syncthreads();  // shared memory of the previous task is free
+#pragma unroll
+    for (int c = 0; c < NR; ++c)
+        for (int k = tid; k < n; k += BAT_THREADS)
+            Xs[k * NR + c] = c < nrhs ? df_split_scaled(__ldcg(X + (long)c * n + k), ex[c]) : make_float2(0.0f, 0.0f);
+    __syncthreads();
+    const int row = 64 * t.i + (tid & 63), kg = tid >> 6;
+    const double *Ai = a.A + s.a_off + min(row, n - 1);
+    double acc[NR];
+#pragma unroll
+    for (int c = 0; c < NR; ++c) acc[c] = 0.0;
+    for (int j0 = kg; j0 < n; j0 += 512) {  // 128 terms of this thread
+        float sh[NR], sl[NR];
+#pragma unroll
+        for (int c = 0; c < NR; ++c) sh[c] = 0.0f, sl[c] = 0.0f;
+        const int j1 = min(n, j0 + 512);
+        for (int j = j0; j < j1; j += 32) {
+            double av[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) av[u] = j + 4 * u < j1 ? Ai[(long)(j + 4 * u) * n] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float2 v = bat_split(av[u], ea);
+                const float2 *x = Xs + min(j + 4 * u, n - 1) * NR;
+#pragma unroll
+                for (int c = 0; c < NR; ++c) df_mac(sh[c], sl[c], v.x, v.y, x[c].x, x[c].y);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NR; ++c) acc[c] += ldexp((double)sh[c] + (double)sl[c], ea + ex[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < NR; ++c) part[(kg * NR + c) * 64 + (tid & 63)] = acc[c];
+    __syncthreads();
+    for (int e = tid; e < 64 * NR; e += BAT_THREADS) {
+        const int c = e >> 6, i = 64 * t.i + (e & 63);
+        double m = 0.0;
+        if (c < nrhs && i < n) {
+            const double *p = part + c * 64 + (e & 63);
+            const double r = B[(long)c * n + i] - ((p[0] + p[64 * NR]) + (p[128 * NR] + p[192 * NR]));
+            a.R[s.r_off + (long)c * n + i] = r;
+            m = fabs(r);
+        }
+        m = bat_warp_max(isnan(m) ? 0.0 : m);  // a warp's elements are of one right-hand side
+        if ((tid & 31) == 0 && c < nrhs) atomicMax(&st.rmax[c], (unsigned long long)__double_as_longlong(m));
+    }
+}
+
+template <int NR> __global__ void __launch_bounds__(BAT_THREADS, 2) batched_dposv_kernel(const BatchedArgs a)
+{
+    extern __shared__ __align__(16) unsigned char bat_smem[];
+    __shared__ int cnt[BAT_BUCKETS * BAT_CNT];
+    __shared__ uint64_t bar[16];
+    __shared__ double red[BAT_THREADS];
+    float *smem = (float *)bat_smem;
+    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    for (int e = threadIdx.x; e < BAT_BUCKETS * BAT_CNT; e += BAT_THREADS) cnt[e] = a.cnt[e];
+    cp_panel_init(bar);
+    __syncthreads();
+    BatTask t;
+    for (int q = blockIdx.x; bat_find_rows(a, cnt, q, t); q += gridDim.x) bat_convert(a, t, red);
+    grid.sync();
+    uint32_t panels = 0;
+    for (int k = 0; k < a.steps; ++k) {
+        for (int q = blockIdx.x; bat_find_panel(a, cnt, k, q, t); q += gridDim.x)
+            bat_panel(a, t, *(CpPanel<float, 2> *)bat_smem, bar, panels++ & 1);
+        grid.sync();
+        for (int q = blockIdx.x; bat_find_update(a, cnt, k, q, t); q += gridDim.x)
+            bat_update(a, t, smem, smem + DC_B * DC_LD);
+        grid.sync();
+    }
+    for (int round = 0;; ++round) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.active[(round + 1) % 3] = 0;  // counted in the next round
+        for (int q = blockIdx.x; q < a.nsys; q += gridDim.x) bat_round<NR>(a, q, round, smem, red);
+        grid.sync();
+        if (__ldcg(&a.active[round % 3]) == 0) break;
+        for (int q = blockIdx.x; bat_find_rows(a, cnt, q, t); q += gridDim.x) bat_residual<NR>(a, t, smem);
+        grid.sync();
     }
 }
 

@@ -93,12 +93,15 @@ template <typename T, typename F> __device__ __forceinline__ void cp_each(CpBloc
             for (int h = 0; h < 2; ++h) f(v[g][c][h], 32 * h + lane, 32 * g + 4 * warp + c);
 }
 
-// the published columns of step s (bounded: the publisher never waits for this warp)
+// the published columns of step s; bounded (a step takes well below a
+// microsecond, and the publisher never waits for this warp)
 __device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity)
 {
-    for (int i = 0; i < (1 << 22); ++i)
-        if (ptx::mbar_try_wait(bar, parity)) return true;
-    return false;
+    if (ptx::mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = ptx::globaltimer();
+    while (!ptx::mbar_try_wait(bar, parity))
+        if (ptx::globaltimer() - t0 > 20000000ull) return false;  // 20 ms
+    return true;
 }
 
 // rank-4 update of the column groups G .. LAST by a published step
@@ -247,7 +250,10 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         ok = cp_wait(&bar[w - 1], phase) && ok;
         cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
     }
+    // (every mbarrier completes in every panel, so that all keep one parity)
     if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w]));
+    else ptx::mbar_arrive(&bar[w]);
+    if (8 + w >= steps) ptx::mbar_arrive(&bar[8 + w]);
     __syncwarp();
     if (steps <= 8) return ok;
     if (w > 0) cp_update<T, NX, 1, 1>(d, x, pan[w - 1]);

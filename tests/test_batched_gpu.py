@@ -152,3 +152,27 @@ def test_dense_autotuner_stores_the_schedule_beside_the_perfmodels(gpu, tmp_path
     dense = [r for r in rows if r[0] == "dense"]
     assert len(dense) == 1 and int(dense[0][1]) == 1024 and int(dense[0][2]) == out["la"]
     assert len([r for r in rows if r[0] != "dense"]) == 6  # the batched lines are kept
+
+
+@pytest.mark.parametrize("nrhs", [1, 4, 5, 8])
+@pytest.mark.parametrize("sizes", [[1], [16, 17, 31, 32, 33], [64, 65, 127, 128, 129], [513, 576, 577, 5, 1023]])
+def test_batched_block_edges(gpu, oracle, sizes, nrhs):
+    systems = [make_system(oracle, n, 500 + n, nrhs) for n in sizes]
+    status, berr, Xs = run_batched(gpu, systems, nrhs)
+    for (A, B), X, st, be in zip(systems, Xs, status, berr):
+        ob, _ = oracle.backward_error(A, X, B)
+        assert st >= 0 and be <= 1e-12 and ob <= 1e-12, (A.shape, st, be, ob)
+
+
+@pytest.mark.parametrize("k", [1, 16, 33, 64, 65, 100, 128])
+def test_batched_first_bad_pivot(gpu, oracle, k):
+    A, B = make_system(oracle, 128, 900)
+    A[k - 1, k - 1] = -5.0
+    status, berr, _ = run_batched(gpu, [(A, B), make_system(oracle, 40, 901)])
+    assert status[0] == -k and np.isinf(berr[0]) and status[1] >= 0
+
+
+def test_batched_iteration_limit(gpu, oracle):
+    systems = [make_system(oracle, n, 910 + n) for n in (60, 200)]
+    status, berr, _ = run_batched(gpu, systems, tol=0.0, max_iter=2)
+    assert np.all(np.asarray(status) == -1000) and np.all(np.asarray(berr) < 1e-12)
