@@ -14,7 +14,7 @@
 
 namespace gb300 {
 
-// smallest trailing matrix whose FP64 update runs on the tensor cores
+// fewest rows of an FP64 product or trailing update that runs on the tensor cores
 constexpr int SLICE_MIN_M = 128;
 // largest FP32 matrix (or diagonal tile) that one cooperative launch factors:
 // 1522 us at n = 4096 against 2417 us in tiles of 256 with a launch per tile,
@@ -23,6 +23,33 @@ constexpr int SLICE_MIN_M = 128;
 constexpr int COOP_MAX_N = 4096;
 
 static inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
+
+// C[m x n] -= A B^T in FP64 on the tensor cores (kernels/slice_update.cuh), A
+// m x k and B n x k with the given element strides.  GEMM: any k, guarded;
+// else k <= 64, for a panel of an SPD matrix.
+template <bool GEMM>
+static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const double *A, long a_rs, long a_ks,
+                         const double *B, long b_rs, long b_ks, double *C, long ldc, int *err)
+{
+    if (m <= 0 || n <= 0 || k <= 0) return;
+    if (gb300_func_dyn_smem((const void *)slice_update_kernel<GEMM>, SU_SMEM)) return;
+    SliceUpdateArgs a;
+    a.A = A, a.a_rs = a_rs, a.a_ks = a_ks, a.B = B, a.b_rs = b_rs, a.b_ks = b_ks;
+    a.C = C, a.ldc = ldc, a.m = m, a.n = n, a.k = k, a.lower = lower ? 1 : 0;
+    a.col_tiles = (n + SU_BN - 1) / SU_BN;
+    a.err = err;
+    a.wait_budget_ns = 2000000000ull;  // 2 s per wait: far above any legitimate stall
+    a.total = 0;
+    for (int rb = 0; rb * SU_BM < m; ++rb)
+        a.total += lower ? std::min(a.col_tiles, (SU_BM / SU_BN) * (rb + 1)) : a.col_tiles;
+    gb300_count_launch(), slice_update_kernel<GEMM>
+        <<<std::min(a.total, gb300_device_sms()), SU_THREADS, SU_SMEM, s>>>(a);
+}
+
+// Elements of C from which an FP64 product (alpha = -1, beta = 1) runs on the
+// tensor cores: 64 columns of A and B take a launch of 8 to 9 us there until the
+// tiles make more than a wave, and m n / 7700 us on the FP64 units.
+constexpr long SLICE_MIN_ELEMENTS = 96 * 1024;
 
 template <typename T, bool TA, bool TB, int BM, int BN, int BK, int TM, int TN>
 static void gemm_launch(cudaStream_t s, bool lower, int m, int n, int k, T alpha, const T *A, long lda, const T *B,
@@ -78,7 +105,10 @@ template <> struct simt_cfg<double> {
     static void run(cudaStream_t s, bool lower, int m, int n, int k, double al, const double *A, long lda,
                     const double *B, long ldb, double be, double *C, long ldc)
     {
-        if (!lower && n <= 16)
+        if (al == -1.0 && be == 1.0 && m >= SLICE_MIN_M && n >= 16 && k >= 16 &&
+            (lower ? (long)m * (m + 1) / 2 : (long)m * n) >= SLICE_MIN_ELEMENTS)
+            slice_update<true>(s, lower, m, n, k, A, TA ? lda : 1, TA ? 1 : lda, B, TB ? 1 : ldb, TB ? ldb : 1, C, ldc, nullptr);
+        else if (!lower && n <= 16)
             gemm_launch<double, TA, TB, 64, 16, 8, 4, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
         else if (gemm_ctas(lower, m, n, 64) >= 4 * 152)
             gemm_launch<double, TA, TB, 64, 64, 8, 4, 4>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
@@ -200,37 +230,6 @@ template <typename T> void trsm_runu(cudaStream_t s, int m, int n, const T *U, l
     trsm_slab<T>(s, {m, n, U, ldu, 1, B, 1, ldb, true});
 }
 
-// C[m x n] -= A B^T in FP64 on the tensor cores (kernels/slice_update.cuh), A
-// m x k and B n x k with the given element strides, k cut into launches of 64.
-static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const double *A, long a_rs, long a_ks,
-                         const double *B, long b_rs, long b_ks, double *C, long ldc, int *err)
-{
-    if (m <= 0 || n <= 0 || k <= 0) return;
-    if (gb300_func_dyn_smem((const void *)slice_update_kernel, SU_SMEM)) return;
-    SliceUpdateArgs a;
-    a.a_rs = a_rs, a.a_ks = a_ks, a.b_rs = b_rs, a.b_ks = b_ks;
-    a.C = C, a.ldc = ldc, a.m = m, a.n = n, a.lower = lower ? 1 : 0;
-    a.row_blocks = (m + SU_BM - 1) / SU_BM;
-    a.col_tiles = (n + SU_BN - 1) / SU_BN;
-    a.err = err;
-    a.wait_budget_ns = 2000000000ull;  // 2 s per wait: far above any legitimate stall
-    const int sms = gb300_device_sms();
-    auto tiles = [&](int rb) { return lower ? std::min(a.col_tiles, (SU_BM / SU_BN) * (rb + 1)) : a.col_tiles; };
-    long total = 0;
-    for (int rb = 0; rb < a.row_blocks; ++rb) total += tiles(rb);
-    // a work item cuts its 128 rows of A once (about the time of a tile):
-    // long items, but four or more per SM to balance them
-    a.seg = (int)std::max(1L, std::min(16L, total / (4L * sms)));
-    a.items = 0;
-    for (int rb = 0; rb < a.row_blocks; ++rb) a.items += (tiles(rb) + a.seg - 1) / a.seg;
-    for (int k0 = 0; k0 < k; k0 += SU_K) {
-        a.A = A + k0 * a_ks;
-        a.B = B + k0 * b_ks;
-        a.k = std::min(SU_K, k - k0);
-        gb300_count_launch(), slice_update_kernel<<<std::min(a.items, sms), SU_THREADS, SU_SMEM, s>>>(a);
-    }
-}
-
 // Trailing update of one step: C (m x m, lower) -= P P^T, P m x k.
 static void trailing_update(cudaStream_t s, int m, int k, const float *P, long ldp, float *C, long ldc, int *)
 {
@@ -239,7 +238,7 @@ static void trailing_update(cudaStream_t s, int m, int k, const float *P, long l
 static void trailing_update(cudaStream_t s, int m, int k, const double *P, long ldp, double *C, long ldc, int *err)
 {
     if (m < SLICE_MIN_M) gemm<double>(s, false, true, true, m, m, k, -1.0, P, ldp, P, ldp, 1.0, C, ldc);
-    else slice_update(s, true, m, m, k, P, 1, ldp, P, 1, ldp, C, ldc, err);
+    else slice_update<false>(s, true, m, m, k, P, 1, ldp, P, 1, ldp, C, ldc, err);
 }
 
 // Right-looking tiled Cholesky with tile nb: POTRF(k), TRSM of the whole
@@ -291,6 +290,15 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
             <<<cdiv(nrhs, CB), 256, sm_blk, s>>>(w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
         const int rest = TRANS ? j0 : n - j0 - w;
         if (rest <= 0) continue;
+        if constexpr (std::is_same<T, double>::value) {
+            // B_rest -= L X (or L^T X) on the tensor cores: 64 columns of L in
+            // 8 to 9 us, against rest nrhs / 8800 us on the FP64 units
+            if (rest >= SLICE_MIN_M && nrhs >= 16 && (long)rest * nrhs >= SLICE_MIN_ELEMENTS) {
+                slice_update<true>(s, false, rest, nrhs, w, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl,
+                             TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, nullptr);
+                continue;
+            }
+        }
         gb300_count_launch(), trsv_upd_kernel<T, CU, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, CU)), 256, sm_upd, s>>>(
             rest, w, nrhs, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl, ldl, B + j0, TRANS ? B : B + j0 + w, ldb);
     }

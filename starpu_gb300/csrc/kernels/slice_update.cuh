@@ -1,5 +1,5 @@
-// FP64 update C[m x n] -= A[m x k] B[n x k]^T (k <= 64, all column-major or
-// strided) on the tensor cores, with at least the accuracy of FP64 FMAs.
+// FP64 update C[m x n] -= A[m x k] B[n x k]^T (all column-major or strided) on
+// the tensor cores, to the accuracy of FP64 FMAs.
 //
 // GB300 has 2 FP64 FMAs per clock and SM but 4096 FP16 ones on its tensor
 // cores.  Row i of an operand is taken as fixed point relative to a power of
@@ -17,23 +17,38 @@
 //
 // For the Schur complements of an SPD matrix this error is bounded like the
 // classical one, by eps sqrt(A_ii A_jj): a row of L never exceeds sqrt(A_ii).
-// A row that holds Inf or NaN gives NaN.
+// A row that holds Inf or NaN gives NaN there.
+//
+// GEMM = false: k <= 64 (the trailing update of a panel), A stays cut over the
+// tiles of a row block.  GEMM = true: any k in chunks of 64, a tile's chunks
+// summed in registers and C rounded once, as an FMA loop does; A is cut again
+// for every tile and chunk.
+//
+// Products of other matrices (GEMM = true) run guarded: FP64's error is bounded by
+// eps sum_k |a_ik| |b_jk|, which may be far below eps max|a_i| max|b_j| (large
+// elements of a_i that meet small ones of b_j).  One more product, of the
+// magnitudes of the leading digits, estimates that sum from below; an element
+// whose estimate is under half of 2^(e_i + e_j) is formed by FP64 FMAs instead.
+// So are zero rows and rows with Inf or NaN.
 //
 // The operands are cut in the kernel, so no workspace is needed.  A CTA (one
 // per SM, persistent) keeps the slices of 128 rows of A in shared memory and
 // goes along the row in tiles of 32 columns:
-//   warps 8-11  read B's 32 x 64 tile (FP64), find the row exponents and
-//               write its 7 slices (128-byte swizzle), double-buffered; per
-//               work item the same for A's 128 rows
-//   warp 12     issues 7 MMAs per 16 k: slice a_t times the slices
-//               b_1 .. b_{8-t} stacked as 32 (8 - t) rows, so that the 7
-//               scales d land side by side in 224 accumulator columns
-//   warps 0-7   read the accumulator (two, in turn) and update C
+//   warps 16-19  read B's 32 x 64 tile (FP64), find the row exponents and
+//                write its 7 slices (128-byte swizzle), double-buffered
+//   warp 20      issues 7 MMAs per 16 k: slice a_t times the slices
+//                b_1 .. b_{8-t} stacked as 32 (8 - t) rows, so that the 7
+//                scales d land side by side in 224 accumulator columns
+//   warps 0-15   cut A's 128 rows when a work item starts (32 rows per four
+//                warps), then read the accumulators (two, in turn) and update
+//                C, 8 columns per warp
 // The exponents live in rings of four: before tile (item) i + 4's are written,
 // the MMAs of tile (item) i + 2 (i + 3) are done, which the epilogue of tile
 // (item) i has let start.
-// Measured bounds per 128 x 32 tile: 1792 clocks of tensor pipe, 2048 of the
-// FP64 pipe (one add per element), the rest close below.
+// Bounds per 128 x 32 tile: 1792 clocks of tensor pipe (2200 measured), 2400 of
+// the FP64 pipe (one add per element), about 2000 of issue slots.  The epilogue
+// takes 16 warps because its chain of integer operations per element is long
+// (with 8 warps a tile took 9000 clocks).
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -46,9 +61,11 @@ namespace gb300 {
 constexpr int SU_BM = 128, SU_BN = 32, SU_K = 64, SU_S = 7;
 constexpr int SU_SLICE_A = SU_BM * SU_K * 2;  // 16 KB: one 128-byte row per matrix row
 constexpr int SU_SLICE_B = SU_BN * SU_K * 2;  // 4 KB
-constexpr int SU_A_BYTES = SU_S * SU_SLICE_A, SU_B_BYTES = SU_S * SU_SLICE_B;
-constexpr int SU_THREADS = 13 * 32, SU_EPI = 8 * 32, SU_CONV = 4 * 32;
-constexpr int SU_SMEM = SU_A_BYTES + 2 * SU_B_BYTES + 1024 /*align*/ + 4096 /*exponents, barriers*/;
+constexpr int SU_ABS = SU_S;  // slice of the leading digits' magnitudes (guarded products)
+constexpr int SU_A_BYTES = (SU_S + 1) * SU_SLICE_A, SU_B_BYTES = (SU_S + 1) * SU_SLICE_B;
+constexpr int SU_EPI = 16 * 32, SU_CONV = 4 * 32, SU_THREADS = SU_EPI + SU_CONV + 32;
+constexpr int SU_MMA_WARP = (SU_EPI + SU_CONV) / 32;
+constexpr int SU_SMEM = SU_A_BYTES + 2 * SU_B_BYTES + 1024 /*align*/ + 8192 /*exponents, barriers*/;
 constexpr uint32_t SU_TMEM_COLS = 512, SU_ACC_STRIDE = 256;
 constexpr int SU_NONFINITE = 1 << 24;  // exponent of a row with Inf or NaN
 constexpr int SU_ERR_TIMEOUT = -1000;  // *err when a wait inside the kernel ran out
@@ -60,33 +77,48 @@ struct SliceUpdateArgs {
     long ldc;
     int m, n, k;
     int lower;     // 1 (m == n): only elements with row >= column
-    int seg;       // column tiles of one work item
-    int row_blocks, col_tiles, items;
+    int col_tiles, total;  // column tiles of a row block, tiles of all row blocks
     int *err;      // may be null
     unsigned long long wait_budget_ns;
 };
 
-// Work items: row blocks from the last (the longest, when lower) to the
-// first, each cut into segments of `seg` column tiles.
+// The column tiles of all row blocks, row block after row block, are cut into
+// equal ranges, one per CTA; a work item is the part of a range inside one row
+// block.  A CTA cuts A once per item, so hardly more than once.
 struct SliceItems {
-    int rb, base;  // row block and the index of its first item
-    __device__ __forceinline__ SliceItems(const SliceUpdateArgs &a) : rb(a.row_blocks - 1), base(0) {}
+    int rb;        // row block of the current item
+    int next, end; // tiles still to do, counted from the current row block's first
     __device__ __forceinline__ static int tiles(const SliceUpdateArgs &a, int rb)
     {
         return a.lower ? min(a.col_tiles, (SU_BM / SU_BN) * (rb + 1)) : a.col_tiles;
     }
-    // item id (ascending over calls) -> row block rb, column tiles [t0, t1)
-    __device__ __forceinline__ void find(const SliceUpdateArgs &a, int id, int &t0, int &t1)
+    __device__ __forceinline__ SliceItems(const SliceUpdateArgs &a)
     {
-        int nt = tiles(a, rb), ns = (nt + a.seg - 1) / a.seg;
-        while (id >= base + ns) {
-            base += ns;
-            --rb;
-            nt = tiles(a, rb);
-            ns = (nt + a.seg - 1) / a.seg;
+        const long lo = (long)a.total * blockIdx.x / gridDim.x, hi = (long)a.total * (blockIdx.x + 1) / gridDim.x;
+        rb = 0;
+        next = (int)lo;
+        end = (int)hi;
+        skip(a);
+    }
+    __device__ __forceinline__ void skip(const SliceUpdateArgs &a)
+    {
+        while (next < end) {
+            const int nt = tiles(a, rb);
+            if (next < nt) break;
+            next -= nt;
+            end -= nt;
+            ++rb;
         }
-        t0 = (id - base) * a.seg;
-        t1 = min(nt, t0 + a.seg);
+    }
+    // the next item: column tiles [t0, t1) of row block rb; false: no more
+    __device__ __forceinline__ bool item(const SliceUpdateArgs &a, int &t0, int &t1)
+    {
+        skip(a);
+        if (next >= end) return false;
+        t0 = next;
+        t1 = min(end, tiles(a, rb));
+        next = t1;
+        return true;
     }
 };
 
@@ -133,12 +165,66 @@ __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, ui
         for (int t = 0; t < SU_S; ++t)
             *reinterpret_cast<uint4 *>(dst + t * slice_bytes + row * 128 + chunk * 16) =
                 make_uint4(d[t][0], d[t][1], d[t][2], d[t][3]);
+        constexpr uint32_t MAG = 0x7FFF7FFFu;
+        *reinterpret_cast<uint4 *>(dst + SU_ABS * slice_bytes + row * 128 + chunk * 16) =
+            make_uint4(d[0][0] & MAG, d[0][1] & MAG, d[0][2] & MAG, d[0][3] & MAG);
     }
 }
 
-// acc 2^(e - 2098) as FP64, rounded to nearest (e: sum of two biased exponents)
-__device__ __forceinline__ double su_to_double(long long acc, int e)
+// one element of A B^T by FP64 FMAs
+__device__ __noinline__ double su_dot(const SliceUpdateArgs &a, int row, int col)
 {
+    const double *p = a.A + row * a.a_rs, *q = a.B + col * a.b_rs;
+    double v = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < a.k; ++k) v = fma(p[k * a.a_ks], q[k * a.b_ks], v);
+    return v;
+}
+
+// Rows row0 .. row0 + 31 of an operand, cut by a group of four warps (member
+// cw holds k = k0 + 16 cw ..): this thread's 16 elements of row row0 + lane.
+__device__ __forceinline__ void su_load(const double *src, long rs, long ks, int row0, int rows, int k0, int k, int cw, double (&v)[16])
+{
+    const int lane = threadIdx.x & 31;
+    k0 += 16 * cw;
+    const double *p = src + (row0 + lane) * rs + k0 * ks;
+    const bool in = row0 + lane < rows;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = in && k0 + i < k ? p[i * ks] : 0.0;
+}
+// their exponents to ex[0 .. 31] and slices to dst; rmax: [2][4][32] of the
+// group, rp alternates; bar: the group's named barrier
+__device__ __forceinline__ void su_convert(const double (&v)[16], int *ex, uint8_t *dst, int slice_bytes, int row, int cw,
+                                           unsigned *rmax, int &rp, int bar)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned mx = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) mx = max(mx, (unsigned)__double2hiint(v[i]) & 0x7FFFFFFFu);
+    unsigned *r = rmax + rp * 128;
+    rp ^= 1;
+    r[cw * 32 + lane] = mx;
+    asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+    const int e = (int)(max(max(r[lane], r[32 + lane]), max(r[64 + lane], r[96 + lane])) >> 20);
+    if (cw == 0) ex[lane] = e == 0x7FF ? SU_NONFINITE : e;
+    su_write_digits(v, e, dst, slice_bytes, row, cw);
+}
+// A bounded wait that all four warps of a group pass or none does (they meet
+// at barriers afterwards); bar: a named barrier for the vote.
+__device__ __forceinline__ bool su_wait_group(uint64_t *mbar, uint32_t parity, volatile int *abort, uint64_t budget_ns, int bar)
+{
+    uint32_t all, mine = ptx::wait_parity(mbar, parity, abort, budget_ns) ? 1 : 0;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(all)
+                 : "r"(mine), "r"(bar)
+                 : "memory");
+    return all != 0;
+}
+
+// acc 2^(e - 2098) as FP64, rounded to nearest (e: sum of two biased exponents)
+__device__ __noinline__ double su_to_double_any(long long acc, int e)
+{
+    if (e >= SU_NONFINITE) return __longlong_as_double(0x7FF8000000000000ll);
     if (acc == 0) return 0.0;
     const unsigned long long mag = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
     const int lz = __clzll((long long)mag);
@@ -156,16 +242,44 @@ __device__ __forceinline__ double su_to_double(long long acc, int e)
     }
     return __longlong_as_double((long long)(bits | sign));
 }
+// the same for the usual case: 32 or more significant bits, a normal result
+__device__ __forceinline__ double su_to_double(long long acc, int e)
+{
+    const uint32_t sgn = (uint32_t)((unsigned long long)acc >> 32) & 0x80000000u;
+    const unsigned long long mag = (unsigned long long)(acc < 0 ? -acc : acc);
+    const uint32_t hi = (uint32_t)(mag >> 32), lo = (uint32_t)mag;
+    const int lz = __clz((int)hi), ex = e - 1012 - lz;
+    if (hi == 0 || (unsigned)(ex - 1) >= 2045u) return su_to_double_any(acc, e);
+    const uint32_t nh = __funnelshift_l(lo, hi, lz), nl = lo << lz;
+    const unsigned long long m = ((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11);
+    const unsigned long long bits = m + ((nl >> 10) & 1u) + ((unsigned long long)(uint32_t)(ex - 1) << 52);
+    return __hiloint2double((int)((uint32_t)(bits >> 32) | sgn), (int)(uint32_t)bits);
+}
 
-__global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const SliceUpdateArgs a)
+// sum_d S_d 2^{8 (7 - d)}, d = 2 .. 8, the last one rounded.  The integers held
+// by floats are taken on the FMA pipe: |S| <= 2^22 (d <= 5) by adding 1.5 2^23,
+// S_8 / 256 by adding 1.5 2^31; S_6 and S_7 may reach 2^22.6 and are converted.
+__device__ __forceinline__ long long su_combine(const uint32_t (&r)[SU_S][4], int j)
+{
+    constexpr int K22 = 0x4B400000, K30 = 0x4F400000;  // the bits of those sums for S = 0
+    auto f = [&](int d) { return __uint_as_float(r[d][j]); };
+    auto raw = [&](int d) { return __float_as_int(f(d) + 12582912.0f); };
+    const int t1 = (int)((unsigned)raw(1) * 256u + (unsigned)raw(2) - (unsigned)K22 * 257u);
+    const int t2 = __float2int_rn(f(4)) * 256 + __float2int_rn(f(5)) + (__float_as_int(f(6) + 3221225472.0f) - K30);
+    const long long lo = (long long)(raw(3) - K22) * 65536 + t2;
+    const long long mid = (long long)t1 * 16777216 + lo;
+    return mid + ((long long)((raw(0) - K22) * 256) << 32);
+}
+
+template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const SliceUpdateArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sA = smem, *sB = smem + SU_A_BYTES;
-    int *ea = (int *)(sB + 2 * SU_B_BYTES);       // [4][128] row exponents of A, by item
-    int *eb = ea + 4 * SU_BM;                     // [4][32] of B, by tile
-    unsigned *rmax = (unsigned *)(eb + 4 * SU_BN);  // [2][4][32]
-    uint64_t *bars = (uint64_t *)(rmax + 2 * 4 * 32);
+    int *ea = (int *)(sB + 2 * SU_B_BYTES);         // [4][128] row exponents of A, by item
+    int *eb = ea + 4 * SU_BM;                       // [4][32] of B, by tile
+    unsigned *rmax = (unsigned *)(eb + 4 * SU_BN);  // [5 groups][2][4][32]
+    uint64_t *bars = (uint64_t *)(rmax + 5 * 2 * 4 * 32);
     uint64_t *b_full = bars, *b_empty = bars + 2, *acc_full = bars + 4, *acc_empty = bars + 6;
     uint64_t *a_full = bars + 8, *a_empty = bars + 9, *drain = bars + 10;
     uint32_t *tmem_slot = (uint32_t *)(bars + 11);
@@ -179,13 +293,13 @@ __global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const Slice
             ptx::mbar_init(&acc_full[i], 1);
             ptx::mbar_init(&acc_empty[i], SU_EPI);
         }
-        ptx::mbar_init(a_full, SU_CONV);
+        ptx::mbar_init(a_full, SU_EPI);
         ptx::mbar_init(a_empty, 1);
         ptx::mbar_init(drain, 1);
         *abort_flag = 0;
         ptx::fence_mbarrier_init();
     }
-    if (warp == 12) {
+    if (warp == SU_MMA_WARP) {
         ptx::tmem_alloc(tmem_slot, SU_TMEM_COLS);
         ptx::tmem_relinquish();
     }
@@ -194,100 +308,61 @@ __global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const Slice
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
+    const int chunks = GEMM ? (a.k + SU_K - 1) / SU_K : 1;
 
-    if (warp >= 8 && warp < 12) {
-        // ------------------------------------------------ operand slices
-        const int cw = warp - 8;
-        int tile = 0, item = 0, rp = 0;
+    if (warp >= SU_EPI / 32 && warp < SU_MMA_WARP) {
+        // ---------------------------------------------------- B's slices
+        const int cw = warp & 3;
+        int tile = 0, rp = 0;  // tile counts accumulators: column tiles times chunks
         SliceItems it(a);
-        // 32 rows starting at row0: exponents to ex[0..31], slices to dst
-        auto load = [&](const double *src, long rs, long ks, int row0, int rows, double (&v)[16]) {
-            const double *p = src + (row0 + lane) * rs + 16 * cw * ks;
-            const bool in = row0 + lane < rows;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = in && 16 * cw + i < a.k ? p[i * ks] : 0.0;
-        };
-        auto convert = [&](const double (&v)[16], int *ex, uint8_t *dst, int slice_bytes, int row) {
-            unsigned mx = 0;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) mx = max(mx, (unsigned)__double2hiint(v[i]) & 0x7FFFFFFFu);
-            unsigned *r = rmax + rp * 128;
-            rp ^= 1;
-            r[cw * 32 + lane] = mx;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            const int e = (int)(max(max(r[lane], r[32 + lane]), max(r[64 + lane], r[96 + lane])) >> 20);
-            if (cw == 0) ex[lane] = e == 0x7FF ? SU_NONFINITE : e;
-            su_write_digits(v, e, dst, slice_bytes, row, cw);
-        };
-        // all four warps go on or none does: they meet at barriers below
-        auto wait_all = [&](uint64_t *bar, uint32_t parity) {
-            uint32_t all, mine = ptx::wait_parity(bar, parity, abort_flag, a.wait_budget_ns) ? 1 : 0;
-            asm volatile(
-                "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, 2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
-                : "=r"(all)
-                : "r"(mine)
-                : "memory");
-            return all != 0;
-        };
-        for (int id = blockIdx.x; id < a.items && ok; id += gridDim.x, ++item) {
-            int t0, t1;
-            it.find(a, id, t0, t1);
+        for (int t0, t1; ok && it.item(a, t0, t1);) {
             double v[16];
-            load(a.A, a.a_rs, a.a_ks, it.rb * SU_BM, a.m, v);
-            if (!(ok = wait_all(a_empty, (item & 1) ^ 1))) break;
-#pragma unroll 1
-            for (int g = 0; g < 4; ++g) {
-                double nx[16];
-                if (g < 3) load(a.A, a.a_rs, a.a_ks, it.rb * SU_BM + 32 * (g + 1), a.m, nx);
-                else load(a.B, a.b_rs, a.b_ks, t0 * SU_BN, a.n, nx);
-                convert(v, ea + (item & 3) * SU_BM + 32 * g, sA, SU_SLICE_A, 32 * g + lane);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = nx[i];
-            }
-            ptx::fence_proxy_async_smem();
-            ptx::mbar_arrive(a_full);
-            for (int t = t0; t < t1; ++t, ++tile) {
+            su_load(a.B, a.b_rs, a.b_ks, t0 * SU_BN, a.n, 0, a.k, cw, v);
+            for (int t = t0, ch = 0; t < t1; ++tile) {
                 const int buf = tile & 1;
-                if (!(ok = wait_all(&b_empty[buf], ((tile >> 1) & 1) ^ 1))) break;
-                double nx[16];
-                if (t + 1 < t1) load(a.B, a.b_rs, a.b_ks, (t + 1) * SU_BN, a.n, nx);
-                convert(v, eb + (tile & 3) * SU_BN, sB + buf * SU_B_BYTES, SU_SLICE_B, lane);
+                if (!(ok = su_wait_group(&b_empty[buf], ((tile >> 1) & 1) ^ 1, abort_flag, a.wait_budget_ns, 1))) break;
+                su_convert(v, eb + (tile & 3) * SU_BN, sB + buf * SU_B_BYTES, SU_SLICE_B, lane, cw, rmax + 4 * 256, rp, 2);
                 ptx::fence_proxy_async_smem();
                 ptx::mbar_arrive(&b_full[buf]);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = nx[i];
+                if (++ch == chunks) ch = 0, ++t;
+                if (t < t1) su_load(a.B, a.b_rs, a.b_ks, t * SU_BN, a.n, ch * SU_K, a.k, cw, v);
             }
         }
-    } else if (warp == 12) {
+    } else if (warp == SU_MMA_WARP) {
         // ---------------------------------------------------- MMA issuer
         if (ptx::elect_one()) {
-            int tile = 0, item = 0;
+            int tile = 0, item = 0;  // item counts the times A was cut
             SliceItems it(a);
-            const int ks = (a.k + 15) / 16;
-            for (int id = blockIdx.x; id < a.items && ok; id += gridDim.x, ++item) {
-                int t0, t1;
-                it.find(a, id, t0, t1);
-                ok = ptx::wait_parity(a_full, item & 1, abort_flag, a.wait_budget_ns);
-                for (int t = t0; t < t1 && ok; ++t, ++tile) {
+            for (int t0, t1; ok && it.item(a, t0, t1);) {
+                if (!GEMM) ok = ptx::wait_parity(a_full, item & 1, abort_flag, a.wait_budget_ns);
+                for (int t = t0, ch = 0; t < t1 && ok; ++tile) {
                     const int buf = tile & 1;
                     const uint32_t par = (tile >> 1) & 1;
-                    ok = ptx::wait_parity(&acc_empty[buf], par ^ 1, abort_flag, a.wait_budget_ns) &&
+                    ok = (!GEMM || ptx::wait_parity(a_full, item & 1, abort_flag, a.wait_budget_ns)) &&
+                         ptx::wait_parity(&acc_empty[buf], par ^ 1, abort_flag, a.wait_budget_ns) &&
                          ptx::wait_parity(&b_full[buf], par, abort_flag, a.wait_budget_ns);
                     if (!ok) break;
                     ptx::tc_fence_after();
                     const uint32_t d = tmem_base + (uint32_t)buf * SU_ACC_STRIDE;
                     const uint32_t aA = ptx::smem_u32(sA), aB = ptx::smem_u32(sB + buf * SU_B_BYTES);
+                    const int ks = (min(SU_K, a.k - ch * SU_K) + 15) / 16;
                     for (int k = 0; k < ks; ++k) {
                         const uint64_t bd = ptx::make_sdesc_k128(aB + k * 32);
 #pragma unroll
                         for (int s = 0; s < SU_S; ++s)
                             ptx::mma_f16_ss(d + s * SU_BN, ptx::make_sdesc_k128(aA + s * SU_SLICE_A + k * 32), bd,
                                             ptx::make_idesc(SU_BM, SU_BN * (SU_S - s), ptx::FMT_F16), (k | s) ? 1u : 0u);
+                        if (GEMM)
+                            ptx::mma_f16_ss(d + SU_ABS * SU_BN, ptx::make_sdesc_k128(aA + SU_ABS * SU_SLICE_A + k * 32),
+                                            ptx::make_sdesc_k128(aB + SU_ABS * SU_SLICE_B + k * 32),
+                                            ptx::make_idesc(SU_BM, SU_BN, ptx::FMT_F16), k ? 1u : 0u);
                     }
                     ptx::mma_commit(&b_empty[buf]);
                     ptx::mma_commit(&acc_full[buf]);
+                    if (GEMM) ptx::mma_commit(a_empty), ++item;
+                    if (++ch == chunks) ch = 0, ++t;
                 }
-                if (ok) ptx::mma_commit(a_empty);
+                if (!GEMM && ok) ptx::mma_commit(a_empty), ++item;
             }
             // every MMA issued has read its operands before the CTA ends
             ptx::mma_commit(drain);
@@ -295,57 +370,84 @@ __global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const Slice
             ptx::wait_parity(drain, 0, &never, a.wait_budget_ns);
         }
     } else {
-        // ------------------------------------------------------ epilogue
-        const int quarter = warp & 3, chalf = warp >> 2;
-        int tile = 0, item = 0;
+        // ------------------------------------------ A's slices, epilogue
+        const int quarter = warp & 3, group = warp >> 2;  // TMEM lanes; 32 rows of A, 8 columns of a tile
+        int tile = 0, item = 0, rp = 0;
         SliceItems it(a);
-        for (int id = blockIdx.x; id < a.items && ok; id += gridDim.x, ++item) {
-            int t0, t1;
-            it.find(a, id, t0, t1);
+        auto cut_a = [&](int k0) {
+            double v[16];
+            su_load(a.A, a.a_rs, a.a_ks, it.rb * SU_BM + 32 * group, a.m, k0, a.k, quarter, v);
+            if (!su_wait_group(a_empty, (item & 1) ^ 1, abort_flag, a.wait_budget_ns, 3 + group)) return false;
+            su_convert(v, ea + (item & 3) * SU_BM + 32 * group, sA, SU_SLICE_A, 32 * group + lane, quarter,
+                       rmax + group * 256, rp, 7 + group);
+            ptx::fence_proxy_async_smem();
+            ptx::mbar_arrive(a_full);
+            return true;
+        };
+        for (int t0, t1; ok && it.item(a, t0, t1); ++item) {
+            if (!GEMM && !(ok = cut_a(0))) break;
             const int rl = quarter * 32 + lane, row = it.rb * SU_BM + rl;
-            for (int t = t0; t < t1 && ok; ++t, ++tile) {
-                const int buf = tile & 1;
-                const uint32_t tb = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * SU_ACC_STRIDE;
-                const int col0 = t * SU_BN + 16 * chalf;
+            for (int t = t0; t < t1 && ok; ++t) {
+                const int col0 = t * SU_BN + 8 * group;
                 double *crow = a.C + row + (long)col0 * a.ldc;
-                auto inside = [&](int j) { return row < a.m && col0 + j < a.n && (!a.lower || row >= col0 + j); };
-                double c[16];
+                // the tile is inside C, on or below the diagonal
+                const bool whole = (it.rb + 1) * SU_BM <= a.m && (t + 1) * SU_BN <= a.n &&
+                                   (!a.lower || it.rb * SU_BM >= (t + 1) * SU_BN - 1);
+                const int jn = whole ? 8 : (row < a.m ? min(8, min(a.n, a.lower ? row + 1 : a.n) - col0) : 0);  // columns of this row
+                double c[8];  // GEMM: the sum over the chunks; else C, read before the wait
 #pragma unroll
-                for (int j = 0; j < 16; ++j) c[j] = inside(j) ? crow[(long)j * a.ldc] : 0.0;
-                ok = ptx::wait_parity(&acc_full[buf], (tile >> 1) & 1, abort_flag, a.wait_budget_ns);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                ptx::tc_fence_after();
-                const int er = ea[(item & 3) * SU_BM + rl];
-                const int *ec = eb + (tile & 3) * SU_BN + 16 * chalf;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t r[SU_S][8];
-#pragma unroll
-                    for (int d = 0; d < SU_S; ++d) ptx::tmem_ld_32x32b_x8(tb + d * SU_BN + 16 * chalf + 8 * h, r[d]);
+                for (int j = 0; j < 8; ++j) c[j] = !GEMM && j < jn ? crow[(long)j * a.ldc] : 0.0;
+                unsigned weak = 0;  // GEMM: columns that need FMAs
+                for (int ch = 0; ch < chunks; ++ch, ++tile) {
+                    if (GEMM && !(ok = cut_a(ch * SU_K))) break;
+                    const int buf = tile & 1;
+                    const uint32_t tb = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * SU_ACC_STRIDE + 8 * group;
+                    ok = ptx::wait_parity(&acc_full[buf], (tile >> 1) & 1, abort_flag, a.wait_budget_ns);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const int er = ea[(item & 3) * SU_BM + rl];
+                    const int *ec = eb + (tile & 3) * SU_BN + 8 * group;
                     int ev[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) ev[j] = er + ec[8 * h + j];
-                    ptx::tmem_ld_wait();
-                    if (h == 1) {
-                        ptx::tc_fence_before();
-                        ptx::mbar_arrive(&acc_empty[buf]);
-                    }
+                    for (int j = 0; j < 8; ++j) ev[j] = er + ec[j];
+                    // 128 x 128 / 2 for 64 terms: half the product of two largest elements
+                    const float least = 128.0f * (float)min(SU_K, a.k - ch * SU_K);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        int s[SU_S];
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t r[SU_S][4], mag[4];
 #pragma unroll
-                        for (int d = 0; d < SU_S; ++d) s[d] = (int)__uint_as_float(r[d][j]);
-                        // sum of s[d] 2^{8 (5 - d)}, d = 0 .. 6, the last one rounded off
-                        const long long hi = (long long)s[0] * 65536 + (s[1] * 256 + s[2]);
-                        const long long lo = (long long)s[3] * 65536 + (s[4] * 256 + s[5] + ((s[6] + 128) >> 8));
-                        const int e = ev[j];
-                        double val = su_to_double((hi << 24) + lo, e);
-                        if (e >= SU_NONFINITE) val = __longlong_as_double(0x7FF8000000000000ll);
-                        if (inside(8 * h + j)) crow[(long)(8 * h + j) * a.ldc] = c[8 * h + j] - val;
+                        for (int d = 0; d < SU_S; ++d) ptx::tmem_ld_32x32b_x4(tb + d * SU_BN + 4 * h, r[d]);
+                        if (GEMM) ptx::tmem_ld_32x32b_x4(tb + SU_ABS * SU_BN + 4 * h, mag);
+                        ptx::tmem_ld_wait();
+                        if (h == 1) {
+                            ptx::tc_fence_before();
+                            ptx::mbar_arrive(&acc_empty[buf]);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const double v = su_to_double(su_combine(r, j), ev[4 * h + j]);
+                            if (GEMM) {
+                                if (__uint_as_float(mag[j]) < least) weak |= 1u << (4 * h + j);
+                                c[4 * h + j] += v;
+                            } else if (4 * h + j < jn) {
+                                crow[(long)(4 * h + j) * a.ldc] = c[4 * h + j] - v;
+                            }
+                        }
                     }
+                    if (GEMM) ++item;
+                }
+                if (!GEMM || !ok) continue;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < jn && !(weak >> j & 1)) crow[(long)j * a.ldc] -= c[j];
+                if (jn < 8) weak &= (1u << max(jn, 0)) - 1;
+                for (; weak; weak &= weak - 1) {
+                    const int j = __ffs((int)weak) - 1;
+                    crow[(long)j * a.ldc] -= su_dot(a, row, col0 + j);
                 }
             }
+            if (GEMM) --item;  // counted per chunk
         }
     }
     if (!ok) {
@@ -355,7 +457,7 @@ __global__ void __launch_bounds__(SU_THREADS, 1) slice_update_kernel(const Slice
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    if (warp == 12) ptx::tmem_dealloc(tmem_base, SU_TMEM_COLS);
+    if (warp == SU_MMA_WARP) ptx::tmem_dealloc(tmem_base, SU_TMEM_COLS);
 }
 
 } // namespace gb300

@@ -157,3 +157,52 @@ def test_lu_panel_solves(gpu, dtype, m, n):
             u = t64 + np.eye(k)
             got, mag = x @ u, np.abs(x) @ np.abs(u)
         assert np.all(np.abs(got - b) <= 4 * k * EPS[dtype] * (mag + np.abs(b)))
+
+
+@pytest.mark.parametrize("form", ["syrk", "nt", "nn"])
+@pytest.mark.parametrize("m,n,k", [(512, 192, 16), (129, 800, 65), (641, 640, 200), (130, 2000, 17)])
+@pytest.mark.parametrize("kind", ["random", "graded", "sparse", "special"])
+def test_fp64_products_keep_the_componentwise_bound(gpu, form, m, n, k, kind):
+    rng = np.random.default_rng(m + n + k)
+    n = max(m, 500) if form == "syrk" else n
+    m = n if form == "syrk" else m
+    a, b, c = rng.standard_normal((m, k)), rng.standard_normal((n, k)), rng.standard_normal((m, n))
+    if kind == "graded":  # large elements of A meet small ones of B
+        s = np.power(10.0, np.linspace(-7, 7, k))
+        a, b = a * s, b / s
+    elif kind == "sparse":
+        a[rng.uniform(size=a.shape) < 0.97] = 0
+        b[::3] = 0
+    elif kind == "special":
+        a[3, 1], a[7, 0], b[5, 2 % k], a[11] = np.nan, np.inf, -np.inf, 1e-310
+    if form == "syrk":
+        b = a
+    da, dc = up(a), up(c)
+    db = up(b.T if form == "nn" else b)
+    if form == "syrk":
+        check(gpu.starpu_gb300_dsyrk_ln_tile(None, n, k, -1.0, da.ptr, n, 1.0, dc.ptr, n))
+    elif form == "nt":
+        check(gpu.starpu_gb300_dgemm_nt_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    else:
+        check(gpu.starpu_gb300_dgemm_nn_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, k, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float64)
+    with np.errstate(all="ignore"):
+        ref = c - a @ b.T
+        bound = (k + 2) * EPS[np.float64] * (np.abs(c) + np.abs(a) @ np.abs(b).T)
+    keep = np.tril(np.ones((m, n), bool)) if form == "syrk" else np.ones((m, n), bool)
+    assert np.array_equal(out[~keep], c[~keep])
+    fine = np.isfinite(ref) & keep
+    assert np.all(np.abs(out - ref)[fine] <= bound[fine])
+    assert np.array_equal(np.isfinite(out)[keep], np.isfinite(ref)[keep])
+
+
+@pytest.mark.parametrize("n,nrhs", [(3000, 40), (1900, 64)])
+def test_potrs_many_columns_graded(gpu, n, nrhs):
+    d = np.power(10.0, np.random.default_rng(n).uniform(-5, 5, n))
+    l = np.linalg.cholesky(spd(n, n, d))
+    b = np.random.default_rng(nrhs).uniform(-1, 1, (n, nrhs))
+    dl, db = up(l), up(b)
+    check(gpu.starpu_gb300_dpotrs(None, n, nrhs, dl.ptr, n, db.ptr, n))
+    x = db.download((n, nrhs), np.float64)
+    y = np.abs(l.T) @ np.abs(x)
+    assert np.all(np.abs(l @ (l.T @ x) - b) <= 8 * n * EPS[np.float64] * (np.abs(l) @ y + np.abs(b)))
