@@ -275,19 +275,19 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
 // POTRS with a lower factor: L y = b (forward), then L^T x = y (backward),
 // in blocks of CP_SB rows: solve the block, update the rows to come.
 // min-dgels/base/SRC/dpotrs.c does the same two sweeps through dtrsm.
-// CB right-hand sides per CTA in the block solve, CU in the update.
-template <typename T, int CB, int CU, bool TRANS>
+// C right-hand sides per CTA in the update.
+template <typename T, int C, bool TRANS>
 static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
-    constexpr size_t sm_blk = cp_trsv_smem<T, CB>(TRANS), sm_upd = cp_upd_smem<T, CU>(TRANS);
-    if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, CB, TRANS>, (int)sm_blk) ||
-        gb300_func_dyn_smem((const void *)trsv_upd_kernel<T, CU, TRANS>, (int)sm_upd))
+    constexpr size_t sm_blk = cp_trsv_smem<T>(TRANS), sm_upd = cp_upd_smem<T, C>(TRANS);
+    if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, TRANS>, (int)sm_blk) ||
+        gb300_func_dyn_smem((const void *)trsv_upd_kernel<T, C, TRANS>, (int)sm_upd))
         return;
     const int nblk = (n + CP_SB - 1) / CP_SB;
     for (int b = 0; b < nblk; ++b) {
         const int j0 = (TRANS ? nblk - 1 - b : b) * CP_SB, w = std::min(CP_SB, n - j0);
-        gb300_count_launch(), trsv_blk_kernel<T, CB, TRANS>
-            <<<cdiv(nrhs, CB), 256, sm_blk, s>>>(w, nrhs, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb);
+        gb300_count_launch(), trsv_blk_kernel<T, TRANS>
+            <<<nrhs, 256, sm_blk, s>>>(w, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb, nullptr);
         const int rest = TRANS ? j0 : n - j0 - w;
         if (rest <= 0) continue;
         if constexpr (std::is_same<T, double>::value) {
@@ -295,32 +295,28 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
             // 8 to 9 us, against rest nrhs / 8800 us on the FP64 units
             if (rest >= SLICE_MIN_M && nrhs >= 16 && (long)rest * nrhs >= SLICE_MIN_ELEMENTS) {
                 slice_update<true>(s, false, rest, nrhs, w, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl,
-                             TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, nullptr);
+                                   TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, nullptr);
                 continue;
             }
         }
-        gb300_count_launch(), trsv_upd_kernel<T, CU, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, CU)), 256, sm_upd, s>>>(
+        gb300_count_launch(), trsv_upd_kernel<T, C, TRANS><<<dim3(cdiv(rest, 32), cdiv(nrhs, C)), 256, sm_upd, s>>>(
             rest, w, nrhs, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl, ldl, B + j0, TRANS ? B : B + j0 + w, ldb);
     }
 }
 
-template <typename T, int CB, int CU>
-static void potrs_sweeps(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
+template <typename T, int C> static void potrs_sweeps(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
-    potrs_sweep_blocks<T, CB, CU, false>(s, n, nrhs, L, ldl, B, ldb);
-    potrs_sweep_blocks<T, CB, CU, true>(s, n, nrhs, L, ldl, B, ldb);
+    potrs_sweep_blocks<T, C, false>(s, n, nrhs, L, ldl, B, ldb);
+    potrs_sweep_blocks<T, C, true>(s, n, nrhs, L, ldl, B, ldb);
 }
 
 template <typename T>
 void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
 {
     if (n <= 0 || nrhs <= 0) return;
-    // The block solve takes one right-hand side per CTA while there are SMs for
-    // them: its rows' products share one SM's FMA units.
-    if (nrhs == 1) potrs_sweeps<T, 1, 1>(s, n, nrhs, L, ldl, B, ldb);
-    else if (nrhs <= 4) potrs_sweeps<T, 1, 4>(s, n, nrhs, L, ldl, B, ldb);
-    else if (nrhs <= 152) potrs_sweeps<T, 1, 8>(s, n, nrhs, L, ldl, B, ldb);
-    else potrs_sweeps<T, 4, 8>(s, n, nrhs, L, ldl, B, ldb);
+    if (nrhs == 1) potrs_sweeps<T, 1>(s, n, nrhs, L, ldl, B, ldb);
+    else if (nrhs <= 4) potrs_sweeps<T, 4>(s, n, nrhs, L, ldl, B, ldb);
+    else potrs_sweeps<T, 8>(s, n, nrhs, L, ldl, B, ldb);
 }
 
 // ---- single-launch POTRS sweeps with inverted 64 x 64 diagonal blocks ------

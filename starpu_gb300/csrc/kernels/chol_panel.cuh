@@ -470,117 +470,107 @@ template <typename T, int SR> __global__ void __launch_bounds__(256) trsm_slab_k
 // one launch that solves the block (trsv_blk_kernel) and one that updates the
 // rows still to come (trsv_upd_kernel), forward with L, backward with L^T.
 //
-// trsv_blk_kernel: C right-hand sides per CTA (8 warps).  The block goes in
-// 32-row pieces: warp c solves column c's piece by shuffles (lane = row)
-// while the CTA's loads of the piece's off-diagonal part are in flight, then
-// thread = row (forward) or column (backward) applies them.  Bound by the
-// chain of dependent rows.  FP64 solves a piece scaled to a unit diagonal, one
+// trsv_blk_kernel: one right-hand side per CTA.  Thread = row (forward) or
+// column (backward) of the block, warp = 32 of them.  A warp waits for the
+// pieces solved before its own (an mbarrier each, no CTA barrier), subtracts
+// their products, solves its piece by shuffles and publishes it; its operands
+// of the next piece are on their way meanwhile.  Bound by the chain of
+// dependent rows: per piece 32 steps of a shuffle and an FMA.  FP32 sums the
+// products apart from the right-hand side, so that each rounding is relative to
+// their (smaller) sum; FP64 solves a piece scaled to a unit diagonal, one
 // operation (64 clocks) per row in the chain instead of three.
 // ---------------------------------------------------------------------------
 constexpr int CP_SB = 256;
 
-template <typename T, int C> constexpr size_t cp_trsv_smem(bool trans)
+template <typename T> constexpr size_t cp_trsv_smem(bool trans)
 {
-    return ((size_t)(C + 1) * CP_SB + 32 * 33 + (trans ? (size_t)CP_SB * 33 : 0)) * sizeof(T);
+    return ((size_t)CP_SB + (trans ? 8 * 32 * 33 : 0)) * sizeof(T);
 }
 
-template <typename T, int C, bool TRANS>
-__global__ void __launch_bounds__(256) trsv_blk_kernel(int w, int nrhs, const T *__restrict__ L, long ldl,
-                                                       T *__restrict__ B, long ldb)
+template <typename T, bool TRANS>
+__global__ void __launch_bounds__(256) trsv_blk_kernel(int w, const T *__restrict__ L, long ldl, T *__restrict__ B, long ldb,
+                                                       int *err)
 {
     extern __shared__ __align__(16) unsigned char cp_smem[];
-    T *xs = (T *)cp_smem;         // [C][CP_SB]
-    T *dinv = xs + C * CP_SB;     // [CP_SB]: 1 / L(r, r)
-    T *Ld = dinv + CP_SB;         // [32][33]: forward Ld[j][i] = L(i, j), backward Ld[j][i] = L(j, i)
-    T *Lt = Ld + 32 * 33;         // backward: [CP_SB][33], Lt[c][i] = L(piece row i, c)
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int c0 = blockIdx.x * C, nc = min(C, nrhs - c0);
-    for (int e = tid; e < C * CP_SB; e += 256) {
-        const int r = e % CP_SB, c = e / CP_SB;
-        xs[e] = (r < w && c < nc) ? B[r + (long)(c0 + c) * ldb] : T(0);
-    }
-    dinv[tid] = tid < w ? T(1) / L[tid + (long)tid * ldl] : T(1);
-    __syncthreads();
+    __shared__ uint64_t bar[16];
     constexpr bool SCALED = sizeof(T) == 8;
+    T *xs = (T *)cp_smem;  // [CP_SB]: solved pieces
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = 32 * warp + lane;
+    T *stage = xs + CP_SB + warp * 32 * 33;
+    T *b = B + (long)blockIdx.x * ldb;
     const int np = (w + 31) / 32;
-    for (int s = 0; s < np; ++s) {
-        const int p0 = 32 * (TRANS ? np - 1 - s : s), pw = min(32, w - p0);
-        // the off-diagonal part of this piece, in flight during the solve
-        T l[32];
+    cp_panel_init(bar);
+    __syncthreads();
+    if (warp >= np) return;
+    // l[j]: this row's elements of piece p, L(r, 32 p + j), or its column's, L(32 p + j, r)
+    auto load = [&](T(&l)[32], int p) {
         if (!TRANS) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                l[j] = (tid >= p0 + 32 && tid < w) ? L[tid + (long)(p0 + j) * ldl] : T(0);
+            for (int j = 0; j < 32; ++j) l[j] = r < w && 32 * p + j < w ? L[r + (long)(32 * p + j) * ldl] : T(0);
         } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int c = warp + 8 * j;
-                l[j] = (c < p0 && lane < pw) ? L[(p0 + lane) + (long)c * ldl] : T(0);
+            for (int j = 0; j < 32; ++j) {  // column 32 warp + j, lane = row: coalesced, then turned
+                const int row = 32 * p + lane, col = 32 * warp + j;
+                l[j] = row < w && col < w ? L[row + (long)col * ldl] : T(0);
             }
         }
-        for (int e = tid; e < 32 * 32; e += 256) {
-            const int i = e & 31, j = e >> 5;  // L(i, j) of the piece's diagonal block
-            T v = (i < pw && j <= i) ? L[(p0 + i) + (long)(p0 + j) * ldl] : T(i == j ? 1 : 0);
-            if (SCALED) v *= dinv[p0 + (TRANS ? j : i)];
-            Ld[TRANS ? i * 33 + j : j * 33 + i] = v;
-        }
-        __syncthreads();
-        for (int c = warp; c < C; c += 8) {
-            // the products are summed apart from the right-hand side, so that
-            // each rounding is relative to their (smaller) sum
-            const T d = dinv[p0 + lane];
-            if (SCALED) {
-                T v = xs[c * CP_SB + p0 + lane] * d;
-#pragma unroll 8
-                for (int i = 0; i < 32; ++i) {
-                    const int j = TRANS ? 31 - i : i;
-                    const T xj = __shfl_sync(0xffffffffu, v, j);
-                    if (TRANS ? lane < j : lane > j) v = fma(-Ld[j * 33 + lane], xj, v);
-                }
-                xs[c * CP_SB + p0 + lane] = v;
-                continue;
-            }
-            const T v = xs[c * CP_SB + p0 + lane];
-            T acc = T(0);
-            if (!TRANS) {
-#pragma unroll 8
-                for (int j = 0; j < 32; ++j) {
-                    const T xj = __shfl_sync(0xffffffffu, (v - acc) * d, j);
-                    if (lane > j) acc = fma(Ld[j * 33 + lane], xj, acc);
-                }
-            } else {
-#pragma unroll 8
-                for (int j = 31; j >= 0; --j) {
-                    const T xj = __shfl_sync(0xffffffffu, (v - acc) * d, j);
-                    if (lane < j) acc = fma(Ld[j * 33 + lane], xj, acc);
-                }
-            }
-            xs[c * CP_SB + p0 + lane] = (v - acc) * d;
-        }
-        if (TRANS) {
+    };
+    auto turn = [&](T(&l)[32]) {
+        if (!TRANS) return;
+        __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) Lt[(warp + 8 * j) * 33 + lane] = l[j];
+        for (int j = 0; j < 32; ++j) stage[j * 33 + lane] = l[j];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) l[j] = stage[lane * 33 + j];
+    };
+    const T v = r < w ? b[r] : T(0), d = r < w ? T(1) / L[r + (long)r * ldl] : T(1);
+    T m[32], l[32], sum = T(0);
+    load(m, warp);  // the piece's own block
+    const int n = TRANS ? np - 1 - warp : warp;  // pieces before this one
+    if (n > 0) load(l, TRANS ? np - 1 : 0);
+    turn(m);
+    if (SCALED)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) m[j] *= d;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+        const int p = TRANS ? np - 1 - i : i;
+        turn(l);
+        ok = cp_wait(&bar[p], 0) && ok;
+        const Quad<T> *x = reinterpret_cast<const Quad<T> *>(xs + 32 * p);
+        T acc[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const Quad<T> y = x[j / 4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = fma(l[j + q], y.v[q], acc[q]);
         }
-        __syncthreads();
-        if (TRANS ? tid < p0 : (tid >= p0 + 32 && tid < w)) {
-            if (TRANS) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) l[j] = Lt[tid * 33 + j];
-            }
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                T acc[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-                for (int j = 0; j < 32; ++j) acc[j & 3] = fma(l[j], xs[c * CP_SB + p0 + j], acc[j & 3]);
-                xs[c * CP_SB + tid] -= (acc[0] + acc[1]) + (acc[2] + acc[3]);
-            }
-        }
-        __syncthreads();
+        if (i + 1 < n) load(l, TRANS ? p - 1 : p + 1);
+        sum += (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
-    for (int e = tid; e < C * CP_SB; e += 256) {
-        const int r = e % CP_SB, c = e / CP_SB;
-        if (r < w && c < nc) B[r + (long)(c0 + c) * ldb] = xs[e];
+    T y;
+    if (SCALED) {
+        y = (v - sum) * d;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const int j = TRANS ? 31 - i : i;
+            const T xj = __shfl_sync(0xffffffffu, y, j);
+            if (TRANS ? lane < j : lane > j) y = fma(-m[j], xj, y);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const int j = TRANS ? 31 - i : i;
+            const T xj = __shfl_sync(0xffffffffu, (v - sum) * d, j);
+            if (TRANS ? lane < j : lane > j) sum = fma(m[j], xj, sum);
+        }
+        y = (v - sum) * d;
     }
+    xs[r] = y;
+    ptx::mbar_arrive(&bar[warp]);
+    if (r < w) b[r] = y;
+    if (!ok && err) atomicCAS(err, 0, CP_ERR_TIMEOUT);
 }
 
 // C right-hand sides of Y[m x nrhs] -= op(L) X[w x nrhs] (w <= CP_SB): op(L) =
