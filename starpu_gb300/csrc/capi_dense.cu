@@ -79,6 +79,20 @@ static long gemm_ctas(bool lower, int m, int n, int bm)
     return lower ? tm * (tm + 1) / 2 : tm * tn;
 }
 
+static bool aligned16(const float *p, long ld) { return ((uintptr_t)p & 15) == 0 && (ld & 3) == 0; }
+
+static void gemm_nt_f32(cudaStream_t s, bool lower, int m, int n, int k, float alpha, const float *A, long lda,
+                        const float *B, long ldb, float beta, float *C, long ldc)
+{
+    const unsigned tm = cdiv(m, 128), tn = cdiv(n, 128);
+    if (lower)
+        gb300_count_launch(), gemm_nt_f32_kernel<true>
+            <<<tm * (tm + 1) / 2, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+    else
+        gb300_count_launch(), gemm_nt_f32_kernel<false>
+            <<<dim3(tm, tn), 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+
 // FP32: 128x128 block tiles, 8x8 per thread, when they make at least half a
 // wave; smaller ones otherwise (the 64 and 32 tiles take a third and an eighth
 // of the 128 tile's time each, so up to two waves of them are faster).
@@ -90,6 +104,8 @@ template <> struct simt_cfg<float> {
     {
         if (!lower && n <= 32)
             gemm_launch<float, TA, TB, 128, 32, 8, 8, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
+        else if (!TA && TB && gemm_ctas(lower, m, n, 128) > 76 && aligned16(A, lda) && aligned16(B, ldb) && aligned16(C, ldc))
+            gemm_nt_f32(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
         else if (gemm_ctas(lower, m, n, 128) > 76)
             gemm_launch<float, TA, TB, 128, 128, 8, 8, 8>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
         else if (gemm_ctas(lower, m, n, 64) > 76)
@@ -258,7 +274,7 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
         const int kb = std::min(nb, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
         if (kb <= CP_W)
-            gb300_count_launch(), potf2_leaf_kernel<T><<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
+            gb300_count_launch(), potf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
         else if (std::is_same<T, float>::value && kb <= COOP_MAX_N)
             potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0);
         else

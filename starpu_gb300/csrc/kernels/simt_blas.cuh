@@ -182,6 +182,120 @@ gemm_simt_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long lda
 }
 
 // ---------------------------------------------------------------------------
+// The FP32 N,T product C = beta C + alpha A B^T for large matrices: the same
+// sums in the same order as gemm_simt_kernel's 128 x 128 tile (thread = 8 x 8,
+// k ascending), with the operands read 16 bytes at a time, 16 k per barrier and
+// whole tiles stored without per-element tests: the scalar form spent a third of
+// its issue slots on addresses and tests.  A, B and C 16-byte aligned with
+// leading dimensions divisible by 4.
+// ---------------------------------------------------------------------------
+template <bool LOWER>
+__global__ void __launch_bounds__(256, 2) gemm_nt_f32_kernel(int m, int n, int k, float alpha, const float *__restrict__ A,
+                                                             long lda, const float *__restrict__ B, long ldb, float beta,
+                                                             float *__restrict__ C, long ldc)
+{
+    constexpr int BM = 128, BK = 16, LD = BM + 4;
+    __shared__ __align__(16) float As[2][BK][LD], Bs[2][BK][LD];
+    int bi, bj;
+    if (LOWER) {
+        const int t = blockIdx.x;
+        int r = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+        while ((r + 1) * (r + 2) / 2 <= t) ++r;
+        while (r * (r + 1) / 2 > t) --r;
+        bi = r;
+        bj = t - r * (r + 1) / 2;
+    } else {
+        bi = blockIdx.x;
+        bj = blockIdx.y;
+    }
+    const int m0 = bi * BM, n0 = bj * BM, tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+    // this thread's loads: 4 rows from 4 (tid % 32), k = tid / 32 and + 8
+    const int lr = 4 * (tid & 31), lk = tid >> 5;
+    const float *pa = A + m0 + lr + (long)lk * lda, *pb = B + n0 + lr + (long)lk * ldb;
+    const bool wa = m0 + BM <= m, wb = n0 + BM <= n;
+    float4 ra[2], rb[2];
+    auto load4 = [](const float *p, bool whole, int rows, bool in) {
+        if (whole && in) return *reinterpret_cast<const float4 *>(p);
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (in) {
+            if (rows > 0) v.x = p[0];
+            if (rows > 1) v.y = p[1];
+            if (rows > 2) v.z = p[2];
+            if (rows > 3) v.w = p[3];
+        }
+        return v;
+    };
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const bool in = k0 + lk + 8 * q < k;
+            ra[q] = load4(pa + (long)(k0 + 8 * q) * lda, wa, m - m0 - lr, in);
+            rb[q] = load4(pb + (long)(k0 + 8 * q) * ldb, wb, n - n0 - lr, in);
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            *reinterpret_cast<float4 *>(&As[buf][lk + 8 * q][lr]) = ra[q];
+            *reinterpret_cast<float4 *>(&Bs[buf][lk + 8 * q][lr]) = rb[q];
+        }
+    };
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    const int nk = (k + BK - 1) / BK;
+    if (nk > 0) {
+        load(0);
+        store(0);
+    }
+    __syncthreads();
+    for (int kt = 0; kt < nk; ++kt) {
+        const int cur = kt & 1;
+        if (kt + 1 < nk) load((kt + 1) * BK);
+#pragma unroll
+        for (int p = 0; p < BK; ++p) {
+            float a[8], b[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 x = *reinterpret_cast<const float4 *>(&As[cur][p][64 * h + 4 * tr]);
+                const float4 y = *reinterpret_cast<const float4 *>(&Bs[cur][p][64 * h + 4 * tc]);
+                a[4 * h] = x.x, a[4 * h + 1] = x.y, a[4 * h + 2] = x.z, a[4 * h + 3] = x.w;
+                b[4 * h] = y.x, b[4 * h + 1] = y.y, b[4 * h + 2] = y.z, b[4 * h + 3] = y.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        if (kt + 1 < nk) store(cur ^ 1);
+        __syncthreads();
+    }
+    const bool whole = wa && wb && (!LOWER || bi > bj);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int col = n0 + 64 * (j >> 2) + 4 * tc + (j & 3);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = m0 + 64 * h + 4 * tr;
+            float *c = C + row + (long)col * ldc;
+            if (whole) {
+                const float4 o = beta == 0.0f ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : *reinterpret_cast<const float4 *>(c);
+                *reinterpret_cast<float4 *>(c) =
+                    make_float4(fmaf(alpha, acc[4 * h][j], beta * o.x), fmaf(alpha, acc[4 * h + 1][j], beta * o.y),
+                                fmaf(alpha, acc[4 * h + 2][j], beta * o.z), fmaf(alpha, acc[4 * h + 3][j], beta * o.w));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (col < n && row + i < m && (!LOWER || row + i >= col))
+                        c[i] = fmaf(alpha, acc[4 * h + i][j], beta == 0.0f ? 0.0f : beta * c[i]);
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Elementwise helpers.
 // ---------------------------------------------------------------------------
 template <typename TO, typename TI>
