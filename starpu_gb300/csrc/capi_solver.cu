@@ -13,6 +13,8 @@
 #include <algorithm>
 #include <atomic>
 #include <functional>
+#include <memory>
+#include <new>
 #include <vector>
 #include <stdlib.h>
 #include <cuda_runtime.h>
@@ -175,20 +177,45 @@ __global__ void accumulate_kernel(int n, int nrhs, const float *__restrict__ y, 
 // exponent of the largest magnitude of v (0 for zero or non-finite), as FP32 column scales use
 __device__ __forceinline__ int column_exp(double v) { return (v > 0.0 && isfinite(v)) ? ilogb(v) : 0; }
 
-// e_j = exponent of max_i |M_ij| (one CTA per column)
-__global__ void colmax_exp_kernel(int n, const double *__restrict__ M, long ldm, int *__restrict__ exps)
+// |v| as an integer that orders like the magnitude, 0 for NaN (as fmax(0, v)
+// would leave it).  The column maxima below compare these: an FP64 compare
+// holds a sub-partition's only FP64 unit for 64 clocks a warp, an integer one 2.
+__device__ __forceinline__ unsigned long long mag_bits(double v)
 {
-    const long j = blockIdx.x;
-    double m = 0.0;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, fabs(M[i + j * ldm]));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    __shared__ double red[32];
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return u > 0x7ff0000000000000ull ? 0ull : u;
+}
+
+// max over the CTA, in thread 0 (red: one word per warp, free on entry)
+__device__ __forceinline__ unsigned long long cta_max_bits(unsigned long long m, unsigned long long *red)
+{
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-        exps[j] = column_exp(m);
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0ull;
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
+    return m;
+}
+
+// The column kernels run one CTA per right-hand side: they are bound by the
+// latency of their loads, so a CTA holds as many threads as it can.  With
+// 256 threads, FP64 maxima and three status reads a round instead of one, the
+// mixed solve took 675 us at n = 777 and 2729 us at n = 4096; so 570 and 2561.
+static constexpr int COL_T = 1024;
+
+// e_j = exponent of max_i |M_ij| (one CTA per column)
+__global__ void __launch_bounds__(COL_T) colmax_exp_kernel(int n, const double *__restrict__ M, long ldm,
+                                                           int *__restrict__ exps)
+{
+    const double *m = M + (long)blockIdx.x * ldm;
+    unsigned long long b = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += COL_T) b = max(b, mag_bits(m[i]));
+    __shared__ unsigned long long red[32];
+    b = cta_max_bits(b, red);
+    if (threadIdx.x == 0) exps[blockIdx.x] = column_exp(__longlong_as_double((long long)b));
 }
 
 // R = B (copy) before the GEMM R -= A X
@@ -295,7 +322,7 @@ static int residual_mixed(cudaStream_t s, int n, int nrhs, const double *A, long
     }
     const long cap = (long)(residual_partials(n, nrhs) / ((size_t)n * nrhs));
     const int kc = residual_tc_kchunk(n, nrhs, (int)cap);
-    gb300_count_launch(), df_split_x_kernel<<<nrhs, 256, 0, s>>>(n, X, ldx, xs, sx);
+    gb300_count_launch(), colmax_exp_kernel<<<nrhs, COL_T, 0, s>>>(n, X, ldx, sx);
     int rc = residual_tc(s, n, nrhs, rtc_a, X, ldx, sx, anorm_bits + 2, kc, rtc_xs, partials, d_err);
     if (rc) return rc;
     const unsigned gx = (unsigned)std::min<long>(((long)n + 255) / 256, 1024);
@@ -306,36 +333,28 @@ static int residual_mixed(cudaStream_t s, int n, int nrhs, const double *A, long
 
 // Per right-hand side j (one CTA): berr_j = ||r_j||_inf / (||A||_inf ||x_j||_inf + ||b_j||_inf);
 // done_j = berr_j <= tol.
-__global__ void backward_error_kernel(int n, const double *__restrict__ R, long ldr, const double *__restrict__ X,
-                                      long ldx, const double *__restrict__ B, long ldb,
-                                      const unsigned long long *anorm_bits, double tol, double *berr, int *done,
-                                      int *rexp)
+__global__ void __launch_bounds__(COL_T) backward_error_kernel(int n, const double *__restrict__ R, long ldr,
+                                                               const double *__restrict__ X, long ldx,
+                                                               const double *__restrict__ B, long ldb,
+                                                               const unsigned long long *anorm_bits, double tol,
+                                                               double *berr, int *done, int *rexp)
 {
     const long j = blockIdx.x;
-    double rm = 0, xm = 0, bm = 0;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) {
-        rm = fmax(rm, fabs(R[i + j * ldr]));
-        xm = fmax(xm, fabs(X[i + j * ldx]));
-        bm = fmax(bm, fabs(B[i + j * ldb]));
+    const double *r = R + j * ldr, *x = X + j * ldx, *b = B + j * ldb;
+    unsigned long long rb = 0, xb = 0, bb = 0;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < n; i += COL_T) {
+        rb = max(rb, mag_bits(r[i]));
+        xb = max(xb, mag_bits(x[i]));
+        bb = max(bb, mag_bits(b[i]));
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        rm = fmax(rm, __shfl_down_sync(0xffffffffu, rm, o));
-        xm = fmax(xm, __shfl_down_sync(0xffffffffu, xm, o));
-        bm = fmax(bm, __shfl_down_sync(0xffffffffu, bm, o));
-    }
-    __shared__ double s[3][32];
-    if ((threadIdx.x & 31) == 0) {
-        s[0][threadIdx.x >> 5] = rm;
-        s[1][threadIdx.x >> 5] = xm;
-        s[2][threadIdx.x >> 5] = bm;
-    }
-    __syncthreads();
+    __shared__ unsigned long long red[3][32];
+    rb = cta_max_bits(rb, red[0]);
+    xb = cta_max_bits(xb, red[1]);
+    bb = cta_max_bits(bb, red[2]);
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            rm = fmax(rm, s[0][w]);
-            xm = fmax(xm, s[1][w]);
-            bm = fmax(bm, s[2][w]);
-        }
+        const double rm = __longlong_as_double((long long)rb), xm = __longlong_as_double((long long)xb),
+                     bm = __longlong_as_double((long long)bb);
         const double an = __longlong_as_double((long long)*anorm_bits);
         const double den = an * xm + bm;
         const double e = den > 0 ? rm / den : (rm > 0 ? INFINITY : 0.0);
@@ -459,32 +478,35 @@ __global__ void __launch_bounds__(512) pcg_step_kernel(int n, const double *__re
 
 // max_i L_ii^2 / min_i L_ii^2 of the FP32 factor (one CTA): the ratio of the
 // largest to the smallest Cholesky pivot, a lower bound of kappa_2(A) (every
-// pivot lies between the extreme eigenvalues).
-__global__ void pivot_ratio_kernel(int n, const float *__restrict__ W, long ldw, double *ratio)
+// pivot lies between the extreme eigenvalues).  The extremes are found in FP32
+// and squared in FP64, which orders them alike.
+__global__ void __launch_bounds__(COL_T) pivot_ratio_kernel(int n, const float *__restrict__ W, long ldw, double *ratio)
 {
-    __shared__ double rmx[32], rmn[32];
-    double mx = 0.0, mn = INFINITY;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) {
-        const double d = (double)W[i + i * ldw];
-        mx = fmax(mx, d * d);
-        mn = fmin(mn, d * d);
+    __shared__ float rmx[32], rmn[32];
+    float mx = 0.0f, mn = INFINITY;
+#pragma unroll 4
+    for (long i = threadIdx.x; i < n; i += COL_T) {
+        const float d = fabsf(W[i + i * ldw]);
+        mx = fmaxf(mx, d);
+        mn = fminf(mn, d);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-        mn = fmin(mn, __shfl_down_sync(0xffffffffu, mn, o));
-    }
+    auto warp = [&] {
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        }
+    };
+    warp();
     if ((threadIdx.x & 31) == 0) {
         rmx[threadIdx.x >> 5] = mx;
         rmn[threadIdx.x >> 5] = mn;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mx = fmax(mx, rmx[w]);
-            mn = fmin(mn, rmn[w]);
-        }
-        *ratio = mn > 0.0 ? mx / mn : INFINITY;
-    }
+    if (threadIdx.x >= 32) return;
+    mx = rmx[threadIdx.x];
+    mn = rmn[threadIdx.x];
+    warp();
+    if (threadIdx.x == 0) *ratio = mn > 0.0f ? ((double)mx * mx) / ((double)mn * mn) : INFINITY;
 }
 
 // F (n x n, ld n) = the lower triangle of A, zeros above: the FP64 copy the
@@ -516,7 +538,8 @@ struct SolverWs {
     double *rho;           // nrhs: r.z of the conjugate-gradient steps
     int *brk;              // breakdown word of the conjugate-gradient steps
     int *rexp;             // nrhs: power-of-two scales of the FP32 right-hand sides
-    unsigned long long *anorm_bits;
+    unsigned long long *anorm_bits;  // status words: [0] ||A||_inf, [1] info and err, [2] max |A_ij|, [3] brk
+    double *ratio;                   // [4] pivot ratio; berr follows 256 bytes after anorm_bits
     int *info, *err;
     size_t panel_bytes;
 };
@@ -637,10 +660,10 @@ static size_t layout(int n, int nrhs, int nb, void *base, SolverWs *ws)
     const size_t oZ = tiles ? take(tsw_scratch_bytes(n, nb)) : 0;
     const size_t oA = take(residual_tc_a_bytes(n));
     const size_t oN = take((size_t)((n + 63) / 64) * n * sizeof(float));
-    const size_t oS = take(4 * sizeof(unsigned long long));
+    const size_t oS = take(4 * sizeof(unsigned long long) + sizeof(double));
+    const size_t oE = take((size_t)nrhs * sizeof(double));  // follows the status words: one read takes both
     const size_t oR = take((size_t)n * nrhs * sizeof(double));
     const size_t oY = take((size_t)n * nrhs * sizeof(float));
-    const size_t oE = take((size_t)nrhs * sizeof(double));
     const size_t oD = take((size_t)nrhs * sizeof(int));
     const size_t oQ = take(residual_partials(n, nrhs) * sizeof(double));
     const size_t oX = take((size_t)n * 16 * ((nrhs + 15) / 16) * sizeof(float2));
@@ -648,7 +671,7 @@ static size_t layout(int n, int nrhs, int nb, void *base, SolverWs *ws)
     const size_t oJ = take((size_t)nrhs * sizeof(int));
     const size_t oK = take(residual_tc_xs_bytes(n, nrhs));
     const size_t oG = take(3 * (size_t)n * nrhs * sizeof(double));
-    const size_t oH = take((size_t)nrhs * sizeof(double) + 16);
+    const size_t oH = take((size_t)nrhs * sizeof(double));
     if (ws && base) {
         char *b = (char *)base;
         ws->W = (float *)(b + oW);
@@ -672,11 +695,12 @@ static size_t layout(int n, int nrhs, int nb, void *base, SolverWs *ws)
         ws->Qn = ws->P + (size_t)n * nrhs;
         ws->Zp = ws->Qn + (size_t)n * nrhs;
         ws->rho = (double *)(b + oH);
-        ws->brk = (int *)(ws->rho + nrhs);
         ws->done = (int *)(b + oD);
         ws->anorm_bits = (unsigned long long *)(b + oS);
         ws->info = (int *)(b + oS + 8);
         ws->err = (int *)(b + oS + 12);  // read back together with info
+        ws->brk = (int *)(b + oS + 24);
+        ws->ratio = (double *)(b + oS + 32);
     }
     return off;
 }
@@ -908,35 +932,47 @@ int dsposv_refine(cudaStream_t s, int n, int nrhs, const double *A, int lda, con
     cudaMemsetAsync(ws.done, 0, nrhs * sizeof(int), s);
     cudaMemsetAsync(ws.err, 0, sizeof(int), s);
     cudaMemsetAsync(ws.brk, 0, sizeof(int), s);
-    gb300_count_launch(), colmax_exp_kernel<<<nrhs, 256, 0, s>>>(n, B, ldb, ws.rexp);
+    gb300_count_launch(), colmax_exp_kernel<<<nrhs, COL_T, 0, s>>>(n, B, ldb, ws.rexp);
     gb300_count_launch(), to_f32_kernel<<<dim3(gx, nrhs), 256, 0, s>>>(n, nrhs, B, ldb, ws.Y, n, ws.rexp);
     int slot = gb300_prof_begin(s, GB300_PROF_SOLVE);
     correction_solve(s, n, nrhs, nb, ws);
     gb300_prof_end(s, slot, 2.0 * n * (double)n * nrhs, 4.0 * n * (double)n);
     gb300_count_launch(), accumulate_kernel<<<dim3(gx, nrhs), 256, 0, s>>>(n, nrhs, ws.Y, n, X, ldx, 0, nullptr,
                                                                            ws.rexp);
-    double *hberr = (double *)malloc(sizeof(double) * (size_t)nrhs);
+    // the status words and the backward errors, as one block
+    const size_t hoff = (size_t)((char *)ws.berr - (char *)ws.anorm_bits);
+    const size_t hbytes = hoff + sizeof(double) * (size_t)nrhs;
+    std::unique_ptr<char[]> host(new (std::nothrow) char[hbytes]);
+    if (!host) return GB300_ENOMEM;
     int status = GB300_ETIMEDOUT;
     int it = 0, rc = 0;
     const int mode = refine_mode();
     bool pcg = false, restart = true, true_residual = true;
     double hratio = 0.0;
-    if (mode == 2) {  // the factor's pivot ratio, read with the first backward error
-        gb300_count_launch(), pivot_ratio_kernel<<<1, 1024, 0, s>>>(n, ws.W, n, ws.rho);
-        cudaMemcpyAsync(&hratio, ws.rho, sizeof(double), cudaMemcpyDeviceToHost, s);
-    }
-    double worst = INFINITY, prev = INFINITY, best = INFINITY;
+    if (mode == 2)  // the factor's pivot ratio, read with the first backward error
+        gb300_count_launch(), pivot_ratio_kernel<<<1, COL_T, 0, s>>>(n, ws.W, n, ws.ratio);
+    double worst = INFINITY, prev = INFINITY, best = INFINITY, anorm = 0.0;
     int since_best = 0;
     // read the backward errors (and the wait-timeout word) of the step just queued
     auto read_berr = [&](int *herr, int *hbreak) -> int {
-        int r = gb300_record_cuda_error(cudaMemcpyAsync(hberr, ws.berr, sizeof(double) * nrhs,
+        int r = gb300_record_cuda_error(cudaMemcpyAsync(host.get(), ws.anorm_bits, hbytes,
                                                         cudaMemcpyDeviceToHost, s));
-        if (!r) r = gb300_record_cuda_error(cudaMemcpyAsync(herr, ws.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-        if (!r) r = gb300_record_cuda_error(cudaMemcpyAsync(hbreak, ws.brk, sizeof(int), cudaMemcpyDeviceToHost, s));
         if (!r) r = gb300_record_cuda_error(cudaStreamSynchronize(s));
+        if (r) return r;
+        auto word = [&](const void *d, void *h, size_t bytes) {
+            memcpy(h, host.get() + ((const char *)d - (const char *)ws.anorm_bits), bytes);
+        };
+        word(ws.err, herr, sizeof(int));
+        word(ws.brk, hbreak, sizeof(int));
+        word(ws.anorm_bits, &anorm, sizeof anorm);
+        if (mode == 2) word(ws.ratio, &hratio, sizeof hratio);
         worst = 0;
-        for (int j = 0; j < nrhs; ++j) worst = fmax(worst, hberr[j]);
-        return r;
+        for (int j = 0; j < nrhs; ++j) {
+            double e;
+            memcpy(&e, host.get() + hoff + sizeof(double) * (size_t)j, sizeof e);
+            worst = fmax(worst, e);
+        }
+        return 0;
     };
     for (;;) {
         int herr = 0, hbreak = 0;
@@ -947,7 +983,7 @@ int dsposv_refine(cudaStream_t s, int n, int nrhs, const double *A, int lda, con
                                      ws.rtc_a, ws.rtc_xs, ws.anorm_bits, ws.err)))
                 break;
             gb300_prof_end(s, slot, 2.0 * n * (double)n * nrhs, 8.0 * n * (double)n + 32.0 * n * nrhs);
-            gb300_count_launch(), backward_error_kernel<<<nrhs, 256, 0, s>>>(n, ws.R, n, X, ldx, B, ldb,
+            gb300_count_launch(), backward_error_kernel<<<nrhs, COL_T, 0, s>>>(n, ws.R, n, X, ldx, B, ldb,
                                                                              ws.anorm_bits, tol, ws.berr, ws.done,
                                                                              ws.rexp);
             if ((rc = read_berr(&herr, &hbreak))) break;
@@ -1009,19 +1045,13 @@ int dsposv_refine(cudaStream_t s, int n, int nrhs, const double *A, int lda, con
         true_residual = worst <= tol || hbreak;
         if (hbreak) cudaMemsetAsync(ws.brk, 0, sizeof(int), s);
     }
-    free(hberr);
     if (rc) return rc;
     if (out) {
         out->iterations = it;
         out->backward_error = worst;
         out->status = status;
         out->method = pcg ? 1 : 0;
-        unsigned long long ab = 0;
-        cudaMemcpyAsync(&ab, ws.anorm_bits, sizeof ab, cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
-        double an;
-        memcpy(&an, &ab, sizeof an);
-        out->anorm = an;
+        out->anorm = anorm;
     }
     return status;
 }
@@ -1063,7 +1093,7 @@ int dsposv_fp64(cudaStream_t s, int n, int nrhs, const double *A, int lda, const
     if ((rc = residual_mixed(s, n, nrhs, A, lda, X, ldx, B, ldb, ws.R, n, ws.partials, ws.xs, ws.sx, ws.rtc_a,
                              ws.rtc_xs, ws.anorm_bits, ws.err)))
         return rc;
-    gb300_count_launch(), backward_error_kernel<<<nrhs, 256, 0, s>>>(n, ws.R, n, X, ldx, B, ldb, ws.anorm_bits, tol,
+    gb300_count_launch(), backward_error_kernel<<<nrhs, COL_T, 0, s>>>(n, ws.R, n, X, ldx, B, ldb, ws.anorm_bits, tol,
                                                                      ws.berr, ws.done, nullptr);
     std::vector<double> hb((size_t)nrhs);
     unsigned long long ab = 0;
@@ -1604,7 +1634,7 @@ int starpu_gb300_backward_error(void *stream, int n, int nrhs, const double *A, 
     cudaMemsetAsync(an, 0, sizeof *an, s);
     gb300_count_launch(), convert_lower_norm_kernel<<<n, 256, 0, s>>>(n, A, lda, nullptr, 0, an);
     residual_f64(s, n, nrhs, A, lda, X, ldx, B, ldb, R, n, partials);
-    gb300_count_launch(), backward_error_kernel<<<nrhs, 256, 0, s>>>(n, R, n, X, ldx, B, ldb, an, 0.0, berr, done, nullptr);
+    gb300_count_launch(), backward_error_kernel<<<nrhs, COL_T, 0, s>>>(n, R, n, X, ldx, B, ldb, an, 0.0, berr, done, nullptr);
     int rc = gb300_record_cuda_error(cudaMemcpyAsync(berr_host, berr, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, s));
     if (rc) return rc;
     return gb300_record_cuda_error(cudaStreamSynchronize(s));

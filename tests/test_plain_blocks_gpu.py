@@ -3,6 +3,8 @@ blocking changes: leaf and panel remainders, the row counts that pick the
 panel solve's slab, the product tiles, the solve's block and column groups,
 and the FP64 update on the tensor cores (tile, segment and row-block edges).
 Reference: numpy in FP64."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -206,3 +208,31 @@ def test_potrs_many_columns_graded(gpu, n, nrhs):
     x = db.download((n, nrhs), np.float64)
     y = np.abs(l.T) @ np.abs(x)
     assert np.all(np.abs(l @ (l.T @ x) - b) <= 8 * n * EPS[np.float64] * (np.abs(l) @ y + np.abs(b)))
+
+
+@pytest.mark.parametrize("n,nrhs,extreme", [(1, 1, None), (33, 3, None), (1023, 2, None), (1025, 5, None),
+                                            (1500, 2, np.nan), (1500, 2, np.inf)])
+def test_backward_error_column_maxima(gpu, n, nrhs, extreme):
+    rng = np.random.default_rng(n)
+    a = rng.uniform(-1, 1, (n, n))
+    a = np.tril(a) + np.tril(a, -1).T
+    x, b = rng.uniform(-1, 1, (n, nrhs)), rng.uniform(-3, 3, (n, nrhs))
+    x[n - 1, 0], b[n // 2, nrhs - 1] = -5.0, 9.0  # maxima in the last row and in the middle
+    if extreme is not None:
+        b[7, 1] = extreme
+    with np.errstate(invalid="ignore"):
+        r = np.abs(b - a @ x)
+    anorm = np.abs(a).sum(1).max()
+    ref = np.nanmax(r, 0) / (anorm * np.abs(x).max(0) + np.nanmax(np.abs(b), 0))  # NaN entries do not count
+    da, dx, db = up(a), up(x), up(b)
+    gpu.starpu_gb300_backward_error_workspace.restype = ctypes.c_size_t
+    lwork = gpu.starpu_gb300_backward_error_workspace(n, nrhs)
+    work, got = DeviceBuffer(lwork), (ctypes.c_double * nrhs)()
+    vp = ctypes.c_void_p
+    check(gpu.starpu_gb300_backward_error(vp(), n, nrhs, vp(da.ptr), n, vp(dx.ptr), n, vp(db.ptr), n, vp(work.ptr),
+                                          ctypes.c_size_t(lwork), got))
+    got = np.array(got)
+    finite = np.isfinite(ref)
+    # both residuals are within (n + 2) u of (|A| |x| + |b|), the denominator's bound
+    assert np.all(np.abs(got - ref)[finite] <= 4 * (n + 2) * EPS[np.float64])
+    assert np.all(np.isnan(got[~finite]))  # inf / inf
