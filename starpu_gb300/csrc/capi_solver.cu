@@ -587,42 +587,41 @@ static void tile_sweeps(cudaStream_t s, int n, int nrhs, int nb, const float *L,
     a.budget_ns = gb300_wait_budget_ns();
     // persistent CTAs: as many as fit on the device, and at least one per slab
     // of a tile row (the diagonal tasks of a tile row wait for one another)
-    const void *fns[3] = {(const void *)tile_sweep_kernel<false, false>, (const void *)tile_sweep_kernel<true, false>,
-                          (const void *)tile_sweep_kernel<true, true>};
-    static thread_local int per_sm[16][3];
+    using Fn = void (*)(TileSweepArgs);
+    static const Fn fns[3][2] = {{tile_sweep_kernel<false, 4>, tile_sweep_kernel<true, 4>},
+                                 {tile_sweep_kernel<false, 8>, tile_sweep_kernel<true, 8>},
+                                 {tile_sweep_kernel<false, 16>, tile_sweep_kernel<true, 16>}};
+    const int warps = tsw_warps(nb), w = warps == 4 ? 0 : warps == 8 ? 1 : 2, smem = tsw_dsmem(warps);
+    static thread_local int per_sm[16][3][2];
     int dev = 0;
     cudaGetDevice(&dev);
-    int *per = per_sm[dev & 15];
+    int *per = per_sm[dev & 15][w];
     if (!per[0]) {
-        // the table is filled only once all three kernels are set up
-        int occ[3];
-        for (int i = 0; i < 3; ++i) {
-            if (gb300_func_dyn_smem(fns[i], TSW_DSMEM) ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[i], fns[i], TSW_T, TSW_DSMEM) != cudaSuccess) {
+        // the table is filled only once both kernels are set up
+        int occ[2];
+        for (int i = 0; i < 2; ++i) {
+            if (gb300_func_dyn_smem((const void *)fns[w][i], smem) ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[i], fns[w][i], 32 * warps, smem) != cudaSuccess) {
                 // the kernels cannot run on this device: report it in the error word
                 if (err) cudaMemsetAsync(err, 1, 1, s);
                 return;
             }
         }
-        for (int i = 2; i >= 0; --i) per[i] = std::max(occ[i], 1);
+        for (int i = 1; i >= 0; --i) per[i] = std::max(occ[i], 1);
     }
     const int sms = gb300_device_sms();
-    auto grid = [&](int which) {
-        const long g = std::min<long>((long)a.total, (long)per[which] * sms);
-        return (unsigned)std::max<long>(g, a.spt);
-    };
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    const bool vec = al(L) && al(band) && (!band_t || al(band_t)) && ldl % 4 == 0 && ldk % 4 == 0;
+    a.vec_l = al(L) && ldl % 4 == 0;
+    a.vec_d = al(band) && (!band_t || al(band_t)) && ldk % 4 == 0;
     const size_t cbytes = (3 * (size_t)a.ntiles + 1) * sizeof(int);
     for (int c0 = 0; c0 < nrhs; c0 += 16) {
         a.nrhs = std::min(16, nrhs - c0);
         a.B = Y + (long)c0 * ldy;
-        a.vec = vec;
-        cudaMemsetAsync(cnt, 0, cbytes, s);
-        gb300_count_launch(), tile_sweep_kernel<false, false><<<grid(0), TSW_T, TSW_DSMEM, s>>>(a);
-        cudaMemsetAsync(cnt, 0, cbytes, s);
-        if (upper) gb300_count_launch(), tile_sweep_kernel<true, true><<<grid(2), TSW_T, TSW_DSMEM, s>>>(a);
-        else gb300_count_launch(), tile_sweep_kernel<true, false><<<grid(1), TSW_T, TSW_DSMEM, s>>>(a);
+        for (int back = 0; back < 2; ++back) {
+            const long g = std::max<long>(std::min<long>((long)a.total, (long)per[back] * sms), a.spt);
+            cudaMemsetAsync(cnt, 0, cbytes, s);
+            gb300_count_launch(), fns[w][back]<<<(unsigned)g, 32 * warps, smem, s>>>(a);
+        }
     }
 }
 

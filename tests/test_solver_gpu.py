@@ -349,6 +349,32 @@ def test_spotrs_inv_tiles_matches_fp64_triangular_solves(gpu, oracle, n, nb, nrh
     assert np.max(np.abs(outs[0] - ref)) / np.max(np.abs(ref)) < 2e-5
 
 
+@pytest.mark.parametrize("n,nb,nrhs", [(1537, 512, 17), (1600, 480, 16), (1025, 1024, 2), (13 * 1024 + 36, 1024, 3)])
+def test_spotrs_inv_tiles_cta_sizes_and_long_rows(gpu, n, nb, nrhs):
+    """Tile orders on either side of the CTA sizes, rows of L off the 16-byte
+    grid, and tile rows long enough that a CTA takes tickets ahead."""
+    from scipy.linalg import solve_triangular
+    rng = np.random.default_rng(n)
+    L32 = np.asfortranarray(np.tril(rng.uniform(-1, 1, (n, n)).astype(np.float32) / n, -1))
+    L32[np.arange(n), np.arange(n)] = rng.uniform(1, 2, n)
+    band, ldd = inv_tile_band(L32, nb)
+    B = rng.uniform(-1, 1, (n, nrhs)).astype(np.float32)
+    dL, dD, dB = DeviceBuffer.from_array(L32), DeviceBuffer.from_array(band), DeviceBuffer.from_array(B)
+    lw = gpu.starpu_gb300_spotrs_inv_tiles_workspace(n, nb)
+    W, err = DeviceBuffer(lw), DeviceBuffer.from_array(np.zeros(1, np.int32))
+    check(gpu.starpu_gb300_spotrs_inv_tiles(None, n, nrhs, nb, dL.ptr, n, dD.ptr, ldd, dB.ptr, n, W.ptr, lw, err.ptr))
+    out = dB.download((n, nrhs), np.float32)
+    assert err.download((1,), np.int32)[0] == 0
+    L64 = L32.astype(np.float64)
+    y = solve_triangular(L64, B.astype(np.float64), lower=True, check_finite=False)
+    ref = solve_triangular(L64, y, lower=True, trans=1, check_finite=False)
+    # rows of |L| off the diagonal sum to about 1/2 (diagonal 1 .. 2), so a sweep at
+    # most doubles an error; a row's error is (16 MMA steps + 16 warps + tile rows) 2^-24
+    # + 3 2^-21 of its sum
+    depth = 32 + (n + nb - 1) // nb
+    assert np.max(np.abs(out - ref)) <= 4 * (depth * 2.0**-24 + 3 * 2.0**-21) * np.max(np.abs(B)) * 2
+
+
 def test_spotrs_inv_tiles_rejects_bad_tiles(gpu):
     assert gpu.starpu_gb300_spotrs_inv_tiles_workspace(100, 48) == 0  # nb not a multiple of 32
     assert gpu.starpu_gb300_spotrs_inv_tiles(None, 100, 1, 48, None, 100, None, 64, None, 100, None, 0, None) == -22
