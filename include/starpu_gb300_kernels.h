@@ -14,6 +14,9 @@
  * Numeric failure (a non-positive pivot) is not a return code: it is written
  * to the device status word *d_info (LAPACK convention: 0 = success, k > 0 =
  * the leading minor of order k is not positive definite) without trapping.
+ * Kernels that hand work on between warps or CTAs bound every wait; one that
+ * runs out (it cannot on a healthy device) leaves a negative *d_info and an
+ * unspecified result.
  */
 #ifndef STARPU_GB300_KERNELS_H
 #define STARPU_GB300_KERNELS_H

@@ -218,14 +218,6 @@ __global__ void __launch_bounds__(COL_T) colmax_exp_kernel(int n, const double *
     if (threadIdx.x == 0) exps[blockIdx.x] = column_exp(__longlong_as_double((long long)b));
 }
 
-// R = B (copy) before the GEMM R -= A X
-__global__ void copy_f64_kernel(int n, const double *__restrict__ B, long ldb, double *__restrict__ R, long ldr)
-{
-    const long j = blockIdx.y;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        R[i + j * ldr] = B[i + j * ldb];
-}
-
 // R = B + sum_z P_z, the K-split partials of -A X, added in a fixed order
 // (B null: R = -A X, the product the conjugate-gradient steps need)
 __global__ void residual_reduce_kernel(int n, int nrhs, int nk, const double *__restrict__ B, long ldb,

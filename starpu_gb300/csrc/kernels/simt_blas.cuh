@@ -295,34 +295,4 @@ __global__ void __launch_bounds__(256, 2) gemm_nt_f32_kernel(int m, int n, int k
     }
 }
 
-// ---------------------------------------------------------------------------
-// Elementwise helpers.
-// ---------------------------------------------------------------------------
-template <typename TO, typename TI>
-__global__ void convert_lower_kernel(int n, const TI *__restrict__ in, long ldi, TO *__restrict__ out, long ldo, int lower_only)
-{
-    const long j = blockIdx.y;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        if (lower_only && i < j) continue;
-        out[i + j * ldo] = (TO)in[i + j * ldi];
-    }
-}
-
-template <typename TO, typename TI>
-__global__ void convert_rect_kernel(int m, int n, const TI *__restrict__ in, long ldi, TO *__restrict__ out, long ldo)
-{
-    const long j = blockIdx.y;
-    if (j >= n) return;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (long)gridDim.x * blockDim.x)
-        out[i + j * ldo] = (TO)in[i + j * ldi];
-}
-
-template <typename T>
-__global__ void zero_upper_kernel(int n, T *__restrict__ A, long lda)
-{
-    const long j = blockIdx.y;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < j && i < n; i += (long)gridDim.x * blockDim.x)
-        A[i + j * lda] = T(0);
-}
-
 } // namespace gb300
