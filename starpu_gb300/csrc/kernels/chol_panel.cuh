@@ -261,8 +261,8 @@ static __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, float *__
 // (Four warps, one per unit, so that nothing shares a unit with the chain, took
 // 3 us more: each warp then trails its own backlog.)
 template <int H0>  // columns 32 H0 .. 32 H0 + 31, rows 32 H0 .. 63
-__device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*col)[CP_W], uint64_t *bar, int n, int *info,
-                                               int info_base)
+__device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*col)[CP_W], double2 *pv, uint64_t *bar, int n,
+                                               int *info, int info_base)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bool ok = true;
@@ -306,6 +306,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
                 col[mine][32 * h + lane] = a[H0][q][h];
             }
             ptx::mbar_arrive(&bar[mine]);
+            if (lane == 0) pv[mine] = make_double2(piv, r);
             if (!(piv > 0.0) && lane == 0 && info) atomicCAS(info, 0, info_base + mine + 1);
             __syncwarp();
             if (w > 0) rest(mine - 1, q + 1);
@@ -324,6 +325,7 @@ static __global__ void __launch_bounds__(256)
 potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_base)
 {
     __shared__ double col[CP_W][CP_W];
+    __shared__ double2 pv[CP_W];  // pivots and the factors their columns were scaled with
     __shared__ uint64_t bar[CP_W];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double a[2][4][2];  // [half of the columns][q][row half]: column 32 g + 4 q + w
@@ -339,12 +341,18 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
     };
     each([&](double &v, int r, int c) { v = r < n && c <= r ? A[r + (long)c * lda] : 0.0; });
     __syncthreads();
-    bool ok = cp_leaf64_half<0>(a, col, bar, n, info, info_base);
-    if (n > 32) ok = cp_leaf64_half<1>(a, col, bar, n, info, info_base) && ok;
+    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base);
+    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base) && ok;
     if (!ok && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
     each([&](double &v, int r, int c) {
-        if (r < n && c <= r) A[r + (long)c * lda] = v;
+        if (r < n && c < r) A[r + (long)c * lda] = v;
     });
+    // the diagonal, sqrt(pivot): the product is off by up to an ulp, one step makes it exact
+    __syncthreads();
+    if (threadIdx.x < n) {
+        const double d = pv[threadIdx.x].x, r = pv[threadIdx.x].y, l = d * r;
+        A[threadIdx.x * (lda + 1)] = cp_normal(d) ? fma(fma(-l, l, d), 0.5 * r, l) : sqrt(d);
+    }
 }
 
 // ---------------------------------------------------------------------------

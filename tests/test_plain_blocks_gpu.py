@@ -236,3 +236,15 @@ def test_backward_error_column_maxima(gpu, n, nrhs, extreme):
     # both residuals are within (n + 2) u of (|A| |x| + |b|), the denominator's bound
     assert np.all(np.abs(got - ref)[finite] <= 4 * (n + 2) * EPS[np.float64])
     assert np.all(np.isnan(got[~finite]))  # inf / inf
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64])
+def test_dpotrf_leaf_diagonal_is_the_square_root(gpu, n):
+    d = np.random.default_rng(n).uniform(1e-3, 1e3, n)
+    d[0] = 5e-320  # below the normal range: the plain functions
+    da, info = up(np.diag(d)), up(np.zeros(1, np.int32))
+    check(gpu.starpu_gb300_dpotrf_tile(None, n, da.ptr, n, info.ptr))
+    assert info.download((1,), np.int32)[0] == 0
+    got, ref = np.diag(da.download((n, n), np.float64)), np.sqrt(d)
+    # half an ulp, and the residual's and the step's rounding (2^-53 of the ulp-sized step)
+    assert np.all(np.abs(got - ref) <= np.spacing(ref))
