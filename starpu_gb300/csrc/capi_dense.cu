@@ -81,21 +81,26 @@ static long gemm_ctas(bool lower, int m, int n, int bm)
 
 static bool aligned16(const float *p, long ld) { return ((uintptr_t)p & 15) == 0 && (ld & 3) == 0; }
 
-static void gemm_nt_f32(cudaStream_t s, bool lower, int m, int n, int k, float alpha, const float *A, long lda,
-                        const float *B, long ldb, float beta, float *C, long ldc)
+template <bool TB>
+static void gemm_f32(cudaStream_t s, bool lower, int m, int n, int k, float alpha, const float *A, long lda,
+                     const float *B, long ldb, float beta, float *C, long ldc)
 {
     const unsigned tm = cdiv(m, 128), tn = cdiv(n, 128);
-    if (lower)
-        gb300_count_launch(), gemm_nt_f32_kernel<true>
+    if (TB && lower)
+        gb300_count_launch(), gemm_f32_kernel<true, true>
             <<<tm * (tm + 1) / 2, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
     else
-        gb300_count_launch(), gemm_nt_f32_kernel<false>
+        gb300_count_launch(), gemm_f32_kernel<false, TB>
             <<<dim3(tm, tn), 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }
 
-// FP32: 128x128 block tiles, 8x8 per thread, when they make at least half a
-// wave; smaller ones otherwise (the 64 and 32 tiles take a third and an eighth
-// of the 128 tile's time each, so up to two waves of them are faster).
+// FP32: 128x128 block tiles, 8x8 per thread, from 64 of them on; smaller ones
+// otherwise (the 64 and 32 tiles take a third and an eighth of the 128 tile's
+// time each, so up to two waves of them are faster).  Alone, a 1024^3 product is
+// faster in 64 tiles (86 us against 108) and a 512^3 one in 32 tiles (27 and 33),
+// but a task graph runs eight of them side by side, where a third or a half
+// more work per product counts: LU of order 16384 takes 218 ms in 32 x 32 tiles,
+// 307 with smaller product tiles, and 143 and 164 ms in 16 x 16.
 // Narrow variant for few columns.
 template <> struct simt_cfg<float> {
     template <bool TA, bool TB>
@@ -104,11 +109,11 @@ template <> struct simt_cfg<float> {
     {
         if (!lower && n <= 32)
             gemm_launch<float, TA, TB, 128, 32, 8, 8, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else if (!TA && TB && gemm_ctas(lower, m, n, 128) > 76 && aligned16(A, lda) && aligned16(B, ldb) && aligned16(C, ldc))
-            gemm_nt_f32(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else if (gemm_ctas(lower, m, n, 128) > 76)
+        else if (!TA && gemm_ctas(lower, m, n, 128) >= 64 && aligned16(A, lda) && aligned16(B, ldb) && aligned16(C, ldc))
+            gemm_f32<TB>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
+        else if (gemm_ctas(lower, m, n, 128) >= 64)
             gemm_launch<float, TA, TB, 128, 128, 8, 8, 8>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else if (gemm_ctas(lower, m, n, 64) > 76)
+        else if (gemm_ctas(lower, m, n, 64) >= 64)
             gemm_launch<float, TA, TB, 64, 64, 16, 4, 4>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
         else
             gemm_launch<float, TA, TB, 32, 32, 32, 2, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);

@@ -182,17 +182,19 @@ gemm_simt_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long lda
 }
 
 // ---------------------------------------------------------------------------
-// The FP32 N,T product C = beta C + alpha A B^T for large matrices: the same
-// sums in the same order as gemm_simt_kernel's 128 x 128 tile (thread = 8 x 8,
-// k ascending), with the operands read 16 bytes at a time, 16 k per barrier and
-// whole tiles stored without per-element tests: the scalar form spent a third of
-// its issue slots on addresses and tests.  A, B and C 16-byte aligned with
-// leading dimensions divisible by 4.
+// The FP32 products C = beta C + alpha A B^T (TB) and beta C + alpha A B for
+// large matrices: the same sums in the same order as gemm_simt_kernel's 128 x
+// 128 tile (thread = 8 x 8, k ascending), with the operands read 16 bytes at a
+// time, 16 k per barrier and whole tiles stored without per-element tests: the
+// scalar form spent a third of its issue slots on addresses and tests (order
+// 2048: A B^T 474 -> 362 us, A B 474 -> 411; B's columns are turned on the way
+// into shared memory).  A, B and C 16-byte aligned with leading dimensions
+// divisible by 4.
 // ---------------------------------------------------------------------------
-template <bool LOWER>
-__global__ void __launch_bounds__(256, 2) gemm_nt_f32_kernel(int m, int n, int k, float alpha, const float *__restrict__ A,
-                                                             long lda, const float *__restrict__ B, long ldb, float beta,
-                                                             float *__restrict__ C, long ldc)
+template <bool LOWER, bool TB>
+__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int m, int n, int k, float alpha, const float *__restrict__ A,
+                                                          long lda, const float *__restrict__ B, long ldb, float beta,
+                                                          float *__restrict__ C, long ldc)
 {
     constexpr int BM = 128, BK = 16, LD = BM + 4;
     __shared__ __align__(16) float As[2][BK][LD], Bs[2][BK][LD];
@@ -211,7 +213,10 @@ __global__ void __launch_bounds__(256, 2) gemm_nt_f32_kernel(int m, int n, int k
     const int m0 = bi * BM, n0 = bj * BM, tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
     // this thread's loads: 4 rows from 4 (tid % 32), k = tid / 32 and + 8
     const int lr = 4 * (tid & 31), lk = tid >> 5;
-    const float *pa = A + m0 + lr + (long)lk * lda, *pb = B + n0 + lr + (long)lk * ldb;
+    // (B not transposed: 4 k from 4 (tid % 4), columns tid / 4 and + 64)
+    const int bk = 4 * (tid & 3), bc = tid >> 2;
+    const float *pa = A + m0 + lr + (long)lk * lda;
+    const float *pb = TB ? B + n0 + lr + (long)lk * ldb : B + bk + (long)(n0 + bc) * ldb;
     const bool wa = m0 + BM <= m, wb = n0 + BM <= n;
     float4 ra[2], rb[2];
     auto load4 = [](const float *p, bool whole, int rows, bool in) {
@@ -230,14 +235,22 @@ __global__ void __launch_bounds__(256, 2) gemm_nt_f32_kernel(int m, int n, int k
         for (int q = 0; q < 2; ++q) {
             const bool in = k0 + lk + 8 * q < k;
             ra[q] = load4(pa + (long)(k0 + 8 * q) * lda, wa, m - m0 - lr, in);
-            rb[q] = load4(pb + (long)(k0 + 8 * q) * ldb, wb, n - n0 - lr, in);
+            if (TB) rb[q] = load4(pb + (long)(k0 + 8 * q) * ldb, wb, n - n0 - lr, in);
+            else rb[q] = load4(pb + k0 + (long)(64 * q) * ldb, k0 + BK <= k, k - k0 - bk, n0 + bc + 64 * q < n);
         }
     };
     auto store = [&](int buf) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             *reinterpret_cast<float4 *>(&As[buf][lk + 8 * q][lr]) = ra[q];
-            *reinterpret_cast<float4 *>(&Bs[buf][lk + 8 * q][lr]) = rb[q];
+            if (TB) {
+                *reinterpret_cast<float4 *>(&Bs[buf][lk + 8 * q][lr]) = rb[q];
+            } else {
+                Bs[buf][bk][bc + 64 * q] = rb[q].x;
+                Bs[buf][bk + 1][bc + 64 * q] = rb[q].y;
+                Bs[buf][bk + 2][bc + 64 * q] = rb[q].z;
+                Bs[buf][bk + 3][bc + 64 * q] = rb[q].w;
+            }
         }
     };
     float acc[8][8];

@@ -84,6 +84,18 @@ def test_product_tiles(gpu, dtype, m, n, k, lower):
     assert np.array_equal(out[~keep], c[~keep])
 
 
+# k a multiple of 4 with a remainder of 16, ragged tiles; ld of B (k) and of A and C (m) off the 16-byte grid
+@pytest.mark.parametrize("m,n,k", [(1024, 1024, 32), (1100, 1033, 36), (1156, 1000, 4), (1028, 1030, 33), (1027, 1024, 64), (1024, 1, 8)])
+def test_product_nn_tiles(gpu, m, n, k):
+    rng = np.random.default_rng(m + k)
+    a, b, c = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, n), (m, n)))
+    da, db, dc = up(a), up(b), up(c)
+    check(gpu.starpu_gb300_sgemm_nn_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, k, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float32).astype(np.float64)
+    a, b, c = (v.astype(np.float64) for v in (a, b, c))
+    assert np.all(np.abs(out - (c - a @ b)) <= (k + 2) * EPS[np.float32] * (np.abs(c) + np.abs(a) @ np.abs(b)))
+
+
 @BOTH
 @pytest.mark.parametrize("n,nb", [(63, 64), (65, 16), (127, 64), (191, 64), (192, 512), (193, 512), (321, 100), (700, 512), (1281, 256), (3001, 512), (4097, 1024)])
 def test_potrf_blocks(gpu, dtype, n, nb):
