@@ -577,8 +577,8 @@ static void tile_sweeps(cudaStream_t s, int n, int nrhs, int nb, const float *L,
     a.err = err;
     a.upper = upper;
     a.budget_ns = gb300_wait_budget_ns();
-    // persistent CTAs: as many as fit on the device, and at least one per slab
-    // of a tile row (the diagonal tasks of a tile row wait for one another)
+    // persistent CTAs: as many as fit on the device (fewer may run at a time
+    // beside other kernels), and at least one per slab of a tile row
     using Fn = void (*)(TileSweepArgs);
     static const Fn fns[3][2] = {{tile_sweep_kernel<false, 4>, tile_sweep_kernel<true, 4>},
                                  {tile_sweep_kernel<false, 8>, tile_sweep_kernel<true, 8>},

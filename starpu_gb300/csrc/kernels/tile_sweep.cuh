@@ -19,13 +19,13 @@
 // then its diagonal tasks, then tile row u + 1.  The products of a tile row
 // therefore spread over all CTAs, and the chain of a tile row is one product
 // with the newest tile row, one product with the inverse and the two
-// hand-overs between them.  A CTA waits only on tasks with smaller tickets or,
-// in a diagonal task, on the other diagonal tasks of its tile row, which
-// publish before they wait.  While it works on a product a CTA holds the next
-// ticket too, in long tile rows the next two (operands are loaded meanwhile),
-// but never while it works on a diagonal task: the smallest unfinished ticket is always being worked on, and
-// with at least as many CTAs as slabs per tile row the sweep cannot deadlock
-// however CTAs are scheduled.  Every wait is bounded by a %globaltimer budget;
+// hand-overs between them.  A CTA waits only on tasks with smaller tickets: the
+// s of a tile row are claimed one by one, normally one by each diagonal task,
+// but a waiting task claims those that nobody works on.  While it works on a
+// product a CTA holds the next ticket too, in long tile rows the next two
+// (operands are loaded meanwhile); the smallest unfinished ticket is always
+// being worked on, so the sweep cannot deadlock however few CTAs run at a time
+// and however they are scheduled beside other kernels.  Every wait is bounded by a %globaltimer budget;
 // on timeout the CTA records an error and stops waiting, so the launch ends.
 //
 // The products M (32 x K) V (K x 16), K <= nb, run on the tensor cores with
@@ -46,7 +46,7 @@
 // Against a 6-stage cp.async ring for both operands, 8 warps, two rounded
 // conversions a split and z exchanged on the chain: a product of 32 x 1024 took
 // 8 us behind its flag (two CTAs on an SM 13 us) and a sweep 19 us at n =
-// 1024, 115 at 4096, 1170 at 32768.  So: 3 us, and 15, 57 and 735 us (a
+// 1024, 115 at 4096, 1170 at 32768.  So: 3 us, and 15, 60 and 760 us (a
 // sweep's factor is 2.1 GB there: 0.32 ms of DRAM time; what is left is the
 // products' own latency with one CTA of 128 registers a thread on an SM).
 #pragma once
@@ -81,7 +81,8 @@ struct TileSweepArgs {
     const float *DinvT;  // optional: tile T's inverse transposed at DinvT + T * dstride (ld ldd)
     unsigned *ticket;
     // per tile row of the solve order, zero at launch.  pcount: products of the
-    // tile rows before the newest in the low half, of the newest in the high
+    // tile rows before the newest in the low half, of the newest in the high;
+    // zcount: slabs whose s is there in the low half, slabs claimed in the high
     int *zcount, *ycount, *pcount;
     int *err;
     unsigned long long budget_ns;
@@ -148,6 +149,31 @@ __device__ __forceinline__ void tsw_wait(const TileSweepArgs &a, const int *cnt,
         }
         __nanosleep(20);
     }
+}
+
+// Thread 0 waits until the s of every slab of a tile row is there (low half of
+// *cnt; slabs claimed in the high half): -1.  Where some stay unclaimed for 20 us
+// -- the CTAs that hold those diagonal tasks are not running yet, because other
+// kernels hold their SMs -- it claims one more: its number.
+__device__ __forceinline__ int tsw_wait_slabs(const TileSweepArgs &a, int *cnt, bool &skip)
+{
+    uint64_t t0 = 0;
+    while (!skip) {
+        const int w = tsw_ld_acquire(cnt);
+        if ((w & 0xffff) >= a.spt) break;
+        const uint64_t t = tsw_timer();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > 20000 && (w >> 16) < a.spt) {
+            const int slab = atomicAdd(cnt, 0x10000) >> 16;
+            if (slab < a.spt) return slab;
+        }
+        if (*(volatile int *)a.err || t - t0 > a.budget_ns) {
+            atomicCAS(a.err, 0, 1);
+            skip = true;
+        }
+        __nanosleep(20);
+    }
+    return -1;
 }
 
 // Every thread's stores become visible with the count (raised by the last
@@ -472,9 +498,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W) tile_sweep_kernel(TileSweepArg
             loaded = tn < a.total;
             if (loaded) tsw_task<TRANS, W>(a, t, tn, true, k);
             t = tn;
-            // a further ticket only if the next task is a product (no CTA
-            // holds one while it works on a diagonal task) of a tile row with
-            // two rounds of them or more: it saves the ticket's and V's latency
+            // a further ticket only if the next task is a product of a tile
+            // row with two rounds of them or more: it saves the ticket's and V's latency
             // a product (n = 32768: 860 us without, 730 with), but in a short
             // row delays a product the chain waits for (8192: 111 and 122 us)
             ahead = loaded && k.v < k.u && (unsigned)(k.u * a.spt) >= 2 * gridDim.x;
@@ -491,25 +516,37 @@ __global__ void __launch_bounds__(32 * W, 16 / W) tile_sweep_kernel(TileSweepArg
             tsw_publish(&a.pcount[c.u], c.v == c.u - 1 ? 0x10000 : 1);
             if (!loaded) return;
         } else {
-            // s = b - the products of the tile rows before the newest
-            if (k.u > 1 && tid == 0) tsw_wait(a, &a.pcount[k.u], 0, 0xffff, (k.u - 1) * a.spt, skip);
+            // s = b - the products of the tile rows before the newest, of the
+            // next slab of the tile row that nobody has claimed
+            if (tid == 0) {
+                s_ticket = (unsigned)atomicAdd(&a.zcount[k.u], 0x10000) >> 16;
+                if (k.u > 1) tsw_wait(a, &a.pcount[k.u], 0, 0xffff, (k.u - 1) * a.spt, skip);
+            }
             __syncthreads();  // (red has been read, too)
             const float *P = a.Zp + (long)k.u * (k.u - 1) / 2 * (long)a.nb * 16;
+            for (int slab = (int)s_ticket; slab >= 0;) {
+                if (slab < a.spt) {
+                    const int c0 = slab * TSW_SLAB;
 #pragma unroll
-            for (int e = tid; e < 512; e += NT) {
-                const int r = e >> 4, c = e & 15;
-                if (r < k.op.rows && c < a.nrhs) {
-                    const float b = __ldcg(&a.B[(long)(k.r0 + r) + (long)c * a.ldb]);
-                    const float *Ps = P + (long)k.s * TSW_SLAB * 16 + e;
-                    float sum = 0.0f;
+                    for (int e = tid; e < 512; e += NT) {
+                        const int r = c0 + (e >> 4), c = e & 15;
+                        if (r < k.kbT && c < a.nrhs) {
+                            const float b = __ldcg(&a.B[(long)(k.t0 + r) + (long)c * a.ldb]);
+                            const float *Ps = P + (long)c0 * 16 + e;
+                            float sum = 0.0f;
 #pragma unroll 8
-                    for (int v = 0; v < k.u - 1; ++v) sum += __ldcg(Ps + (long)v * a.nb * 16);
-                    a.Zt[(long)(k.r0 + r) * 16 + c] = b - sum;
+                            for (int v = 0; v < k.u - 1; ++v) sum += __ldcg(Ps + (long)v * a.nb * 16);
+                            a.Zt[(long)(k.t0 + r) * 16 + c] = b - sum;
+                        }
+                    }
+                    tsw_publish(&a.zcount[k.u], 1);
+                } else {
+                    __syncthreads();  // s_ticket has been read
                 }
+                if (tid == 0) s_ticket = (unsigned)tsw_wait_slabs(a, &a.zcount[k.u], skip);
+                __syncthreads();
+                slab = (int)s_ticket;
             }
-            tsw_publish(&a.zcount[k.u], 1);
-            if (tid == 0) tsw_wait(a, &a.zcount[k.u], 0, 0x7fffffff, a.spt, skip);
-            __syncthreads();
             float *zb = k.u > 0 ? sb : vb;
             tsw_load_v<W>(zb, a.Zt + (long)k.v0 * 16, k.op.K);
             if (k.u > 0) {

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from starpu_gb300 import DeviceBuffer
-from starpu_gb300.native import IrInfo, check
+from starpu_gb300.native import IrInfo, Stream, check
 
 pytestmark = pytest.mark.gpu
 
@@ -373,6 +373,35 @@ def test_spotrs_inv_tiles_cta_sizes_and_long_rows(gpu, n, nb, nrhs):
     # + 3 2^-21 of its sum
     depth = 32 + (n + nb - 1) // nb
     assert np.max(np.abs(out - ref)) <= 4 * (depth * 2.0**-24 + 3 * 2.0**-21) * np.max(np.abs(B)) * 2
+
+
+def test_spotrs_inv_tiles_on_many_streams(gpu):
+    """Sweeps that share the SMs, each with fewer of its CTAs running than a tile
+    row has slabs: every result as alone."""
+    n, nb, nrhs, many = 2100, 1024, 4, 8
+    rng = np.random.default_rng(5)
+    L32 = np.asfortranarray(np.tril(rng.uniform(-1, 1, (n, n)).astype(np.float32) / n, -1))
+    L32[np.arange(n), np.arange(n)] = rng.uniform(1, 2, n)
+    band, ldd = inv_tile_band(L32, nb)
+    dL, dD = DeviceBuffer.from_array(L32), DeviceBuffer.from_array(band)
+    B = rng.uniform(-1, 1, (n, nrhs)).astype(np.float32)
+    lw = gpu.starpu_gb300_spotrs_inv_tiles_workspace(n, nb)
+    err = DeviceBuffer.from_array(np.zeros(1, np.int32))
+
+    def solve(streams):
+        xs, works = [DeviceBuffer.from_array(B) for _ in streams], [DeviceBuffer(lw) for _ in streams]
+        for _ in range(3):  # three right-hand sides in turn: B, A^-1 B, A^-2 B
+            for s, x, w in zip(streams, xs, works):
+                check(gpu.starpu_gb300_spotrs_inv_tiles(s.handle, n, nrhs, nb, dL.ptr, n, dD.ptr, ldd, x.ptr, n, w.ptr, lw,
+                                                        err.ptr))
+        for s in streams:
+            s.sync()
+        return [x.download((n, nrhs), np.float32) for x in xs]
+
+    alone = solve([Stream()])[0]
+    for x in solve([Stream() for _ in range(many)]):
+        np.testing.assert_array_equal(x, alone)
+    assert err.download((1,), np.int32)[0] == 0
 
 
 def test_spotrs_inv_tiles_rejects_bad_tiles(gpu):
