@@ -38,7 +38,7 @@ static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const 
     a.C = C, a.ldc = ldc, a.m = m, a.n = n, a.k = k, a.lower = lower ? 1 : 0;
     a.col_tiles = (n + SU_BN - 1) / SU_BN;
     a.err = err;
-    a.wait_budget_ns = 2000000000ull;  // 2 s per wait: far above any legitimate stall
+    a.wait_budget_ns = gb300_wait_budget_ns();
     a.total = 0;
     for (int rb = 0; rb * SU_BM < m; ++rb)
         a.total += lower ? std::min(a.col_tiles, (SU_BM / SU_BN) * (rb + 1)) : a.col_tiles;

@@ -69,6 +69,7 @@ constexpr int SU_SMEM = SU_A_BYTES + 2 * SU_B_BYTES + 1024 /*align*/ + 8192 /*ex
 constexpr uint32_t SU_TMEM_COLS = 512, SU_ACC_STRIDE = 256;
 constexpr int SU_NONFINITE = 1 << 24;  // exponent of a row with Inf or NaN
 constexpr int SU_ERR_TIMEOUT = -1000;  // *err when a wait inside the kernel ran out
+constexpr uint64_t SU_DRAIN_NS = 2000000000ull;  // limit of the wait for the MMAs in flight
 
 struct SliceUpdateArgs {
     const double *A, *B;
@@ -210,10 +211,12 @@ __device__ __forceinline__ void su_convert(const double (&v)[16], int *ex, uint8
     su_write_digits(v, e, dst, slice_bytes, row, cw);
 }
 // A bounded wait that all four warps of a group pass or none does (they meet
-// at barriers afterwards); bar: a named barrier for the vote.
-__device__ __forceinline__ bool su_wait_group(uint64_t *mbar, uint32_t parity, volatile int *abort, uint64_t budget_ns, int bar)
+// at barriers afterwards); bar: a named barrier for the vote.  bad: this warp
+// has given up on another wait and votes against.
+__device__ __forceinline__ bool su_wait_group(uint64_t *mbar, uint32_t parity, volatile int *abort, uint64_t budget_ns, int bar,
+                                              bool bad = false)
 {
-    uint32_t all, mine = ptx::wait_parity(mbar, parity, abort, budget_ns) ? 1 : 0;
+    uint32_t all, mine = !bad && ptx::wait_parity(mbar, parity, abort, budget_ns) ? 1 : 0;
     asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
                  : "=r"(all)
                  : "r"(mine), "r"(bar)
@@ -364,20 +367,25 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                 }
                 if (!GEMM && ok) ptx::mma_commit(a_empty), ++item;
             }
-            // every MMA issued has read its operands before the CTA ends
+            // every MMA issued has read its operands before the CTA ends,
+            // whatever the limit of the other waits is
             ptx::mma_commit(drain);
             volatile int never = 0;
-            ptx::wait_parity(drain, 0, &never, a.wait_budget_ns);
+            ptx::wait_parity(drain, 0, &never, SU_DRAIN_NS);
         }
     } else {
         // ------------------------------------------ A's slices, epilogue
         const int quarter = warp & 3, group = warp >> 2;  // TMEM lanes; 32 rows of A, 8 columns of a tile
         int tile = 0, item = 0, rp = 0;
+        // Set when the wait for an accumulator runs out.  The warps of a group
+        // meet at named barriers in cut_a, so this warp goes on to the next of
+        // them without touching data and all four leave there together.
+        bool bad = false;
         SliceItems it(a);
         auto cut_a = [&](int k0) {
             double v[16];
             su_load(a.A, a.a_rs, a.a_ks, it.rb * SU_BM + 32 * group, a.m, k0, a.k, quarter, v);
-            if (!su_wait_group(a_empty, (item & 1) ^ 1, abort_flag, a.wait_budget_ns, 3 + group)) return false;
+            if (!su_wait_group(a_empty, (item & 1) ^ 1, abort_flag, a.wait_budget_ns, 3 + group, bad)) return false;
             su_convert(v, ea + (item & 3) * SU_BM + 32 * group, sA, SU_SLICE_A, 32 * group + lane, quarter,
                        rmax + group * 256, rp, 7 + group);
             ptx::fence_proxy_async_smem();
@@ -402,9 +410,13 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                     if (GEMM && !(ok = cut_a(ch * SU_K))) break;
                     const int buf = tile & 1;
                     const uint32_t tb = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * SU_ACC_STRIDE + 8 * group;
-                    ok = ptx::wait_parity(&acc_full[buf], (tile >> 1) & 1, abort_flag, a.wait_budget_ns);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
+                    bad = bad || !ptx::wait_parity(&acc_full[buf], (tile >> 1) & 1, abort_flag, a.wait_budget_ns);
+                    bad = __any_sync(0xffffffffu, bad);
+                    if (bad) {
+                        *abort_flag = 1;
+                        if (GEMM) ++item;
+                        continue;
+                    }
                     ptx::tc_fence_after();
                     const int er = ea[(item & 3) * SU_BM + rl];
                     const int *ec = eb + (tile & 3) * SU_BN + 8 * group;
@@ -437,7 +449,7 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                     }
                     if (GEMM) ++item;
                 }
-                if (!GEMM || !ok) continue;
+                if (!GEMM || !ok || bad) continue;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if (j < jn && !(weak >> j & 1)) crow[(long)j * a.ldc] -= c[j];
@@ -449,9 +461,10 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
             }
             if (GEMM) --item;  // counted per chunk
         }
+        ok = ok && !bad;
     }
     if (!ok) {
-        if (!*abort_flag && a.err) atomicCAS(a.err, 0, SU_ERR_TIMEOUT);
+        if (a.err) atomicCAS(a.err, 0, SU_ERR_TIMEOUT);
         *abort_flag = 1;
     }
     ptx::tc_fence_before();
