@@ -21,7 +21,8 @@ extern "C" {
 
 /* Waits for the submitted tasks, then returns the LAPACK-style info of the
  * first non-positive pivot met by any POTRF tile since the last reset
- * (0 = every tile factored); reset != 0 clears it. */
+ * (0 = every tile factored; negative: a wait inside a kernel ran out and the
+ * result is not valid); reset != 0 clears it. */
 int starpu_gb300_chol_status(int reset);
 
 #ifdef __cplusplus

@@ -16,7 +16,8 @@
  * the leading minor of order k is not positive definite) without trapping.
  * Kernels that hand work on between warps or CTAs bound every wait; one that
  * runs out (it cannot on a healthy device) leaves a negative *d_info and an
- * unspecified result.
+ * unspecified result.  Calls without a status word, or given none, record it
+ * in a word of the library's own (starpu_gb300_take_wait_status).
  */
 #ifndef STARPU_GB300_KERNELS_H
 #define STARPU_GB300_KERNELS_H
@@ -176,12 +177,21 @@ int starpu_gb300_spotrs_noalloc(void *stream, int n, int nrhs, const float *L, i
 
 /* Limit of every bounded wait of the sweeps (starpu_gb300_spotrs_sweep,
  * _noalloc, _inv_tiles and the mixed solve's correction solves) on a flag
- * that another CTA of the same launch publishes; a wait that runs out sets
- * the call's error word and the launch still ends.  Default 2 s; 0 restores
- * it.  Returns the previous limit.  The tensor-core kernels' pipeline waits
+ * that another CTA of the same launch publishes, and of the waits between the
+ * warps of a CTA in the factorisations of diagonal blocks, the blocked solves
+ * and the FP64 products; a wait that runs out sets the call's error word and
+ * the launch still ends.  Default 2 s; 0 restores it.  Returns the previous
+ * limit.  The pipeline waits of the FP32 tensor-core kernels and the residual
  * keep their own fixed limit.  No counterpart in the reference (its CUDA
  * path has no device-side waits). */
 unsigned long long starpu_gb300_set_wait_budget_ns(unsigned long long ns);
+
+/* GB300_ETIMEDOUT when a wait ran out, since the last such answer, in a call
+ * on the current device that has no status word (POTRS, TRSM, SYRK and GEMM)
+ * or was given none, on any stream; the results of those calls are then
+ * invalid.  0 otherwise.  Waits for `stream`: the calls asked about are those
+ * that are complete when its work is.  The answer clears the word. */
+int starpu_gb300_take_wait_status(void *stream);
 
 /* Host-only self-check of the per-device bookkeeping of kernel attributes
  * (dynamic shared memory limits are set once per function and device).

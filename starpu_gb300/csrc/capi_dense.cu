@@ -37,7 +37,8 @@ static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const 
     a.A = A, a.a_rs = a_rs, a.a_ks = a_ks, a.B = B, a.b_rs = b_rs, a.b_ks = b_ks;
     a.C = C, a.ldc = ldc, a.m = m, a.n = n, a.k = k, a.lower = lower ? 1 : 0;
     a.col_tiles = (n + SU_BN - 1) / SU_BN;
-    a.err = err;
+    a.err = err ? err : gb300_wait_status();
+    if (!a.err) return;
     a.wait_budget_ns = gb300_wait_budget_ns();
     a.total = 0;
     for (int rb = 0; rb * SU_BM < m; ++rb)
@@ -272,6 +273,8 @@ template <typename T>
 void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
 {
     if (nb <= 0) nb = n;
+    const CpWait wait{gb300_wait_budget_ns(), info ? info : gb300_wait_status()};
+    if (!wait.err) return;
     if (std::is_same<T, float>::value && n <= COOP_MAX_N) nb = n;
     // FP64: the FP64 units would bound wider panels, the tensor-core update takes 64 columns
     if (std::is_same<T, double>::value) nb = std::min(nb, CP_W);
@@ -279,16 +282,16 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
         const int kb = std::min(nb, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
         if (kb <= CP_W)
-            gb300_count_launch(), potf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0);
+            gb300_count_launch(), potf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0, wait);
         else if (std::is_same<T, float>::value && kb <= COOP_MAX_N)
-            potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0);
+            potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0, wait.err);
         else
             potrf_tiled<T>(s, kb, Akk, lda, CP_W, info, info_base + k0);
         const int m = n - k0 - kb;
         if (m > 0) {
             T *P = A + (k0 + kb) + (long)k0 * lda;
             trsm_rltn<T>(s, m, kb, Akk, lda, P, lda);
-            trailing_update(s, m, kb, P, lda, A + (k0 + kb) + (long)(k0 + kb) * lda, lda, info);
+            trailing_update(s, m, kb, P, lda, A + (k0 + kb) + (long)(k0 + kb) * lda, lda, wait.err);
         }
     }
 }
@@ -298,7 +301,7 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
 // min-dgels/base/SRC/dpotrs.c does the same two sweeps through dtrsm.
 // C right-hand sides per CTA in the update.
 template <typename T, int C, bool TRANS>
-static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
+static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb, const CpWait &wait)
 {
     constexpr size_t sm_blk = cp_trsv_smem<T>(TRANS), sm_upd = cp_upd_smem<T, C>(TRANS);
     if (gb300_func_dyn_smem((const void *)trsv_blk_kernel<T, TRANS>, (int)sm_blk) ||
@@ -308,7 +311,7 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
     for (int b = 0; b < nblk; ++b) {
         const int j0 = (TRANS ? nblk - 1 - b : b) * CP_SB, w = std::min(CP_SB, n - j0);
         gb300_count_launch(), trsv_blk_kernel<T, TRANS>
-            <<<nrhs, 256, sm_blk, s>>>(w, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb, nullptr);
+            <<<nrhs, 256, sm_blk, s>>>(w, L + j0 + (long)j0 * ldl, ldl, B + j0, ldb, wait);
         const int rest = TRANS ? j0 : n - j0 - w;
         if (rest <= 0) continue;
         if constexpr (std::is_same<T, double>::value) {
@@ -316,7 +319,7 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
             // 8 to 9 us, against rest nrhs / 8800 us on the FP64 units
             if (rest >= SLICE_MIN_M && nrhs >= 16 && (long)rest * nrhs >= SLICE_MIN_ELEMENTS) {
                 slice_update<true>(s, false, rest, nrhs, w, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl,
-                                   TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, nullptr);
+                                   TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, wait.err);
                 continue;
             }
         }
@@ -325,19 +328,22 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
     }
 }
 
-template <typename T, int C> static void potrs_sweeps(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
+template <typename T, int C>
+static void potrs_sweeps(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb, const CpWait &wait)
 {
-    potrs_sweep_blocks<T, C, false>(s, n, nrhs, L, ldl, B, ldb);
-    potrs_sweep_blocks<T, C, true>(s, n, nrhs, L, ldl, B, ldb);
+    potrs_sweep_blocks<T, C, false>(s, n, nrhs, L, ldl, B, ldb, wait);
+    potrs_sweep_blocks<T, C, true>(s, n, nrhs, L, ldl, B, ldb, wait);
 }
 
 template <typename T>
-void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb)
+void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb, int *err)
 {
     if (n <= 0 || nrhs <= 0) return;
-    if (nrhs == 1) potrs_sweeps<T, 1>(s, n, nrhs, L, ldl, B, ldb);
-    else if (nrhs <= 4) potrs_sweeps<T, 4>(s, n, nrhs, L, ldl, B, ldb);
-    else potrs_sweeps<T, 8>(s, n, nrhs, L, ldl, B, ldb);
+    const CpWait wait{gb300_wait_budget_ns(), err ? err : gb300_wait_status()};
+    if (!wait.err) return;
+    if (nrhs == 1) potrs_sweeps<T, 1>(s, n, nrhs, L, ldl, B, ldb, wait);
+    else if (nrhs <= 4) potrs_sweeps<T, 4>(s, n, nrhs, L, ldl, B, ldb, wait);
+    else potrs_sweeps<T, 8>(s, n, nrhs, L, ldl, B, ldb, wait);
 }
 
 // ---- single-launch POTRS sweeps with inverted 64 x 64 diagonal blocks ------
@@ -402,8 +408,8 @@ template void trsm_runu<double>(cudaStream_t, int, int, const double *, long, do
 template void potrf_tiled<float>(cudaStream_t, int, float *, long, int, int *, int);
 template void trtri_lower<float>(cudaStream_t, int, const float *, long, float *, long, float *);
 template void potrf_tiled<double>(cudaStream_t, int, double *, long, int, int *, int);
-template void potrs_blocked<float>(cudaStream_t, int, int, const float *, long, float *, long);
-template void potrs_blocked<double>(cudaStream_t, int, int, const double *, long, double *, long);
+template void potrs_blocked<float>(cudaStream_t, int, int, const float *, long, float *, long, int *);
+template void potrs_blocked<double>(cudaStream_t, int, int, const double *, long, double *, long, int *);
 
 } // namespace gb300
 
@@ -516,14 +522,14 @@ int starpu_gb300_dpotrf(void *stream, int n, double *A, int lda, int nb, int *d_
 int starpu_gb300_spotrs(void *stream, int n, int nrhs, const float *L, int ldl, float *B, int ldb)
 {
     if (n < 0 || nrhs < 0 || ldl < (n > 1 ? n : 1) || ldb < (n > 1 ? n : 1)) return GB300_EINVAL;
-    potrs_blocked<float>(GB300_STREAM(stream), n, nrhs, L, ldl, B, ldb);
+    potrs_blocked<float>(GB300_STREAM(stream), n, nrhs, L, ldl, B, ldb, nullptr);
     return gb300_last_launch_status();
 }
 
 int starpu_gb300_dpotrs(void *stream, int n, int nrhs, const double *L, int ldl, double *B, int ldb)
 {
     if (n < 0 || nrhs < 0 || ldl < (n > 1 ? n : 1) || ldb < (n > 1 ? n : 1)) return GB300_EINVAL;
-    potrs_blocked<double>(GB300_STREAM(stream), n, nrhs, L, ldl, B, ldb);
+    potrs_blocked<double>(GB300_STREAM(stream), n, nrhs, L, ldl, B, ldb, nullptr);
     return gb300_last_launch_status();
 }
 

@@ -24,11 +24,13 @@ template <typename T>
 static void getrf_blocked(cudaStream_t s, int n, T *A, long lda, T thr, int *d_first, int *info)
 {
     constexpr int W = sizeof(T) == 4 ? 64 : 32;
+    const CpWait wait{gb300_wait_budget_ns(), info ? info : gb300_wait_status()};
+    if (!wait.err) return;
     for (int k0 = 0; k0 < n; k0 += W) {
         const int kb = std::min(W, n - k0);
         T *Akk = A + k0 + (long)k0 * lda;
         if constexpr (sizeof(T) == 4)
-            gb300_count_launch(), getf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0);
+            gb300_count_launch(), getf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0, wait);
         else
             gb300_count_launch(), getf2_small_kernel<T, W><<<1, 256, 0, s>>>(kb, Akk, lda, thr, d_first, info, k0);
         const int rest = n - k0 - kb;

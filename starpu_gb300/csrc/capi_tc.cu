@@ -456,6 +456,8 @@ static int diag_factor_inverse(cudaStream_t s, int n, float *A, long lda, float 
     a.info_base = info_base;
     a.bar = bar;
     a.err = err;
+    a.err_code = bar ? DC_ERR_TIMEOUT : CP_ERR_TIMEOUT;
+    a.wait_ns = gb300_wait_budget_ns();
     a.invert = invert ? 1 : 0;
     void *args[] = {&a};
     gb300_count_launch();
@@ -463,9 +465,9 @@ static int diag_factor_inverse(cudaStream_t s, int n, float *A, long lda, float 
         cudaLaunchCooperativeKernel((const void *)diag_coop_kernel, dim3(grid), dim3(DC_T), args, 0, s));
 }
 
-int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base)
+int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base, int *err)
 {
-    return diag_factor_inverse(s, n, A, lda, nullptr, 0, nullptr, nullptr, info, info_base, nullptr, false);
+    return diag_factor_inverse(s, n, A, lda, nullptr, 0, nullptr, nullptr, info, info_base, err, false);
 }
 
 // A high-priority stream and a fork / join event pair per host thread and

@@ -192,6 +192,23 @@ extern "C" int gb300_device_sms(void)
 
 extern "C" unsigned long long gb300_wait_budget_ns(void) { return g_wait_budget_ns.load(std::memory_order_relaxed); }
 
+// ---- waits that ran out in calls without a status word ----------------------
+static __device__ int g_wait_status;
+
+static std::atomic<int *> g_wait_status_dev[kMaxDevices];  // the word's address per device
+
+int *gb300::gb300_wait_status()
+{
+    int dev = 0;
+    if (gb300_record_cuda_error(cudaGetDevice(&dev))) return nullptr;
+    int *p = dev >= 0 && dev < kMaxDevices ? g_wait_status_dev[dev].load(std::memory_order_acquire) : nullptr;
+    if (p) return p;
+    void *v = nullptr;
+    if (gb300_record_cuda_error(cudaGetSymbolAddress(&v, g_wait_status))) return nullptr;
+    if (dev >= 0 && dev < kMaxDevices) g_wait_status_dev[dev].store((int *)v, std::memory_order_release);
+    return (int *)v;
+}
+
 extern "C" int gb300_last_launch_status(void)
 {
     return gb300_record_cuda_error(cudaGetLastError());
@@ -204,6 +221,21 @@ const char *starpu_gb300_last_error(void) { return g_last_error; }
 unsigned long long starpu_gb300_set_wait_budget_ns(unsigned long long ns)
 {
     return g_wait_budget_ns.exchange(ns ? ns : kDefaultWaitBudgetNs);
+}
+
+int starpu_gb300_take_wait_status(void *stream)
+{
+    cudaStream_t s = (cudaStream_t)stream;
+    int *w = gb300::gb300_wait_status(), h = 0;
+    if (!w) return GB300_ECUDA;
+    int rc = gb300_record_cuda_error(cudaMemcpyAsync(&h, w, sizeof h, cudaMemcpyDeviceToHost, s));
+    if (!rc) rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
+    if (rc || !h) return rc;
+    rc = gb300_record_cuda_error(cudaMemsetAsync(w, 0, sizeof h, s));
+    if (!rc) rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
+    if (rc) return rc;
+    gb300_set_error("a wait inside a kernel ran out; the results of the calls since the last check are invalid");
+    return GB300_ETIMEDOUT;
 }
 
 int starpu_gb300_selftest_attr_book(void)

@@ -253,14 +253,16 @@ void cholesky_kernel_fini(void)
 }
 
 /* LAPACK-style info of the first non-positive pivot met by the POTRF tiles
- * since the last reset (0 = every tile factored). */
+ * since the last reset (0 = every tile factored); negative when a wait inside
+ * a kernel ran out (in the SYRK and GEMM tiles, which have no word of their
+ * own, since the last call). */
 int starpu_gb300_chol_status(int reset)
 {
     int h = 0;
     if (!d_status) return 0;
     starpu_task_wait_for_all();
     starpu_gb300_memcpy_d2h(NULL, &h, d_status, sizeof h);
-    starpu_gb300_stream_sync(NULL);
+    if (starpu_gb300_take_wait_status(NULL) != 0 && !h) h = GB300_ETIMEDOUT;
     if (reset) {
         starpu_gb300_memset(NULL, d_status, 0, sizeof(int));
         starpu_gb300_stream_sync(NULL);

@@ -117,7 +117,10 @@ int main(int argc, char **argv)
         STARPU_CHECK_RETURN_VALUE(ret, "starpu_task_insert");
         if (ms < best) best = ms;
         int info = starpu_gb300_chol_status(1);
-        if (info) {
+        if (info < 0) {
+            fprintf(stderr, "factorisation failed: a wait inside a kernel ran out\n");
+            status = 2;
+        } else if (info) {
             fprintf(stderr, "factorisation failed: leading minor %d is not positive definite\n", info);
             status = 2;
         }

@@ -12,8 +12,13 @@ namespace gb300 {
 constexpr int GB300_DIAG_TILE_MAX = 1024;
 
 // FP32 lower Cholesky of the whole n x n matrix in one cooperative launch,
-// no workspace (capi_tc.cu)
-int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base);
+// no workspace (capi_tc.cu); err gets a negative word when a wait runs out
+int potrf_coop(cudaStream_t s, int n, float *A, long lda, int *info, int info_base, int *err);
+
+// The word of the current device in which the calls without a status word of
+// their own record that a wait inside a kernel ran out (capi_util.cu); null
+// when its address cannot be had, which is then the calling thread's CUDA error.
+int *gb300_wait_status();
 
 // residual partials P_z = -(A X) on the tensor cores (capi_tc.cu)
 size_t residual_tc_a_bytes(int n);
@@ -89,7 +94,9 @@ template <typename T> void trsm_runu(cudaStream_t s, int m, int n, const T *U, l
 template <typename T> void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base);
 // Linv = inverse of the lower triangle of L (n x n, ld ldi, upper part zeroed); scratch >= n*n/4 elements
 template <typename T> void trtri_lower(cudaStream_t s, int n, const T *L, long ldl, T *Linv, long ldi, T *scratch);
-template <typename T> void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb);
+// err: the word that gets a negative code when a wait runs out; null: gb300_wait_status()
+template <typename T>
+void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb, int *err);
 // single-launch sweeps: workspace = inverted 64x64 diagonal blocks + flags
 template <typename T> size_t potrs_sweep_workspace(int n);
 template <typename T> void potrs_sweep_prepare(cudaStream_t s, int n, const T *L, long ldl, void *ws);

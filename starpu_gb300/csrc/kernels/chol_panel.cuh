@@ -74,6 +74,16 @@ template <typename T, int NX> using CpPanel = Quad<T>[16][CP_W + 32 * NX];
 
 constexpr int CP_ERR_TIMEOUT = -1000;
 
+// How long a warp waits for what another warp of its CTA publishes, and the
+// word that CP_ERR_TIMEOUT goes to when that runs out (never null).  It takes
+// the place of a pivot's info: what follows a wait that ran out is garbage, bad
+// pivots too.
+struct CpWait {
+    unsigned long long ns;
+    int *err;
+    __device__ __forceinline__ void report() const { atomicMin(err, CP_ERR_TIMEOUT); }
+};
+
 // Once per kernel, before a CTA barrier.
 __device__ __forceinline__ void cp_panel_init(uint64_t (&bar)[16])
 {
@@ -94,13 +104,16 @@ template <typename T, typename F> __device__ __forceinline__ void cp_each(CpBloc
 }
 
 // the published columns of step s; bounded (a step takes well below a
-// microsecond, and the publisher never waits for this warp)
-__device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity)
+// microsecond and the publisher never waits for this warp, but a process may be
+// switched out meanwhile)
+__device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity, unsigned long long ns)
 {
+    // a limit below the suspended wait's own (some microseconds): look once
+    if (ns < 1000) return ptx::mbar_test_wait(bar, parity);
     if (ptx::mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = ptx::globaltimer();
     while (!ptx::mbar_try_wait(bar, parity))
-        if (ptx::globaltimer() - t0 > 20000000ull) return false;  // 20 ms
+        if (ptx::globaltimer() - t0 > ns) return false;
     return true;
 }
 
@@ -199,7 +212,7 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
 // False: a wait ran out.
 template <typename T, int NX>
 __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T, NX> &pan, uint64_t (&bar)[16], uint32_t phase,
-                                         int n, int *info, int info_base, bool report)
+                                         int n, int *info, int info_base, bool report, unsigned long long ns)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int steps = (n + 3) / 4;
@@ -210,11 +223,11 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
     };
 #pragma unroll 1
     for (int i = 0; i < min(w, steps) - 1; ++i) {
-        ok = cp_wait(&bar[i], phase) && ok;
+        ok = cp_wait(&bar[i], phase, ns) && ok;
         cp_update<T, NX, 0, 1>(d, x, pan[i]);
     }
     if (w > 0 && w <= steps) {
-        ok = cp_wait(&bar[w - 1], phase) && ok;
+        ok = cp_wait(&bar[w - 1], phase, ns) && ok;
         cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
     }
     // (every mbarrier completes in every panel, so that all keep one parity)
@@ -227,7 +240,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
     cp_update<T, NX, 1, 1>(d, x, pan[w]);
 #pragma unroll 1
     for (int i = w + 1; i < min(8 + w, steps); ++i) {
-        ok = cp_wait(&bar[i], phase) && ok;
+        ok = cp_wait(&bar[i], phase, ns) && ok;
         cp_update<T, NX, 1, 1>(d, x, pan[i]);
     }
     if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w]));
@@ -235,7 +248,8 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
 }
 
 // Cholesky of the n x n (n <= 64) lower block A, in place, by one CTA.
-static __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_base)
+static __global__ void __launch_bounds__(256)
+potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_base, const CpWait wait)
 {
     __shared__ CpPanel<float, 0> pan;
     __shared__ uint64_t bar[16];
@@ -244,7 +258,7 @@ static __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, float *__
     // rows and columns past n continue the block as the identity
     cp_each<float>(a, [&](float &v, int r, int c) { v = (r < n && c <= r) ? A[r + (long)c * lda] : (r == c ? 1.0f : 0.0f); });
     __syncthreads();
-    if (!cp_panel<float, 0>(a, a, pan, bar, 0, n, info, info_base, true) && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
+    if (!cp_panel<float, 0>(a, a, pan, bar, 0, n, info, info_base, true, wait.ns)) wait.report();
     cp_each<float>(a, [&](float &v, int r, int c) {
         if (r < n && c <= r) A[r + (long)c * lda] = v;
     });
@@ -262,7 +276,7 @@ static __global__ void __launch_bounds__(256) potf2_leaf_kernel(int n, float *__
 // 3 us more: each warp then trails its own backlog.)
 template <int H0>  // columns 32 H0 .. 32 H0 + 31, rows 32 H0 .. 63
 __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*col)[CP_W], double2 *pv, uint64_t *bar, int n,
-                                               int *info, int info_base)
+                                               int *info, int info_base, unsigned long long ns)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bool ok = true;
@@ -293,7 +307,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
         if (j0 >= n) break;
 #pragma unroll 1
         for (int j = j0; j < min(mine, n); ++j) {  // columns of this round before mine
-            ok = cp_wait(&bar[j], 0) && ok;
+            ok = cp_wait(&bar[j], 0, ns) && ok;
             next(j, q);
             if (j + 1 < mine) rest(j, q + 1);
         }
@@ -314,7 +328,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
         }
 #pragma unroll 1
         for (int j = mine + 1; j < min(j0 + 8, n); ++j) {  // and after it
-            ok = cp_wait(&bar[j], 0) && ok;
+            ok = cp_wait(&bar[j], 0, ns) && ok;
             rest(j, q + 1);
         }
     }
@@ -322,7 +336,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
 }
 
 static __global__ void __launch_bounds__(256)
-potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_base)
+potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_base, const CpWait wait)
 {
     __shared__ double col[CP_W][CP_W];
     __shared__ double2 pv[CP_W];  // pivots and the factors their columns were scaled with
@@ -341,9 +355,9 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
     };
     each([&](double &v, int r, int c) { v = r < n && c <= r ? A[r + (long)c * lda] : 0.0; });
     __syncthreads();
-    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base);
-    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base) && ok;
-    if (!ok && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
+    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base, wait.ns);
+    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base, wait.ns) && ok;
+    if (!ok) wait.report();
     each([&](double &v, int r, int c) {
         if (r < n && c < r) A[r + (long)c * lda] = v;
     });
@@ -560,7 +574,7 @@ template <typename T> constexpr size_t cp_trsv_smem(bool trans)
 
 template <typename T, bool TRANS>
 __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, const T *__restrict__ L, long ldl, T *__restrict__ B, long ldb,
-                                                       int *err)
+                                                       const CpWait wait)
 {
     extern __shared__ __align__(16) unsigned char cp_smem[];
     __shared__ uint64_t bar[16];
@@ -608,7 +622,7 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, const T *__restric
     for (int i = 0; i < n; ++i) {
         const int p = TRANS ? np - 1 - i : i;
         turn(l);
-        ok = cp_wait(&bar[p], 0) && ok;
+        ok = cp_wait(&bar[p], 0, wait.ns) && ok;
         const Quad<T> *x = reinterpret_cast<const Quad<T> *>(xs + 32 * p);
         T acc[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
@@ -641,7 +655,7 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, const T *__restric
     xs[r] = y;
     ptx::mbar_arrive(&bar[warp]);
     if (r < w) b[r] = y;
-    if (!ok && err) atomicCAS(err, 0, CP_ERR_TIMEOUT);
+    if (!ok) wait.report();
 }
 
 // C right-hand sides of Y[m x nrhs] -= op(L) X[w x nrhs] (w <= CP_SB): op(L) =

@@ -62,9 +62,18 @@ struct DiagCoopArgs {
     int *info;
     int info_base;
     unsigned *bar;  // barrier counter, zero at launch; null: the launch's own grid barrier
-    int *err;       // (with bar)
+    int *err;       // word that err_code goes to when a wait ran out
+    int err_code;   // DC_ERR_TIMEOUT (with bar), or CP_ERR_TIMEOUT where err is an info word
+    unsigned long long wait_ns;  // limit of a wait inside a panel
     int invert;  // 0: factor only (no inverse is written)
 };
+
+// a negative code takes the place of a pivot's info
+__device__ __forceinline__ void dc_report(const DiagCoopArgs &a)
+{
+    if (a.err_code < 0) atomicMin(a.err, a.err_code);
+    else atomicCAS(a.err, 0, a.err_code);
+}
 
 __device__ __forceinline__ unsigned dc_ld_acquire(const unsigned *p)
 {
@@ -90,7 +99,7 @@ __device__ __forceinline__ bool dc_sync(const DiagCoopArgs &a, unsigned phase, i
             const uint64_t t0 = dc_timer();
             while (dc_ld_acquire(a.bar) < target) {
                 if (*(volatile int *)a.err || dc_timer() - t0 > DC_WAIT_NS) {
-                    atomicCAS(a.err, 0, DC_ERR_TIMEOUT);
+                    dc_report(a);
                     ok = 0;
                     break;
                 }
@@ -215,8 +224,8 @@ __global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
                     else v = (r < ri && c < bk) ? __ldcg(Aik + r + (long)c * a.lda) : 0.0f;
                 });
                 __syncthreads();  // pan of the previous task is free
-                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, bk, a.info, a.info_base + k0, t == 0) && a.err)
-                    atomicCAS(a.err, 0, DC_ERR_TIMEOUT);
+                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, bk, a.info, a.info_base + k0, t == 0, a.wait_ns))
+                    dc_report(a);
                 ++panels;
                 if (t > 0)
                     cp_each<float>(x, [&](float &v, int r, int c) {

@@ -201,7 +201,7 @@ __device__ __forceinline__ void getf_own(CpBlock<float> &a, GetfPanel &s, int n,
 }
 
 __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restrict__ A, long lda, float thr, int *d_first,
-                                                         int *info, int info_base)
+                                                         int *info, int info_base, const CpWait wait)
 {
     __shared__ GetfPanel s;
     const int w = threadIdx.x >> 5, steps = (n + 3) / 4;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restric
     bool ok = true;
 #pragma unroll 1
     for (int i = 0; i < min(w, steps); ++i) {
-        ok = cp_wait(&s.bar[i], 0) && ok;
+        ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
         getf_update<0>(a, s, i);
         if (i < w - 1) getf_update<1>(a, s, i);  // the next owner publishes first
     }
@@ -222,12 +222,12 @@ __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restric
         getf_update<1>(a, s, w);
 #pragma unroll 1
         for (int i = w + 1; i < min(8 + w, steps); ++i) {
-            ok = cp_wait(&s.bar[i], 0) && ok;
+            ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
             getf_update<1>(a, s, i);
         }
         if (8 + w < steps) getf_own<1>(a, s, n, thr, d_first, info, info_base);
     }
-    if (!ok && info) atomicCAS(info, 0, CP_ERR_TIMEOUT);
+    if (!ok) wait.report();
     cp_each<float>(a, [&](float &v, int r, int c) {
         if (r < n && c < n) A[r + (long)c * lda] = v;
     });

@@ -79,7 +79,7 @@ struct SliceUpdateArgs {
     int m, n, k;
     int lower;     // 1 (m == n): only elements with row >= column
     int col_tiles, total;  // column tiles of a row block, tiles of all row blocks
-    int *err;      // may be null
+    int *err;      // gets SU_ERR_TIMEOUT when a wait ran out
     unsigned long long wait_budget_ns;
 };
 
@@ -464,7 +464,7 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
         ok = ok && !bad;
     }
     if (!ok) {
-        if (a.err) atomicCAS(a.err, 0, SU_ERR_TIMEOUT);
+        atomicMin(a.err, SU_ERR_TIMEOUT);  // (in place of a pivot's info)
         *abort_flag = 1;
     }
     ptx::tc_fence_before();

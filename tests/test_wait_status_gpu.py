@@ -15,6 +15,9 @@ from starpu_gb300.native import check
 pytestmark = pytest.mark.gpu
 
 TIMEOUT_INFO = -1000
+GB300_ETIMEDOUT = -110
+P = {np.float32: "s", np.float64: "d"}
+EPS = {np.float32: 2.0**-24, np.float64: 2.0**-53}
 
 
 def up(a):
@@ -51,22 +54,93 @@ def test_fp64_product_ends_when_a_wait_runs_out(gpu, m, n, k):
     with short_waits(gpu):
         for _ in range(3):
             product()
+            assert gpu.starpu_gb300_take_wait_status(None) == GB300_ETIMEDOUT
+    assert gpu.starpu_gb300_take_wait_status(None) == 0
     bound = (k + 2) * 2.0**-53 * (np.abs(c) + np.abs(a) @ np.abs(b).T)
     assert np.all(np.abs(product() - (c - a @ b.T)) <= bound)
 
 
-@pytest.mark.parametrize("n", [400, 1500])
-def test_fp64_factorisation_reports_a_wait_that_runs_out(gpu, n):
-    a = spd(n, n)
+# FP32: the leaf, one cooperative launch, and panels; FP64: the leaf, with updates on the tensor cores
+@pytest.mark.parametrize("dtype,n", [(np.float32, 64), (np.float32, 300), (np.float32, 4200), (np.float64, 64),
+                                     (np.float64, 400), (np.float64, 1500)])
+@pytest.mark.parametrize("has_info", [True, False])
+def test_factorisation_reports_a_wait_that_runs_out(gpu, dtype, n, has_info):
+    a = spd(n, n).astype(dtype)
 
     def factor():
         da, info = up(a), up(np.full(1, 7, np.int32))
-        check(gpu.starpu_gb300_dpotrf(None, n, da.ptr, n, 512, info.ptr))
+        check(getattr(gpu, f"starpu_gb300_{P[dtype]}potrf")(None, n, da.ptr, n, 512, info.ptr if has_info else None))
         check(gpu.starpu_gb300_stream_sync(None))
-        return np.tril(da.download((n, n), np.float64)), int(info.download((1,), np.int32)[0])
+        return np.tril(da.download((n, n), dtype)).astype(np.float64), int(info.download((1,), np.int32)[0])
 
     with short_waits(gpu):
-        assert factor()[1] == TIMEOUT_INFO
+        assert factor()[1] == (TIMEOUT_INFO if has_info else 7)
+    assert gpu.starpu_gb300_take_wait_status(None) == (0 if has_info else GB300_ETIMEDOUT)
     l, info = factor()
-    assert info == 0
-    assert np.all(np.abs(a - l @ l.T) <= 2 * (n + 1) * 2.0**-53 * np.sqrt(np.outer(np.diag(a), np.diag(a))))
+    assert info == (0 if has_info else 7) and gpu.starpu_gb300_take_wait_status(None) == 0
+    bound = 2 * (n + 1) * EPS[dtype] * np.sqrt(np.outer(np.diag(a), np.diag(a)).astype(np.float64))
+    assert np.all(np.abs(a - l @ l.T) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("has_info", [True, False])
+def test_lu_leaf_reports_a_wait_that_runs_out(gpu, dtype, has_info):
+    n = 200
+    a = (np.random.default_rng(n).uniform(-1, 1, (n, n)) + n * np.eye(n)).astype(dtype)
+
+    def factor():
+        da, info = up(a), up(np.full(1, 7, np.int32))
+        check(getattr(gpu, f"starpu_gb300_{P[dtype]}getrf_tile")(None, n, da.ptr, n, info.ptr if has_info else None))
+        check(gpu.starpu_gb300_stream_sync(None))
+        return da.download((n, n), dtype).astype(np.float64), int(info.download((1,), np.int32)[0])
+
+    with short_waits(gpu):
+        info = factor()[1]
+    taken = gpu.starpu_gb300_take_wait_status(None)
+    if dtype == np.float32:  # the FP64 leaf has CTA barriers, no waits
+        assert info == (TIMEOUT_INFO if has_info else 7) and taken == (0 if has_info else GB300_ETIMEDOUT)
+    out, info = factor()
+    assert info == (0 if has_info else 7) and gpu.starpu_gb300_take_wait_status(None) == 0
+    l, u = np.tril(out), np.triu(out, 1) + np.eye(n)
+    assert np.all(np.abs(l @ u - a) <= 2 * (n + 1) * EPS[dtype] * (np.abs(l) @ np.abs(u)))
+
+
+@pytest.mark.parametrize("dtype,n,nrhs", [(np.float32, 600, 3), (np.float64, 600, 3), (np.float64, 2300, 64)])
+def test_solve_reports_a_wait_that_runs_out(gpu, dtype, n, nrhs):
+    l = np.linalg.cholesky(spd(n, n)).astype(dtype)
+    b = np.random.default_rng(n).uniform(-1, 1, (n, nrhs)).astype(dtype)
+    dl = up(l)
+
+    def solve():
+        db = up(b)
+        check(getattr(gpu, f"starpu_gb300_{P[dtype]}potrs")(None, n, nrhs, dl.ptr, n, db.ptr, n))
+        status = gpu.starpu_gb300_take_wait_status(None)
+        return db.download((n, nrhs), dtype).astype(np.float64), status
+
+    with short_waits(gpu):
+        assert solve()[1] == GB300_ETIMEDOUT
+    x, status = solve()
+    assert status == 0
+    l64 = l.astype(np.float64)
+    bound = 8 * n * EPS[dtype] * (np.abs(l64) @ (np.abs(l64.T) @ np.abs(x)) + np.abs(b))
+    assert np.all(np.abs(l64 @ (l64.T @ x) - b) <= bound)
+
+
+def test_batched_solve_reports_a_wait_that_runs_out(gpu):
+    sizes = np.array([300, 64, 20], np.int32)
+    mats = [spd(n, n) for n in sizes]
+    rhs = [np.ones((n, 2)) for n in sizes]
+    cat = lambda v: np.concatenate([m.ravel(order="F") for m in v])
+    off = lambda v: np.concatenate([[0], np.cumsum([m.size for m in v])])[:-1].astype(np.int64)
+    da, db, ao, bo = up(cat(mats)), up(cat(rhs)), off(mats), off(rhs)
+    lw = gpu.starpu_gb300_dposv_batched_workspace(3, sizes.ctypes.data, 2)
+    work, dx, status = DeviceBuffer(lw), up(cat(rhs)), np.zeros(3, np.int32)
+
+    def solve():
+        check(gpu.starpu_gb300_dposv_batched(None, 3, sizes.ctypes.data, da.ptr, ao.ctypes.data, db.ptr, bo.ctypes.data,
+                                             dx.ptr, 2, 1e-13, 20, work.ptr, lw, status.ctypes.data, None))
+        return status.copy()
+
+    with short_waits(gpu):
+        assert solve()[0] == -1000
+    assert np.all(solve() >= 0)
