@@ -270,11 +270,12 @@ static void trailing_update(cudaStream_t s, int m, int k, const double *P, long 
 // matrices up to COOP_MAX_N, are factored by one cooperative launch
 // (kernels/diag_coop.cuh); FP64 goes in panels of CP_W columns.
 template <typename T>
-void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
+int potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base)
 {
+    int rc = GB300_OK;
     if (nb <= 0) nb = n;
     const CpWait wait{gb300_wait_budget_ns(), info ? info : gb300_wait_status()};
-    if (!wait.err) return;
+    if (!wait.err) return GB300_ECUDA;
     if (std::is_same<T, float>::value && n <= COOP_MAX_N) nb = n;
     // FP64: the FP64 units would bound wider panels, the tensor-core update takes 64 columns
     if (std::is_same<T, double>::value) nb = std::min(nb, CP_W);
@@ -284,9 +285,10 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
         if (kb <= CP_W)
             gb300_count_launch(), potf2_leaf_kernel<<<1, 256, 0, s>>>(kb, Akk, lda, info, info_base + k0, wait);
         else if (std::is_same<T, float>::value && kb <= COOP_MAX_N)
-            potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0, wait.err);
+            rc = potrf_coop(s, kb, (float *)Akk, lda, info, info_base + k0, wait.err);
         else
-            potrf_tiled<T>(s, kb, Akk, lda, CP_W, info, info_base + k0);
+            rc = potrf_tiled<T>(s, kb, Akk, lda, CP_W, info, info_base + k0);
+        if (rc) return rc;  // nothing is enqueued on a block that is not factored
         const int m = n - k0 - kb;
         if (m > 0) {
             T *P = A + (k0 + kb) + (long)k0 * lda;
@@ -294,6 +296,7 @@ void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int i
             trailing_update(s, m, kb, P, lda, A + (k0 + kb) + (long)(k0 + kb) * lda, lda, wait.err);
         }
     }
+    return GB300_OK;
 }
 
 // POTRS with a lower factor: L y = b (forward), then L^T x = y (backward),
@@ -405,9 +408,9 @@ template void trsm_llnn<float>(cudaStream_t, int, int, const float *, long, floa
 template void trsm_llnn<double>(cudaStream_t, int, int, const double *, long, double *, long);
 template void trsm_runu<float>(cudaStream_t, int, int, const float *, long, float *, long);
 template void trsm_runu<double>(cudaStream_t, int, int, const double *, long, double *, long);
-template void potrf_tiled<float>(cudaStream_t, int, float *, long, int, int *, int);
+template int potrf_tiled<float>(cudaStream_t, int, float *, long, int, int *, int);
 template void trtri_lower<float>(cudaStream_t, int, const float *, long, float *, long, float *);
-template void potrf_tiled<double>(cudaStream_t, int, double *, long, int, int *, int);
+template int potrf_tiled<double>(cudaStream_t, int, double *, long, int, int *, int);
 template void potrs_blocked<float>(cudaStream_t, int, int, const float *, long, float *, long, int *);
 template void potrs_blocked<double>(cudaStream_t, int, int, const double *, long, double *, long, int *);
 
@@ -425,30 +428,34 @@ int starpu_gb300_spotrf_tile(void *stream, int n, float *A, int lda, int *d_info
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_dpotrf_tile(void *stream, int n, double *A, int lda, int *d_info)
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_info, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_spotrf_tile_status(void *stream, int n, float *A, int lda, int *d_status)
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
-    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_dpotrf_tile_status(void *stream, int n, double *A, int lda, int *d_status)
 {
     if (n < 0 || lda < (n > 1 ? n : 1)) return GB300_EINVAL;
-    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, CP_W, d_status, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_strsm_rltn_tile(void *stream, int m, int n, float alpha, const float *L, int ldl, float *B, int ldb)
@@ -507,16 +514,18 @@ int starpu_gb300_spotrf(void *stream, int n, float *A, int lda, int nb, int *d_i
 {
     if (n < 0 || lda < (n > 1 ? n : 1) || nb < 0) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, nb ? nb : 512, d_info, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<float>(GB300_STREAM(stream), n, A, lda, nb ? nb : 512, d_info, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_dpotrf(void *stream, int n, double *A, int lda, int nb, int *d_info)
 {
     if (n < 0 || lda < (n > 1 ? n : 1) || nb < 0) return GB300_EINVAL;
     if (d_info) cudaMemsetAsync(d_info, 0, sizeof(int), GB300_STREAM(stream));
-    if (n) potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, nb ? nb : 512, d_info, 0);
-    return gb300_last_launch_status();
+    const int rc = n ? potrf_tiled<double>(GB300_STREAM(stream), n, A, lda, nb ? nb : 512, d_info, 0) : GB300_OK;
+    const int last = gb300_last_launch_status();
+    return rc ? rc : last;
 }
 
 int starpu_gb300_spotrs(void *stream, int n, int nrhs, const float *L, int ldl, float *B, int ldb)

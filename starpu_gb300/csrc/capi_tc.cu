@@ -588,8 +588,8 @@ static int panel_diag(cudaStream_t s, int n, float *A, long lda, int k0, int kb,
         rc = diag_factor_inverse(s, kb, Akk, lda, linv, ldk, w.scratch, w.bar, d_info, k0, d_err, m > 0 || linv_band,
                                  sms);
     } else {
-        potrf_tiled<float>(s, kb, Akk, lda, 64, d_info, k0);
-        if (m > 0) trtri_lower<float>(s, kb, Akk, lda, linv, ldk, w.scratch);
+        rc = potrf_tiled<float>(s, kb, Akk, lda, 64, d_info, k0);
+        if (!rc && m > 0) trtri_lower<float>(s, kb, Akk, lda, linv, ldk, w.scratch);
     }
     // the inverse split from its row maxima (its elements have no bound from A)
     if (!rc && m > 0) rc = split_f16s(s, kb, kb, linv, ldk, w.inv, ldk);

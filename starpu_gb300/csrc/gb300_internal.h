@@ -91,7 +91,8 @@ void gemm(cudaStream_t s, bool ta, bool tb, bool lower, int m, int n, int k, T a
 template <typename T> void trsm_rltn(cudaStream_t s, int m, int nc, const T *L, long ldl, T *B, long ldb);
 template <typename T> void trsm_llnn(cudaStream_t s, int m, int n, const T *L, long ldl, T *B, long ldb);
 template <typename T> void trsm_runu(cudaStream_t s, int m, int n, const T *U, long ldu, T *B, long ldb);
-template <typename T> void potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base);
+// the first error met: nothing is enqueued behind a launch that failed
+template <typename T> int potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int info_base);
 // Linv = inverse of the lower triangle of L (n x n, ld ldi, upper part zeroed); scratch >= n*n/4 elements
 template <typename T> void trtri_lower(cudaStream_t s, int n, const T *L, long ldl, T *Linv, long ldi, T *scratch);
 // err: the word that gets a negative code when a wait runs out; null: gb300_wait_status()
