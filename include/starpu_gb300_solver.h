@@ -38,7 +38,8 @@ typedef struct starpu_gb300_ir_info {
     int status;            /* 0 converged; GB300_EDOM factor failed; GB300_ETIMEDOUT not converged */
     int iterations;        /* refinement corrections applied (each: one solve with the factor) */
     int factor_terms;      /* products per trailing-update term (1: BF16; 3: split operands) */
-    int potrf_info;        /* LAPACK-style info of the last factorisation (mixed, or FP64 after a fallback) */
+    int potrf_info;        /* LAPACK-style info of the last factorisation (mixed, or FP64 after a fallback);
+                              negative: a wait inside it ran out (status GB300_ETIMEDOUT) */
     double backward_error; /* max over RHS of ||b - A x||_inf / (||A||_inf ||x||_inf + ||b||_inf) */
     double anorm;          /* ||A||_inf */
     int method;            /* refinement at the end: 0 classic corrections, 1 preconditioned conjugate gradients */

@@ -866,7 +866,7 @@ int dsposv_factor(cudaStream_t s, int n, int nrhs, const double *A, int lda, int
         out->potrf_info = hinfo[0];
         out->factor_terms = nterms;
     }
-    if (hinfo[1]) {
+    if (hinfo[1] || hinfo[0] < 0) {  // a wait ran out
         if (out) out->status = GB300_ETIMEDOUT;
         return GB300_ETIMEDOUT;
     }
@@ -1068,15 +1068,17 @@ int dsposv_fp64(cudaStream_t s, int n, int nrhs, const double *A, int lda, const
     if (!rc) rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
     if (rc) return rc;
     if (out) out->potrf_info = hinfo;
-    if (hinfo) {
-        if (out) out->status = GB300_EDOM;
-        return GB300_EDOM;
+    if (hinfo) {  // negative: a wait ran out
+        const int failed = hinfo < 0 ? GB300_ETIMEDOUT : GB300_EDOM;
+        if (out) out->status = failed;
+        return failed;
     }
-    if ((rc = starpu_gb300_dpotrs(s, n, nrhs, F, n, X, ldx))) return rc;
+    cudaMemsetAsync(ws.anorm_bits, 0, 4 * sizeof(unsigned long long), s);  // and the error word
+    potrs_blocked<double>(s, n, nrhs, F, n, X, ldx, ws.err);
+    if ((rc = gb300_last_launch_status())) return rc;
     // the factor is no longer needed: A is cut into its digit slices again
     // (max |A_ij| and ||A||_inf from the lower triangle on the way) and
     // r = b - A x is formed as the refinement forms it
-    cudaMemsetAsync(ws.anorm_bits, 0, 4 * sizeof(unsigned long long), s);
     gb300_count_launch(), convert_lower_max_kernel<<<n, 256, 0, s>>>(n, A, lda, nullptr, 0, ws.anorm_bits + 2);
     if ((rc = residual_tc_slice_a(s, n, A, lda, ws.anorm_bits + 2, ws.rtc_a, ws.rowsum))) return rc;
     gb300_count_launch(), norm_from_rowsums_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, (n + 63) / 64, ws.rowsum,
@@ -1088,13 +1090,15 @@ int dsposv_fp64(cudaStream_t s, int n, int nrhs, const double *A, int lda, const
                                                                      ws.berr, ws.done, nullptr);
     std::vector<double> hb((size_t)nrhs);
     unsigned long long ab = 0;
+    int herr = 0;
     rc = gb300_record_cuda_error(cudaMemcpyAsync(hb.data(), ws.berr, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, s));
     if (!rc) rc = gb300_record_cuda_error(cudaMemcpyAsync(&ab, ws.anorm_bits, sizeof ab, cudaMemcpyDeviceToHost, s));
+    if (!rc) rc = gb300_record_cuda_error(cudaMemcpyAsync(&herr, ws.err, sizeof herr, cudaMemcpyDeviceToHost, s));
     if (!rc) rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
     if (rc) return rc;
     double worst = 0;
     for (double v : hb) worst = fmax(worst, v);
-    const int status = worst <= tol ? GB300_OK : GB300_ETIMEDOUT;
+    const int status = worst <= tol && !herr ? GB300_OK : GB300_ETIMEDOUT;
     if (out) {
         out->backward_error = worst;
         memcpy(&out->anorm, &ab, sizeof ab);

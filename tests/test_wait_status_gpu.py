@@ -5,12 +5,13 @@ The limit of a wait is set to 1 ns (starpu_gb300_set_wait_budget_ns), so that a
 wait which is not satisfied at once runs out; results of those calls are
 discarded.  Reference: numpy in FP64."""
 import contextlib
+import ctypes as C
 
 import numpy as np
 import pytest
 
 from starpu_gb300 import DeviceBuffer
-from starpu_gb300.native import check
+from starpu_gb300.native import IrInfo, check
 
 pytestmark = pytest.mark.gpu
 
@@ -144,3 +145,21 @@ def test_batched_solve_reports_a_wait_that_runs_out(gpu):
     with short_waits(gpu):
         assert solve()[0] == -1000
     assert np.all(solve() >= 0)
+
+
+def test_mixed_solve_does_not_take_a_wait_that_runs_out_for_a_bad_pivot(gpu):
+    n, nb = 2500, 1280  # diagonal tiles above 1024: the plain factorisation, whose info is negative then
+    a, b = spd(n, n), np.ones((n, 1))
+    da, db, dx = up(a), up(b), up(b)
+    lw = gpu.starpu_gb300_dsposv_workspace(n, 1, nb)
+    work = DeviceBuffer(lw)
+
+    def solve():
+        info = IrInfo()
+        rc = gpu.starpu_gb300_dsposv(None, n, 1, da.ptr, n, db.ptr, n, dx.ptr, n, nb, 3, 1e-12, 30, work.ptr, lw,
+                                     C.byref(info))
+        return rc, info.status, info.fallback
+
+    with short_waits(gpu):
+        assert solve() == (GB300_ETIMEDOUT, GB300_ETIMEDOUT, 0)
+    assert solve() == (0, 0, 0)
