@@ -17,7 +17,7 @@
 //
 // For the Schur complements of an SPD matrix this error is bounded like the
 // classical one, by eps sqrt(A_ii A_jj): a row of L never exceeds sqrt(A_ii).
-// A row that holds Inf or NaN gives NaN there.
+// Elements of a row that holds Inf or NaN are formed by FP64 FMAs.
 //
 // GEMM = false: k <= 64 (the trailing update of a panel), A stays cut over the
 // tiles of a row block.  GEMM = true: any k in chunks of 64, a tile's chunks
@@ -224,10 +224,10 @@ __device__ __forceinline__ bool su_wait_group(uint64_t *mbar, uint32_t parity, v
     return all != 0;
 }
 
-// acc 2^(e - 2098) as FP64, rounded to nearest (e: sum of two biased exponents)
+// acc 2^(e - 2098) as FP64, rounded to nearest (e: sum of two biased
+// exponents, finite)
 __device__ __noinline__ double su_to_double_any(long long acc, int e)
 {
-    if (e >= SU_NONFINITE) return __longlong_as_double(0x7FF8000000000000ll);
     if (acc == 0) return 0.0;
     const unsigned long long mag = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
     const int lz = __clzll((long long)mag);
@@ -405,7 +405,7 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                 double c[8];  // GEMM: the sum over the chunks; else C, read before the wait
 #pragma unroll
                 for (int j = 0; j < 8; ++j) c[j] = !GEMM && j < jn ? crow[(long)j * a.ldc] : 0.0;
-                unsigned weak = 0;  // GEMM: columns that need FMAs
+                unsigned weak = 0;  // columns that need FMAs
                 for (int ch = 0; ch < chunks; ++ch, ++tile) {
                     if (GEMM && !(ok = cut_a(ch * SU_K))) break;
                     const int buf = tile & 1;
@@ -420,9 +420,16 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                     ptx::tc_fence_after();
                     const int er = ea[(item & 3) * SU_BM + rl];
                     const int *ec = eb + (tile & 3) * SU_BN + 8 * group;
-                    int ev[8];
+                    int ev[8], special = 0;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) ev[j] = er + ec[j];
+                    for (int j = 0; j < 8; ++j) ev[j] = er + ec[j], special |= ev[j];
+                    if (__any_sync(0xffffffffu, special >= SU_NONFINITE)) {  // all of the warp's elements by FMAs
+                        weak = 0xff;
+                        ptx::tc_fence_before();
+                        ptx::mbar_arrive(&acc_empty[buf]);
+                        if (GEMM) ++item;
+                        continue;
+                    }
                     // 128 x 128 / 2 for 64 terms: half the product of two largest elements
                     const float least = 128.0f * (float)min(SU_K, a.k - ch * SU_K);
 #pragma unroll
@@ -449,10 +456,12 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                     }
                     if (GEMM) ++item;
                 }
-                if (!GEMM || !ok || bad) continue;
+                if (!ok || bad) continue;
+                if (GEMM) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (j < jn && !(weak >> j & 1)) crow[(long)j * a.ldc] -= c[j];
+                    for (int j = 0; j < 8; ++j)
+                        if (j < jn && !(weak >> j & 1)) crow[(long)j * a.ldc] -= c[j];
+                }
                 if (jn < 8) weak &= (1u << max(jn, 0)) - 1;
                 for (; weak; weak &= weak - 1) {
                     const int j = __ffs((int)weak) - 1;

@@ -260,3 +260,49 @@ def test_dpotrf_leaf_diagonal_is_the_square_root(gpu, n):
     got, ref = np.diag(da.download((n, n), np.float64)), np.sqrt(d)
     # half an ulp, and the residual's and the step's rounding (2^-53 of the ulp-sized step)
     assert np.all(np.abs(got - ref) <= np.spacing(ref))
+
+
+# an element of the result is Inf, NaN or finite as the FMA sum makes it: one and
+# two infinities in a row, zeros against them, short and ragged last chunks
+@pytest.mark.parametrize("form", ["syrk", "nt", "nn"])
+@pytest.mark.parametrize("k", [16, 17, 32, 64, 80, 129])
+def test_fp64_products_of_infinities(gpu, form, k):
+    m, n = 512, 512 if form == "syrk" else 400
+    rng = np.random.default_rng(k)
+    a, b, c = rng.standard_normal((m, k)), rng.standard_normal((n, k)), rng.standard_normal((m, n))
+    a[3, 1], a[200, k - 1], a[7, 0], a[7, 5] = np.inf, -np.inf, np.inf, -np.inf
+    a[9, 2] = np.nan
+    b[5, 1], b[6, 1], b[300, 3] = 0.0, -0.0, -np.inf
+    c[3, 20], c[100, 40] = np.inf, -np.inf
+    if form == "syrk":
+        b = a
+    with np.errstate(invalid="ignore"):
+        ref = c.copy()
+        for p in range(k):  # (a BLAS may treat infinities in blocks)
+            ref -= a[:, p, None] * b[None, :, p]
+    da, dc = up(a), up(c)
+    db = up(b.T if form == "nn" else b)
+    if form == "syrk":
+        check(gpu.starpu_gb300_dsyrk_ln_tile(None, n, k, -1.0, da.ptr, n, 1.0, dc.ptr, n))
+    elif form == "nt":
+        check(gpu.starpu_gb300_dgemm_nt_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    else:
+        check(gpu.starpu_gb300_dgemm_nn_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, k, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float64)
+    keep = np.tril(np.ones((m, n), bool)) if form == "syrk" else np.ones((m, n), bool)
+    for f in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(f(out)[keep], f(ref)[keep])
+
+
+def test_fp64_trailing_update_of_an_infinity(gpu):
+    # the panel's row i is infinite: C_ij -= inf l_j, so -inf or +inf by the sign of l_j
+    n, i = 400, 250
+    a = spd(n, n)
+    a[i, 10] = a[10, i] = np.inf
+    da, info = up(a), up(np.zeros(1, np.int32))
+    check(gpu.starpu_gb300_dpotrf(None, n, da.ptr, n, 64, info.ptr))
+    assert info.download((1,), np.int32)[0] == i + 1
+    out = da.download((n, n), np.float64)
+    ref = np.linalg.cholesky(spd(n, n)[:i, :i])
+    assert np.allclose(np.tril(out[:i, :i]), ref, rtol=0, atol=1e-13)
+    assert np.isposinf(out[i, 10])
