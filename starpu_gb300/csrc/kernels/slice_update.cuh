@@ -124,7 +124,8 @@ struct SliceItems {
 };
 
 // The 16 elements v (k = 16 g .. 16 g + 15 of row `row`) as digits relative to
-// biased exponent e, written to the 7 slices at `dst` (row pitch 128 bytes,
+// biased exponent e >= 1 (subnormal numbers have exponent 1 and no leading one),
+// written to the 7 slices at `dst` (row pitch 128 bytes,
 // 128-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)).
 __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, uint8_t *dst, int slice_bytes, int row, int g)
 {
@@ -139,8 +140,8 @@ __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, ui
                 const unsigned long long u = (unsigned long long)__double_as_longlong(v[8 * half + 2 * p + q]);
                 const int ex = (int)(u >> 52) & 0x7FF;
                 // |x| 2^(55 + 1) / 2^(e - 1022), shifted down and rounded to the last place
-                unsigned long long F = ex ? ((u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 3 : 0ull;
-                F = ((F >> min(e - ex, 63)) + 1) >> 1;
+                unsigned long long F = ((u & 0xFFFFFFFFFFFFFull) | (ex ? 0x10000000000000ull : 0ull)) << 3;
+                F = ((F >> min(e - max(ex, 1), 63)) + 1) >> 1;
                 const unsigned long long G =
                     ((long long)u < 0 ? 0ull - F : F) + 0x0080808080808080ull;  // every digit + 128
                 h[q] = (uint32_t)(G >> 32);
@@ -206,7 +207,7 @@ __device__ __forceinline__ void su_convert(const double (&v)[16], int *ex, uint8
     rp ^= 1;
     r[cw * 32 + lane] = mx;
     asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
-    const int e = (int)(max(max(r[lane], r[32 + lane]), max(r[64 + lane], r[96 + lane])) >> 20);
+    const int e = max((int)(max(max(r[lane], r[32 + lane]), max(r[64 + lane], r[96 + lane])) >> 20), 1);
     if (cw == 0) ex[lane] = e == 0x7FF ? SU_NONFINITE : e;
     su_write_digits(v, e, dst, slice_bytes, row, cw);
 }

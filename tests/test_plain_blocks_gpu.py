@@ -306,3 +306,20 @@ def test_fp64_trailing_update_of_an_infinity(gpu):
     ref = np.linalg.cholesky(spd(n, n)[:i, :i])
     assert np.allclose(np.tril(out[:i, :i]), ref, rtol=0, atol=1e-13)
     assert np.isposinf(out[i, 10])
+
+
+# rows in or near the subnormal range, elements spread over 52 powers of two, against large ones
+@pytest.mark.parametrize("k", [16, 64, 100])
+@pytest.mark.parametrize("top", [-1074, -1060, -1022, -1000, -970, -960])
+def test_fp64_products_of_subnormal_rows(gpu, k, top):
+    m, n = 512, 400
+    rng = np.random.default_rng(k - top)
+    a = np.ldexp(rng.uniform(0.5, 1, (m, k)), rng.integers(top - 50, top + 2, (m, k)))  # some round to subnormals or 0
+    b = np.ldexp(rng.uniform(0.5, 1, (n, k)), 900)
+    c = np.zeros((m, n))
+    da, db, dc = up(a), up(b), up(c)
+    check(gpu.starpu_gb300_dgemm_nt_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float64)
+    # scaled into the normal range (exact: powers of two), summed there
+    ref, mag = -(np.ldexp(a, 600) @ np.ldexp(b, -900).T), np.abs(np.ldexp(a, 600)) @ np.abs(np.ldexp(b, -900)).T
+    assert np.all(np.abs(np.ldexp(out, -300) - ref) <= 2 * (k + 2) * EPS[np.float64] * mag)
