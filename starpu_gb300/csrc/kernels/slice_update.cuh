@@ -236,13 +236,13 @@ __device__ __noinline__ double su_to_double_any(long long acc, int e)
     const int ex = e - 1012 - lz;  // biased exponent of the result
     const unsigned long long sign = (unsigned long long)acc & 0x8000000000000000ull;
     unsigned long long bits;
-    if (ex > 0 && ex < 2046) {
+    if (ex > 0 && ex < 2047) {  // (rounding up from the largest exponent gives Inf)
         bits = ((unsigned long long)(ex - 1) << 52) + (norm >> 11) + ((norm >> 10) & 1);
-    } else if (ex >= 2046) {
+    } else if (ex >= 2047) {
         bits = 0x7FF0000000000000ull;
     } else {  // below the normal range
         const int s = 12 - ex;
-        bits = s < 64 ? ((norm >> (s - 1)) + 1) >> 1 : 0ull;
+        bits = s <= 64 ? ((norm >> (s - 1)) + 1) >> 1 : 0ull;
     }
     return __longlong_as_double((long long)(bits | sign));
 }
@@ -253,7 +253,7 @@ __device__ __forceinline__ double su_to_double(long long acc, int e)
     const unsigned long long mag = (unsigned long long)(acc < 0 ? -acc : acc);
     const uint32_t hi = (uint32_t)(mag >> 32), lo = (uint32_t)mag;
     const int lz = __clz((int)hi), ex = e - 1012 - lz;
-    if (hi == 0 || (unsigned)(ex - 1) >= 2045u) return su_to_double_any(acc, e);
+    if (hi == 0 || (unsigned)(ex - 1) >= 2046u) return su_to_double_any(acc, e);
     const uint32_t nh = __funnelshift_l(lo, hi, lz), nl = lo << lz;
     const unsigned long long m = ((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11);
     const unsigned long long bits = m + ((nl >> 10) & 1u) + ((unsigned long long)(uint32_t)(ex - 1) << 52);

@@ -323,3 +323,22 @@ def test_fp64_products_of_subnormal_rows(gpu, k, top):
     # scaled into the normal range (exact: powers of two), summed there
     ref, mag = -(np.ldexp(a, 600) @ np.ldexp(b, -900).T), np.abs(np.ldexp(a, 600)) @ np.abs(np.ldexp(b, -900)).T
     assert np.all(np.abs(np.ldexp(out, -300) - ref) <= 2 * (k + 2) * EPS[np.float64] * mag)
+
+
+# single products in the last binade and beyond it, and around half the smallest number
+@pytest.mark.parametrize("k", [16, 64])
+@pytest.mark.parametrize("top", [True, False])
+def test_fp64_products_at_the_ends_of_the_range(gpu, k, top):
+    m, n = 512, 400
+    rng = np.random.default_rng(k)
+    a, b, c = np.zeros((m, k)), np.zeros((n, k)), np.zeros((m, n))
+    a[:, 3] = np.ldexp(rng.uniform(1, 2, m), (511 + np.arange(m) % 3) if top else (-540 - np.arange(m) % 4))
+    b[:, 3] = np.ldexp(rng.uniform(1, 2, n), 511 if top else -535)
+    with np.errstate(over="ignore", under="ignore"):
+        ref = -(a[:, 3, None] * b[None, :, 3])  # one rounding
+    da, db, dc = up(a), up(b), up(c)
+    check(gpu.starpu_gb300_dgemm_nt_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float64)
+    fine = np.isfinite(ref)
+    assert np.array_equal(np.isneginf(out), ~fine) and fine.any() and (not top or not fine.all())
+    assert np.all(np.abs(out - ref)[fine] <= np.spacing(np.abs(ref))[fine])
