@@ -9,27 +9,44 @@
 // product is sum_d 2^{8 (14 - d)} S_d, S_d = sum_{t+u=d} a_t b_u; every S_d
 // over 64 terms is an integer below 2^23 (at most 7 pairs x 2^14 x 64), so
 // the tensor cores' FP32 accumulation is exact.  The pairs with t + u <= 8
-// are formed (28 products).  Error: F resolves a quarter of the last bit of
-// the row's largest element, the dropped pairs weigh below 2^-58 of
-// 2^(e_i + e_j) per term; an FP64 FMA rounds to 2^-53 of the running sum at
-// every term.  The epilogue adds the S_d as 64-bit integers (units of d = 7)
-// and rounds once to FP64.
+// are formed (28 products).  The scheme is the error-free splitting of matrix
+// products of Ozaki, Ogita, Oishi and Rump (Numerical Algorithms 59, 2012),
+// with the operands cut at fixed points.  The epilogue adds the S_d as 64-bit
+// integers (units of d = 7) and rounds once to FP64.
 //
-// For the Schur complements of an SPD matrix this error is bounded like the
-// classical one, by eps sqrt(A_ii A_jj): a row of L never exceeds sqrt(A_ii).
-// Elements of a row that holds Inf or NaN are formed by FP64 FMAs.
+// Error, in units of 2^(e_i + e_j), per term with two nonzero elements: F
+// rounds to half a unit, 2^-56 of either row's power of two, 2^-55 together; a
+// dropped diagonal d has 15 - d pairs of at most 2^14 2^{8 (14 - d)} / 2^110:
+// d = 9 has 6 2^-56, below 2^-53.4, and the rest 2^-61.7.  Once per 64 terms
+// S_8 is rounded: 2^-55.  With random digits the sum over d = 9 is some 2^-56
+// a term; with every low digit at -128 it is 2^-53.4.  An FP64 FMA rounds to
+// 2^-53 of the running sum at every term.
+//
+// For the Schur complements of an SPD matrix the running sum is bounded by
+// sqrt(A_ii A_jj), and so is 2^(e_i + e_j) within a factor of 4 (a row of L
+// never exceeds sqrt(A_ii)): an error of the same order even where every digit
+// is at its worst.  Elements of a row that holds Inf or NaN are formed by FP64
+// FMAs.
 //
 // GEMM = false: k <= 64 (the trailing update of a panel), A stays cut over the
 // tiles of a row block.  GEMM = true: any k in chunks of 64, a tile's chunks
 // summed in registers and C rounded once, as an FMA loop does; A is cut again
 // for every tile and chunk.
 //
-// Products of other matrices (GEMM = true) run guarded: FP64's error is bounded by
-// eps sum_k |a_ik| |b_jk|, which may be far below eps max|a_i| max|b_j| (large
-// elements of a_i that meet small ones of b_j).  One more product, of the
-// magnitudes of the leading digits, estimates that sum from below; an element
-// whose estimate is under half of 2^(e_i + e_j) is formed by FP64 FMAs instead.
-// So are zero rows and rows with Inf or NaN.
+// Products of other matrices (GEMM = true) run guarded: the error of an FP64
+// FMA loop is bounded by k 2^-53 G, G = sum_k |a_ik| |b_jk|, which may be far
+// below k 2^-53 2^(e_i + e_j) (large elements of a_i that meet small ones of
+// b_j).  Here the pairs with t + u = 9 are formed, too (scaled by 2^-8 in the
+// accumulator of d = 8, whose roundings weigh 2^-61), so that the error of a
+// chunk of c terms, z of them with two nonzero elements, is below
+// (z (2^-55 + 2^-61.7) + 2^-55 + 2^-57) 2^(e_i + e_j), and one more product, of
+// the top seven bits of |a_ik| 2^-e_i and |b_jk| 2^-e_j cut off, gives 2^14 G
+// from below.  Where that is below (4200 z + 5200) / c the error might exceed
+// c 2^-53 G, and the element is formed by FP64 FMAs; z = 0 needs none (z: the
+// smaller of the two rows' nonzero elements).  An element formed by FMAs costs
+// its products twice: with nearly all of them so (columns graded over 14 orders of
+// magnitude) 512^3 takes 598 us where FMAs alone took 545 and random operands,
+// which need none, take 79; 512 x 512 x 16 44, 35 and 25 us.
 //
 // The operands are cut in the kernel, so no workspace is needed.  A CTA (one
 // per SM, persistent) keeps the slices of 128 rows of A in shared memory and
@@ -61,11 +78,11 @@ namespace gb300 {
 constexpr int SU_BM = 128, SU_BN = 32, SU_K = 64, SU_S = 7;
 constexpr int SU_SLICE_A = SU_BM * SU_K * 2;  // 16 KB: one 128-byte row per matrix row
 constexpr int SU_SLICE_B = SU_BN * SU_K * 2;  // 4 KB
-constexpr int SU_ABS = SU_S;  // slice of the leading digits' magnitudes (guarded products)
+constexpr int SU_ABS = SU_S;  // slice of the top bits of the magnitudes (guarded products)
 constexpr int SU_A_BYTES = (SU_S + 1) * SU_SLICE_A, SU_B_BYTES = (SU_S + 1) * SU_SLICE_B;
 constexpr int SU_EPI = 16 * 32, SU_CONV = 4 * 32, SU_THREADS = SU_EPI + SU_CONV + 32;
 constexpr int SU_MMA_WARP = (SU_EPI + SU_CONV) / 32;
-constexpr int SU_SMEM = SU_A_BYTES + 2 * SU_B_BYTES + 1024 /*align*/ + 8192 /*exponents, barriers*/;
+constexpr int SU_SMEM = SU_A_BYTES + 2 * SU_B_BYTES + 1024 /*align*/ + 11264 /*exponents, least sums, barriers*/;
 constexpr uint32_t SU_TMEM_COLS = 512, SU_ACC_STRIDE = 256;
 constexpr int SU_NONFINITE = 1 << 24;  // exponent of a row with Inf or NaN
 constexpr int SU_ERR_TIMEOUT = -1000;  // *err when a wait inside the kernel ran out
@@ -127,14 +144,15 @@ struct SliceItems {
 // biased exponent e >= 1 (subnormal numbers have exponent 1 and no leading one),
 // written to the 7 slices at `dst` (row pitch 128 bytes,
 // 128-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)).
+template <bool GEMM>
 __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, uint8_t *dst, int slice_bytes, int row, int g)
 {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        uint32_t d[SU_S][4];
+        uint32_t d[SU_S][4], mag[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            uint32_t h[2], l[2];
+            uint32_t h[2], l[2], m[2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const unsigned long long u = (unsigned long long)__double_as_longlong(v[8 * half + 2 * p + q]);
@@ -142,6 +160,7 @@ __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, ui
                 // |x| 2^(55 + 1) / 2^(e - 1022), shifted down and rounded to the last place
                 unsigned long long F = ((u & 0xFFFFFFFFFFFFFull) | (ex ? 0x10000000000000ull : 0ull)) << 3;
                 F = ((F >> min(e - max(ex, 1), 63)) + 1) >> 1;
+                m[q] = (uint32_t)(F >> 32);
                 const unsigned long long G =
                     ((long long)u < 0 ? 0ull - F : F) + 0x0080808080808080ull;  // every digit + 128
                 h[q] = (uint32_t)(G >> 32);
@@ -161,15 +180,21 @@ __device__ __forceinline__ void su_write_digits(const double (&v)[16], int e, ui
                 const __half2 x = __hadd2(*reinterpret_cast<const __half2 *>(&w[t]), off);
                 d[t][p] = *reinterpret_cast<const uint32_t *>(&x);
             }
+            if (GEMM) {  // F >> 48 as the FP16 1024 + it, minus 1024
+                const uint32_t w7 = __byte_perm(m[0], m[1], 0x7632) | 0x64006400u;
+                const __half2 x = __hadd2(*reinterpret_cast<const __half2 *>(&w7),
+                                          __half2half2(__ushort_as_half((unsigned short)0xE400)));
+                mag[p] = *reinterpret_cast<const uint32_t *>(&x);
+            }
         }
         const int chunk = (2 * g + half) ^ (row & 7);
 #pragma unroll
         for (int t = 0; t < SU_S; ++t)
             *reinterpret_cast<uint4 *>(dst + t * slice_bytes + row * 128 + chunk * 16) =
                 make_uint4(d[t][0], d[t][1], d[t][2], d[t][3]);
-        constexpr uint32_t MAG = 0x7FFF7FFFu;
-        *reinterpret_cast<uint4 *>(dst + SU_ABS * slice_bytes + row * 128 + chunk * 16) =
-            make_uint4(d[0][0] & MAG, d[0][1] & MAG, d[0][2] & MAG, d[0][3] & MAG);
+        if (GEMM)
+            *reinterpret_cast<uint4 *>(dst + SU_ABS * slice_bytes + row * 128 + chunk * 16) =
+                make_uint4(mag[0], mag[1], mag[2], mag[3]);
     }
 }
 
@@ -194,22 +219,36 @@ __device__ __forceinline__ void su_load(const double *src, long rs, long ks, int
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = in && k0 + i < k ? p[i * ks] : 0.0;
 }
-// their exponents to ex[0 .. 31] and slices to dst; rmax: [2][4][32] of the
-// group, rp alternates; bar: the group's named barrier
-__device__ __forceinline__ void su_convert(const double (&v)[16], int *ex, uint8_t *dst, int slice_bytes, int row, int cw,
+// their exponents to ex[0 .. 31], (GEMM) the least sums that their nonzero
+// elements of a chunk of `terms` ask for to least[0 .. 31], and their slices to
+// dst; rmax: [2][4][32] of the group, rp alternates; bar: the group's named barrier
+template <bool GEMM>
+__device__ __forceinline__ void su_convert(const double (&v)[16], int *ex, float *least, int terms, uint8_t *dst, int slice_bytes, int row, int cw,
                                            unsigned *rmax, int &rp, int bar)
 {
     const int lane = threadIdx.x & 31;
     unsigned mx = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) mx = max(mx, (unsigned)__double2hiint(v[i]) & 0x7FFFFFFFu);
+    if (GEMM) {  // the exponent, and the number of nonzero elements below it
+        mx &= 0x7FF00000u;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            mx += (((unsigned)__double2hiint(v[i]) << 1) | (unsigned)__double2loint(v[i])) != 0 ? 1u : 0u;
+    }
     unsigned *r = rmax + rp * 128;
     rp ^= 1;
     r[cw * 32 + lane] = mx;
     asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
     const int e = max((int)(max(max(r[lane], r[32 + lane]), max(r[64 + lane], r[96 + lane])) >> 20), 1);
-    if (cw == 0) ex[lane] = e == 0x7FF ? SU_NONFINITE : e;
-    su_write_digits(v, e, dst, slice_bytes, row, cw);
+    if (cw == 0) {
+        ex[lane] = e == 0x7FF ? SU_NONFINITE : e;
+        if (GEMM) {
+            const unsigned z = (r[lane] + r[32 + lane] + r[64 + lane] + r[96 + lane]) & 0x7FFu;
+            least[lane] = z ? (4200.0f * (float)z + 5200.0f) / (float)terms : 0.0f;
+        }
+    }
+    su_write_digits<GEMM>(v, e, dst, slice_bytes, row, cw);
 }
 // A bounded wait that all four warps of a group pass or none does (they meet
 // at barriers afterwards); bar: a named barrier for the vote.  bad: this warp
@@ -282,7 +321,8 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
     uint8_t *sA = smem, *sB = smem + SU_A_BYTES;
     int *ea = (int *)(sB + 2 * SU_B_BYTES);         // [4][128] row exponents of A, by item
     int *eb = ea + 4 * SU_BM;                       // [4][32] of B, by tile
-    unsigned *rmax = (unsigned *)(eb + 4 * SU_BN);  // [5 groups][2][4][32]
+    float *la = (float *)(eb + 4 * SU_BN), *lb = la + 4 * SU_BM;  // GEMM: least sums, like ea and eb
+    unsigned *rmax = (unsigned *)(lb + 4 * SU_BN);  // [5 groups][2][4][32]
     uint64_t *bars = (uint64_t *)(rmax + 5 * 2 * 4 * 32);
     uint64_t *b_full = bars, *b_empty = bars + 2, *acc_full = bars + 4, *acc_empty = bars + 6;
     uint64_t *a_full = bars + 8, *a_empty = bars + 9, *drain = bars + 10;
@@ -325,7 +365,8 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
             for (int t = t0, ch = 0; t < t1; ++tile) {
                 const int buf = tile & 1;
                 if (!(ok = su_wait_group(&b_empty[buf], ((tile >> 1) & 1) ^ 1, abort_flag, a.wait_budget_ns, 1))) break;
-                su_convert(v, eb + (tile & 3) * SU_BN, sB + buf * SU_B_BYTES, SU_SLICE_B, lane, cw, rmax + 4 * 256, rp, 2);
+                su_convert<GEMM>(v, eb + (tile & 3) * SU_BN, lb + (tile & 3) * SU_BN, min(SU_K, a.k - ch * SU_K),
+                                 sB + buf * SU_B_BYTES, SU_SLICE_B, lane, cw, rmax + 4 * 256, rp, 2);
                 ptx::fence_proxy_async_smem();
                 ptx::mbar_arrive(&b_full[buf]);
                 if (++ch == chunks) ch = 0, ++t;
@@ -350,16 +391,30 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                     const uint32_t d = tmem_base + (uint32_t)buf * SU_ACC_STRIDE;
                     const uint32_t aA = ptx::smem_u32(sA), aB = ptx::smem_u32(sB + buf * SU_B_BYTES);
                     const int ks = (min(SU_K, a.k - ch * SU_K) + 15) / 16;
+                    constexpr uint32_t N1 = ptx::make_idesc(SU_BM, SU_BN, ptx::FMT_F16);
+                    if (GEMM)  // S_9, where S_8 goes
+                        for (int k = 0; k < ks; ++k)
+#pragma unroll
+                            for (int s = 1; s < SU_S; ++s)
+                                ptx::mma_f16_ss(d + (SU_S - 1) * SU_BN, ptx::make_sdesc_k128(aA + s * SU_SLICE_A + k * 32),
+                                                ptx::make_sdesc_k128(aB + (SU_S - s) * SU_SLICE_B + k * 32), N1,
+                                                (k || s > 1) ? 1u : 0u);
                     for (int k = 0; k < ks; ++k) {
                         const uint64_t bd = ptx::make_sdesc_k128(aB + k * 32);
+                        if (GEMM && k == 0) {  // s = 0: a start for S_2 .. S_7, S_9 2^-8 goes on as S_8
+                            ptx::mma_f16_ss(d, ptx::make_sdesc_k128(aA), bd,
+                                            ptx::make_idesc(SU_BM, SU_BN * (SU_S - 1), ptx::FMT_F16), 0u);
+                            ptx::mma_f16_ss_scale8(d + (SU_S - 1) * SU_BN, ptx::make_sdesc_k128(aA),
+                                                   ptx::make_sdesc_k128(aB + (SU_S - 1) * SU_SLICE_B), N1);
+                        }
 #pragma unroll
                         for (int s = 0; s < SU_S; ++s)
-                            ptx::mma_f16_ss(d + s * SU_BN, ptx::make_sdesc_k128(aA + s * SU_SLICE_A + k * 32), bd,
-                                            ptx::make_idesc(SU_BM, SU_BN * (SU_S - s), ptx::FMT_F16), (k | s) ? 1u : 0u);
+                            if (!(GEMM && k == 0 && s == 0))
+                                ptx::mma_f16_ss(d + s * SU_BN, ptx::make_sdesc_k128(aA + s * SU_SLICE_A + k * 32), bd,
+                                                ptx::make_idesc(SU_BM, SU_BN * (SU_S - s), ptx::FMT_F16), (k | s) ? 1u : 0u);
                         if (GEMM)
                             ptx::mma_f16_ss(d + SU_ABS * SU_BN, ptx::make_sdesc_k128(aA + SU_ABS * SU_SLICE_A + k * 32),
-                                            ptx::make_sdesc_k128(aB + SU_ABS * SU_SLICE_B + k * 32),
-                                            ptx::make_idesc(SU_BM, SU_BN, ptx::FMT_F16), k ? 1u : 0u);
+                                            ptx::make_sdesc_k128(aB + SU_ABS * SU_SLICE_B + k * 32), N1, k ? 1u : 0u);
                     }
                     ptx::mma_commit(&b_empty[buf]);
                     ptx::mma_commit(&acc_full[buf]);
@@ -387,8 +442,9 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
             double v[16];
             su_load(a.A, a.a_rs, a.a_ks, it.rb * SU_BM + 32 * group, a.m, k0, a.k, quarter, v);
             if (!su_wait_group(a_empty, (item & 1) ^ 1, abort_flag, a.wait_budget_ns, 3 + group, bad)) return false;
-            su_convert(v, ea + (item & 3) * SU_BM + 32 * group, sA, SU_SLICE_A, 32 * group + lane, quarter,
-                       rmax + group * 256, rp, 7 + group);
+            su_convert<GEMM>(v, ea + (item & 3) * SU_BM + 32 * group, la + (item & 3) * SU_BM + 32 * group,
+                             min(SU_K, a.k - k0), sA, SU_SLICE_A, 32 * group + lane, quarter, rmax + group * 256, rp,
+                             7 + group);
             ptx::fence_proxy_async_smem();
             ptx::mbar_arrive(a_full);
             return true;
@@ -431,8 +487,8 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                         if (GEMM) ++item;
                         continue;
                     }
-                    // 128 x 128 / 2 for 64 terms: half the product of two largest elements
-                    const float least = 128.0f * (float)min(SU_K, a.k - ch * SU_K);
+                    const float lr = GEMM ? la[(item & 3) * SU_BM + rl] : 0.0f;
+                    const float *lc = lb + (tile & 3) * SU_BN + 8 * group;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         uint32_t r[SU_S][4], mag[4];
@@ -448,7 +504,7 @@ template <bool GEMM> __global__ void __launch_bounds__(SU_THREADS, 1) slice_upda
                         for (int j = 0; j < 4; ++j) {
                             const double v = su_to_double(su_combine(r, j), ev[4 * h + j]);
                             if (GEMM) {
-                                if (__uint_as_float(mag[j]) < least) weak |= 1u << (4 * h + j);
+                                if (__uint_as_float(mag[j]) < fminf(lr, lc[4 * h + j])) weak |= 1u << (4 * h + j);
                                 c[4 * h + j] += v;
                             } else if (4 * h + j < jn) {
                                 crow[(long)(4 * h + j) * a.ldc] = c[4 * h + j] - v;

@@ -342,3 +342,29 @@ def test_fp64_products_at_the_ends_of_the_range(gpu, k, top):
     fine = np.isfinite(ref)
     assert np.array_equal(np.isneginf(out), ~fine) and fine.any() and (not top or not fine.all())
     assert np.all(np.abs(out - ref)[fine] <= np.spacing(np.abs(ref))[fine])
+
+
+# one pair of larger elements, from a hundredth of the rows' maxima up to both, among elements whose digits
+# below the first are all -128, so that the digit products left out add up; some of the elements zero
+@pytest.mark.parametrize("k", [16, 17, 32, 64, 100])
+@pytest.mark.parametrize("zeros", [0.0, 0.8])
+def test_fp64_products_keep_the_bound_at_the_worst_digits(gpu, k, zeros):
+    m, n = 512, 400
+    rng = np.random.default_rng(k)
+    low = sum(2.0 ** (8 * (7 - t)) for t in range(2, 8))
+    cut = lambda first: np.ldexp(first * 2.0**48 - 128.0 * low, -55)  # first digit, then -128s: exact in FP64
+    a, b = np.full((m, k), cut(1.0)), np.full((n, k), cut(1.0))
+    a[:, 2:][rng.uniform(size=(m, k - 2)) < zeros] = 0
+    b[:, 2:][rng.uniform(size=(n, k - 2)) < zeros] = 0
+    a[:, 0], b[:, 0] = cut(128.0), 0.0  # the rows' maxima, against nothing
+    a[:, 1], b[:, 1] = cut(1.0 + np.arange(m) % 128), cut(1.0 + np.arange(n) % 128)
+    b[:, 0] = np.where(np.arange(n) % 2, 0.0, -cut(1.0))
+    c = np.zeros((m, n))
+    da, db, dc = up(a), up(b), up(c)
+    check(gpu.starpu_gb300_dgemm_nt_tile(None, m, n, k, -1.0, da.ptr, m, db.ptr, n, 1.0, dc.ptr, m))
+    out = dc.download((m, n), np.float64)
+    ref, mag = np.zeros((m, n), np.longdouble), np.zeros((m, n))
+    for p in range(k):
+        ref -= a[:, p, None].astype(np.longdouble) * b[None, :, p]
+        mag += np.abs(a[:, p, None] * b[None, :, p])
+    assert np.all(np.abs((out - ref).astype(np.float64)) <= (k + 2) * EPS[np.float64] * mag)
