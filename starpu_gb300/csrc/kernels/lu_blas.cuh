@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(256) getf2_small_kernel(int n, T *__restrict__
 // step factors its 4 x 4 block in every lane, forms its columns of L and
 // publishes them with the reciprocal pivots; the others form their elements
 // of the four rows of U from the 4 x 4 block (four shuffles per column) and
-// apply the rank-4 update.  Bound by the chain of 16 steps: 10 us against 36
+// apply the rank-4 update to the rows below (the rows above are finished, and
+// stay as they are where a zero pivot makes U infinite).  Bound by the chain of 16 steps: 10 us against 36
 // for a barrier and a double-precision reciprocal per column.  Same status words
 // and threshold as getf2_small_kernel.
 // ---------------------------------------------------------------------------
@@ -100,20 +101,21 @@ struct GetfPanel {
     uint64_t bar[16];
 };
 
-template <int G> __device__ __forceinline__ void getf_update(CpBlock<float> &a, const GetfPanel &s, int step)
+// HS = step / 8: the half of the rows that holds the step's
+template <int G, int HS> __device__ __forceinline__ void getf_update(CpBlock<float> &a, const GetfPanel &s, int step)
 {
-    const int lane = threadIdx.x & 31, hs = step >> 3, blk = step & 7;
+    const int lane = threadIdx.x & 31, blk = step & 7;
     const Quad<float> *p = s.pan[step];
     Quad<float> li[2], l[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) li[h] = p[32 * h + lane];
+    for (int h = HS; h < 2; ++h) li[h] = p[32 * h + lane];
 #pragma unroll
     for (int i = 0; i < 4; ++i) l[i] = p[4 * step + i];
     const Quad<float> inv = s.inv[step];
-    const bool in = (lane >> 2) == blk;
+    const bool in = (lane >> 2) == blk, below = (lane >> 2) > blk;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const float v = hs ? a[G][c][1] : a[G][c][0];
+        const float v = a[G][c][HS];
         Quad<float> u;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -123,10 +125,9 @@ template <int G> __device__ __forceinline__ void getf_update(CpBlock<float> &a, 
             u.v[i] = t * inv.v[i];
         }
         const float mine = (lane & 2) ? ((lane & 1) ? u.v[3] : u.v[2]) : ((lane & 1) ? u.v[1] : u.v[0]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (in && h == hs) a[G][c][h] = mine;
-            else if (h >= hs) a[G][c][h] = cp_dot_sub(a[G][c][h], li[h], u);
+        const float upd = cp_dot_sub(v, li[HS], u);
+        a[G][c][HS] = in ? mine : below ? upd : v;
+        if (HS == 0) a[G][c][1] = cp_dot_sub(a[G][c][1], li[1], u);
     }
 }
 
@@ -213,17 +214,22 @@ __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restric
 #pragma unroll 1
     for (int i = 0; i < min(w, steps); ++i) {
         ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
-        getf_update<0>(a, s, i);
-        if (i < w - 1) getf_update<1>(a, s, i);  // the next owner publishes first
+        getf_update<0, 0>(a, s, i);
+        if (i < w - 1) getf_update<1, 0>(a, s, i);  // the next owner publishes first
     }
     if (w < steps) getf_own<0>(a, s, n, thr, d_first, info, info_base);
     if (steps > 8) {
-        if (w > 0) getf_update<1>(a, s, w - 1);
-        getf_update<1>(a, s, w);
+        if (w > 0) getf_update<1, 0>(a, s, w - 1);
+        getf_update<1, 0>(a, s, w);
 #pragma unroll 1
-        for (int i = w + 1; i < min(8 + w, steps); ++i) {
+        for (int i = w + 1; i < 8; ++i) {
             ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
-            getf_update<1>(a, s, i);
+            getf_update<1, 0>(a, s, i);
+        }
+#pragma unroll 1
+        for (int i = 8; i < min(8 + w, steps); ++i) {
+            ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
+            getf_update<1, 1>(a, s, i);
         }
         if (8 + w < steps) getf_own<1>(a, s, n, thr, d_first, info, info_base);
     }
