@@ -156,8 +156,11 @@ template <bool ANY> __device__ __forceinline__ void cp_factor4(float (&l)[4][4],
     }
 }
 
+// The first pivot of the four that is not positive, or -1.  Of a panel's steps
+// only the first that has one says so: it sets `found` before its columns are
+// published, so that the steps behind them see it.
 template <int NX, int G>
-__device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Quad<float> *p)
+__device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Quad<float> *p, volatile int *found)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float l[4][4], r[4];
@@ -187,6 +190,11 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
 #pragma unroll
         for (int j = 3; j >= 0; --j)
             if (!(l[j][j] > 0.0f)) bad = j;
+        if (bad >= 0) {
+            if (*found) bad = -1;
+            __syncwarp();
+            *found = 1;
+        }
     }
     auto solve = [&](float(&c)[4][2], int h, int row) {
         Quad<float> y;
@@ -208,11 +216,12 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
 }
 
 // The whole panel; `phase` is the parity of the mbarriers (0 for the first
-// panel of a kernel, then in turn), with a CTA barrier between two panels.
-// False: a wait ran out.
+// panel of a kernel, then in turn), with a CTA barrier between two panels;
+// found: a word of shared memory.  False: a wait ran out.
 template <typename T, int NX>
 __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T, NX> &pan, uint64_t (&bar)[16], uint32_t phase,
-                                         int n, int *info, int info_base, bool report, unsigned long long ns)
+                                         volatile int *found, int n, int *info, int info_base, bool report,
+                                         unsigned long long ns)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int steps = (n + 3) / 4;
@@ -221,6 +230,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         ptx::mbar_arrive(&bar[step]);
         if (bad >= 0 && report && lane == 0 && info && 4 * step + bad < n) atomicCAS(info, 0, info_base + 4 * step + bad + 1);
     };
+    if (threadIdx.x == 0) *found = 0;  // (warp 0 owns step 0, which every other step waits for)
 #pragma unroll 1
     for (int i = 0; i < min(w, steps) - 1; ++i) {
         ok = cp_wait(&bar[i], phase, ns) && ok;
@@ -231,7 +241,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
     }
     // (every mbarrier completes in every panel, so that all keep one parity)
-    if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w]));
+    if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w], found));
     else ptx::mbar_arrive(&bar[w]);
     if (8 + w >= steps) ptx::mbar_arrive(&bar[8 + w]);
     __syncwarp();
@@ -243,7 +253,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         ok = cp_wait(&bar[i], phase, ns) && ok;
         cp_update<T, NX, 1, 1>(d, x, pan[i]);
     }
-    if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w]));
+    if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w], found));
     return ok;
 }
 
@@ -253,12 +263,13 @@ potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_ba
 {
     __shared__ CpPanel<float, 0> pan;
     __shared__ uint64_t bar[16];
+    __shared__ int found;
     CpBlock<float> a;
     cp_panel_init(bar);
     // rows and columns past n continue the block as the identity
     cp_each<float>(a, [&](float &v, int r, int c) { v = (r < n && c <= r) ? A[r + (long)c * lda] : (r == c ? 1.0f : 0.0f); });
     __syncthreads();
-    if (!cp_panel<float, 0>(a, a, pan, bar, 0, n, info, info_base, true, wait.ns)) wait.report();
+    if (!cp_panel<float, 0>(a, a, pan, bar, 0, &found, n, info, info_base, true, wait.ns)) wait.report();
     cp_each<float>(a, [&](float &v, int r, int c) {
         if (r < n && c <= r) A[r + (long)c * lda] = v;
     });
@@ -313,7 +324,14 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
         }
         if (mine < n) {
             const double piv = __shfl_sync(0xffffffffu, a[H0][q][H0], 8 * q + w);
-            const double r = cp_normal(piv) ? cp_rsqrt(piv) : cp_rsqrt_any(piv);
+            double r;
+            if (cp_normal(piv)) {
+                r = cp_rsqrt(piv);
+            } else {
+                r = cp_rsqrt_any(piv);
+                // (before the column is published: the first bad pivot is the first to get there)
+                if (!(piv > 0.0) && lane == 0 && info) atomicCAS(info, 0, info_base + mine + 1);
+            }
 #pragma unroll
             for (int h = H0; h < 2; ++h) {
                 a[H0][q][h] *= r;
@@ -321,7 +339,6 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
             }
             ptx::mbar_arrive(&bar[mine]);
             if (lane == 0) pv[mine] = make_double2(piv, r);
-            if (!(piv > 0.0) && lane == 0 && info) atomicCAS(info, 0, info_base + mine + 1);
             __syncwarp();
             if (w > 0) rest(mine - 1, q + 1);
             rest(mine, q + 1);

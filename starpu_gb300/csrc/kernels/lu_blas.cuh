@@ -131,6 +131,14 @@ template <int G, int HS> __device__ __forceinline__ void getf_update(CpBlock<flo
     }
 }
 
+// the zeros among the pivots of columns z .. z + 3
+static __device__ __noinline__ void getf_report_zero(Quad<float> piv, int z, int n, int *info, int info_base)
+{
+    if ((threadIdx.x & 31) == 0 && info)
+        for (int j = 0; j < 4; ++j)
+            if (piv.v[j] == 0.0f && z + j < n) atomicCAS(info, 0, info_base + z + j + 1);
+}
+
 // the owner's part of step 8 G + warp
 template <int G>
 __device__ __forceinline__ void getf_own(CpBlock<float> &a, GetfPanel &s, int n, float thr, int *d_first, int *info,
@@ -188,15 +196,15 @@ __device__ __forceinline__ void getf_own(CpBlock<float> &a, GetfPanel &s, int n,
         p[32 * h + lane] = y;
     }
     if (lane == 0) s.inv[step] = {inv[0], inv[1], inv[2], inv[3]};
+    // (before the step is published: the first zero pivot is the first to get
+    // there; every lane knows the pivots, so the branch is the whole warp's)
+    if (fminf(fminf(fabsf(l[0][0]), fabsf(l[1][1])), fminf(fabsf(l[2][2]), fabsf(l[3][3]))) == 0.0f)
+        getf_report_zero({l[0][0], l[1][1], l[2][2], l[3][3]}, 4 * step, n, info, info_base);
     ptx::mbar_arrive(&s.bar[step]);
-    if (lane == 0) {
+    if (lane == 0 && thr > 0.0f && d_first) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int z = 4 * step + j;
-            if (z >= n) break;
-            if (l[j][j] == 0.0f && info) atomicCAS(info, 0, info_base + z + 1);
-            if (thr > 0.0f && !(fabsf(l[j][j]) >= thr) && d_first) atomicMin(d_first, info_base + z);
-        }
+        for (int j = 0; j < 4; ++j)
+            if (4 * step + j < n && !(fabsf(l[j][j]) >= thr)) atomicMin(d_first, info_base + 4 * step + j);
     }
     __syncwarp();
 }

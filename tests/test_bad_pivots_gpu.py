@@ -31,3 +31,18 @@ def test_zero_pivot_leaves_earlier_rows_as_they_are(gpu, dtype, n, z):
     assert np.all(np.isfinite(out[:z]))
     l, u = np.tril(out[:z, :z]), np.triu(out[:z], 1) + np.eye(z, n)
     assert np.all(np.abs(l @ u - a[:z]) <= 2 * (n + 1) * EPS[dtype] * (np.abs(l) @ np.abs(u)))
+
+
+@BOTH
+@pytest.mark.parametrize("n", [5, 64, 200])
+def test_the_first_of_many_bad_pivots_is_reported(gpu, dtype, n):
+    # from pivot z on every pivot is bad, and each is known at once to the warp that owns it
+    for z in (0, 1, 2, 3, 4, n // 2, n - 1):
+        chol, lu = np.eye(n, dtype=dtype), np.eye(n, dtype=dtype)
+        chol[range(z, n), range(z, n)] = -1
+        lu[range(z, n), range(z, n)] = 0
+        for _ in range(20):
+            dc, dl, info = up(chol), up(lu), up(np.zeros(2, np.int32))
+            check(getattr(gpu, f"starpu_gb300_{P[dtype]}potrf")(None, n, dc.ptr, n, 64, info.ptr))
+            check(getattr(gpu, f"starpu_gb300_{P[dtype]}getrf_tile")(None, n, dl.ptr, n, info.ptr + 4))
+            assert info.download((2,), np.int32).tolist() == [z + 1, z + 1]
