@@ -277,7 +277,7 @@ static int run_batched(cudaStream_t s, int nsys, const int *n, const double *A, 
     a.nrhs = nrhs;
     a.max_iter = max_iter;
     a.tol = tol;
-    a.wait_ns = gb300_wait_budget_ns();
+    a.wait_us = gb300_wait_us();
     a.sys = ws.sys;
     a.state = ws.state;
     a.cnt = ws.cnt;

@@ -274,7 +274,7 @@ int potrf_tiled(cudaStream_t s, int n, T *A, long lda, int nb, int *info, int in
 {
     int rc = GB300_OK;
     if (nb <= 0) nb = n;
-    const CpWait wait{gb300_wait_budget_ns(), info ? info : gb300_wait_status()};
+    const CpWait wait{gb300_wait_us(), info ? info : gb300_wait_status()};
     if (!wait.err) return GB300_ECUDA;
     if (std::is_same<T, float>::value && n <= COOP_MAX_N) nb = n;
     // FP64: the FP64 units would bound wider panels, the tensor-core update takes 64 columns
@@ -342,7 +342,7 @@ template <typename T>
 void potrs_blocked(cudaStream_t s, int n, int nrhs, const T *L, long ldl, T *B, long ldb, int *err)
 {
     if (n <= 0 || nrhs <= 0) return;
-    const CpWait wait{gb300_wait_budget_ns(), err ? err : gb300_wait_status()};
+    const CpWait wait{gb300_wait_us(), err ? err : gb300_wait_status()};
     if (!wait.err) return;
     if (nrhs == 1) potrs_sweeps<T, 1>(s, n, nrhs, L, ldl, B, ldb, wait);
     else if (nrhs <= 4) potrs_sweeps<T, 4>(s, n, nrhs, L, ldl, B, ldb, wait);

@@ -24,7 +24,7 @@ template <typename T>
 static void getrf_blocked(cudaStream_t s, int n, T *A, long lda, T thr, int *d_first, int *info)
 {
     constexpr int W = sizeof(T) == 4 ? 64 : 32;
-    const CpWait wait{gb300_wait_budget_ns(), info ? info : gb300_wait_status()};
+    const CpWait wait{gb300_wait_us(), info ? info : gb300_wait_status()};
     if (!wait.err) return;
     for (int k0 = 0; k0 < n; k0 += W) {
         const int kb = std::min(W, n - k0);

@@ -457,7 +457,7 @@ static int diag_factor_inverse(cudaStream_t s, int n, float *A, long lda, float 
     a.bar = bar;
     a.err = err;
     a.err_code = bar ? DC_ERR_TIMEOUT : CP_ERR_TIMEOUT;
-    a.wait_ns = gb300_wait_budget_ns();
+    a.wait_us = gb300_wait_us();
     a.invert = invert ? 1 : 0;
     void *args[] = {&a};
     gb300_count_launch();

@@ -125,6 +125,12 @@ extern "C" int gb300_device_sms(void);
 // Limit of one bounded wait on a flag or counter written by another CTA of
 // the same launch (starpu_gb300_set_wait_budget_ns; default 2 s).
 extern "C" unsigned long long gb300_wait_budget_ns(void);
+// the same in microseconds, 0 for less than one (waits between warps look once then)
+static inline unsigned gb300_wait_us()
+{
+    const unsigned long long us = gb300_wait_budget_ns() / 1000;
+    return us < 0xffffffffull ? (unsigned)us : 0xffffffffu;
+}
 
 // Per-kernel-class timing (the profiling mode of starpu_gb300_profiling_*):
 // prof_begin/prof_end bracket one launch with CUDA events on its stream when

@@ -63,7 +63,7 @@ struct BatchedState {
 struct BatchedArgs {
     int nsys, nrhs, max_iter, steps;
     double tol;
-    unsigned long long wait_ns;  // limit of a wait inside a panel
+    unsigned wait_us;           // limit of a wait inside a panel
     const BatchedSystem *sys;   // [nsys] largest first
     BatchedState *state;        // [nsys], zeroed
     const int *cnt;             // [BAT_BUCKETS][BAT_CNT]: systems of the bucket with n > 16 v
@@ -234,7 +234,7 @@ __device__ void bat_panel(const BatchedArgs &a, const BatTask &t, CpPanel<float,
     });
     cp_each<float>(x, [&](float &v, int r, int c) { v = (r < rows && c < bk) ? __ldcg(P + r + (long)c * ld) : 0.0f; });
     __syncthreads();  // pan of the previous task is free
-    if (!cp_panel<float, 2>(d, x, pan, bar, phase, found, bk, &a.state[t.pos].info, t.k0, t.i == 0, a.wait_ns))
+    if (!cp_panel<float, 2>(d, x, pan, bar, phase, found, bk, &a.state[t.pos].info, t.k0, t.i == 0, a.wait_us))
         atomicMax(&a.state[t.pos].info, BAT_MAXN + 1);  // a wait ran out: the system is reported as failed
     if (t.i > 0) {
         cp_each<float>(x, [&](float &v, int r, int c) {

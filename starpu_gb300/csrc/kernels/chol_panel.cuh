@@ -79,7 +79,7 @@ constexpr int CP_ERR_TIMEOUT = -1000;
 // the place of a pivot's info: what follows a wait that ran out is garbage, bad
 // pivots too.
 struct CpWait {
-    unsigned long long ns;
+    unsigned us;
     int *err;
     __device__ __forceinline__ void report() const { atomicMin(err, CP_ERR_TIMEOUT); }
 };
@@ -106,14 +106,14 @@ template <typename T, typename F> __device__ __forceinline__ void cp_each(CpBloc
 // the published columns of step s; bounded (a step takes well below a
 // microsecond and the publisher never waits for this warp, but a process may be
 // switched out meanwhile)
-__device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity, unsigned long long ns)
+__device__ __forceinline__ bool cp_wait(uint64_t *bar, uint32_t parity, unsigned us)
 {
-    // a limit below the suspended wait's own (some microseconds): look once
-    if (ns < 1000) return ptx::mbar_test_wait(bar, parity);
+    // a limit below a microsecond, which the suspended wait alone may exceed: look once
+    if (us == 0) return ptx::mbar_test_wait(bar, parity);
     if (ptx::mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = ptx::globaltimer();
     while (!ptx::mbar_try_wait(bar, parity))
-        if (ptx::globaltimer() - t0 > ns) return false;
+        if (ptx::globaltimer() - t0 > 1000ull * us) return false;
     return true;
 }
 
@@ -221,7 +221,7 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
 template <typename T, int NX>
 __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T, NX> &pan, uint64_t (&bar)[16], uint32_t phase,
                                          volatile int *found, int n, int *info, int info_base, bool report,
-                                         unsigned long long ns)
+                                         unsigned us)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int steps = (n + 3) / 4;
@@ -233,11 +233,11 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
     if (threadIdx.x == 0) *found = 0;  // (warp 0 owns step 0, which every other step waits for)
 #pragma unroll 1
     for (int i = 0; i < min(w, steps) - 1; ++i) {
-        ok = cp_wait(&bar[i], phase, ns) && ok;
+        ok = cp_wait(&bar[i], phase, us) && ok;
         cp_update<T, NX, 0, 1>(d, x, pan[i]);
     }
     if (w > 0 && w <= steps) {
-        ok = cp_wait(&bar[w - 1], phase, ns) && ok;
+        ok = cp_wait(&bar[w - 1], phase, us) && ok;
         cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
     }
     // (every mbarrier completes in every panel, so that all keep one parity)
@@ -250,7 +250,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
     cp_update<T, NX, 1, 1>(d, x, pan[w]);
 #pragma unroll 1
     for (int i = w + 1; i < min(8 + w, steps); ++i) {
-        ok = cp_wait(&bar[i], phase, ns) && ok;
+        ok = cp_wait(&bar[i], phase, us) && ok;
         cp_update<T, NX, 1, 1>(d, x, pan[i]);
     }
     if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w], found));
@@ -269,7 +269,7 @@ potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_ba
     // rows and columns past n continue the block as the identity
     cp_each<float>(a, [&](float &v, int r, int c) { v = (r < n && c <= r) ? A[r + (long)c * lda] : (r == c ? 1.0f : 0.0f); });
     __syncthreads();
-    if (!cp_panel<float, 0>(a, a, pan, bar, 0, &found, n, info, info_base, true, wait.ns)) wait.report();
+    if (!cp_panel<float, 0>(a, a, pan, bar, 0, &found, n, info, info_base, true, wait.us)) wait.report();
     cp_each<float>(a, [&](float &v, int r, int c) {
         if (r < n && c <= r) A[r + (long)c * lda] = v;
     });
@@ -287,7 +287,7 @@ potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_ba
 // 3 us more: each warp then trails its own backlog.)
 template <int H0>  // columns 32 H0 .. 32 H0 + 31, rows 32 H0 .. 63
 __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*col)[CP_W], double2 *pv, uint64_t *bar, int n,
-                                               int *info, int info_base, unsigned long long ns)
+                                               int *info, int info_base, unsigned us)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bool ok = true;
@@ -318,7 +318,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
         if (j0 >= n) break;
 #pragma unroll 1
         for (int j = j0; j < min(mine, n); ++j) {  // columns of this round before mine
-            ok = cp_wait(&bar[j], 0, ns) && ok;
+            ok = cp_wait(&bar[j], 0, us) && ok;
             next(j, q);
             if (j + 1 < mine) rest(j, q + 1);
         }
@@ -345,7 +345,7 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
         }
 #pragma unroll 1
         for (int j = mine + 1; j < min(j0 + 8, n); ++j) {  // and after it
-            ok = cp_wait(&bar[j], 0, ns) && ok;
+            ok = cp_wait(&bar[j], 0, us) && ok;
             rest(j, q + 1);
         }
     }
@@ -372,8 +372,8 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
     };
     each([&](double &v, int r, int c) { v = r < n && c <= r ? A[r + (long)c * lda] : 0.0; });
     __syncthreads();
-    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base, wait.ns);
-    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base, wait.ns) && ok;
+    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base, wait.us);
+    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base, wait.us) && ok;
     if (!ok) wait.report();
     each([&](double &v, int r, int c) {
         if (r < n && c < r) A[r + (long)c * lda] = v;
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(256) trsv_blk_kernel(int w, const T *__restric
     for (int i = 0; i < n; ++i) {
         const int p = TRANS ? np - 1 - i : i;
         turn(l);
-        ok = cp_wait(&bar[p], 0, wait.ns) && ok;
+        ok = cp_wait(&bar[p], 0, wait.us) && ok;
         const Quad<T> *x = reinterpret_cast<const Quad<T> *>(xs + 32 * p);
         T acc[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll

@@ -64,7 +64,7 @@ struct DiagCoopArgs {
     unsigned *bar;  // barrier counter, zero at launch; null: the launch's own grid barrier
     int *err;       // word that err_code goes to when a wait ran out
     int err_code;   // DC_ERR_TIMEOUT (with bar), or CP_ERR_TIMEOUT where err is an info word
-    unsigned long long wait_ns;  // limit of a wait inside a panel
+    unsigned wait_us;  // limit of a wait inside a panel
     int invert;  // 0: factor only (no inverse is written)
 };
 
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
                     else v = (r < ri && c < bk) ? __ldcg(Aik + r + (long)c * a.lda) : 0.0f;
                 });
                 __syncthreads();  // pan of the previous task is free
-                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, &found, bk, a.info, a.info_base + k0, t == 0, a.wait_ns))
+                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, &found, bk, a.info, a.info_base + k0, t == 0, a.wait_us))
                     dc_report(a);
                 ++panels;
                 if (t > 0)

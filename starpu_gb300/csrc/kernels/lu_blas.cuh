@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restric
     bool ok = true;
 #pragma unroll 1
     for (int i = 0; i < min(w, steps); ++i) {
-        ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
+        ok = cp_wait(&s.bar[i], 0, wait.us) && ok;
         getf_update<0, 0>(a, s, i);
         if (i < w - 1) getf_update<1, 0>(a, s, i);  // the next owner publishes first
     }
@@ -231,12 +231,12 @@ __global__ void __launch_bounds__(256) getf2_leaf_kernel(int n, float *__restric
         getf_update<1, 0>(a, s, w);
 #pragma unroll 1
         for (int i = w + 1; i < 8; ++i) {
-            ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
+            ok = cp_wait(&s.bar[i], 0, wait.us) && ok;
             getf_update<1, 0>(a, s, i);
         }
 #pragma unroll 1
         for (int i = 8; i < min(8 + w, steps); ++i) {
-            ok = cp_wait(&s.bar[i], 0, wait.ns) && ok;
+            ok = cp_wait(&s.bar[i], 0, wait.us) && ok;
             getf_update<1, 1>(a, s, i);
         }
         if (8 + w < steps) getf_own<1>(a, s, n, thr, d_first, info, info_base);
