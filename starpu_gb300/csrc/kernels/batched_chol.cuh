@@ -221,7 +221,7 @@ __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
 
 // ---- panel: diagonal block and (i > 0) 64 rows below it
 __device__ void bat_panel(const BatchedArgs &a, const BatTask &t, CpPanel<float, 2> &pan, uint64_t (&bar)[16], uint32_t phase,
-                          int *found)
+                          CpState &st)
 {
     const BatchedSystem s = a.sys[t.pos];
     const int n = s.n, ld = bat_ldw(n), bk = min(t.nb, n - t.k0), r0 = t.k0 + t.nb + 64 * (t.i - 1), rows = t.i > 0 ? min(64, n - r0) : 0;
@@ -234,7 +234,7 @@ __device__ void bat_panel(const BatchedArgs &a, const BatTask &t, CpPanel<float,
     });
     cp_each<float>(x, [&](float &v, int r, int c) { v = (r < rows && c < bk) ? __ldcg(P + r + (long)c * ld) : 0.0f; });
     __syncthreads();  // pan of the previous task is free
-    if (!cp_panel<float, 2>(d, x, pan, bar, phase, found, bk, &a.state[t.pos].info, t.k0, t.i == 0, a.wait_us))
+    if (!cp_panel<float, 2>(d, x, pan, bar, phase, st, bk, &a.state[t.pos].info, t.k0, t.i == 0, a.wait_us))
         atomicMax(&a.state[t.pos].info, BAT_MAXN + 1);  // a wait ran out: the system is reported as failed
     if (t.i > 0) {
         cp_each<float>(x, [&](float &v, int r, int c) {
@@ -242,7 +242,10 @@ __device__ void bat_panel(const BatchedArgs &a, const BatTask &t, CpPanel<float,
         });
     } else {
         float *D = a.D + (long)t.pos * (DC_B * DC_B);
-        cp_each<float>(d, [&](float &v, int r, int c) { D[r + DC_B * c] = v; });
+        cp_each<float>(d, [&](float &v, int r, int c) {
+            if (r != c) D[r + DC_B * c] = v;
+        });
+        st.diagonal([&](int c, float v) { D[c * (DC_B + 1)] = v; });
     }
 }
 
@@ -522,7 +525,7 @@ template <int NR> __global__ void __launch_bounds__(BAT_THREADS, 2) batched_dpos
     __shared__ int cnt[BAT_BUCKETS * BAT_CNT];
     __shared__ uint64_t bar[16];
     __shared__ double red[BAT_THREADS];
-    __shared__ int found;
+    __shared__ CpState st;
     float *smem = (float *)bat_smem;
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     for (int e = threadIdx.x; e < BAT_BUCKETS * BAT_CNT; e += BAT_THREADS) cnt[e] = a.cnt[e];
@@ -534,7 +537,7 @@ template <int NR> __global__ void __launch_bounds__(BAT_THREADS, 2) batched_dpos
     uint32_t panels = 0;
     for (int k = 0; k < a.steps; ++k) {
         for (int q = blockIdx.x; bat_find_panel(a, cnt, k, q, t); q += gridDim.x)
-            bat_panel(a, t, *(CpPanel<float, 2> *)bat_smem, bar, panels++ & 1, &found);
+            bat_panel(a, t, *(CpPanel<float, 2> *)bat_smem, bar, panels++ & 1, st);
         grid.sync();
         for (int q = blockIdx.x; bat_find_update(a, cnt, k, q, t); q += gridDim.x)
             bat_update(a, t, smem, smem + DC_B * DC_LD);

@@ -156,11 +156,25 @@ template <bool ANY> __device__ __forceinline__ void cp_factor4(float (&l)[4][4],
     }
 }
 
+// What a panel's warps keep beside the columns: the pivots, whose roots the
+// diagonal holds in the end (a product with the reciprocal root, which the
+// columns take, is off by up to an ulp), and whether a bad one was found.
+struct CpState {
+    Quad<float> piv[16];
+    int found;
+    // the diagonal: f(column, root), a warp for its own columns
+    template <typename F> __device__ __forceinline__ void diagonal(F f) const
+    {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = 32 * (lane >> 2) + 4 * warp + (lane & 3);
+        if (lane < 8) f(c, sqrtf(((const volatile float *)piv)[c]));
+    }
+};
+
 // The first pivot of the four that is not positive, or -1.  Of a panel's steps
-// only the first that has one says so: it sets `found` before its columns are
+// only the first that has one says so: it sets st.found before its columns are
 // published, so that the steps behind them see it.
 template <int NX, int G>
-__device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Quad<float> *p, volatile int *found)
+__device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Quad<float> *p, CpState &st)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float l[4][4], r[4];
@@ -191,11 +205,13 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
         for (int j = 3; j >= 0; --j)
             if (!(l[j][j] > 0.0f)) bad = j;
         if (bad >= 0) {
+            volatile int *found = &st.found;
             if (*found) bad = -1;
             __syncwarp();
             *found = 1;
         }
     }
+    if (lane == 0) st.piv[8 * G + warp] = {l[0][0], l[1][1], l[2][2], l[3][3]};
     auto solve = [&](float(&c)[4][2], int h, int row) {
         Quad<float> y;
 #pragma unroll
@@ -215,12 +231,12 @@ __device__ __forceinline__ int cp_solve4(CpBlock<float> &d, CpBlock<float> &x, Q
     return bad;
 }
 
-// The whole panel; `phase` is the parity of the mbarriers (0 for the first
+// The whole panel (but for d's diagonal, CpState::diagonal); `phase` is the parity of the mbarriers (0 for the first
 // panel of a kernel, then in turn), with a CTA barrier between two panels;
-// found: a word of shared memory.  False: a wait ran out.
+// st: in shared memory.  False: a wait ran out.
 template <typename T, int NX>
 __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T, NX> &pan, uint64_t (&bar)[16], uint32_t phase,
-                                         volatile int *found, int n, int *info, int info_base, bool report,
+                                         CpState &st, int n, int *info, int info_base, bool report,
                                          unsigned us)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -230,7 +246,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         ptx::mbar_arrive(&bar[step]);
         if (bad >= 0 && report && lane == 0 && info && 4 * step + bad < n) atomicCAS(info, 0, info_base + 4 * step + bad + 1);
     };
-    if (threadIdx.x == 0) *found = 0;  // (warp 0 owns step 0, which every other step waits for)
+    if (threadIdx.x == 0) *(volatile int *)&st.found = 0;  // (warp 0 owns step 0, which every other step waits for)
 #pragma unroll 1
     for (int i = 0; i < min(w, steps) - 1; ++i) {
         ok = cp_wait(&bar[i], phase, us) && ok;
@@ -241,7 +257,7 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         cp_update<T, NX, 0, 0>(d, x, pan[w - 1]);
     }
     // (every mbarrier completes in every panel, so that all keep one parity)
-    if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w], found));
+    if (w < steps) own(w, cp_solve4<NX, 0>(d, x, pan[w], st));
     else ptx::mbar_arrive(&bar[w]);
     if (8 + w >= steps) ptx::mbar_arrive(&bar[8 + w]);
     __syncwarp();
@@ -253,7 +269,8 @@ __device__ __forceinline__ bool cp_panel(CpBlock<T> &d, CpBlock<T> &x, CpPanel<T
         ok = cp_wait(&bar[i], phase, us) && ok;
         cp_update<T, NX, 1, 1>(d, x, pan[i]);
     }
-    if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w], found));
+    if (8 + w < steps) own(8 + w, cp_solve4<NX, 1>(d, x, pan[8 + w], st));
+    __syncwarp();  // st.piv
     return ok;
 }
 
@@ -263,15 +280,18 @@ potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_ba
 {
     __shared__ CpPanel<float, 0> pan;
     __shared__ uint64_t bar[16];
-    __shared__ int found;
+    __shared__ CpState st;
     CpBlock<float> a;
     cp_panel_init(bar);
     // rows and columns past n continue the block as the identity
     cp_each<float>(a, [&](float &v, int r, int c) { v = (r < n && c <= r) ? A[r + (long)c * lda] : (r == c ? 1.0f : 0.0f); });
     __syncthreads();
-    if (!cp_panel<float, 0>(a, a, pan, bar, 0, &found, n, info, info_base, true, wait.us)) wait.report();
+    if (!cp_panel<float, 0>(a, a, pan, bar, 0, st, n, info, info_base, true, wait.us)) wait.report();
     cp_each<float>(a, [&](float &v, int r, int c) {
-        if (r < n && c <= r) A[r + (long)c * lda] = v;
+        if (r < n && c < r) A[r + (long)c * lda] = v;
+    });
+    st.diagonal([&](int c, float v) {
+        if (c < n) A[c * (lda + 1)] = v;
     });
 }
 

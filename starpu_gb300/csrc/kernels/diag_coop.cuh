@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
     float *s0 = (float *)shared, *s1 = (float *)(shared + TILE);
     CpPanel<float, 2> &pan = *(CpPanel<float, 2> *)shared;
     __shared__ uint64_t bar[16];
-    __shared__ int s_ok, found;
+    __shared__ int s_ok;
+    __shared__ CpState st;
     const int n = a.n, nblk = (n + DC_B - 1) / DC_B, G = gridDim.x, b = blockIdx.x;
     const bool vec = ((reinterpret_cast<uintptr_t>(a.A) & 15) == 0) && ((a.lda & 3) == 0);
     const bool vec_inv = ((reinterpret_cast<uintptr_t>(a.Linv) & 15) == 0) && ((a.ldi & 3) == 0);
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
                     else v = (r < ri && c < bk) ? __ldcg(Aik + r + (long)c * a.lda) : 0.0f;
                 });
                 __syncthreads();  // pan of the previous task is free
-                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, &found, bk, a.info, a.info_base + k0, t == 0, a.wait_us))
+                if (!cp_panel<float, 2>(d, x, pan, bar, panels & 1, st, bk, a.info, a.info_base + k0, t == 0, a.wait_us))
                     dc_report(a);
                 ++panels;
                 if (t > 0)
@@ -240,10 +241,14 @@ __global__ void __launch_bounds__(DC_T, 2) diag_coop_kernel(DiagCoopArgs a)
             }
         }
         if (!dc_sync(a, ++phase, &s_ok)) return;
-        if (b == 0)  // the factored block: every CTA has read the unfactored one
+        if (b == 0) {  // the factored block: every CTA has read the unfactored one
             cp_each<float>(d, [&](float &v, int r, int c) {
-                if (r < bk && c <= r) Akk[r + (long)c * a.lda] = v;
+                if (r < bk && c < r) Akk[r + (long)c * a.lda] = v;
             });
+            st.diagonal([&](int c, float v) {
+                if (c < bk) Akk[c * (a.lda + 1)] = v;
+            });
+        }
         if (k == nblk - 1) break;
         // ---- phase B
         // (CTA 0, which stores the factored block, takes its tile last)

@@ -368,3 +368,14 @@ def test_fp64_products_keep_the_bound_at_the_worst_digits(gpu, k, zeros):
         ref -= a[:, p, None].astype(np.longdouble) * b[None, :, p]
         mag += np.abs(a[:, p, None] * b[None, :, p])
     assert np.all(np.abs((out - ref).astype(np.float64)) <= (k + 2) * EPS[np.float64] * mag)
+
+
+# the leaf, one cooperative launch of several blocks, and panels
+@pytest.mark.parametrize("n", [1, 31, 64, 65, 200, 4200])
+def test_spotrf_diagonal_is_the_square_root(gpu, n):
+    d = np.random.default_rng(n).uniform(1e-3, 1e3, n).astype(np.float32)
+    d[0] = 1e-41  # below the normal range
+    da, info = up(np.diag(d)), up(np.zeros(1, np.int32))
+    check(gpu.starpu_gb300_spotrf(None, n, da.ptr, n, 512, info.ptr))
+    assert info.download((1,), np.int32)[0] == 0
+    assert np.array_equal(np.diag(da.download((n, n), np.float32)), np.sqrt(d))
