@@ -379,3 +379,34 @@ def test_spotrf_diagonal_is_the_square_root(gpu, n):
     check(gpu.starpu_gb300_spotrf(None, n, da.ptr, n, 512, info.ptr))
     assert info.download((1,), np.int32)[0] == 0
     assert np.array_equal(np.diag(da.download((n, n), np.float32)), np.sqrt(d))
+
+
+# L of [[d, t], [t, 2.5 t^2 / d]] has t / sqrt(d) below the diagonal (t a power of two): 32 such blocks a
+# matrix, d over the normal range and its powers of two, and beyond it
+@BOTH
+def test_leaf_reciprocal_root(gpu, dtype):
+    lo, hi, t = (-126, 128, 2.0**-20) if dtype == np.float32 else (-1022, 1024, 2.0**-60)
+    rng = np.random.default_rng(11)
+    edges = np.concatenate([[1.0, 1.5, np.nextafter(dtype(2), dtype(0)), 2.0, 3.0, np.nextafter(dtype(4), dtype(0))]] * 8)
+    e = rng.integers(lo, hi, 32 * 400)
+    d = np.ldexp(rng.uniform(1, 2, e.size).astype(dtype), np.minimum(e, hi - 1))
+    d[: edges.size] = np.ldexp(edges.astype(dtype), rng.integers(lo + 2, hi - 4, edges.size))
+    d[-64:] = np.ldexp(dtype(1), np.linspace(lo - 10, lo, 64).astype(int)).astype(dtype)  # some subnormal
+    d = d[np.isfinite(d)][: e.size // 32 * 32]
+    info = up(np.zeros(1, np.int32))
+    worst = 0.0
+    for block in d.reshape(-1, 32):
+        a = np.zeros((64, 64), dtype)
+        i = 2 * np.arange(32)
+        a[i, i], a[i + 1, i] = block, t
+        a[i + 1, i + 1] = np.maximum(2.5 * t * (t / block.astype(np.float64)), 1e-30)
+        da = up(a)
+        check(fn(gpu, dtype, "potrf_tile")(None, 64, da.ptr, 64, info.ptr))
+        r = da.download((64, 64), dtype)[i + 1, i].astype(np.longdouble) / t
+        exact = 1 / np.sqrt(block.astype(np.longdouble))
+        normal = block >= np.finfo(dtype).tiny
+        err = np.abs(r / exact - 1).astype(np.float64) / EPS[dtype]
+        # 1.5 u; outside the normal range 1 / sqrt(d) of two rounded operations, 2 u
+        assert np.all(err <= np.where(normal, 1.5, 2.0) * (1 + 2.0**-9)), (block[np.argmax(err)], err.max())
+        worst = max(worst, err.max())
+    assert worst > 0.5
