@@ -179,6 +179,17 @@ __device__ __forceinline__ float2 bat_split(double a, int ea)
                        __uint_as_float(sign | __float_as_uint(__fmul_rn(r, __uint_as_float((uint32_t)(fe - 52) << 23)))));
 }
 
+// v as (float)v gives it, by bit operations where the result is a normal number
+// (a conversion holds the FP64 pipe)
+__device__ __forceinline__ float bat_to_float(double v)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    if (((hi >> 20) & 0x7FF) - 897u > 253u) return (float)v;
+    uint32_t f = __funnelshift_l(lo, hi & 0x7FFFFFFFu, 3) - (896u << 23);  // truncated, then to nearest even
+    f += (lo & 0x1FFFFFFFu) + (f & 1) > 0x10000000u ? 1u : 0u;
+    return __uint_as_float(f | (hi & 0x80000000u));
+}
+
 // ---- convert: 64 rows of one system.  The row sums run in double-float
 // relative to the largest diagonal element (FP64 additions and conversions,
 // one each per element, took 530 us for 1024 systems: the FP64 pipe's time).
@@ -192,8 +203,6 @@ __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
     for (int i = threadIdx.x & 31; i < n; i += 32) dm = max(dm, (unsigned)__double2hiint(A0[(long)i * (n + 1)]) & 0x7FFFFFFFu);
     dm = __reduce_max_sync(0xffffffffu, dm);
     const int ex = (int)(dm >> 20), ea = ex == 0 || ex == 0x7FF ? 0 : ex - 1023;
-    const bool plain = ea < -100 || ea > 100;  // 2^ea leaves FP32's range: convert element by element
-    const float back = plain ? 0.0f : __int_as_float((ea + 127) << 23);
     float sh = 0.0f, sl = 0.0f;
     if (row < n)
         for (int c0 = cg; c0 < n; c0 += 64) {
@@ -206,7 +215,7 @@ __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
                 const float h = fabsf(p.x), l = fabsf(p.y), q = __fadd_rn(sh, h), z = __fsub_rn(q, sh);
                 sl = __fadd_rn(sl, __fadd_rn(l, __fadd_rn(__fsub_rn(sh, __fsub_rn(q, z)), __fsub_rn(h, z))));
                 sh = q;
-                if (c0 + 4 * u <= row) W[(long)(c0 + 4 * u) * ldw] = plain ? (float)v[u] : __fmul_rn(__fadd_rn(p.x, p.y), back);
+                if (c0 + 4 * u <= row) W[(long)(c0 + 4 * u) * ldw] = bat_to_float(v[u]);
             }
         }
     __syncthreads();

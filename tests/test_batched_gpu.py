@@ -176,3 +176,16 @@ def test_batched_iteration_limit(gpu, oracle):
     systems = [make_system(oracle, n, 910 + n) for n in (60, 200)]
     status, berr, _ = run_batched(gpu, systems, tol=0.0, max_iter=2)
     assert np.all(np.asarray(status) == -1000) and np.all(np.asarray(berr) < 1e-12)
+
+
+@pytest.mark.parametrize("n", [40, 130])
+def test_batched_graded_diagonal(gpu, oracle, n):
+    """Elements far below the largest, but within FP32's range, keep their value in
+    the factor: they are no zero pivots."""
+    d = np.logspace(30, -20, n)
+    A = np.asfortranarray(np.diag(d))
+    B = np.asfortranarray(oracle.uniform_rhs(n, 2, 920))
+    status, berr, X = run_batched(gpu, [(A, B)], nrhs=2, tol=1e-6)
+    assert status[0] >= 0
+    # d to FP32, its root, its reciprocal, two products and b to FP32: below 12 ulps of 2^-24
+    assert np.all(np.abs(X[0] * d[:, None] - B) <= 12 * 2.0**-24 * np.abs(B))
