@@ -190,9 +190,13 @@ __device__ __forceinline__ float bat_to_float(double v)
     return __uint_as_float(f | (hi & 0x80000000u));
 }
 
-// ---- convert: 64 rows of one system.  The row sums run in double-float
-// relative to the largest diagonal element (FP64 additions and conversions,
-// one each per element, took 530 us for 1024 systems: the FP64 pipe's time).
+// ---- convert: 64 rows of one system.  A row's sum is taken in 64-bit integers,
+// units of 2^-54 of the largest diagonal element's binade, which bounds the
+// elements of an SPD matrix: an element's rounding is 2^-55, below that of an
+// FP64 addition to a sum of that size, and the largest sum is no smaller.  Rows
+// with a larger element (or of a matrix without a finite diagonal) are added in
+// FP64.  (FP64 additions and conversions, one each per element, took 530 us for
+// 1024 systems: the FP64 pipe's time.)
 __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
 {
     const BatchedSystem s = a.sys[t.pos];
@@ -202,8 +206,9 @@ __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
     unsigned dm = 0;
     for (int i = threadIdx.x & 31; i < n; i += 32) dm = max(dm, (unsigned)__double2hiint(A0[(long)i * (n + 1)]) & 0x7FFFFFFFu);
     dm = __reduce_max_sync(0xffffffffu, dm);
-    const int ex = (int)(dm >> 20), ea = ex == 0 || ex == 0x7FF ? 0 : ex - 1023;
-    float sh = 0.0f, sl = 0.0f;
+    const int ex = dm >= 0x7FF00000u ? -1 : max((int)(dm >> 20), 1);  // biased; -1: every row in FP64
+    unsigned long long F = 0;
+    int wide = 0;  // an exponent above ex was met
     if (row < n)
         for (int c0 = cg; c0 < n; c0 += 64) {
             double v[16];
@@ -211,19 +216,24 @@ __device__ void bat_convert(const BatchedArgs &a, const BatTask &t, double *red)
             for (int u = 0; u < 16; ++u) v[u] = c0 + 4 * u < n ? A[(long)(c0 + 4 * u) * n] : 0.0;
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
-                const float2 p = bat_split(v[u], ea);
-                const float h = fabsf(p.x), l = fabsf(p.y), q = __fadd_rn(sh, h), z = __fsub_rn(q, sh);
-                sl = __fadd_rn(sl, __fadd_rn(l, __fadd_rn(__fsub_rn(sh, __fsub_rn(q, z)), __fsub_rn(h, z))));
-                sh = q;
+                const unsigned long long m = (unsigned long long)__double_as_longlong(v[u]);
+                const int e = (int)(m >> 52) & 0x7FF, down = ex - max(e, 1);
+                wide |= down;
+                F += ((((m & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull)) << 3 >> min((unsigned)down, 63u)) + 1) >> 1;
                 if (c0 + 4 * u <= row) W[(long)(c0 + 4 * u) * ldw] = bat_to_float(v[u]);
             }
         }
+    double sum = ldexp(__ull2double_rn(F), ex - (1023 + 54));
+    if (wide < 0) {
+        sum = 0.0;
+        for (int c = cg; c < n; c += 4) sum += fabs(A[(long)c * n]);
+    }
     __syncthreads();
-    red[threadIdx.x] = ldexp((double)sh + (double)sl, ea);
+    red[threadIdx.x] = sum;
     __syncthreads();
     if (threadIdx.x < 64) {
         double m = (red[threadIdx.x] + red[64 + threadIdx.x]) + (red[128 + threadIdx.x] + red[192 + threadIdx.x]);
-        m = bat_warp_max(m);
+        m = bat_warp_max(isnan(m) ? 0.0 : m);
         if ((threadIdx.x & 31) == 0) atomicMax(&a.state[t.pos].anorm, (unsigned long long)__double_as_longlong(m));
     }
 }
