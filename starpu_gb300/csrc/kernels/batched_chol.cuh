@@ -22,9 +22,11 @@
 // task is a fixed sequence of operations on its system's data, so a system's
 // result does not depend on which other systems share the launch.
 //
-// The residual runs in double-float arithmetic on the FP32 pipe (A split per
-// element, X split once per task into shared memory, FP64 flush every 128
-// terms; ~2^-47 relative per block): the FP64 pipe is 64 times slower.
+// The residual of a system with n nrhs <= BAT_DF_TERMS runs in double-float
+// arithmetic on the FP32 pipe (A split per element, X split once per task into
+// shared memory, FP64 flush every 128 terms; ~2^-47 relative per block): the
+// FP64 pipe is 64 times slower.  Larger ones, with seven or eight right-hand
+// sides, keep FP64 FMAs.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -39,6 +41,7 @@ namespace gb300 {
 constexpr int BAT_THREADS = 256;
 constexpr int BAT_MAXN = 1024;
 constexpr int BAT_MAXRHS = 8;
+constexpr int BAT_DF_TERMS = 6688;        // n nrhs up to which the residual may be double-float
 constexpr int BAT_BUCKETS = 6;            // n <= 32, 64, 128, 256, 512, 1024
 constexpr int BAT_GRAIN = 16;             // cnt is kept for every multiple of this order
 constexpr int BAT_CNT = BAT_MAXN / BAT_GRAIN + 1;
@@ -161,7 +164,7 @@ template <int NR> struct BatSmem {
     static constexpr size_t PAN = sizeof(CpPanel<float, 2>);
     // solve: right-hand sides, diagonal block, its inverse pivots, the block's rows
     static constexpr size_t SOLVE = ((size_t)NR * BAT_MAXN + CP_W * CP_LP + CP_W + 8 * CP_LP) * sizeof(float);
-    // residual: X split, partial sums
+    // residual: X split (or X), partial sums
     static constexpr size_t RES = (size_t)NR * BAT_MAXN * sizeof(float2) + 4 * 64 * NR * sizeof(double);
     static constexpr size_t M1 = TILES > PAN ? TILES : PAN, M2 = SOLVE > RES ? SOLVE : RES;
     static constexpr size_t BYTES = M1 > M2 ? M1 : M2;
@@ -475,8 +478,8 @@ template <int NR> __device__ void bat_round(const BatchedArgs &a, int pos, int r
 
 // ---- residual: 64 rows of R = B - A X in double-float arithmetic on the
 // FP32 pipe (A scaled by the exponent of ||A||_inf and split per element by bit
-// operations, each column of X scaled by its own exponent), thread = row and
-// every fourth column, the four sums added in a fixed order.
+// operations, each column of X scaled by its own exponent) or by FP64 FMAs,
+// thread = row and every fourth column, the four sums added in a fixed order.
 template <int NR> __device__ void bat_residual(const BatchedArgs &a, const BatTask &t, float *smem)
 {
     const BatchedSystem s = a.sys[t.pos];
@@ -490,18 +493,36 @@ template <int NR> __device__ void bat_residual(const BatchedArgs &a, const BatTa
 #pragma unroll
     for (int c = 0; c < NR; ++c) ex[c] = c < nrhs ? df_scale_exp(__ldcg(&st.xmax[c])) : 0;
     const int ea = df_scale_exp(__longlong_as_double((long long)__ldcg(&st.anorm)));
+    const bool fp64 = NR * BAT_MAXN > BAT_DF_TERMS && n * nrhs > BAT_DF_TERMS;
+    double *Xd = reinterpret_cast<double *>(smem);  // fp64: [n][NR]
     __syncthreads();  // shared memory of the previous task is free
 #pragma unroll
     for (int c = 0; c < NR; ++c)
-        for (int k = tid; k < n; k += BAT_THREADS)
-            Xs[k * NR + c] = c < nrhs ? df_split_scaled(__ldcg(X + (long)c * n + k), ex[c]) : make_float2(0.0f, 0.0f);
+        for (int k = tid; k < n; k += BAT_THREADS) {
+            const double x = c < nrhs ? __ldcg(X + (long)c * n + k) : 0.0;
+            if (fp64) Xd[k * NR + c] = x;
+            else Xs[k * NR + c] = df_split_scaled(x, ex[c]);
+        }
     __syncthreads();
     const int row = 64 * t.i + (tid & 63), kg = tid >> 6;
     const double *Ai = a.A + s.a_off + min(row, n - 1);
     double acc[NR];
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[c] = 0.0;
-    for (int j0 = kg; j0 < n; j0 += 512) {  // 128 terms of this thread
+    if (fp64)
+        for (int j0 = kg; j0 < n; j0 += 32) {
+            double av[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) av[u] = j0 + 4 * u < n ? Ai[(long)(j0 + 4 * u) * n] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (j0 + 4 * u >= n) break;
+                const double *x = Xd + (j0 + 4 * u) * NR;
+#pragma unroll
+                for (int c = 0; c < NR; ++c) acc[c] = fma(av[u], x[c], acc[c]);
+            }
+        }
+    for (int j0 = fp64 ? n : kg; j0 < n; j0 += 512) {  // 128 terms of this thread
         float sh[NR], sl[NR];
 #pragma unroll
         for (int c = 0; c < NR; ++c) sh[c] = 0.0f, sl[c] = 0.0f;

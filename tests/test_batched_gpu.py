@@ -189,3 +189,25 @@ def test_batched_graded_diagonal(gpu, oracle, n):
     assert status[0] >= 0
     # d to FP32, its root, its reciprocal, two products and b to FP32: below 12 ulps of 2^-24
     assert np.all(np.abs(X[0] * d[:, None] - B) <= 12 * 2.0**-24 * np.abs(B))
+
+
+@pytest.mark.parametrize("n,nrhs", [(836, 8), (837, 8), (1000, 8), (1024, 7)])
+def test_batched_residual_of_many_right_hand_sides(gpu, oracle, n, nrhs):
+    """With n nrhs > 6688 the residual is an FP64 one: on a tridiagonal matrix no
+    element of it takes more than 8 roundings (3 products, 3 sums of the four
+    threads' parts, b less that, with one to spare), each half an ulp of a value
+    no larger than |A| |x| + |b|.  After one correction x has some 48 bits."""
+    rng = np.random.default_rng(n + nrhs)
+    off = rng.uniform(-1, 1, n - 1)
+    A = np.asfortranarray(np.diag(rng.uniform(3, 4, n)) + np.diag(off, 1) + np.diag(off, -1))
+    B = oracle.uniform_rhs(n, nrhs, 930)
+    _, berr, X = run_batched(gpu, [(A, B)], nrhs=nrhs, tol=0.0, max_iter=1)
+    r = np.empty((n, nrhs), dtype=np.longdouble)
+    for c in range(nrhs):
+        x = X[0][:, c].astype(np.longdouble)
+        r[:, c] = B[:, c] - np.diag(A) * x
+        r[:-1, c] -= off * x[1:]
+        r[1:, c] -= off * x[:-1]
+    den = np.abs(A).sum(1).max() * np.abs(X[0]).max(0) + np.abs(B).max(0)
+    true = float((np.abs(r).max(0) / den).max())
+    assert abs(berr[0] - true) <= (8 if n * nrhs > 6688 else 2**8) * 2.0**-53, (berr[0], true)
