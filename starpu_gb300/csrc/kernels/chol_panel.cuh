@@ -309,15 +309,20 @@ potf2_leaf_kernel(int n, float *__restrict__ A, long lda, int *info, int info_ba
 // instructions, 1 in the lower half), takes 1/sqrt (5), scales (2 or 1),
 // publishes, and catches up on its other columns afterwards.  Bound by the chain
 // and by the 3000 instructions of the block (48000 clocks over four units).
+// The products go into sums of their own, which a column takes in where its group
+// of 16 begins, so that most roundings are relative to a sum of products: with
+// every product rounded into its element (64 times) the factor of a matrix of
+// order 1000 was off by 1.6e-16, with a 32-column leaf, as before, by 1.4e-16, and
+// is by 1.1e-16 (to 80 bits, on the CPU).
 // (Four warps, one per unit, so that nothing shares a unit with the chain, took
 // 3 us more: each warp then trails its own backlog.)
 template <int H0>  // columns 32 H0 .. 32 H0 + 31, rows 32 H0 .. 63
-__device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*col)[CP_W], double2 *pv, uint64_t *bar, int n,
-                                               int *info, int info_base, unsigned us)
+__device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], const double (&e)[2][4][2], double (*col)[CP_W],
+                                               double2 *pv, uint64_t *bar, int n, int *info, int info_base, unsigned us)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bool ok = true;
-    // with published column j: column 32 H0 + 4 q + w, and all right of it
+    // with published column j: column 32 H0 + 8 q + w, and all right of it
     auto next = [&](int j, int q) {
         const double lc = col[j][32 * H0 + 8 * q + w];
 #pragma unroll
@@ -339,9 +344,14 @@ __device__ __forceinline__ bool cp_leaf64_half(double (&a)[2][4][2], double (*co
             for (int q = 0; q < 4; ++q) a[1][q][1] = fma(-l[1], col[j][32 + 8 * q + w], a[1][q][1]);
     };
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {  // this warp's next column: 32 H0 + 4 q + w
+    for (int q = 0; q < 4; ++q) {  // this warp's next column: 32 H0 + 8 q + w
         const int j0 = 32 * H0 + 8 * q, mine = j0 + w;
         if (j0 >= n) break;
+        if (q % 2 == 0 && H0 + q > 0)  // a group of 16 begins: its elements, less the products so far
+#pragma unroll
+            for (int u = q; u < q + 2; ++u)
+#pragma unroll
+                for (int h = H0; h < 2; ++h) a[H0][u][h] += e[H0][u][h];
 #pragma unroll 1
         for (int j = j0; j < min(mine, n); ++j) {  // columns of this round before mine
             ok = cp_wait(&bar[j], 0, us) && ok;
@@ -385,7 +395,7 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
     __shared__ double2 pv[CP_W];  // pivots and the factors their columns were scaled with
     __shared__ uint64_t bar[CP_W];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double a[2][4][2];  // [half of the columns][q][row half]: column 32 g + 4 q + w
+    double a[2][4][2], e[2][4][2];  // [half of the columns][q][row half]: column 32 g + 8 q + w
     if (threadIdx.x < CP_W) ptx::mbar_init(&bar[threadIdx.x], 32);
     ptx::fence_mbarrier_init();
     auto each = [&](auto f) {
@@ -397,9 +407,18 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
                 for (int h = 0; h < 2; ++h) f(a[g][q][h], 32 * h + lane, 32 * g + 8 * q + w);
     };
     each([&](double &v, int r, int c) { v = r < n && c <= r ? A[r + (long)c * lda] : 0.0; });
+#pragma unroll
+    for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                e[g][q][h] = a[g][q][h];
+                if (g > 0 || q >= 2) a[g][q][h] = 0.0;
+            }
     __syncthreads();
-    bool ok = cp_leaf64_half<0>(a, col, pv, bar, n, info, info_base, wait.us);
-    if (n > 32) ok = cp_leaf64_half<1>(a, col, pv, bar, n, info, info_base, wait.us) && ok;
+    bool ok = cp_leaf64_half<0>(a, e, col, pv, bar, n, info, info_base, wait.us);
+    if (n > 32) ok = cp_leaf64_half<1>(a, e, col, pv, bar, n, info, info_base, wait.us) && ok;
     if (!ok) wait.report();
     each([&](double &v, int r, int c) {
         if (r < n && c < r) A[r + (long)c * lda] = v;

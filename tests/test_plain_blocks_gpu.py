@@ -410,3 +410,16 @@ def test_leaf_reciprocal_root(gpu, dtype):
         assert np.all(err <= np.where(normal, 1.5, 2.0) * (1 + 2.0**-9)), (block[np.argmax(err)], err.max())
         worst = max(worst, err.max())
     assert worst > 0.5
+
+
+def test_dpotrf_leaf_sums_products_apart(gpu):
+    """48 products of 2^-54 count 3 2^-50 together and nothing one by one beside 1:
+    rounded into their element at every column they would be lost."""
+    l = np.eye(64)
+    l[48:, :48] = 2.0**-27
+    a = l @ l.T  # exact
+    da = up(a)
+    check(gpu.starpu_gb300_dpotrf(None, 64, da.ptr, 64, 64, None))
+    out = np.tril(da.download((64, 64), np.float64))
+    assert np.all(np.diag(out) == 1.0)
+    assert np.all(np.abs(out - l) <= 2.0**-52 * l)
