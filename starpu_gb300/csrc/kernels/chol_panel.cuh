@@ -446,7 +446,11 @@ potf2_leaf_kernel(int n, double *__restrict__ A, long lda, int *info, int info_b
 //   solve   16 lanes per row, 4 columns each, passed on by shuffles (no
 //           barrier).  FP32: 4 neighbouring columns per lane, 4 at a time.
 //           FP64: every 16th column, one at a time, on M scaled to a unit
-//           diagonal: 164 FP64 operations per row pair instead of 416.
+//           diagonal: 167 FP64 operations per row pair instead of 416.  Of
+//           the columns past the first 16 the products are summed apart until
+//           their group of 16 begins, as in the leaf: rounded into the scaled
+//           right-hand side they cost the factor 0.15e-16 of 1.6e-16 at order
+//           1000.
 // SR is 16 where that fills the GPU, else 8 or 4.
 // ---------------------------------------------------------------------------
 constexpr int CP_TRSM_MAXN = 1024;  // columns of one launch (shared memory: SR n elements)
@@ -501,11 +505,12 @@ template <int SR> __device__ __forceinline__ void cp_slab_solve(float *S, const 
 template <int SR> __device__ __forceinline__ void cp_slab_solve(double *S, const double *Ls, const double *inv)
 {
     const int r = threadIdx.x >> 4, l = threadIdx.x & 15, src = threadIdx.x & 16;
-    double x[4];
+    double x[4], b[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) x[q] = S[r * CP_LP + 16 * q + l] * inv[16 * q + l];
+    for (int q = 0; q < 4; ++q) b[q] = S[r * CP_LP + 16 * q + l] * inv[16 * q + l], x[q] = 0.0;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
+        x[g] = g ? b[g] + x[g] : b[0];
 #pragma unroll 4
         for (int s = 0; s < 16; ++s) {
             const double y = __shfl_sync(0xffffffffu, x[g], src | s);

@@ -423,3 +423,18 @@ def test_dpotrf_leaf_sums_products_apart(gpu):
     out = np.tril(da.download((64, 64), np.float64))
     assert np.all(np.diag(out) == 1.0)
     assert np.all(np.abs(out - l) <= 2.0**-52 * l)
+
+
+@pytest.mark.parametrize("m", [1, 33, 800, 2100])
+def test_dtrsm_slab_sums_products_apart(gpu, m):
+    """The panel solve's counterpart of the leaf's: X = 1 in the last group of 16
+    columns once the 48 products before it are summed apart."""
+    l = np.eye(64)
+    l[48:, :48] = 2.0**-27
+    x = np.ones((m, 64))
+    x[:, :48] = 2.0**-27
+    b = x.copy()
+    b[:, 48:] += 3 * 2.0**-50
+    dl, db = up(l), up(b)
+    check(gpu.starpu_gb300_dtrsm_rltn_tile(None, m, 64, 1.0, dl.ptr, 64, db.ptr, m))
+    np.testing.assert_array_equal(db.download((m, 64), np.float64), x)
