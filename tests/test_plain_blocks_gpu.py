@@ -438,3 +438,27 @@ def test_dtrsm_slab_sums_products_apart(gpu, m):
     dl, db = up(l), up(b)
     check(gpu.starpu_gb300_dtrsm_rltn_tile(None, m, 64, 1.0, dl.ptr, 64, db.ptr, m))
     np.testing.assert_array_equal(db.download((m, 64), np.float64), x)
+
+
+def test_dpotrs_sums_products_apart(gpu):
+    """The same in the solve's blocks of 32 rows, whose groups are of eight: forward
+    the last group has 24 products of 2^-54 before it, backward the others eight."""
+    l = np.eye(32)
+    l[24:, :24] = 2.0**-27
+    b = np.full((32, 1), 2.0**-27)
+    b[24:] = 1 + 3 * 2.0**-51
+    x = np.full((32, 1), -7 * 2.0**-27)
+    x[24:] = 1.0
+    dl, db = up(l), up(b)
+    check(gpu.starpu_gb300_dpotrs(None, 32, 1, dl.ptr, 32, db.ptr, 32))
+    np.testing.assert_array_equal(db.download((32, 1), np.float64), x)
+
+    sign = np.where(np.arange(24) % 2 == 0, 1.0, -1.0)  # so that forward every sum is exact
+    l[24:, :24] = 2.0**-27 * sign
+    b = np.full((32, 1), 2.0**-27 + 3 * 2.0**-75)
+    b[:24, 0] = 1 + sign * 2.0**-51
+    x = np.full((32, 1), 2.0**-27)
+    x[:24] = 1.0
+    dl, db = up(l), up(b)
+    check(gpu.starpu_gb300_dpotrs(None, 32, 1, dl.ptr, 32, db.ptr, 32))
+    np.testing.assert_array_equal(db.download((32, 1), np.float64), x)
