@@ -16,10 +16,12 @@ namespace gb300 {
 
 // fewest rows of an FP64 product or trailing update that runs on the tensor cores
 constexpr int SLICE_MIN_M = 128;
-// largest FP32 matrix (or diagonal tile) that one cooperative launch factors:
-// 1522 us at n = 4096 against 2417 us in tiles of 256 with a launch per tile,
-// panel and update; beyond, its 64-wide updates would read and write the
-// trailing matrix too often
+// largest FP32 matrix (or diagonal tile) that one cooperative launch factors.
+// Against tiles of 256, 512 or 1024 with a launch per tile, panel and update, the
+// fastest of them: n = 600 131 and 187 us, 2048 543 and 588, 3000 958 and 1132,
+// 4096 1562 and 1693; 5000 2394 and 2556, 6000 3496 and 3696, 8192 7383 and 6587.
+// The line is below the crossing, since the launch rounds the trailing matrix
+// every 64 columns instead of every tile.
 constexpr int COOP_MAX_N = 4096;
 
 static inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
@@ -132,7 +134,7 @@ template <> struct simt_cfg<double> {
             slice_update<true>(s, lower, m, n, k, A, TA ? lda : 1, TA ? 1 : lda, B, TB ? 1 : ldb, TB ? ldb : 1, C, ldc, nullptr);
         else if (!lower && n <= 16)
             gemm_launch<double, TA, TB, 64, 16, 8, 4, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-        else if (gemm_ctas(lower, m, n, 64) >= 4 * 152)
+        else if (gemm_ctas(lower, m, n, 64) >= 4L * gb300_device_sms())
             gemm_launch<double, TA, TB, 64, 64, 8, 4, 4>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
         else
             gemm_launch<double, TA, TB, 32, 32, 16, 2, 2>(s, lower, m, n, k, al, A, lda, B, ldb, be, C, ldc);
@@ -218,7 +220,7 @@ template <typename T> void trsm_slab(cudaStream_t s, const SlabArgs<T> &a)
         // 16 rows per CTA once that fills the GPU; below, 4 spread the products
         // over more SMs (8 when one 64-column block has none)
         if (a.m >= 16 * 128) slab_launch<T, 16>(s, c);
-        else if (a.n <= CP_W && a.m > 4 * 152) slab_launch<T, 8>(s, c);
+        else if (a.n <= CP_W && a.m > 4 * gb300_device_sms()) slab_launch<T, 8>(s, c);
         else slab_launch<T, 4>(s, c);
         const int rest = a.n - j0 - c.n;
         if (rest <= 0) break;

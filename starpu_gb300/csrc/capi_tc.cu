@@ -283,16 +283,20 @@ static long tcu_tiles(int m, int n, int lower, int bn)
     return cnt;
 }
 
-// The tile width of an update on `ctas` SMs: a wide tile takes about 2.6 times
-// as long as a narrow one (both measured on a 1024 x 1024 x 1024 update, where
-// the narrow ones are faster by the number of waves), so the fewer waves by
-// that weight win.  A range of tiles [t0, t1) counts in wide ones.
+// The tile width of an update on `ctas` SMs: narrow tiles where they need no more
+// waves than wide ones, that is where the wide ones leave most SMs idle.  A wave
+// of narrow tiles takes 0.6 (k = 1024) to 0.8 (k = 3000) of a wave of wide ones,
+// since they read A four times as often, so that two against one lose.  Tile
+// product codelets, narrow and wide, us: SYRK 512 22 32, 1024 31 42, 1408 40 50
+// (one wave each), 1536 64 53, 2048 84 66 (two and one), 3000 209 144 (four and
+// two); GEMM 1024 41 51 (one each), 1152 60 57, 1536 78 67 (two and one), 2048 160
+// 90 (four and one).  A range of tiles [t0, t1) counts in wide ones.
 static int tcu_bn(int m, int n, int lower, int ctas, int t0, int t1)
 {
     if (t0 > 0 || t1 >= 0) return TCU_BN;
     const long w = (tcu_tiles(m, n, lower, TCU_BN) + ctas - 1) / ctas;
     const long v = (tcu_tiles(m, n, lower, TCU_BN_NARROW) + ctas - 1) / ctas;
-    return 10 * v < 26 * w ? TCU_BN_NARROW : TCU_BN;
+    return v <= w ? TCU_BN_NARROW : TCU_BN;
 }
 
 // max_grid > 0 caps the persistent grid (CTAs, one per SM): the trailing
@@ -554,7 +558,8 @@ static int lookahead_sms(int m2, int kb)
     const double R = rate / S;
     const double f_upd = 3.0 * m2 * (double)m2 * kb, f_trsm = 6.0 * m2 * (double)kb * kb / panel_rate;
     // at least a sixth of the GPU: n = 32768 took 61.8 ms from 24 SMs up, 62.2
-    // from 16 and 62.6 from 38 (a quarter)
+    // from 16 and 62.6 from 38 (a quarter).  n = 8192 and 16384, from an eighth, a
+    // sixth and a quarter: 4.33, 4.37, 4.42 and 12.05, 12.10, 12.20 ms.
     int best = S / 6;
     double best_t = 1e30;
     for (int L = S / 6; L <= S - 16; L += 8) {
