@@ -17,7 +17,10 @@
  * Kernels that hand work on between warps or CTAs bound every wait; one that
  * runs out (it cannot on a healthy device) leaves a negative *d_info and an
  * unspecified result.  Calls without a status word, or given none, record it
- * in a word of the library's own (starpu_gb300_take_wait_status).
+ * in a word of the library's own (starpu_gb300_take_wait_status).  Only the grid
+ * barriers of the plain FP32 POTRF and of the batched solve have no limit: those
+ * are cooperative launches, whose CTAs all run at the same time.  Such a launch
+ * starts once all of its CTAs (up to two on every SM) fit beside what runs.
  */
 #ifndef STARPU_GB300_KERNELS_H
 #define STARPU_GB300_KERNELS_H
@@ -126,7 +129,9 @@ int starpu_gb300_dswap_columns_tile(void *stream, int m, int n, double *A, int l
 /* Tiled right-looking Cholesky of the whole n x n matrix with tile nb (0 =
  * 512): the DAG of examples/cholesky/cholesky_implicit.c:244-318 (POTRF k,
  * TRSM m>k, SYRK/GEMM) with the tasks of one step fused into whole-panel
- * launches.  Only the lower triangle is read and written. */
+ * launches.  Only the lower triangle is read and written.  nb is the width of a
+ * step for FP32 matrices above order 4096; smaller ones are one launch, and FP64
+ * steps are never wider than 64. */
 int starpu_gb300_spotrf(void *stream, int n, float *A, int lda, int nb, int *d_info);
 int starpu_gb300_dpotrf(void *stream, int n, double *A, int lda, int nb, int *d_info);
 

@@ -102,8 +102,8 @@ static void gemm_f32(cudaStream_t s, bool lower, int m, int n, int k, float alph
 // time each, so up to two waves of them are faster).  Alone, a 1024^3 product is
 // faster in 64 tiles (86 us against 108) and a 512^3 one in 32 tiles (27 and 33),
 // but a task graph runs eight of them side by side, where a third or a half
-// more work per product counts: LU of order 16384 takes 218 ms in 32 x 32 tiles,
-// 307 with smaller product tiles, and 143 and 164 ms in 16 x 16.
+// more work per product counts: LU of order 16384 takes 195 ms in 32 x 32 tiles,
+// 290 with smaller product tiles (from 152 instead of 64), and 105 and 127 ms in 16 x 16.
 // Narrow variant for few columns.
 template <> struct simt_cfg<float> {
     template <bool TA, bool TB>

@@ -34,7 +34,7 @@
 // two 128 x BN FP32 accumulators so the epilogue of tile i overlaps the main loop
 // of tile i+1.  A 64-column tile reads its A operand four times as often (its
 // MMAs are bound by shared memory at two thirds of the tensor rate) but makes
-// four times as many tiles: tcu_narrow() takes it where the wide tiles leave SMs
+// four times as many tiles: tcu_bn() takes it where the wide tiles leave SMs
 // idle.  Every element's products are added in the same order either way.
 #pragma once
 #include <cuda.h>

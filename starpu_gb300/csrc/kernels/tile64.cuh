@@ -63,7 +63,7 @@ struct DcTile {
 
 // acc += As * Bs for 64 x 64 shared tiles: As column-major (As[p * DC_LD + r]
 // = A(r, p)), Bs stored p-major (Bs[p * DC_LD + c] = B(p, c)) -- which is how
-// dc_load stores a tile whose transpose is the operand (NT products).
+// DcTile::store leaves a tile whose transpose is the operand (NT products).
 // Thread (tr = tid % 16, tn = tid / 16) owns rows 4 tr .. 4 tr + 3 and
 // columns 4 tn .. 4 tn + 3: two float4 shared loads per 16 FMAs.  kmax: terms.
 __device__ __forceinline__ void dc_mma(const float *As, const float *Bs, float acc[4][4], int kmax = DC_B)
