@@ -50,8 +50,12 @@ static void slice_update(cudaStream_t s, bool lower, int m, int n, int k, const 
 }
 
 // Elements of C from which an FP64 product (alpha = -1, beta = 1) runs on the
-// tensor cores: 64 columns of A and B take a launch of 8 to 9 us there until the
-// tiles make more than a wave, and m n / 7700 us on the FP64 units.
+// tensor cores.  The line is the solve's, which loses below it: POTRS of 64
+// right-hand sides, us, with this line, on the FP64 units alone and with slices
+// throughout: order 1000 488 488 626, 2000 1226 1206 1379, 3000 1893
+// 2136 2061, 8000 5745 10172 5953.  Square products at the line (m = n = 320), slices
+// and FP64 units: k = 16 23 and 17, 64 23 and 28, 256 45 and 77; at 256 23 and 16, 23 and
+// 28, 46 and 79; at 640 24 and 25, 22 and 62, 46 and 207.
 constexpr long SLICE_MIN_ELEMENTS = 96 * 1024;
 
 template <typename T, bool TA, bool TB, int BM, int BN, int BK, int TM, int TN>
@@ -320,8 +324,7 @@ static void potrs_sweep_blocks(cudaStream_t s, int n, int nrhs, const T *L, long
         const int rest = TRANS ? j0 : n - j0 - w;
         if (rest <= 0) continue;
         if constexpr (std::is_same<T, double>::value) {
-            // B_rest -= L X (or L^T X) on the tensor cores: 64 columns of L in
-            // 8 to 9 us, against rest nrhs / 8800 us on the FP64 units
+            // B_rest -= L X (or L^T X) on the tensor cores (SLICE_MIN_ELEMENTS)
             if (rest >= SLICE_MIN_M && nrhs >= 16 && (long)rest * nrhs >= SLICE_MIN_ELEMENTS) {
                 slice_update<true>(s, false, rest, nrhs, w, TRANS ? L + j0 : L + (j0 + w) + (long)j0 * ldl,
                                    TRANS ? ldl : 1, TRANS ? 1 : ldl, B + j0, ldb, 1, TRANS ? B : B + j0 + w, ldb, wait.err);
