@@ -119,7 +119,8 @@ int starpu_gb300_backward_error(void *stream, int n, int nrhs, const double *A, 
  * FP64 until its backward error <= tol or max_iter corrections.  nrhs <= 8.
  * Synchronous: on return status[i] (host, may be NULL) holds the number of
  * corrections (>= 0), -k if the FP32 factor met a non-positive pivot k, or
- * -1000 if it did not converge; berr[i] (host, may be NULL) the final error. */
+ * -1000 if it did not converge or a wait inside the kernel ran out; berr[i]
+ * (host, may be NULL) the final error. */
 size_t starpu_gb300_dposv_batched_workspace(int nsys, const int *n, int nrhs);
 int starpu_gb300_dposv_batched(void *stream, int nsys, const int *n, const double *A, const long long *a_off,
                                const double *B, const long long *b_off, double *X, int nrhs, double tol,

@@ -18,7 +18,8 @@
  * its stream, like the reference's.  The reference asserts on a zero pivot
  * from the host after one synchronisation per column; here nothing waits, so
  * a zero pivot shows as non-finite entries of the factor (the driver's check
- * then fails).
+ * then fails).  The kernels have no status word here either: a wait inside one
+ * that ran out makes the next GETRF_PIVOT, or lu_kernel_fini, abort.
  */
 #include <starpu.h>
 #include <string.h>
@@ -40,6 +41,7 @@ starpu_data_handle_t devInfo = NULL;
 #define THRESHOLD_F64 10e-10
 
 void lu_kernel_fini(void);
+static void free_workspace(void);
 static int *d_ipiv = NULL;     /* pivot record of one GETRF_PIVOT tile */
 static void *d_work = NULL;    /* copy of one tile for the pivoting fallback */
 static size_t work_bytes = 0;
@@ -50,6 +52,13 @@ static int ipiv_cap = 0;
         int _rc = (rc);                                                                                           \
         if (_rc != 0) STARPU_ABORT_MSG("GB300 kernel launch failed (%d): %s", _rc, starpu_gb300_last_error());   \
     } while (0)
+
+/* the tiles factored so far are not valid when a wait inside a kernel ran out */
+static void check_waits(void *stream)
+{
+    if (starpu_gb300_take_wait_status(stream) == GB300_ETIMEDOUT)
+        STARPU_ABORT_MSG("GB300 LU: %s", starpu_gb300_last_error());
+}
 
 #define IS_F64(d) (STARPU_MATRIX_GET_ELEMSIZE(d) == sizeof(double))
 
@@ -78,7 +87,7 @@ static void lu_gb300_getrf_pivot(void *descr[], void *arg)
          * xlu_implicit.c do), so the first pivoting tile sizes the workspace.
          * This codelet synchronises its stream anyway (it fills the host pivot
          * record), so no earlier use of the buffers is still in flight. */
-        lu_kernel_fini();
+        free_workspace();
         work_bytes = starpu_gb300_dgetrf_pivot_tile_workspace(n);
         ipiv_cap = n;
         d_work = starpu_gb300_device_malloc(work_bytes);
@@ -94,6 +103,7 @@ static void lu_gb300_getrf_pivot(void *descr[], void *arg)
     STARPU_ASSERT(h);
     CHECK_LAUNCH(starpu_gb300_memcpy_d2h(s, h, d_ipiv, sizeof(int) * (size_t)n));
     CHECK_LAUNCH(starpu_gb300_stream_sync(s));
+    check_waits(s);
     /* the reference records a step only when it pivoted */
     for (int z = 0; z < n; ++z)
         if (h[z] >= 0) piv->piv[z + piv->first] = (unsigned)h[z] + piv->first;
@@ -245,7 +255,7 @@ void lu_kernel_init(int nb)
     STARPU_ASSERT_MSG(d_work && d_ipiv, "cannot allocate the LU codelet workspace");
 }
 
-void lu_kernel_fini(void)
+static void free_workspace(void)
 {
     if (d_work) starpu_gb300_device_free(d_work);
     if (d_ipiv) starpu_gb300_device_free(d_ipiv);
@@ -253,4 +263,11 @@ void lu_kernel_fini(void)
     d_ipiv = NULL;
     work_bytes = 0;
     ipiv_cap = 0;
+}
+
+/* after the tasks, before starpu_shutdown() */
+void lu_kernel_fini(void)
+{
+    free_workspace();
+    if (starpu_cuda_worker_get_count()) check_waits(NULL);
 }

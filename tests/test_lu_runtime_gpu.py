@@ -56,3 +56,36 @@ def test_lu_with_threshold_pivoting(prec):
 def test_lu_pivot_mode_without_small_pivots_matches_plain():
     r, _ = run_lu(["-size", "1024", "-nblocks", "8", "-check", "-piv"], STARPU_NCPU=0)
     assert r.returncode == 0 and "0 pivoting steps" in r.stderr, r.stdout + r.stderr
+
+
+_WAITS = r"""
+import ctypes as C, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import starpu_gb300
+from starpu_gb300 import DeviceBuffer
+from starpu_gb300.native import check
+L = starpu_gb300.load()
+lu = C.CDLL(sys.argv[1] + "/starpu_gb300/lib/libstarpu_gb300_lu.so")
+assert L.starpu_init(None) == 0 and L.starpu_cuda_worker_get_count() > 0
+n = 200
+a = DeviceBuffer.from_array(np.asfortranarray(np.eye(n, dtype=np.float32)))
+L.starpu_gb300_set_wait_budget_ns(1 if sys.argv[2] == "short" else 0)
+check(L.starpu_gb300_sgetrf_tile(None, n, a.ptr, n, None))
+lu.lu_kernel_fini()
+print("valid", flush=True)
+L.starpu_shutdown()
+"""
+
+
+@pytest.mark.parametrize("waits", ["short", "default"])
+def test_lu_codelets_abort_when_a_wait_ran_out(waits):
+    """The LU drivers have no status to read: lu_kernel_fini ends the program (on the
+    host) when a wait inside a tile's kernel ran out, here one of 1 ns."""
+    import sys
+    r = subprocess.run([sys.executable, "-c", _WAITS, ROOT, waits], env=dict(os.environ, STARPU_NCPU="0"),
+                       capture_output=True, text=True, timeout=300)
+    if waits == "short":
+        assert r.returncode != 0 and "valid" not in r.stdout and "wait inside a kernel ran out" in r.stderr, r.stdout + r.stderr
+    else:
+        assert r.returncode == 0 and "valid" in r.stdout, r.stdout + r.stderr
