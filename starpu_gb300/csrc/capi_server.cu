@@ -131,7 +131,7 @@ static void serve_large(starpu_gb300_server *sv, Exec &e, starpu_gb300_request *
         return;
     }
     CacheEntry *entry = nullptr;
-    bool fresh = false;
+    bool fresh = false, factored = false;
     const size_t ws_bytes = starpu_gb300_dsposv_workspace(n, sv->max_nrhs, NB);
     {
         std::lock_guard<std::mutex> g(sv->mu);
@@ -173,6 +173,7 @@ static void serve_large(starpu_gb300_server *sv, Exec &e, starpu_gb300_request *
         if (!r->A) rc = GB300_EINVAL;  // no cached factor for this id and no matrix given
         if (!rc) rc = copy_in(Adev, r->A, sizeof(double) * (size_t)n * n, s);
         if (!rc) rc = gb300::dsposv_factor(s, n, nrhs, Adev, n, NB, 3, ws, &info);
+        factored = !rc;
     } else if (!rc) {
         r->cache_hit = 1;
     }
@@ -189,9 +190,9 @@ static void serve_large(starpu_gb300_server *sv, Exec &e, starpu_gb300_request *
         if (entry) {
             entry->in_use--;
             if (fresh) {
-                if (rc == GB300_OK || rc == GB300_ETIMEDOUT) {
+                if (factored && (rc == GB300_OK || rc == GB300_ETIMEDOUT)) {
                     entry->ready = true;
-                } else {  // factor failed: do not keep it
+                } else {  // factor failed, or a wait in it ran out: do not keep it
                     cudaFreeAsync(entry->A, s);
                     cudaFreeAsync(entry->ws, s);
                     sv->used -= entry->bytes;

@@ -140,3 +140,26 @@ def test_invalid_requests_are_rejected(gpu):
         assert gpu.starpu_gb300_server_submit(sv, C.byref(r)) == -22  # n > max_n
     finally:
         gpu.starpu_gb300_server_destroy(sv)
+
+
+def test_factor_behind_a_wait_that_ran_out_is_not_kept(gpu, oracle, problems):
+    A, B, _ = problems[5]  # n = 1500, large path
+    sv = gpu.starpu_gb300_server_create(24 * GB, 1, 2048, 16, 0)
+    assert sv, gpu.starpu_gb300_last_error()
+    try:
+        r1, _ = request(A, B, 901)
+        prev = gpu.starpu_gb300_set_wait_budget_ns(1)
+        try:
+            assert gpu.starpu_gb300_server_submit(sv, C.byref(r1)) == 0
+            gpu.starpu_gb300_server_wait(sv, C.byref(r1))
+        finally:
+            gpu.starpu_gb300_set_wait_budget_ns(prev)
+        assert r1.status == -110
+        r2, X2 = request(A, B, 901)
+        assert gpu.starpu_gb300_server_submit(sv, C.byref(r2)) == 0
+        assert gpu.starpu_gb300_server_wait(sv, C.byref(r2)) == 0
+    finally:
+        gpu.starpu_gb300_server_destroy(sv)
+    assert r2.status == 0 and r2.cache_hit == 0
+    be, _ = oracle.backward_error(A, X2, B)
+    assert be <= 1e-12
