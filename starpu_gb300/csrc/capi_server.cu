@@ -55,6 +55,7 @@ struct Exec {
     double *pA = nullptr, *pB = nullptr, *pX = nullptr;  // batch pools
     void *bws = nullptr;
     size_t lbws = 0;
+    int *info = nullptr;  // mode 1
 };
 
 } // namespace
@@ -123,9 +124,12 @@ static void serve_large(starpu_gb300_server *sv, Exec &e, starpu_gb300_request *
     if (sv->mode == 1) {  // plain baseline: FP64 dposv, alone
         rc = copy_in(e.A, r->A, sizeof(double) * (size_t)n * n, s);
         if (!rc) rc = copy_in(e.X, r->B, sizeof(double) * (size_t)n * nrhs, s);
-        if (!rc) rc = starpu_gb300_dposv(s, n, nrhs, e.A, n, e.X, n, 512, nullptr);
+        int info = 0;
+        if (!rc) rc = starpu_gb300_dposv(s, n, nrhs, e.A, n, e.X, n, 512, e.info);
         if (!rc) rc = copy_in(r->X, e.X, sizeof(double) * (size_t)n * nrhs, s);
+        if (!rc) rc = copy_in(&info, e.info, sizeof info, s);
         if (!rc) rc = gb300_record_cuda_error(cudaStreamSynchronize(s));
+        if (!rc && info < 0) rc = GB300_ETIMEDOUT;  // a wait inside a kernel ran out
         r->status = rc;
         finish(sv, r);
         return;
@@ -306,6 +310,7 @@ static void free_exec(Exec &e)
     cudaFree(e.pB);
     cudaFree(e.pX);
     cudaFree(e.bws);
+    cudaFree(e.info);
     if (e.s) cudaStreamDestroy(e.s);
 }
 
@@ -329,6 +334,7 @@ starpu_gb300_server *starpu_gb300_server_create(size_t hbm_budget_bytes, int exe
         ok &= !gb300_record_cuda_error(cudaMalloc(&e.B, sizeof(double) * (size_t)max_n * max_nrhs));
         ok &= !gb300_record_cuda_error(cudaMalloc(&e.X, sizeof(double) * (size_t)max_n * max_nrhs));
         size_t bytes = sizeof(double) * ((size_t)max_n * max_n + 2 * (size_t)max_n * max_nrhs);
+        if (mode == 1) ok &= !gb300_record_cuda_error(cudaMalloc(&e.info, sizeof(int)));
         if (mode == 2) {  // per-request mixed solves: one solver workspace, no batch pools
             e.lws = starpu_gb300_dsposv_workspace(max_n, max_nrhs, NB);
             ok &= !gb300_record_cuda_error(cudaMalloc(&e.ws, e.lws));

@@ -1640,7 +1640,9 @@ int starpu_gb300_dposv(void *stream, int n, int nrhs, double *A, int lda, double
 {
     int rc = starpu_gb300_dpotrf(stream, n, A, lda, nb, d_info);
     if (rc) return rc;
-    return starpu_gb300_dpotrs(stream, n, nrhs, A, lda, B, ldb);
+    if (nrhs < 0 || ldb < (n > 1 ? n : 1)) return GB300_EINVAL;
+    potrs_blocked<double>((cudaStream_t)stream, n, nrhs, A, lda, B, ldb, d_info);
+    return gb300_last_launch_status();
 }
 
 } // extern "C"

@@ -163,3 +163,19 @@ def test_factor_behind_a_wait_that_ran_out_is_not_kept(gpu, oracle, problems):
     assert r2.status == 0 and r2.cache_hit == 0
     be, _ = oracle.backward_error(A, X2, B)
     assert be <= 1e-12
+
+
+def test_plain_request_reports_a_wait_that_ran_out(gpu, oracle, problems):
+    A, B, _ = problems[3]
+    prev = gpu.starpu_gb300_set_wait_budget_ns(1)
+    try:
+        r, _ = request(A, B)
+        serve(gpu, [r], executors=1, mode=1)
+    finally:
+        gpu.starpu_gb300_set_wait_budget_ns(prev)
+    assert r.status == -110
+    assert gpu.starpu_gb300_take_wait_status(None) == 0  # nothing left for another caller
+    r, X = request(A, B)
+    serve(gpu, [r], executors=1, mode=1)
+    be, _ = oracle.backward_error(A, X, B)
+    assert r.status == 0 and be <= 1e-13

@@ -163,3 +163,14 @@ def test_mixed_solve_does_not_take_a_wait_that_runs_out_for_a_bad_pivot(gpu):
     with short_waits(gpu):
         assert solve() == (GB300_ETIMEDOUT, GB300_ETIMEDOUT, 0)
     assert solve() == (0, 0, 0)
+
+
+def test_dposv_reports_both_phases_in_its_info(gpu):
+    n = 600
+    a, b = spd(n, n), np.ones((n, 3))
+    da, db, info = up(a), up(b), up(np.zeros(1, np.int32))
+    with short_waits(gpu):
+        check(gpu.starpu_gb300_dposv(None, n, 3, da.ptr, n, db.ptr, n, 512, info.ptr))
+        check(gpu.starpu_gb300_stream_sync(None))
+    assert int(info.download((1,), np.int32)[0]) == TIMEOUT_INFO
+    assert gpu.starpu_gb300_take_wait_status(None) == 0
