@@ -26,7 +26,9 @@
 // arithmetic on the FP32 pipe (A split per element, X split once per task into
 // shared memory, FP64 flush every 128 terms; ~2^-47 relative per block): the
 // FP64 pipe is 64 times slower.  Larger ones, with seven or eight right-hand
-// sides, keep FP64 FMAs.
+// sides, keep FP64 FMAs (64 systems of order 900 to 1024 with eight: 4.99 ms against
+// 3.94 in double-float, whose backward error is off by some 40 2^-53 there; with six
+// 3.89 ms).
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
